@@ -1,0 +1,95 @@
+"""The atom-pair engine at the sizes where its groups can go wrong: one-atom
+rows to several groups per block, a group with more pairs than the queue
+holds (a pose squeezed until nearly every pair is in reach), block pairs and
+rotamer pairs of such poses, and type parameters without a common fade
+interval (no far class).
+
+float64 energies and gradients against the oracle.  A gradient component is
+a sum of at most a few thousand signed terms, each no larger than the largest
+component's magnitude allows by a factor of ten or so, so its float64 sum is
+good to 1e-12 of the largest component (2.2e-16 x a few thousand); energies
+likewise to 1e-11 relative."""
+
+import numpy
+import pytest
+import torch
+
+from oracle import oracle as O
+from tmol_b200.pose.rotamers import synthetic_rotamer_set
+from tmol_b200.pose.synthetic import synthetic_pose_stack
+from tmol_b200.score.elec_energy_term import ElecEnergyTerm, elec_pose_score_args
+from tmol_b200.score.elec_op import elec_pose_scores
+from tmol_b200.score.ljlk_energy_term import LJLKEnergyTerm, pose_score_args, rotamer_score_args
+from tmol_b200.score.ljlk_op import clear_plan_cache, ljlk_pose_scores, ljlk_rotamer_scores
+from tolerances import E_close
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def close(x, ref, rel):
+    ref = numpy.asarray(ref)
+    err = numpy.abs(x.detach().cpu().numpy() - ref)
+    assert err.max() <= rel * numpy.abs(ref).max() + 1e-9, (err.max(), numpy.abs(ref).max())
+
+
+def on_gpu(args, dtype):
+    return [
+        a.to(DEV, dtype if a.is_floating_point() else a.dtype) if isinstance(a, torch.Tensor) else a for a in args
+    ]
+
+
+@pytest.mark.parametrize("scale", [1.0, 0.5])
+@pytest.mark.parametrize("name", ["ljlk", "elec"])
+@pytest.mark.parametrize("block_pair", [False, True])
+def test_pose_groups(name, block_pair, scale):
+    ps = synthetic_pose_stack([30, 1, 2, 9, 75], [5, 6, 7, 8, 9], spacing=0.0)
+    x = (ps.coords * scale).flatten(0, 1).double()
+    op, args_of, term = {
+        "ljlk": (ljlk_pose_scores, pose_score_args, LJLKEnergyTerm()),
+        "elec": (elec_pose_scores, elec_pose_score_args, ElecEnergyTerm()),
+    }[name]
+    args = args_of(ps, term, block_pair)
+    oc = O.OracleCall(x, args, f64=True, term=name)
+    n = 3 if name == "ljlk" else 1
+    c = x.to(DEV).requires_grad_(True)
+    E, nbr = op(c, *on_gpu(args, torch.float64))
+    Eo, dVo, nbro = oc.pose_scores(block_pair=block_pair, require_gradient=True)
+    close(E, numpy.asarray(Eo)[:n].reshape(E.shape), 1e-11)
+    assert numpy.array_equal(nbr.cpu().numpy(), nbro)
+    E.sum().backward()
+    _, dVo, _ = oc.pose_scores(require_gradient=True)
+    close(c.grad, dVo[:n].sum(0), 1e-12)
+    E32, _ = op(x.to(DEV, torch.float32), *on_gpu(args, torch.float32))
+    E_close(E32.cpu().numpy(), numpy.asarray(Eo)[:n].reshape(E.shape), what=f"{name} float32, scale {scale}")
+    clear_plan_cache()
+
+
+@pytest.mark.parametrize("scale", [1.0, 0.5])
+def test_rotamer_groups(scale):
+    ps = synthetic_pose_stack([12, 3], [15, 16], spacing=0.0)
+    rs = synthetic_rotamer_set(ps, max_rots=40, seed=3)
+    args = rotamer_score_args(ps, rs, LJLKEnergyTerm())
+    x = (rs.coords * scale).double()
+    Eo, ind, _ = O.OracleCall(x, args, f64=True).rotamer_scores()
+    E, indices = ljlk_rotamer_scores(x.to(DEV), *on_gpu(args, torch.float64))
+    assert numpy.array_equal(indices.cpu().numpy(), ind)
+    close(E, Eo, 1e-11)
+    clear_plan_cache()
+
+
+def test_no_common_fade_interval():
+    """A type whose LJ minimum lies inside the fade interval fades on an
+    interval of its own: the general path serves every pair.  (Energies, from
+    the oracle's energy-only form: for such a type the reference's form with
+    derivatives divides attractive and repulsive parts otherwise.)"""
+    ps = synthetic_pose_stack([40, 12], [25, 26], spacing=0.0)
+    args = pose_score_args(ps, LJLKEnergyTerm())
+    params = args[22].clone()
+    params[int(args[17][0, 0]), 0] = 3.1  # the radius of the first block type's first atom's type
+    args[22] = params
+    x = ps.coords.flatten(0, 1).double()
+    E, _ = ljlk_pose_scores(x.to(DEV), *on_gpu(args, torch.float64))
+    Eo, _, _ = O.OracleCall(x, args, f64=True).pose_scores()
+    close(E, Eo, 1e-11)
+    clear_plan_cache()

@@ -17,7 +17,7 @@ SRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "lib", "libtmol_b200_ljlk.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 SOURCES = ["ljlk.cu", "ljlk_noalloc.cu", "screen.cu", "bondsep.cu"]
-HEADERS = ["ljlk_potentials.cuh", "elec_potentials.cuh", "bondsep.cuh"]
+HEADERS = ["ljlk_potentials.cuh", "elec_potentials.cuh", "bondsep.cuh", "pair_engine.cuh", "lkball.cuh"]
 
 
 def nvcc_path():

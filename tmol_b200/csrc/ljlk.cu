@@ -6,7 +6,7 @@
 //   blk_bt[P*B], blk_off[P*B]      block type and first-atom offset per block
 //   pose_last[P]                   1 + index of each pose's last real block
 //   bt_tf[nbt*A]                   per block-type atom: compact atom type | heavy
-//   ljtab, lktab[ntp*ntp]          per atom-type-pair LJ / LK constants
+//   ljtab, lktab, fartab[ntp*ntp]  per atom-type-pair LJ / LK constants
 //   bt_pd[nbt][A][A] (u8)          intra-block bond separation
 //   bt_conn_pd[nbt][C][A] (u8)     bond separation from each connection atom
 //   cp_*[P*B][CP_CAP]              per block: the later blocks within
@@ -17,17 +17,11 @@
 //                                  to each pose's last real block
 //   spheres[P*B][4]                centroid + radius, rebuilt every call
 //
-// Scoring (one persistent launch per call, after the sphere kernel): every
-// warp is an independent worker taking rows from an atomic ticket.  For row
-// (p, b1) it stages b1's atoms (a tile of 32) in its shared-memory slab,
-// tests b1 against all later blocks of the pose with the bounding-sphere rule
-// (32 candidates per ballot) and evaluates each neighbouring block pair at
-// once, in two phases: a screening pass over all atom pairs (distance and
-// count-pair weight) compacts the pairs that contribute into a per-warp
-// queue, split into LJ-only and heavy-atom (LJ + LK) pairs, and a dense pass
-// evaluates the queue with every lane busy.  Energies stay in registers for
-// the whole row; gradients accumulate in the slab (b1's across the whole
-// row) and are flushed to global memory once per block pair (b2) or row (b1).
+//   packed[n_atoms], g4[n_atoms][4]  staged atoms and padded gradient, per call
+//
+// Scoring is one persistent launch per call after the sphere kernel (every
+// warp takes work items from an atomic ticket; pair_engine.cuh), and a copy
+// of the padded gradient into the caller's where one is wanted.
 
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
@@ -243,10 +237,11 @@ __global__ void plan_block_types_kernel(PlanBuildArgs a, const int* type_map,
     if (at < n) {
       if (a.term == kTermLJLK) {
         int t = in.bt_atom_types[i];
-        if (t < 0 || t >= in.n_atom_types || type_map[t] < 0) {
+        const int heavy = a.bt_flags[i] == kHeavy ? 1 : 0;
+        if (t < 0 || t >= in.n_atom_types || type_map[2 * t + heavy] < 0) {
           atomicOr(a.status, kStIndex);
         } else {
-          tf = (uint16_t)(type_map[t] | (a.bt_flags[i] == kHeavy ? 256 : 0));
+          tf = (uint16_t)(type_map[2 * t + heavy] | (heavy << 8));
         }
       }
       for (int at2 = 0; at2 < A; ++at2) {
@@ -274,18 +269,67 @@ __global__ void plan_block_types_kernel(PlanBuildArgs a, const int* type_map,
   }
 }
 
-// Type-pair tables for every ordered pair of the compact atom types.
+// Pairs within a block, per block-type atom `at` and word of 32 atoms of its
+// type: x the atoms it is not scored with (itself and the earlier ones, which
+// hold the pair, and those nearer than four bonds), y those four bonds away
+// (weight 0.2), from the intra-block separation table
+// (ljlk_pose_score.impl.hh:115-134; the ligand 3/4 -> 5 rule is already folded
+// into that table).
+__global__ void plan_intra_masks_kernel(const uint8_t* bt_pd, const int* bt_n_atoms, int nbt, int A, int n_words,
+                                        uint2* out) {
+  const int64_t total = (int64_t)nbt * A * n_words;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t row = i / n_words;
+    const int word = (int)(i - row * n_words), bt = (int)(row / A), at = (int)(row - (int64_t)bt * A);
+    const int n = bt_n_atoms[bt];
+    uint2 m = make_uint2(0xffffffffu, 0u);
+    for (int k = 0; k < 32; ++k) {
+      const int j = 32 * word + k;
+      if (j >= n || at >= n || j <= at) continue;
+      const int sep = bt_pd[row * A + j];
+      if (sep >= 4) m.x &= ~(1u << k);
+      if (sep == 4) m.y |= 1u << k;
+    }
+    out[i] = m;
+  }
+}
+
+// Heavy atoms per block type (work counters), and which coordinates belong to
+// a block or rotamer.
+__global__ void plan_heavy_count_kernel(const uint16_t* bt_tf, const int* bt_n_atoms, int nbt, int A, int* out) {
+  for (int bt = blockIdx.x * blockDim.x + threadIdx.x; bt < nbt; bt += gridDim.x * blockDim.x) {
+    int n = 0;
+    for (int k = 0; k < bt_n_atoms[bt]; ++k) n += bt_tf[(int64_t)bt * A + k] >> 8;
+    out[bt] = n;
+  }
+}
+
+__global__ void plan_real_atoms_kernel(const int* bt_of, const int* off_of, int n, const int* bt_n_atoms,
+                                       uint8_t* real) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    if (bt_of[i] < 0) continue;
+    for (int k = 0; k < bt_n_atoms[bt_of[i]]; ++k) real[(int64_t)off_of[i] + k] = 1;
+  }
+}
+
+// a compact type of hydrogens (atoms not listed heavy): no LK
+constexpr int kTypeLight = 1 << 30;
+
+// Type-pair tables for every ordered pair of the compact atom types; *mixed
+// is set when some pair's LJ fades on another interval than LK.
 template <typename Real>
 __global__ void plan_tables_kernel(const Real* type_params, const Real* gp,
                                    const int* compact_types, int ntp,
-                                   LJRecord<Real>* ljtab, LKRecord<Real>* lktab) {
+                                   Quad<Real>* ljtab, LKRecord<Real>* lktab, Quad<Real>* fartab,
+                                   int* mixed) {
   GlobalParams<Real> g = {gp[0], gp[1], gp[2], gp[3], gp[4]};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntp * ntp;
        i += gridDim.x * blockDim.x) {
     AtomParams<Real> pr[2];
     int ts[2] = {compact_types[i / ntp], compact_types[i % ntp]};
     for (int k = 0; k < 2; ++k) {
-      const Real* r = type_params + 10 * (int64_t)ts[k];
+      const Real* r = type_params + 10 * (int64_t)(ts[k] & ~kTypeLight);
       pr[k].lj_radius = r[0];
       pr[k].lj_wdepth = r[1];
       pr[k].lk_dgfree = r[2];
@@ -299,7 +343,11 @@ __global__ void plan_tables_kernel(const Real* type_params, const Real* gp,
       if (r[9] != 0) f |= kCarbonLK;
       pr[k].flags = f;
     }
-    build_records(pr[0], pr[1], g, ljtab[i], lktab[i]);
+    const bool heavy = !(ts[0] & kTypeLight) && !(ts[1] & kTypeLight);
+    build_records(pr[0], pr[1], g, ljtab[i], ljtab[ntp * ntp + i], lktab[i]);
+    const Quad<Real> fade = ljtab[ntp * ntp + i];
+    fartab[i] = Quad<Real>{fade.b, fade.c, heavy ? lktab[i].fmin_V : Real(0), heavy ? lktab[i].fmin_dp : Real(0)};
+    if (ljtab[i].d != g.max_dis - Real(1.5)) *mixed = 1;
   }
 }
 
@@ -465,9 +513,21 @@ struct ScoreArgs {
   const int* blk_off;
   const int* pose_last;
   const uint16_t* bt_tf;  // per block-type atom: compact type | heavy << 8
-  const LJRecord<Real>* ljtab;
+  const Quad<Real>* ljtab;   // [2][ntp * ntp]: LJ base and fade groups
   const LKRecord<Real>* lktab;
+  const Quad<Real>* fartab;  // [ntp * ntp] fade-out knots of LJ and LK together
   int ntp;  // compact atom types (tables are ntp x ntp)
+  // where the class of far pairs (both potentials fading out) starts; 0: the
+  // plan's types fade on different intervals, no pair takes that class
+  Real far_d;
+  // per block-type atom and word of 32 atoms of its type: which pairs are
+  // excluded within the block and which have weight 0.2
+  const uint2* imask;
+  int n_iwords;
+  const int* bt_n_heavy;  // heavy atoms per block type (work counters)
+  // LJ/LK and elec: the gradient as [n_atoms][4], zeroed by the sphere pass
+  // and copied out by grad_out_kernel
+  Real* g4;
   const uint8_t* bt_pd;
   const uint8_t* bt_conn_pd;
   const int* bt_n_atoms;
@@ -493,7 +553,7 @@ struct ScoreArgs {
   // pair (never honoured for b1 == b2 or count-pair partners)
   const uint32_t* skip;
   int skip_words;  // 32-bit words per row
-  int max_slots;   // neighbouring blocks packed per screening group
+  int max_slots;   // pair energies: block (or rotamer) pairs screened per group
   // elec plans: partial charge per block-type atom [nbt * A] and the
   // potential's per-unit-charge constants (ElecK layout)
   const Real* bt_q;
@@ -580,50 +640,7 @@ __global__ void spheres_kernel(ScoreArgs<Real> s) {
   }
 }
 
-// ---------------------------------------------------------------------------
-// Per-warp shared-memory slab.
-//
-// Side 0 holds a tile (<= 32 atoms) of the row block b1; side 1 packs the
-// atoms of up to MAX_SLOTS neighbouring blocks b2 (at most M1 atoms), so that
-// one screening pass covers several block pairs with every lane busy.  The
-// pair queue collects the atom pairs that contribute (inside max_dis with a
-// non-zero count-pair weight): LJ-only pairs from the front, heavy-atom
-// (LJ + LK) pairs from the back.  Both sides live in one atom array (side 0
-// at [0, TILE), side 1 at [TILE, TILE + M1)), each atom one 16-byte record
-// (x, y, z, type) so that a pair costs two vector loads; an entry packs
-// a (5 bits: a side-0 atom) | k (7 bits: an index into the atom array) |
-// count-pair-weight-0.2 flag (bit 12).  Entries come in runs that share k:
-// screening emits each side-1 atom's pairs together, the intra-tile pass
-// each row's.  One screening chunk (32 side-1 atoms x 32 rows) emits at
-// most 1024 entries, so a queue of QCAP >= 1024 takes any chunk whole.
-
-constexpr int M1 = 96;
-constexpr int MAX_SLOTS = 12;
-// copies of the side-0 force accumulators: lane l adds an entry's force on
-// its side-0 atom into copy l % A_COPIES, so that at most four lanes of a
-// step can meet at one address (shared atomics serialise on a conflict)
-constexpr int A_COPIES = 8;
-constexpr int QCAP = 1024;
-constexpr int kTfHeavy = 256;
-
-enum SlotKind : int {
-  kSlotFar = 0,       // bond separation > 4 everywhere: weight 1
-  kSlotStriking = 1,  // count pair through the connection atoms
-  kSlotIntra = 2,     // another tile of block b1: intra-block separation table
-};
-
-// One staged atom: coordinates and either per block-type atom flags
-// (LJ/LK: compact atom type | heavy << 8) or the partial charge (elec).
-template <typename Real>
-struct alignas(16) AtomRec {
-  Real x, y, z;
-  union {
-    int tf;
-    Real q;
-  };
-};
-
-constexpr int N_ATOMS = TILE + M1;
+#include "pair_engine.cuh"
 
 // Writes block (bt, off)'s atoms as staged records: coordinates and the
 // block-type atom's compact type | heavy flag (LJ/LK) or partial charge
@@ -643,870 +660,8 @@ __device__ __forceinline__ void pack_block(const ScoreArgs<Real>& s, int bt, int
     else
       a.tf = s.bt_tf[(int64_t)bt * s.A + k];
     s.packed[(int64_t)off + k] = a;
+    if (s.g4) reinterpret_cast<Quad<Real>*>(s.g4)[(int64_t)off + k] = Quad<Real>{0, 0, 0, 0};
   }
-}
-
-template <typename Real>
-struct Slab {
-  AtomRec<Real> at[N_ATOMS];            // side 0, then side 1
-  Real gx[N_ATOMS], gy[N_ATOMS], gz[N_ATOMS];  // gradient accumulators
-  Real ga[A_COPIES][3][TILE];  // side-0 forces of entries' a atoms, by copy
-  uint32_t cpd0[TILE];  // bond separation to each connection atom, a byte each
-  uint32_t cpd1[M1];
-  int gidx1[M1];  // global atom index
-  uint8_t slot1[M1];   // slot of the packed atom
-  uint8_t local1[M1];  // atom index within its block
-  uint8_t seps[MAX_SLOTS][16];
-  int slot_kind[MAX_SLOTS], slot_nc[MAX_SLOTS], slot_lig[MAX_SLOTS];
-  Real slot_sph[MAX_SLOTS][4];  // bounding sphere of each slot's block
-  unsigned long long counts[8];
-  uint16_t queue[QCAP];
-};
-
-struct RowInfo {
-  int p, b1, i1, bt1, off1, n1, nc1, lig1;
-  int st1, c1;  // tile of b1 in side 0
-};
-
-
-
-template <typename Real>
-__device__ __forceinline__ Real warp_sum(Real v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-template <typename Real>
-__device__ __forceinline__ uint32_t load_cpd(const ScoreArgs<Real>& s, int bt,
-                                             int nconn, int at) {
-  uint32_t v = 0x06060606u;
-  for (int k = 0; k < nconn; ++k) {
-    uint32_t d = s.bt_conn_pd[((int64_t)bt * s.C + k) * s.A + at];
-    v = (v & ~(0xffu << (8 * k))) | (d << (8 * k));
-  }
-  return v;
-}
-
-// Stage atoms [start, start + cnt) of block (bt, off) into side 0.
-template <typename Real, int TERM = kTermLJLK>
-__device__ __forceinline__ void stage_side0(const ScoreArgs<Real>& s,
-                                            Slab<Real>& w, int bt, int off,
-                                            int start, int cnt, int nconn,
-                                            int lane) {
-  if (lane < cnt) {
-    int at = start + lane;
-    AtomRec<Real> a;
-    if (s.packed) {
-      a = s.packed[(int64_t)off + at];
-    } else {
-      const Real* c = s.coords + 3 * ((int64_t)off + at);
-      a.x = c[0];
-      a.y = c[1];
-      a.z = c[2];
-      if (TERM == kTermElec)
-        a.q = s.bt_q[(int64_t)bt * s.A + at];
-      else
-        a.tf = s.bt_tf[(int64_t)bt * s.A + at];
-    }
-    w.at[lane] = a;
-    w.cpd0[lane] = load_cpd(s, bt, nconn, at);
-    w.gx[lane] = 0;
-    w.gy[lane] = 0;
-    w.gz[lane] = 0;
-  }
-#pragma unroll
-  for (int k = 0; k < A_COPIES; ++k) {
-    w.ga[k][0][lane] = 0;
-    w.ga[k][1][lane] = 0;
-    w.ga[k][2][lane] = 0;
-  }
-}
-
-// Append the atoms of [start, start + cnt) of block (bt, off) that can reach
-// block b1 to side 1 at j0: an atom farther than r1 + max_dis from b1's
-// centroid is farther than max_dis from every b1 atom, and every term is zero
-// there.  Returns the number of atoms kept; with `heavy`, also the number of
-// heavy atoms among all cnt (a work counter).
-template <typename Real, int TERM = kTermLJLK>
-__device__ __forceinline__ int stage_side1(const ScoreArgs<Real>& s,
-                                           Slab<Real>& w, int j0, int slot,
-                                           int bt, int off, int start,
-                                           int cnt, int nconn, Real cx,
-                                           Real cy, Real cz, Real reach2,
-                                           int lane, int* heavy = nullptr) {
-  bool keep = false;
-  AtomRec<Real> a;
-  a.x = a.y = a.z = Real(0);
-  a.tf = 0;
-  int at = start + lane;
-  if (lane < cnt) {
-    if (s.packed) {
-      a = s.packed[(int64_t)off + at];
-    } else {
-      const Real* c = s.coords + 3 * ((int64_t)off + at);
-      a.x = c[0];
-      a.y = c[1];
-      a.z = c[2];
-      if (TERM == kTermElec)
-        a.q = s.bt_q[(int64_t)bt * s.A + at];
-      else
-        a.tf = s.bt_tf[(int64_t)bt * s.A + at];
-    }
-    Real dx = a.x - cx, dy = a.y - cy, dz = a.z - cz;
-    keep = dx * dx + dy * dy + dz * dz < reach2;
-  }
-  if (heavy)
-    *heavy = TERM == kTermLJLK ? __popc(__ballot_sync(0xffffffffu, lane < cnt && (a.tf & kTfHeavy))) : 0;
-  unsigned km = __ballot_sync(0xffffffffu, keep);
-  if (keep) {
-    int j = j0 + __popc(km & ((1u << lane) - 1));
-    w.at[TILE + j] = a;
-    w.cpd1[j] = load_cpd(s, bt, nconn, at);
-    w.gidx1[j] = off + at;
-    w.slot1[j] = (uint8_t)slot;
-    w.local1[j] = (uint8_t)at;
-    w.gx[TILE + j] = 0;
-    w.gy[TILE + j] = 0;
-    w.gz[TILE + j] = 0;
-  }
-  return __popc(km);
-}
-
-template <typename Real>
-__device__ __forceinline__ void flush_side0(const ScoreArgs<Real>& s,
-                                            Slab<Real>& w, int off, int start,
-                                            int cnt, int lane) {
-  if (lane < cnt) {
-    Real* d = s.dcoords + 3 * ((int64_t)off + start + lane);
-    Real gx = w.gx[lane], gy = w.gy[lane], gz = w.gz[lane];
-#pragma unroll
-    for (int k = 0; k < A_COPIES; ++k) {
-      gx += w.ga[k][0][lane];
-      gy += w.ga[k][1][lane];
-      gz += w.ga[k][2][lane];
-    }
-    if (gx != 0) atomicAdd(d + 0, gx);
-    if (gy != 0) atomicAdd(d + 1, gy);
-    if (gz != 0) atomicAdd(d + 2, gz);
-  }
-}
-
-template <typename Real>
-__device__ __forceinline__ void flush_side1(const ScoreArgs<Real>& s,
-                                            Slab<Real>& w, int m, int lane) {
-  for (int j = lane; j < m; j += 32) {
-    Real* d = s.dcoords + 3 * (int64_t)w.gidx1[j];
-    Real gx = w.gx[TILE + j], gy = w.gy[TILE + j], gz = w.gz[TILE + j];
-    if (gx != 0) atomicAdd(d + 0, gx);
-    if (gy != 0) atomicAdd(d + 1, gy);
-    if (gz != 0) atomicAdd(d + 2, gz);
-  }
-}
-
-// What the out-of-line screening and evaluation functions need, by value.
-template <typename Real>
-struct EvalCtx {
-  union {
-    const LJRecord<Real>* ljtab;  // LJ/LK
-    const Real* elec_k;           // elec: ElecK constants
-  };
-  const LKRecord<Real>* lktab;
-  const uint8_t* pd;  // intra-block separations of b1, row st1 (tile start)
-  int ntp, A;
-  Real max_dis;
-  Real wt0, wt1, wt2;  // gradient weights of the three terms (elec: wt0)
-};
-
-template <typename Real>
-struct E3 {
-  Real atr, rep, lk;
-};
-
-__device__ __forceinline__ void cnt_add(unsigned long long* c, int k, long long v, int lane) {
-  if (lane == 0) c[k] += (unsigned long long)v;
-}
-
-// The pair-evaluation helpers below are out of line by default (one copy
-// each: the kernel's code footprint and register budget stay small).
-#ifndef TMOL_B200_LJLK_OUTLINE
-#define TMOL_B200_LJLK_OUTLINE __noinline__
-#endif
-
-// Dense evaluation of one queue (HEAVY: LJ + LK, else LJ only; elec: the
-// elec energy in .atr); returns the lane's energy sums.  Entries come in
-// screening order, so lanes sharing a1 are mostly contiguous: their a1
-// forces are summed with a segmented shuffle reduction and added once per
-// segment.
-template <typename Real, bool GRAD, int TERM = kTermLJLK>
-__device__ TMOL_B200_LJLK_OUTLINE E3<Real> eval_queue(EvalCtx<Real> c, Slab<Real>* wp,
-                                            int nl, int nh, int lane) {
-  Slab<Real>& w = *wp;
-  E3<Real> acc = {0, 0, 0};
-  const Real dmax = c.max_dis;
-  const Real far_dmin = c.max_dis - Real(1.5);
-  const Real far_first = far_dmin > Real(4.5) ? far_dmin : Real(4.5);
-  const Real inv_hf = Real(1) / (dmax - far_dmin);
-  ElecK<Real> K;
-  if (TERM == kTermElec) K = load_elec_k(c.elec_k);
-  // one pass over the LJ-only entries, then the heavy-atom ones: only the
-  // step holding both has lanes on different paths
-  const int n = nl + nh;
-  for (int base = 0; base < n; base += 32) {
-    int i = base + lane;
-    bool act = i < n;
-    const bool heavy = TERM == kTermLJLK && i >= nl;
-    int e = act ? (int)w.queue[heavy ? QCAP - 1 - (i - nl) : i] : 0;
-    // j: the entry's k (runs of equal k are consecutive), a1: its a
-    int a1 = e & 31, j = (e >> 5) & 127;
-    Real wcp = (e >> 12) & 1 ? Real(0.2) : Real(1);
-    Real fx = 0, fy = 0, fz = 0;
-    if (act && TERM == kTermElec) {
-      const AtomRec<Real> p1 = w.at[a1];
-      const AtomRec<Real> p2 = w.at[j];
-      const Real dx = p1.x - p2.x;
-      const Real dy = p1.y - p2.y;
-      const Real dz = p1.z - p2.z;
-      const Real d2 = dx * dx + dy * dy + dz * dz;
-      // coincident atoms take the flat region and add no force
-      const Real inv_d = inv_sqrt(d2);
-      const Real d = d2 > Real(0) ? d2 * inv_d : Real(0);
-      Real f, df = 0;
-      elec_eval<Real, GRAD>(d, K, f, df);
-      const Real wq = wcp * p1.q * p2.q;
-      acc.atr += wq * f;
-      if (GRAD && d != Real(0)) {
-        const Real g = wq * c.wt0 * df * inv_d;
-        fx = g * dx;
-        fy = g * dy;
-        fz = g * dz;
-      }
-    } else if (act) {
-      const AtomRec<Real> p1 = w.at[a1];
-      const AtomRec<Real> p2 = w.at[j];
-      int t1 = p1.tf & 0xff, t2 = p2.tf & 0xff;
-      // records are symmetric in the two types (LJ by construction, LK as
-      // sums of both directions), so only the upper triangle is read (lower
-      // type first): half the tables' footprint in L1
-      Real dx = p1.x - p2.x;
-      Real dy = p1.y - p2.y;
-      Real dz = p1.z - p2.z;
-      const Real d2 = dx * dx + dy * dy + dz * dz;
-      // coincident atoms (d2 = 0) take the linear LJ and flat LK regions,
-      // which never use inv_d, and add no force
-      const Real inv_d = inv_sqrt(d2);
-      const Real d = d2 > Real(0) ? d2 * inv_d : Real(0);
-      int tp = t1 < t2 ? t1 * c.ntp + t2 : t2 * c.ntp + t1;
-      Real atr, rep, datr, drep;
-      lj_eval<Real, GRAD>(d, inv_d, c.ljtab + tp, atr, rep, datr, drep);
-      acc.atr += wcp * atr;
-      acc.rep += wcp * rep;
-      Real dE = c.wt0 * datr + c.wt1 * drep;
-      if (heavy) {
-        Real lk, dlk;
-        lk_eval<Real, GRAD>(d, inv_d, c.lktab + tp, far_dmin, far_first, inv_hf, lk, dlk);
-        acc.lk += wcp * lk;
-        dE += c.wt2 * dlk;
-      }
-      if (GRAD && d != Real(0)) {
-        Real f = wcp * dE * inv_d;
-        fx = f * dx;
-        fy = f * dy;
-        fz = f * dz;
-      }
-    }
-    if (GRAD) {
-      // segments: maximal runs of lanes with equal j (the entry's k); a
-      // run only merges lanes before the next segment head, so j values that
-      // recur later in the warp form separate segments
-      int key = act ? j : -1 - lane;
-      int kprev = __shfl_up_sync(0xffffffffu, key, 1);
-      bool head = lane == 0 || kprev != key;
-      unsigned heads = __ballot_sync(0xffffffffu, head);
-      unsigned after = heads & ~((2u << lane) - 1u);
-      int seg_end = after ? __ffs(after) - 1 : 32;
-      Real sx = fx, sy = fy, sz = fz;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        Real tx = __shfl_down_sync(0xffffffffu, sx, o);
-        Real ty = __shfl_down_sync(0xffffffffu, sy, o);
-        Real tz = __shfl_down_sync(0xffffffffu, sz, o);
-        if (lane + o < seg_end) {
-          sx += tx;
-          sy += ty;
-          sz += tz;
-        }
-      }
-      // segment heads and a targets add with shared-memory atomics: the
-      // same j can head two segments and the same a1 sit in two runs'
-      // entries of one step (cheaper than finding the unique targets)
-      const bool add0 = act && head;
-      if (add0) {
-        atomicAdd(&w.gx[j], -sx);
-        atomicAdd(&w.gy[j], -sy);
-        atomicAdd(&w.gz[j], -sz);
-      }
-      __syncwarp();
-      if (act) {
-        Real(*ga)[TILE] = w.ga[lane & (A_COPIES - 1)];
-        atomicAdd(&ga[0][a1], fx);
-        atomicAdd(&ga[1][a1], fy);
-        atomicAdd(&ga[2][a1], fz);
-      }
-      __syncwarp();  // the next step's adds may touch the same atoms
-    }
-  }
-  return acc;
-}
-
-template <typename Real, bool GRAD, int TERM = kTermLJLK, bool COUNT = true>
-__device__ __forceinline__ void drain_queue(const EvalCtx<Real>& c,
-                                            Slab<Real>* wp, int& nl, int& nh,
-                                            int lane, E3<Real>& acc) {
-  __syncwarp();
-  if (COUNT) {
-    cnt_add(wp->counts, 3, nl + nh, lane);
-    cnt_add(wp->counts, 4, nh, lane);
-  }
-  if (nl + nh) {
-    E3<Real> e = eval_queue<Real, GRAD, TERM>(c, wp, nl, nh, lane);
-    acc.atr += e.atr;
-    acc.rep += e.rep;
-    acc.lk += e.lk;
-  }
-  __syncwarp();
-  nl = 0;
-  nh = 0;
-}
-
-__device__ __forceinline__ void queue_push(uint16_t* queue, bool in, bool hv,
-                                           int entry, int lane, int& nl,
-                                           int& nh) {
-  unsigned lt = (1u << lane) - 1;
-  unsigned mh = __ballot_sync(0xffffffffu, hv);
-  unsigned ml = __ballot_sync(0xffffffffu, in && !hv);
-  if ((mh | ml) == 0) return;
-  if (hv) queue[QCAP - 1 - (nh + __popc(mh & lt))] = (uint16_t)entry;
-  if (in && !hv) queue[nl + __popc(ml & lt)] = (uint16_t)entry;
-  nh += __popc(mh);
-  nl += __popc(ml);
-}
-
-// Pairs inside the side-0 tile of c1 atoms (a1 < a2), weights from the
-// intra-block separation table (ljlk_pose_score.impl.hh:115-134; the ligand
-// 3/4 -> 5 rule is already folded into that table and is not applied again).
-template <typename Real, bool GRAD, int TERM = kTermLJLK, bool COUNT = true>
-__device__ TMOL_B200_LJLK_OUTLINE E3<Real> intra_tile(EvalCtx<Real> c, Slab<Real>* wp,
-                                            int st1, int c1, int lane) {
-  Slab<Real>& w = *wp;
-  E3<Real> acc = {0, 0, 0};
-  const Real maxd2 = c.max_dis * c.max_dis;
-  int nl = 0, nh = 0;
-  int npairs = c1 * c1;
-  int qq = TILE / c1, rr = TILE - qq * c1;
-  int a1 = lane / c1, a2 = lane - a1 * c1;
-  for (int base = 0; base < npairs; base += 32) {
-    bool in = false, hv = false;
-    int wbit = 0;
-    if (base + lane < npairs && a1 < a2) {
-      const AtomRec<Real> p1 = w.at[a1], p2 = w.at[a2];
-      Real dx = p1.x - p2.x;
-      Real dy = p1.y - p2.y;
-      Real dz = p1.z - p2.z;
-      Real d2 = dx * dx + dy * dy + dz * dz;
-      if (d2 < maxd2) {
-        int sep = c.pd[a1 * c.A + st1 + a2];
-        in = sep >= 4;
-        wbit = sep == 4;
-        hv = TERM == kTermLJLK && in && (p1.tf & p2.tf & kTfHeavy);
-      }
-    }
-    // the row a1 is the entry's k (a row's entries are consecutive)
-    queue_push(w.queue, in, hv, a2 | (a1 << 5) | (wbit << 12), lane, nl, nh);
-    a1 += qq;
-    a2 += rr;
-    if (a2 >= c1) {
-      a2 -= c1;
-      a1 += 1;
-    }
-  }
-  drain_queue<Real, GRAD, TERM, COUNT>(c, wp, nl, nh, lane, acc);
-  return acc;
-}
-
-// Screen side 0 (c1 atoms, nc1 connections) against the m packed side-1
-// atoms of `ns` slots, draining the queue whenever it could overflow.  Lanes
-// walk the packed atoms (32 per chunk); side-0 atoms are broadcast one per
-// step, skipping those farther than r_k + max_dis from every slot block's
-// centroid.  Returns the lane's energy sums.
-template <typename Real, bool GRAD, int TERM = kTermLJLK, bool COUNT = true>
-__device__ TMOL_B200_LJLK_OUTLINE E3<Real> screen_slots(EvalCtx<Real> c, Slab<Real>* wp,
-                                              int c1, int nc1, int m, int ns,
-                                              int lane) {
-  Slab<Real>& w = *wp;
-  E3<Real> acc = {0, 0, 0};
-  const Real maxd2 = c.max_dis * c.max_dis;
-  bool act0 = false;
-  if (lane < c1) {
-    const AtomRec<Real> p0 = w.at[lane];
-    for (int k = 0; k < ns; ++k) {
-      Real dx = p0.x - w.slot_sph[k][0];
-      Real dy = p0.y - w.slot_sph[k][1];
-      Real dz = p0.z - w.slot_sph[k][2];
-      Real rr = w.slot_sph[k][3] + c.max_dis;
-      act0 |= dx * dx + dy * dy + dz * dz < rr * rr * Real(1.0001);
-    }
-  }
-  const unsigned rows = __ballot_sync(0xffffffffu, act0);
-  const unsigned heavy_rows =
-      TERM == kTermLJLK ? __ballot_sync(0xffffffffu, lane < c1 && (w.at[lane].tf & kTfHeavy)) : 0u;
-  int nl = 0, nh = 0;
-  for (int cbase = 0; cbase < m; cbase += 32) {
-    const int j = cbase + lane;
-    const bool valid = j < m;
-    const int jj = valid ? j : 0;
-    const AtomRec<Real> pj = w.at[TILE + jj];
-    const Real xj = pj.x, yj = pj.y, zj = pj.z;
-    const int heavy_j = TERM == kTermLJLK && valid ? (pj.tf & kTfHeavy) : 0;
-    const int slot = w.slot1[jj];
-    const int kind = w.slot_kind[slot];
-    // count-pair classes of this lane's pairs with the active rows, once per
-    // chunk: excl (separation < 4, weight 0) and w02 (separation 4, 0.2)
-    unsigned excl = 0, w02 = 0;
-    if (valid && kind != kSlotFar) {
-      const bool lig = w.slot_lig[slot];
-      if (kind == kSlotStriking) {
-        // separation through the connections: min over (u, v) of
-        // pd1[a1][u] + seps[u][v] + pd2[j][v], capped at 5; the minimum
-        // over v depends on this lane only
-        const int nc2 = w.slot_nc[slot];
-        const uint32_t cpdj = w.cpd1[jj];
-        const uint8_t* seps = w.seps[slot];
-        int best[MAX_CONN];
-#pragma unroll
-        for (int u = 0; u < MAX_CONN; ++u) {
-          best[u] = 255;
-          if (u < nc1)
-            for (int v = 0; v < nc2; ++v) {
-              const int t = seps[u * 4 + v] + ((cpdj >> (8 * v)) & 0xff);
-              best[u] = t < best[u] ? t : best[u];
-            }
-        }
-        for (unsigned rm = rows; rm; rm &= rm - 1) {
-          const int a1 = __ffs(rm) - 1;
-          const uint32_t c0 = w.cpd0[a1];
-          int sep = 5;
-#pragma unroll
-          for (int u = 0; u < MAX_CONN; ++u) {
-            const int t = (int)((c0 >> (8 * u)) & 0xff) + best[u];
-            sep = t < sep ? t : sep;
-          }
-          if (lig && (sep == 3 || sep == 4)) sep = 5;
-          excl |= (unsigned)(sep < 4) << a1;
-          w02 |= (unsigned)(sep == 4) << a1;
-        }
-      } else {
-        // another tile of block b1: the intra-block separation table
-        const uint8_t* pd = c.pd + w.local1[jj];
-        for (unsigned rm = rows; rm; rm &= rm - 1) {
-          const int a1 = __ffs(rm) - 1;
-          int sep = pd[a1 * c.A];
-          if (lig && (sep == 3 || sep == 4)) sep = 5;
-          excl |= (unsigned)(sep < 4) << a1;
-          w02 |= (unsigned)(sep == 4) << a1;
-        }
-      }
-    }
-    const unsigned live = valid ? rows & ~excl : 0u;
-    // distance tests of this lane's atom against every active row, as a
-    // row mask (no per-pair ballots)
-    unsigned inm = 0;
-    for (unsigned rm = rows; rm; rm &= rm - 1) {
-      const int a1 = __ffs(rm) - 1;
-      const AtomRec<Real> pa = w.at[a1];
-      const Real dx = pa.x - xj;
-      const Real dy = pa.y - yj;
-      const Real dz = pa.z - zj;
-      const Real d2 = dx * dx + dy * dy + dz * dz;
-      inm |= (d2 < maxd2 ? 1u : 0u) << a1;
-    }
-    inm &= live;
-    const unsigned hm = heavy_j ? inm & heavy_rows : 0u;
-    const unsigned lm = inm & ~hm;
-    // each lane's entries go out together (a run of equal k), at offsets
-    // from a warp scan of the counts (LJ-only low half-word, heavy high)
-    const int cnt = __popc(lm) | (__popc(hm) << 16);
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    const int tot = __shfl_sync(0xffffffffu, incl, 31);
-    const int tl = tot & 0xffff, th = tot >> 16;
-    if (tl + th == 0) continue;
-    if (nl + nh + tl + th > QCAP) drain_queue<Real, GRAD, TERM, COUNT>(c, wp, nl, nh, lane, acc);
-    const int before = incl - cnt;
-    int ql = nl + (before & 0xffff);
-    int qh = nh + (before >> 16);
-    const int kbits = (TILE + j) << 5;
-    for (unsigned b = lm; b; b &= b - 1) {
-      const int a1 = __ffs(b) - 1;
-      w.queue[ql++] = (uint16_t)(a1 | kbits | (int)(((w02 >> a1) & 1u) << 12));
-    }
-    for (unsigned b = hm; b; b &= b - 1) {
-      const int a1 = __ffs(b) - 1;
-      w.queue[QCAP - 1 - qh++] = (uint16_t)(a1 | kbits | (int)(((w02 >> a1) & 1u) << 12));
-    }
-    nl += tl;
-    nh += th;
-  }
-  drain_queue<Real, GRAD, TERM, COUNT>(c, wp, nl, nh, lane, acc);
-  return acc;
-}
-
-// Count-pair lookup for (row block, b2): lanes hold the row's partner list.
-struct RowPartners {
-  int b2;      // this lane's partner block, or -1
-  int minsep;  // its minimum bond separation
-  int entry;   // its cp table entry
-};
-
-// Adds a warp's block-pair energies to entry `o` of the [n_terms, stride]
-// output (the warp owns the entry).
-template <typename Real, int TERM>
-__device__ __forceinline__ void add_pair_energies(Real* out, int64_t stride, int64_t o,
-                                                  const E3<Real>& e, int lane) {
-  const Real v0 = warp_sum(e.atr);
-  if (TERM == kTermElec) {
-    if (lane == 0) out[o] += v0;
-    return;
-  }
-  const Real v1 = warp_sum(e.rep), v2 = warp_sum(e.lk);
-  if (lane == 0) {
-    out[o] += v0;
-    out[stride + o] += v1;
-    out[2 * stride + o] += v2;
-  }
-}
-
-// Scores the staged slots against side 0 and flushes their gradients.
-template <typename Real, bool GRAD, bool BLOCK_PAIR, int TERM, bool COUNT>
-__device__ __forceinline__ void score_group(const ScoreArgs<Real>& s,
-                                            Slab<Real>& w, const EvalCtx<Real>& c,
-                                            const RowInfo& r, int& m, int& ns,
-                                            int lane, E3<Real>& acc,
-                                            int64_t pair_o, bool want_E) {
-  __syncwarp();
-  if (m > 0) {
-    E3<Real> e = screen_slots<Real, GRAD, TERM, COUNT>(c, &w, r.c1, r.nc1, m, ns, lane);
-    if (GRAD) flush_side1(s, w, m, lane);
-    if (BLOCK_PAIR) {
-      if (want_E) add_pair_energies<Real, TERM>(s.energies, (int64_t)s.P * s.B * s.B, pair_o, e, lane);
-    } else {
-      acc.atr += e.atr;
-      acc.rep += e.rep;
-      acc.lk += e.lk;
-    }
-  }
-  __syncwarp();
-  m = 0;
-  ns = 0;
-}
-
-// The fused kernel.  A work item is (pose p, block b1, candidate range
-// [c0, c1) of later blocks b2 >= b1).  Every warp takes items from a global
-// ticket, tests b1 against each candidate with the bounding-sphere rule of
-// tmol/score/common/sphere_overlap.impl.hh:287-351 (32 per ballot) and
-// scores the hits: b1 with itself when b1 is in the range, the other
-// neighbours packed into side 1.  GRAD selects the adjoint (which also
-// yields the energies when s.energies is set); BLOCK_PAIR selects
-// per-block-pair energies / weights instead of per-pose ones (one block pair
-// per group).
-#ifndef TMOL_B200_FLOAT_MIN_CTAS
-#define TMOL_B200_FLOAT_MIN_CTAS 2
-#endif
-
-// float: up to 16 warps per CTA (one CTA of 16 warps per SM measured best),
-// 128 registers; double: up to 8 warps
-template <typename Real, bool GRAD, bool BLOCK_PAIR, int TERM, bool COUNT>
-__global__ void __launch_bounds__(sizeof(Real) == 4 ? 512 : 256, 1)
-    score_kernel(ScoreArgs<Real> s, int items_per_ticket) {
-  if (s.done && *s.done) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  Slab<Real>& w = reinterpret_cast<Slab<Real>*>(smem_raw)[warp];
-  if (lane < N_COUNTS) w.counts[lane] = 0;
-  __syncwarp();
-  const bool want_E = !GRAD || s.energies != nullptr;
-  const int64_t stride = (int64_t)s.P * s.B * s.B;
-  const int max_slots = BLOCK_PAIR ? 1 : s.max_slots;
-  const Real reach_atoms = s.g.max_dis;
-
-  const int n_work = s.ticket[2];
-  for (;;) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(s.ticket, 1);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    int it0 = t * items_per_ticket;
-    if (it0 >= n_work) break;
-    int it1 = min(it0 + items_per_ticket, n_work);
-    for (int item = it0; item < it1; ++item) {
-      // item costs for plan_rebalance: measured by the counting instantiation
-      const long long t_item = COUNT ? clock64() : 0;
-      int4 wi = s.work[item];
-      RowInfo r;
-      r.p = wi.x;
-      r.b1 = wi.y;
-      int cand0 = wi.z, cand1 = wi.w;
-      r.i1 = r.p * s.B + r.b1;
-      if (s.blk_info) {
-        const int4 bi1 = s.blk_info[r.i1];
-        r.bt1 = bi1.x;
-        if (r.bt1 < 0) continue;
-        r.off1 = bi1.y;
-        r.n1 = bi1.z;
-        r.nc1 = bi1.w & 0xff;
-        r.lig1 = bi1.w >> 8;
-      } else {
-        r.bt1 = s.blk_bt[r.i1];
-        if (r.bt1 < 0) continue;
-        r.off1 = s.blk_off[r.i1];
-        r.n1 = s.bt_n_atoms[r.bt1];
-        r.nc1 = s.bt_n_conn[r.bt1];
-        r.lig1 = s.bt_is_ligand[r.bt1];
-      }
-      E3<Real> acc = {0, 0, 0};
-      EvalCtx<Real> ec;
-      if (TERM == kTermElec)
-        ec.elec_k = s.elec_k;
-      else
-        ec.ljtab = s.ljtab;
-      ec.lktab = s.lktab;
-      ec.ntp = s.ntp;
-      ec.A = s.A;
-      ec.max_dis = s.g.max_dis;
-      ec.wt0 = ec.wt1 = ec.wt2 = 0;
-      if (GRAD && !BLOCK_PAIR) {
-        ec.wt0 = s.dTdV[r.p];
-        if (TERM == kTermLJLK) {
-          ec.wt1 = s.dTdV[s.P + r.p];
-          ec.wt2 = s.dTdV[2 * s.P + r.p];
-        }
-      }
-      const Quad<Real> sph1 = reinterpret_cast<const Quad<Real>*>(s.spheres)[r.i1];
-      const Real c1x = sph1.a, c1y = sph1.b, c1z = sph1.c, rad1 = sph1.d;
-      const Real reach1 = rad1 + reach_atoms;
-      const Real reach1_2 = reach1 * reach1 * Real(1.0001);
-
-      // with a skip mask: the row's count-pair partners, which it never skips
-      int skip_ncp = 0, skip_cp = -1;
-      if (s.skip) {
-        skip_ncp = s.cp_count[r.i1];
-        if (lane < skip_ncp) skip_cp = s.cp_b2[r.i1 * CP_CAP + lane];
-      }
-
-      // neighbour tests of the whole range first: one ballot mask per 32
-      // candidates, kept in registers (lane k holds the mask of batch k)
-      unsigned my_mask = 0;
-      int n_batches = (cand1 - cand0 + 31) / 32;
-      for (int bi = 0; bi < n_batches; ++bi) {
-        int b2 = cand0 + bi * 32 + lane;
-        bool hit = false;
-        if (b2 < cand1) {
-          int i2 = r.p * s.B + b2;
-          if (s.blk_bt[i2] >= 0) {
-            const Quad<Real> s2 = reinterpret_cast<const Quad<Real>*>(s.spheres)[i2];
-            Real dx = sub_rn(c1x, s2.a);
-            Real dy = sub_rn(c1y, s2.b);
-            Real dz = sub_rn(c1z, s2.c);
-            Real d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
-            Real thr = add_rn(add_rn(rad1, s2.d), s.reach);
-            hit = d2 < mul_rn(thr, thr);
-          }
-          if (s.nbr) s.nbr[(int64_t)r.i1 * s.B + b2] = hit ? 1 : 0;
-        }
-        if (s.skip) {
-          // a screened-out pair is dropped unless it is b1 itself or one of
-          // b1's count-pair partners (bond separation <= 4)
-          bool drop = hit && b2 != r.b1 &&
-                      ((s.skip[(int64_t)r.i1 * s.skip_words + (b2 >> 5)] >> (b2 & 31)) & 1u);
-          for (int k = 0; k < skip_ncp; ++k)
-            if (__shfl_sync(0xffffffffu, skip_cp, k) == b2) drop = false;
-          if (drop) hit = false;
-        }
-        unsigned mk = __ballot_sync(0xffffffffu, hit);
-        if (lane == bi) my_mask = mk;
-      }
-      bool any = __any_sync(0xffffffffu, my_mask != 0);
-      if (!any) {
-        if (COUNT && s.item_cost && lane == 0)
-          s.item_cost[item] = (int)min((clock64() - t_item) >> 4, (long long)0x7fffffff);
-        continue;
-      }
-
-      // the row's count-pair partners, one per lane
-      RowPartners rp;
-      {
-        int ncp = s.cp_count[r.i1];
-        rp.b2 = -1;
-        rp.minsep = 6;
-        rp.entry = r.i1 * CP_CAP + lane;
-        if (lane < ncp) {
-          rp.b2 = s.cp_b2[rp.entry];
-          rp.minsep = s.cp_minsep[rp.entry];
-        }
-      }
-      int nt1 = (r.n1 + TILE - 1) / TILE;
-      for (int ti = 0; ti < nt1; ++ti) {
-        r.st1 = ti * TILE;
-        r.c1 = min(TILE, r.n1 - r.st1);
-        stage_side0<Real, TERM>(s, w, r.bt1, r.off1, r.st1, r.c1, r.nc1, lane);
-        ec.pd = s.bt_pd + ((int64_t)r.bt1 * s.A + r.st1) * s.A;
-        __syncwarp();
-        int h1 = COUNT && TERM == kTermLJLK
-                     ? __popc(__ballot_sync(0xffffffffu, lane < r.c1 && (w.at[lane].tf & kTfHeavy)))
-                     : 0;
-        int m = 0, ns = 0;
-        int64_t pair_o = 0;
-        for (int bi = 0; bi < n_batches; ++bi) {
-          unsigned mask = __shfl_sync(0xffffffffu, my_mask, bi);
-          while (mask) {
-            int k = __ffs(mask) - 1;
-            mask &= mask - 1;
-            int bb2 = cand0 + bi * 32 + k;
-            if (bb2 == r.b1) {
-              // b1 with itself: this tile with itself, then with b1's later tiles
-              score_group<Real, GRAD, BLOCK_PAIR, TERM, COUNT>(s, w, ec, r, m, ns, lane, acc, pair_o, want_E);
-              pair_o = (int64_t)r.i1 * s.B + r.b1;
-              if (BLOCK_PAIR && GRAD) {
-                ec.wt0 = s.dTdV[pair_o];
-                if (TERM == kTermLJLK) {
-                  ec.wt1 = s.dTdV[stride + pair_o];
-                  ec.wt2 = s.dTdV[2 * stride + pair_o];
-                }
-              }
-              if (COUNT) {
-                if (ti == 0) {
-                  cnt_add(w.counts, 0, 1, lane);
-                  cnt_add(w.counts, 1, (long long)r.n1 * (r.n1 - 1) / 2, lane);
-                }
-                cnt_add(w.counts, 2, (long long)h1 * (h1 - 1) / 2, lane);
-              }
-              {
-                E3<Real> e = intra_tile<Real, GRAD, TERM, COUNT>(ec, &w, r.st1, r.c1, lane);
-                if (BLOCK_PAIR) {
-                  if (want_E) add_pair_energies<Real, TERM>(s.energies, stride, pair_o, e, lane);
-                } else {
-                  acc.atr += e.atr;
-                  acc.rep += e.rep;
-                  acc.lk += e.lk;
-                }
-              }
-              for (int tj = ti + 1; tj < nt1; ++tj) {
-                int st2 = tj * TILE, c2 = min(TILE, r.n1 - st2);
-                if (lane == 0) {
-                  w.slot_kind[0] = kSlotIntra;
-                  w.slot_nc[0] = 0;
-                  w.slot_lig[0] = 0;
-                  w.slot_sph[0][0] = c1x;
-                  w.slot_sph[0][1] = c1y;
-                  w.slot_sph[0][2] = c1z;
-                  w.slot_sph[0][3] = rad1;
-                }
-                int h2 = 0;
-                m = stage_side1<Real, TERM>(s, w, 0, 0, r.bt1, r.off1, st2, c2, 0, c1x, c1y, c1z, reach1_2, lane,
-                                            COUNT ? &h2 : nullptr);
-                if (COUNT) cnt_add(w.counts, 2, (long long)h1 * h2, lane);
-                ns = 1;
-                score_group<Real, GRAD, BLOCK_PAIR, TERM, COUNT>(s, w, ec, r, m, ns, lane, acc, pair_o, want_E);
-              }
-              continue;
-            }
-            int i2 = r.p * s.B + bb2;
-            int bt2, off2, n2, nc2_all, lig2;
-            if (s.blk_info) {
-              const int4 bi2 = s.blk_info[i2];
-              bt2 = bi2.x;
-              off2 = bi2.y;
-              n2 = bi2.z;
-              nc2_all = bi2.w & 0xff;
-              lig2 = bi2.w >> 8;
-            } else {
-              bt2 = s.blk_bt[i2];
-              off2 = s.blk_off[i2];
-              n2 = s.bt_n_atoms[bt2];
-              nc2_all = s.bt_n_conn[bt2];
-              lig2 = s.bt_is_ligand[bt2];
-            }
-            int nt2 = (n2 + TILE - 1) / TILE;
-            unsigned pm = __ballot_sync(0xffffffffu, rp.b2 == bb2);
-            int kind = kSlotFar, nc2 = 0, e = 0;
-            if (pm) {
-              int src = __ffs(pm) - 1;
-              int msep = __shfl_sync(0xffffffffu, rp.minsep, src);
-              e = __shfl_sync(0xffffffffu, rp.entry, src);
-              kind = msep <= 4 ? kSlotStriking : kSlotFar;
-            }
-            if (kind == kSlotStriking) nc2 = nc2_all;
-            int lig = r.lig1 && lig2;
-            const Real* s2 = s.spheres + 4 * (int64_t)i2;
-            if (COUNT && ti == 0) {
-              cnt_add(w.counts, 0, 1, lane);
-              cnt_add(w.counts, 1, (long long)r.n1 * n2, lane);
-            }
-            for (int tj = 0; tj < nt2; ++tj) {
-              int st2 = tj * TILE, c2 = min(TILE, n2 - st2);
-              if (m + c2 > M1 || ns == max_slots)
-                score_group<Real, GRAD, BLOCK_PAIR, TERM, COUNT>(s, w, ec, r, m, ns, lane, acc, pair_o, want_E);
-              if (lane == 0) {
-                w.slot_kind[ns] = kind;
-                w.slot_nc[ns] = nc2;
-                w.slot_lig[ns] = lig;
-              }
-              if (lane < 4) w.slot_sph[ns][lane] = s2[lane];
-              if (kind == kSlotStriking && lane < 16) w.seps[ns][lane] = s.cp_seps[(int64_t)e * 16 + lane];
-              int h2 = 0;
-              int kept = stage_side1<Real, TERM>(s, w, m, ns, bt2, off2, st2, c2, nc2, c1x, c1y, c1z, reach1_2, lane,
-                                                 COUNT ? &h2 : nullptr);
-              if (COUNT) cnt_add(w.counts, 2, (long long)h1 * h2, lane);
-              if (kept > 0) {
-                m += kept;
-                ns += 1;
-              }
-              if (BLOCK_PAIR) {
-                pair_o = (int64_t)r.i1 * s.B + bb2;
-                if (GRAD) {
-                  ec.wt0 = s.dTdV[pair_o];
-                  if (TERM == kTermLJLK) {
-                    ec.wt1 = s.dTdV[stride + pair_o];
-                    ec.wt2 = s.dTdV[2 * stride + pair_o];
-                  }
-                }
-              }
-            }
-          }
-        }
-        score_group<Real, GRAD, BLOCK_PAIR, TERM, COUNT>(s, w, ec, r, m, ns, lane, acc, pair_o, want_E);
-        if (GRAD) flush_side0(s, w, r.off1, r.st1, r.c1, lane);
-        __syncwarp();
-      }
-      if (!BLOCK_PAIR && want_E) {
-        Real v0 = warp_sum(acc.atr);
-        Real v1 = TERM == kTermLJLK ? warp_sum(acc.rep) : Real(0);
-        Real v2 = TERM == kTermLJLK ? warp_sum(acc.lk) : Real(0);
-        if (lane == 0) {
-          if (v0 != Real(0)) atomicAdd(&s.energies[r.p], v0);
-          if (v1 != Real(0)) atomicAdd(&s.energies[s.P + r.p], v1);
-          if (v2 != Real(0)) atomicAdd(&s.energies[2 * s.P + r.p], v2);
-        }
-      }
-      if (COUNT && s.item_cost && lane == 0)
-        s.item_cost[item] = (int)min((clock64() - t_item) >> 4, (long long)0x7fffffff);
-    }
-  }
-  __syncwarp();
-  if (COUNT && s.counts && lane < N_COUNTS && w.counts[lane])
-    atomicAdd(&s.counts[lane], w.counts[lane]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1538,8 +693,10 @@ template <typename Real>
 __global__ void rot_spheres_kernel(ScoreArgs<Real> s, RotArgs ra, Real* rs) {
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < ra.R; r += warps)
+  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < ra.R; r += warps) {
     warp_sphere(s.coords, s.bt_n_atoms, ra.rot_bt[r], ra.rot_off[r], lane, rs + 4 * (int64_t)r);
+    if (s.packed) pack_block(s, ra.rot_bt[r], ra.rot_off[r], lane);
+  }
 }
 
 // Block spheres enclosing all rotamers of each block: the mean of the
@@ -1710,22 +867,24 @@ __global__ void rot_row_fill_kernel(ScoreArgs<Real> s, RotArgs ra) {
   }
 }
 
-// Scoring of work items: rotamer rot1 (side 0, tile by tile) against the
-// rotamers rot2 of one neighbouring block (side 1, one rotamer tile per
-// group), or against itself on the diagonal.  Energies go to the item's
-// pairs (energies[t * n_pairs + d]; the warp owns them), the adjoint
+// Scoring of work items: rotamer rot1 (the rows, tile by tile) against the
+// rotamers rot2 of one neighbouring block (side 1: a word or more each, as
+// block pairs have in score_kernel), or against itself on the diagonal.
+// Energies go to the item's pairs (energies[t * n_pairs + d]), the adjoint
 // weights come from dTdV[t * n_pairs + d].
 template <typename Real, bool GRAD, int TERM, bool COUNT>
-__global__ void __launch_bounds__(256, sizeof(Real) == 4 ? TMOL_B200_FLOAT_MIN_CTAS : 1)
+__global__ void __launch_bounds__(sizeof(Real) == 4 ? 512 : 256, 1)
     rotamer_kernel(ScoreArgs<Real> s, RotArgs ra, const Real* rs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Slab<Real>& w = reinterpret_cast<Slab<Real>*>(smem_raw)[warp];
-  if (lane < N_COUNTS) w.counts[lane] = 0;
-  __syncwarp();
-  const long long np = ra.n_pairs;
-  const bool want_E = s.energies != nullptr;
-  const Real reach_atoms = s.g.max_dis;
+  EvalCtx<Real> ec = eval_ctx(s);
+  ec.energies = s.energies;
+  ec.dTdV = s.dTdV;
+  ec.stride = ra.n_pairs;
+  const int max_words = min(MAXW, s.max_slots);
+  long long n_bp = 0, n_ap = 0, n_in[2] = {0, 0};
+  E3<Real> unused = {0, 0, 0};  // energies go to their pairs
   for (;;) {
     int it = 0;
     if (lane == 0) it = atomicAdd(s.ticket, 1);
@@ -1734,138 +893,132 @@ __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? TMOL_B200_FLOAT_MIN_C
     const int4 item = ra.items[it];
     const int rot1 = item.x, rot2_first = item.y, n_rot2 = item.z;
     const long long pair_first = item.w;
-    RowInfo r;
-    r.p = ra.rot_pose[rot1];
-    r.b1 = ra.rot_block[rot1];
-    r.i1 = r.p * s.B + r.b1;
-    r.bt1 = ra.rot_bt[rot1];
-    r.off1 = ra.rot_off[rot1];
-    r.n1 = s.bt_n_atoms[r.bt1];
-    r.nc1 = s.bt_n_conn[r.bt1];
-    r.lig1 = s.bt_is_ligand[r.bt1];
-    EvalCtx<Real> ec;
-    if (TERM == kTermElec)
-      ec.elec_k = s.elec_k;
-    else
-      ec.ljtab = s.ljtab;
-    ec.lktab = s.lktab;
-    ec.ntp = s.ntp;
-    ec.A = s.A;
-    ec.max_dis = s.g.max_dis;
-    ec.wt0 = ec.wt1 = ec.wt2 = 0;
-    const Real* sph1 = rs + 4 * (int64_t)rot1;
-    const Real c1x = sph1[0], c1y = sph1[1], c1z = sph1[2], rad1 = sph1[3];
-    const Real reach1 = rad1 + reach_atoms;
+    const int p = ra.rot_pose[rot1], b1 = ra.rot_block[rot1];
+    const int64_t i1 = (int64_t)p * s.B + b1;
+    RowSide r;
+    r.bt = ra.rot_bt[rot1];
+    r.nc = s.bt_n_conn[r.bt];
+    r.lig = s.bt_is_ligand[r.bt];
+    const int n1 = s.bt_n_atoms[r.bt], off1 = ra.rot_off[rot1];
+    const Quad<Real> sph1 = reinterpret_cast<const Quad<Real>*>(rs)[rot1];
+    const Real reach1 = sph1.d + s.g.max_dis;
     const Real reach1_2 = reach1 * reach1 * Real(1.0001);
     const bool diag = rot2_first == rot1;
-    // block-level count pair of (b1, b2): kind and connection separations
-    int kind = kSlotFar, cp_entry = 0, b2 = diag ? r.b1 : ra.rot_block[rot2_first];
+    // block-level count pair of (b1, b2): the connection separations
+    const uint8_t* seps = nullptr;
     if (!diag) {
-      const int ncp = s.cp_count[r.i1];
-      const int e = r.i1 * CP_CAP + lane;
-      const bool match = lane < ncp && s.cp_b2[e] == b2;
-      const unsigned pm = __ballot_sync(0xffffffffu, match);
-      if (pm) {
-        const int src = __ffs(pm) - 1;
-        const int msep = __shfl_sync(0xffffffffu, lane < ncp ? s.cp_minsep[e] : 6, src);
-        cp_entry = r.i1 * CP_CAP + src;
-        kind = msep <= 4 ? kSlotStriking : kSlotFar;
-      }
+      const int b2 = ra.rot_block[rot2_first], ncp = s.cp_count[i1];
+      const unsigned pm = __ballot_sync(0xffffffffu, lane < ncp && s.cp_b2[i1 * CP_CAP + lane] == b2);
+      if (pm) seps = s.cp_seps + (i1 * CP_CAP + __ffs(pm) - 1) * 16;
     }
-    const int nt1 = (r.n1 + TILE - 1) / TILE;
-    for (int ti = 0; ti < nt1; ++ti) {
-      r.st1 = ti * TILE;
-      r.c1 = min(TILE, r.n1 - r.st1);
-      stage_side0<Real, TERM>(s, w, r.bt1, r.off1, r.st1, r.c1, r.nc1, lane);
-      ec.pd = s.bt_pd + ((int64_t)r.bt1 * s.A + r.st1) * s.A;
-      __syncwarp();
-      for (int k = 0; k < n_rot2; ++k) {
-        const long long d = pair_first + k;
-        if (GRAD) {
-          ec.wt0 = s.dTdV[d];
-          if (TERM == kTermLJLK) {
-            ec.wt1 = s.dTdV[np + d];
-            ec.wt2 = s.dTdV[2 * np + d];
+    const bool masked = diag || seps != nullptr;
+    for (int ti = 0; ti * TILE < n1; ++ti) {
+      r.st = ti * TILE;
+      r.c1 = min(TILE, n1 - r.st);
+      ec.row0 = (int64_t)off1 + r.st;
+      AtomRec<Real> a1;
+      a1.x = a1.y = a1.z = Real(0);
+      a1.tf = 0;
+      if (lane < r.c1) a1 = s.packed[ec.row0 + lane];
+      w.row[lane] = a1;
+      const unsigned heavy_rows =
+          TERM == kTermLJLK ? __ballot_sync(0xffffffffu, lane < r.c1 && (a1.tf & kTfHeavy)) : 0u;
+      const int at_first = diag ? r.st : 0;
+      int next = 0, batch = 0, at = at_first;
+      unsigned hits = 0;
+      int bt2 = 0, off2 = 0, n2 = 0;  // this lane's rotamer of the batch
+      bool done = false;
+      while (!done) {
+        int m = 0, nw = 0, nsp = 0;
+        for (;;) {
+          if (hits) {
+            const int src = __ffs(hits) - 1;
+            const int off = __shfl_sync(0xffffffffu, off2, src), n = __shfl_sync(0xffffffffu, n2, src);
+            const int cnt = min(32, n - at);
+            if (nw >= max_words || m + 32 > M1 || (masked && nsp == MAXSP)) break;
+            int used = cnt;
+            if (cnt > 0 && masked) {
+              const int bt = __shfl_sync(0xffffffffu, bt2, src);
+              stage_special(s, w, r, m, nsp, bt, (int64_t)off, at, cnt, diag, seps, diag ? 0 : s.bt_n_conn[bt],
+                            !diag && r.lig && s.bt_is_ligand[bt], lane);
+              if (lane < cnt) w.slot[m + lane] = (uint8_t)nw;
+              ++nsp;
+            } else if (cnt > 0) {
+              const bool valid = lane < cnt;
+              const int64_t gi = (int64_t)off + at + lane;
+              AtomRec<Real> a;
+              a.x = a.y = a.z = Real(0);
+              a.tf = 0;
+              if (valid) a = s.packed[gi];
+              used = stage_culled(w, m, valid, a, gi, sph1.a, sph1.b, sph1.c, reach1_2, nw, lane);
+            }
+            if (used > 0) {
+              if (lane == 0) {
+                w.desc[nw] = m | (used << 8) | (masked ? nsp << 16 : 0);
+                w.out[nw] = pair_first + batch + src;
+              }
+              m += (used + 3) & ~3;
+              ++nw;
+            }
+            at += 32;
+            if (at >= n) {
+              at = at_first;
+              hits &= hits - 1;
+            }
+          } else if (next < n_rot2) {
+            // the next 32 rotamers; every atom of rot2 lies within its radius
+            // of its centre: when the spheres are farther apart than both
+            // radii plus the reach no atom pair is in range
+            batch = next;
+            next += 32;
+            bool hit = false;
+            if (batch + lane < n_rot2) {
+              const int rot2 = rot2_first + batch + lane;
+              bt2 = ra.rot_bt[rot2];
+              off2 = ra.rot_off[rot2];
+              n2 = s.bt_n_atoms[bt2];
+              const Quad<Real> q = reinterpret_cast<const Quad<Real>*>(rs)[rot2];
+              const Real sx = q.a - sph1.a, sy = q.b - sph1.b, sz = q.c - sph1.c;
+              const Real lim = reach1 + q.d;
+              hit = diag || sx * sx + sy * sy + sz * sz < lim * lim * Real(1.0001);
+              if (COUNT && ti == 0) {
+                n_bp += 1;
+                n_ap += diag ? (long long)n1 * (n1 - 1) / 2 : (long long)n1 * n2;
+              }
+            }
+            hits = __ballot_sync(0xffffffffu, hit);
+          } else {
+            done = true;
+            break;
           }
         }
-        E3<Real> e = {0, 0, 0};
-        if (ti == 0) {
-          const long long n2a = diag ? 0 : s.bt_n_atoms[ra.rot_bt[rot2_first + k]];
-          if (COUNT) {
-            cnt_add(w.counts, 0, 1, lane);
-            cnt_add(w.counts, 1, diag ? (long long)r.n1 * (r.n1 - 1) / 2 : (long long)r.n1 * n2a, lane);
-          }
-        }
-        if (diag) {
-          // this tile with itself, then with the rotamer's later tiles
-          E3<Real> t = intra_tile<Real, GRAD, TERM, COUNT>(ec, &w, r.st1, r.c1, lane);
-          e.atr += t.atr;
-          e.rep += t.rep;
-          e.lk += t.lk;
-          for (int tj = ti + 1; tj < nt1; ++tj) {
-            const int st2 = tj * TILE, c2 = min(TILE, r.n1 - st2);
-            if (lane == 0) {
-              w.slot_kind[0] = kSlotIntra;
-              w.slot_nc[0] = 0;
-              w.slot_lig[0] = 0;
-              w.slot_sph[0][0] = c1x;
-              w.slot_sph[0][1] = c1y;
-              w.slot_sph[0][2] = c1z;
-              w.slot_sph[0][3] = rad1;
-            }
-            const int m = stage_side1<Real, TERM>(s, w, 0, 0, r.bt1, r.off1, st2, c2, 0, c1x, c1y, c1z, reach1_2, lane);
-            __syncwarp();
-            if (m > 0) {
-              E3<Real> g = screen_slots<Real, GRAD, TERM, COUNT>(ec, &w, r.c1, r.nc1, m, 1, lane);
-              if (GRAD) flush_side1(s, w, m, lane);
-              e.atr += g.atr;
-              e.rep += g.rep;
-              e.lk += g.lk;
-            }
-            __syncwarp();
-          }
-        } else {
-          const int rot2 = rot2_first + k;
-          const int bt2 = ra.rot_bt[rot2], off2 = ra.rot_off[rot2];
-          const int nc2 = kind == kSlotStriking ? s.bt_n_conn[bt2] : 0;
-          const int lig = r.lig1 && s.bt_is_ligand[bt2];
-          const Real* sph2 = rs + 4 * (int64_t)rot2;
-          // every atom of rot2 lies within its radius of its centre: when the
-          // spheres are farther apart than both radii plus the reach, the
-          // atom cull would drop them all, so the pair is left at zero
-          const Real sx = sph2[0] - c1x, sy = sph2[1] - c1y, sz = sph2[2] - c1z;
-          const Real lim = reach1 + sph2[3];
-          const int n2 = sx * sx + sy * sy + sz * sz < lim * lim * Real(1.0001) ? s.bt_n_atoms[bt2] : 0;
-          for (int st2 = 0; st2 < n2; st2 += TILE) {
-            const int c2 = min(TILE, n2 - st2);
-            if (lane == 0) {
-              w.slot_kind[0] = kind;
-              w.slot_nc[0] = nc2;
-              w.slot_lig[0] = lig;
-            }
-            if (lane < 4) w.slot_sph[0][lane] = sph2[lane];
-            if (kind == kSlotStriking && lane < 16) w.seps[0][lane] = s.cp_seps[(int64_t)cp_entry * 16 + lane];
-            const int m = stage_side1<Real, TERM>(s, w, 0, 0, bt2, off2, st2, c2, nc2, c1x, c1y, c1z, reach1_2, lane);
-            __syncwarp();
-            if (m > 0) {
-              E3<Real> g = screen_slots<Real, GRAD, TERM, COUNT>(ec, &w, r.c1, r.nc1, m, 1, lane);
-              if (GRAD) flush_side1(s, w, m, lane);
-              e.atr += g.atr;
-              e.rep += g.rep;
-              e.lk += g.lk;
-            }
-            __syncwarp();
-          }
-        }
-        if (want_E) add_pair_energies<Real, TERM>(s.energies, np, d, e, lane);
+        if (nw > 0)
+          process_group<Real, GRAD, true, TERM, COUNT>(ec, w, nw, r.c1, a1.x, a1.y, a1.z, heavy_rows, lane, unused,
+                                                       n_in);
       }
-      if (GRAD) flush_side0(s, w, r.off1, r.st1, r.c1, lane);
       __syncwarp();
     }
   }
-  __syncwarp();
-  if (COUNT && s.counts && lane < N_COUNTS && w.counts[lane])
-    atomicAdd(&s.counts[lane], w.counts[lane]);
+  if (COUNT && s.counts) {
+    const long long v[N_COUNTS] = {warp_sum(n_bp), warp_sum(n_ap), 0, warp_sum(n_in[0]), warp_sum(n_in[1])};
+    if (lane == 0)
+      for (int k = 0; k < N_COUNTS; ++k)
+        if (v[k]) atomicAdd(&s.counts[k], (unsigned long long)v[k]);
+  }
+}
+
+// The gradient from its padded form: out [n_atoms][3] = hit or miss
+// [n_atoms][4] (hit when *flag is set; a null flag: miss), 0 for atoms that
+// belong to no block.
+template <typename Real>
+__global__ void grad_out_kernel(const int* flag, const Real* hit, const Real* miss, const uint8_t* real, Real* out,
+                                int64_t n_atoms) {
+  const Real* src = flag && *flag ? hit : miss;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * n_atoms;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t a = i / 3;
+    out[i] = real[a] ? src[4 * a + (i - 3 * a)] : Real(0);
+  }
 }
 
 #include "lkball.cuh"
@@ -2052,7 +1205,14 @@ struct tmol_b200_ljlk_plan {
   int* blk_bt = nullptr;
   int* blk_off = nullptr;
   int4* blk_info = nullptr;  // pose plans of LJ/LK and elec: {bt, off, n_atoms, n_conn | ligand << 8}
-  void* packed = nullptr;    // and their atoms as staged records [n_atoms], rewritten every call
+  void* packed = nullptr;    // LJ/LK and elec: atoms as staged records [n_atoms], rewritten every call
+  void* g4 = nullptr;        // and the gradient as [n_atoms][4]
+  uint8_t* real_atom = nullptr;  // [n_atoms] 1 where a block (or rotamer) has the atom
+  uint2* imask = nullptr;        // [nbt * A][n_iwords] pairs within a block type
+  int n_iwords = 0;
+  int* bt_n_heavy = nullptr;
+  void* fartab = nullptr;
+  double far_d = 0;  // where far pairs start, 0: none
   int* pose_last = nullptr;
   uint16_t* bt_tf = nullptr;
   int* type_map = nullptr;
@@ -2075,7 +1235,7 @@ struct tmol_b200_ljlk_plan {
   int n_work = 0;
   int work_cap = 0;  // capacity of work / item_cost
   void* spheres = nullptr;
-  int* counters = nullptr;  // [0] ticket, [1] status, [2] work items
+  int* counters = nullptr;  // [0] ticket, [1] status, [2] work items, [3] pairs fade on mixed intervals
   unsigned long long* counts = nullptr;  // [N_COUNTS] of the last forward
   bool counting = false;  // whole-pose LJ/LK and elec kernels fill `counts`
   // speculative gradient of the pose ops: the weights of the last
@@ -2084,7 +1244,7 @@ struct tmol_b200_ljlk_plan {
   // device flag a backward sets when its weights match those
   void* spec_next = nullptr;  // [n_terms, P]
   void* spec_used = nullptr;  // [n_terms, P]
-  void* spec_g = nullptr;     // [N, 3]
+  void* spec_g = nullptr;     // [N, 4] (LK-ball: [N, 3])
   void* spec_dw = nullptr;    // LK-ball: [N, 4, 3], the waters' gradient
   int* spec_flag = nullptr;
   bool spec_ready = false;  // spec_next holds a backward's weights
@@ -2151,7 +1311,8 @@ void free_plan(tmol_b200_ljlk_plan* pl) {
                   pl->bt_q,      pl->elec_k,      pl->lkb_sites,   pl->lkb_pol,
                   pl->lkb_npol,  pl->lkb_occ,     pl->lkb_nocc,    pl->lkb_par,
                   pl->lkb_waters, pl->lkb_dwaters, pl->lkb_nbocc, pl->lkb_active,
-                  pl->blk_info,  pl->packed,      pl->spec_next,   pl->spec_used, pl->spec_g,
+                  pl->blk_info,  pl->packed,      pl->g4,          pl->real_atom,  pl->imask,
+                  pl->bt_n_heavy, pl->fartab,      pl->spec_next,   pl->spec_used, pl->spec_g,
                   pl->spec_dw,   pl->spec_flag};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -2164,8 +1325,8 @@ void default_launch(tmol_b200_ljlk_launch& l) {
   if (l.warps_per_cta <= 0) l.warps_per_cta = 8;
   if (l.ctas_per_sm <= 0) l.ctas_per_sm = 2;
   if (l.candidates_per_item <= 0) l.candidates_per_item = 64;
-  if (l.slots_per_group <= 0) l.slots_per_group = MAX_SLOTS;
-  l.slots_per_group = std::min(l.slots_per_group, MAX_SLOTS);
+  if (l.slots_per_group <= 0) l.slots_per_group = MAXW;
+  l.slots_per_group = std::min(l.slots_per_group, MAXW);
   l.rows_per_item = std::min(l.rows_per_item, MAX_ROWS_PER_ITEM);
   l.warps_per_cta = std::min(l.warps_per_cta, MAX_WARPS);
   l.candidates_per_item = std::min(l.candidates_per_item, 32 * 32);
@@ -2239,8 +1400,14 @@ ScoreArgs<Real> score_args(tmol_b200_ljlk_plan* pl, const void* coords) {
   s.packed = (AtomRec<Real>*)pl->packed;
   s.pose_last = pl->pose_last;
   s.bt_tf = pl->bt_tf;
-  s.ljtab = (const LJRecord<Real>*)pl->ljtab;
+  s.ljtab = (const Quad<Real>*)pl->ljtab;
   s.lktab = (const LKRecord<Real>*)pl->lktab;
+  s.fartab = (const Quad<Real>*)pl->fartab;
+  s.far_d = (Real)pl->far_d;
+  s.imask = pl->imask;
+  s.n_iwords = pl->n_iwords;
+  s.bt_n_heavy = pl->bt_n_heavy;
+  s.g4 = (Real*)pl->g4;
   s.ntp = pl->ntp;
   s.bt_pd = pl->bt_pd;
   s.bt_conn_pd = pl->bt_conn_pd;
@@ -2283,8 +1450,23 @@ ScoreArgs<Real> score_args(tmol_b200_ljlk_plan* pl, const void* coords) {
   s.counts = pl->counts;
   s.skip = pl->skip;
   s.skip_words = pl->skip_words;
-  s.max_slots = pl->launch.slots_per_group > 0 ? pl->launch.slots_per_group : MAX_SLOTS;
+  s.max_slots = pl->launch.slots_per_group > 0 ? pl->launch.slots_per_group : MAXW;
   return s;
+}
+
+// Warps per CTA and CTAs of a persistent launch over n_tickets: the plan's
+// shape, or fewer warps per CTA when the work cannot fill it, so that a small
+// call is spread over all SMs (one warp alone on an SM runs at its latency)
+// instead of filling a few of them.
+struct GridShape {
+  int warps, grid;
+};
+
+GridShape grid_shape(const tmol_b200_ljlk_plan* pl, int64_t n_tickets, int max_warps) {
+  const int ctas = pl->n_sm * pl->launch.ctas_per_sm;
+  int warps = std::min(pl->launch.warps_per_cta, max_warps);
+  warps = (int)std::min<int64_t>(warps, std::max<int64_t>(1, (n_tickets + ctas - 1) / ctas));
+  return GridShape{warps, (int)std::max<int64_t>(1, std::min<int64_t>((n_tickets + warps - 1) / warps, ctas))};
 }
 
 template <typename Real, bool GRAD, bool BLOCK_PAIR>
@@ -2292,12 +1474,14 @@ int launch_score(tmol_b200_ljlk_plan* pl, ScoreArgs<Real> s, cudaStream_t st) {
   int n_blocks = pl->P * pl->B;
   int threads = 256;
   int grid_s = std::max(1, std::min((n_blocks + 7) / 8, pl->n_sm * 16));
+  if (!GRAD) s.g4 = nullptr;
   spheres_kernel<Real><<<grid_s, threads, 0, st>>>(s);  // also resets the work ticket
   CK(cudaGetLastError());
   if (pl->n_work == 0) return TMOL_B200_OK;
-  int warps = pl->launch.warps_per_cta;
-  if (sizeof(Real) == 8) warps = std::min(warps, 8);  // the float64 kernel: at most 256 threads
-  size_t smem = warps * sizeof(Slab<Real>);
+  const int R = pl->launch.rows_per_item;
+  // the float64 kernel: at most 256 threads
+  const GridShape gs = grid_shape(pl, (pl->n_work + R - 1) / R, sizeof(Real) == 8 ? 8 : MAX_WARPS);
+  size_t smem = gs.warps * sizeof(Slab<Real>);
   // the work counters cost registers and instructions in the item loop:
   // they are compiled into a separate instantiation, used on request
   auto kern = pl->term == kTermElec
@@ -2305,17 +1489,25 @@ int launch_score(tmol_b200_ljlk_plan* pl, ScoreArgs<Real> s, cudaStream_t st) {
                                   : score_kernel<Real, GRAD, BLOCK_PAIR, kTermElec, false>)
                   : (pl->counting ? score_kernel<Real, GRAD, BLOCK_PAIR, kTermLJLK, true>
                                   : score_kernel<Real, GRAD, BLOCK_PAIR, kTermLJLK, false>);
-  int R = pl->launch.rows_per_item;
-  int n_tickets = (pl->n_work + R - 1) / R;
-  int grid = std::max(1, std::min((n_tickets + warps - 1) / warps, pl->n_sm * pl->launch.ctas_per_sm));
   bool prof = pl->profiling && 2 * (size_t)pl->prof_n + 1 < pl->prof_events.size();
   if (prof) CK(cudaEventRecord(pl->prof_events[2 * pl->prof_n], st));
-  kern<<<grid, 32 * warps, smem, st>>>(s, pl->launch.rows_per_item);
+  kern<<<gs.grid, 32 * gs.warps, smem, st>>>(s, R);
   CK(cudaGetLastError());
   if (prof) {
     CK(cudaEventRecord(pl->prof_events[2 * pl->prof_n + 1], st));
     ++pl->prof_n;
   }
+  return TMOL_B200_OK;
+}
+
+// dcoords [N, 3] from the padded gradient (`hit` instead when *flag is set).
+template <typename Real>
+int grad_out(tmol_b200_ljlk_plan* pl, const int* flag, const void* hit, void* dcoords, cudaStream_t st) {
+  if (pl->N == 0) return TMOL_B200_OK;
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((3 * pl->N + 255) / 256, (int64_t)pl->n_sm * 16));
+  grad_out_kernel<Real><<<grid, 256, 0, st>>>(flag, (const Real*)hit, (const Real*)pl->g4, pl->real_atom,
+                                              (Real*)dcoords, pl->N);
+  CK(cudaGetLastError());
   return TMOL_B200_OK;
 }
 
@@ -2342,11 +1534,9 @@ int backward_impl(tmol_b200_ljlk_plan* pl, const void* coords, int block_pair,
                   const void* dTdV, void* dcoords, cudaStream_t st) {
   ScoreArgs<Real> s = score_args<Real>(pl, coords);
   s.dTdV = (const Real*)dTdV;
-  s.dcoords = (Real*)dcoords;
   s.counts = nullptr;
-  s.zero_dcoords = (int64_t)pl->N * 3;  // by the sphere pass
-  if (block_pair) return launch_score<Real, true, true>(pl, s, st);
-  return launch_score<Real, true, false>(pl, s, st);
+  const int rc = block_pair ? launch_score<Real, true, true>(pl, s, st) : launch_score<Real, true, false>(pl, s, st);
+  return rc != TMOL_B200_OK ? rc : grad_out<Real>(pl, nullptr, nullptr, dcoords, st);
 }
 
 template <typename Real>
@@ -2355,13 +1545,12 @@ int energy_and_gradient_impl(tmol_b200_ljlk_plan* pl, const void* coords,
                              cudaStream_t st) {
   ScoreArgs<Real> s = score_args<Real>(pl, coords);
   s.dTdV = (const Real*)weights;
-  s.dcoords = (Real*)dcoords;
   s.energies = (Real*)energies;
   // the sphere pass zeroes the outputs before the scoring launch adds to them
-  s.zero_dcoords = (int64_t)pl->N * 3;
   s.zero_energies = (int64_t)n_terms(pl->term) * pl->P;
   s.zero_counts = 1;
-  return launch_score<Real, true, false>(pl, s, st);
+  const int rc = launch_score<Real, true, false>(pl, s, st);
+  return rc != TMOL_B200_OK ? rc : grad_out<Real>(pl, nullptr, nullptr, dcoords, st);
 }
 
 // Sets *flag to 1 when a[0, n) and b[0, n) are equal element by element
@@ -2397,11 +1586,10 @@ int forward_speculative_impl(tmol_b200_ljlk_plan* pl, const void* coords, void* 
   s.energies = (Real*)energies;
   s.nbr = nbr;
   s.dTdV = (const Real*)pl->spec_used;
-  s.dcoords = (Real*)pl->spec_g;
+  s.g4 = (Real*)pl->spec_g;
   if (nbr) CK(cudaMemsetAsync(nbr, 0, (size_t)pl->P * pl->B * pl->B * sizeof(int32_t), st));
   // energies, the kept gradient and the counters: by the sphere pass
   s.zero_energies = (int64_t)n_terms(pl->term) * pl->P;
-  s.zero_dcoords = (int64_t)pl->N * 3;
   s.zero_counts = 1;
   return launch_score<Real, true, false>(pl, s, st);
 }
@@ -2416,27 +1604,20 @@ template <typename Real>
 int backward_speculative_impl(tmol_b200_ljlk_plan* pl, const void* coords, const void* dTdV, void* dcoords,
                               int speculated, cudaStream_t st) {
   const int n_w = n_terms(pl->term) * pl->P;
-  const int64_t n_g = (int64_t)pl->N * 3;
   if (speculated && pl->spec_taken && n_w > 0) {
     spec_match_kernel<Real><<<1, 1024, 0, st>>>((const Real*)dTdV, (const Real*)pl->spec_used, n_w, pl->spec_flag);
     CK(cudaGetLastError());
   } else {
     CK(cudaMemsetAsync(pl->spec_flag, 0, sizeof(int), st));
   }
-  // a hit copies the kept gradient whole; a miss zeroes dcoords in the
-  // sphere pass (which a hit skips) before the scoring launch
-  if (n_g > 0) {
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n_g + 255) / 256, (int64_t)pl->n_sm * 8));
-    spec_copy_kernel<Real><<<grid, 256, 0, st>>>(pl->spec_flag, (const Real*)pl->spec_g, (Real*)dcoords, n_g);
-    CK(cudaGetLastError());
-  }
   ScoreArgs<Real> s = score_args<Real>(pl, coords);
   s.dTdV = (const Real*)dTdV;
-  s.dcoords = (Real*)dcoords;
   s.counts = nullptr;
   s.done = pl->spec_flag;
-  s.zero_dcoords = n_g;
-  const int rc = launch_score<Real, true, false>(pl, s, st);
+  int rc = launch_score<Real, true, false>(pl, s, st);
+  if (rc != TMOL_B200_OK) return rc;
+  // a hit takes the kept gradient, a miss the one just recomputed
+  rc = grad_out<Real>(pl, pl->spec_flag, pl->spec_g, dcoords, st);
   if (rc != TMOL_B200_OK) return rc;
   if (n_w > 0) CK(cudaMemcpyAsync(pl->spec_next, dTdV, (size_t)n_w * sizeof(Real), cudaMemcpyDeviceToDevice, st));
   pl->spec_ready = true;
@@ -2521,28 +1702,29 @@ int rotamer_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const int32_
   ra.n_pairs = n_pairs;
   s.energies = (Real*)energies;
   s.dTdV = (const Real*)dTdV;
-  s.dcoords = (Real*)dcoords;
+  if (!GRAD) s.g4 = nullptr;
   s.counts = GRAD ? nullptr : pl->counts;
   if (!GRAD) CK(cudaMemsetAsync(pl->counts, 0, N_COUNTS * sizeof(unsigned long long), st));
   if (energies) CK(cudaMemsetAsync(energies, 0, (size_t)n_terms(pl->term) * n_pairs * sizeof(Real), st));
-  if (dcoords) CK(cudaMemsetAsync(dcoords, 0, (size_t)pl->N * 3 * sizeof(Real), st));
-  if (n_items == 0) return TMOL_B200_OK;
+  if (n_items == 0) {
+    if (dcoords) CK(cudaMemsetAsync(dcoords, 0, (size_t)pl->N * 3 * sizeof(Real), st));
+    return TMOL_B200_OK;
+  }
   if (pl->R > 0) {
     int gr = std::max(1, std::min((pl->R + 7) / 8, pl->n_sm * 16));
     rot_spheres_kernel<Real><<<gr, 256, 0, st>>>(s, ra, (Real*)pl->rot_spheres);
     CK(cudaGetLastError());
   }
   CK(cudaMemsetAsync(pl->counters, 0, sizeof(int), st));
-  const int warps = std::min(pl->launch.warps_per_cta, 8);  // a kernel of at most 256 threads
-  const size_t smem = warps * sizeof(Slab<Real>);
-  int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n_items + warps - 1) / warps,
-                                                         (int64_t)pl->n_sm * pl->launch.ctas_per_sm));
+  // the float64 kernel: at most 256 threads
+  const GridShape gs = grid_shape(pl, n_items, sizeof(Real) == 8 ? 8 : MAX_WARPS);
+  const size_t smem = gs.warps * sizeof(Slab<Real>);
   auto kern = pl->term == kTermElec
                   ? (pl->counting ? rotamer_kernel<Real, GRAD, kTermElec, true> : rotamer_kernel<Real, GRAD, kTermElec, false>)
                   : (pl->counting ? rotamer_kernel<Real, GRAD, kTermLJLK, true> : rotamer_kernel<Real, GRAD, kTermLJLK, false>);
-  kern<<<grid, 32 * warps, smem, st>>>(s, ra, (const Real*)pl->rot_spheres);
+  kern<<<gs.grid, 32 * gs.warps, smem, st>>>(s, ra, (const Real*)pl->rot_spheres);
   CK(cudaGetLastError());
-  return TMOL_B200_OK;
+  return GRAD ? grad_out<Real>(pl, nullptr, nullptr, dcoords, st) : TMOL_B200_OK;
 }
 
 template <typename Real>
@@ -3017,9 +2199,9 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   pl->N = in->n_atoms;
   pl->reach = in->max_dis;
   pl->launch = launch ? *launch : tmol_b200_ljlk_launch{0, 0, 0, 0};
-  // float pose plans of LJ/LK and elec: one CTA of 16 warps per SM unless
-  // the caller chose
-  if (real_bytes == 4 && !rotamers && term != kTermLKBall && pl->launch.warps_per_cta <= 0 &&
+  // float plans of LJ/LK and elec: one CTA of 16 warps per SM unless the
+  // caller chose
+  if (real_bytes == 4 && term != kTermLKBall && pl->launch.warps_per_cta <= 0 &&
       pl->launch.ctas_per_sm <= 0) {
     pl->launch.warps_per_cta = 16;
     pl->launch.ctas_per_sm = 1;
@@ -3042,7 +2224,7 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   PCK(dalloc(pl, &pl->blk_off, PB));
   PCK(dalloc(pl, &pl->pose_last, P));
   PCK(dalloc(pl, &pl->bt_tf, (size_t)nbt * A));
-  PCK(dalloc(pl, &pl->type_map, std::max(T, 1)));
+  PCK(dalloc(pl, &pl->type_map, 2 * (size_t)std::max(T, 1)));
   PCK(dalloc(pl, &pl->bt_pd, (size_t)nbt * A * A));
   PCK(dalloc(pl, &pl->bt_conn_pd, (size_t)nbt * C * A));
   PCK(dalloc(pl, &pl->bt_flags, (size_t)nbt * A));
@@ -3054,13 +2236,22 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   PCK(dalloc(pl, &pl->cp_minsep, PB * CP_CAP));
   PCK(dalloc(pl, &pl->cp_seps, PB * CP_CAP * 16));
   PCK(dalloc(pl, (unsigned char**)&pl->spheres, PB * 4 * real_bytes));
+  if (term != kTermLKBall) {
+    const int64_t n_at = std::max<int64_t>(in->n_atoms, 1);
+    PCK(dalloc(pl, (unsigned char**)&pl->packed,
+               n_at * (real_bytes == 4 ? sizeof(AtomRec<float>) : sizeof(AtomRec<double>))));
+    PCK(dalloc(pl, (unsigned char**)&pl->g4, (size_t)n_at * 4 * real_bytes));
+    PCK(dalloc(pl, &pl->real_atom, n_at));
+    PCK(cudaMemsetAsync(pl->real_atom, 0, n_at, st));
+    pl->n_iwords = (A + 31) / 32;
+    PCK(dalloc(pl, &pl->imask, (size_t)nbt * A * pl->n_iwords));
+    PCK(dalloc(pl, &pl->bt_n_heavy, nbt));
+  }
   if (!rotamers && term != kTermLKBall) {
     PCK(dalloc(pl, &pl->blk_info, PB));
-    PCK(dalloc(pl, (unsigned char**)&pl->packed,
-               std::max<int64_t>(in->n_atoms, 1) * (real_bytes == 4 ? sizeof(AtomRec<float>) : sizeof(AtomRec<double>))));
     PCK(dalloc(pl, (unsigned char**)&pl->spec_next, (size_t)n_terms(term) * std::max(P, 1) * real_bytes));
     PCK(dalloc(pl, (unsigned char**)&pl->spec_used, (size_t)n_terms(term) * std::max(P, 1) * real_bytes));
-    PCK(dalloc(pl, (unsigned char**)&pl->spec_g, (size_t)std::max<int64_t>(in->n_atoms, 1) * 3 * real_bytes));
+    PCK(dalloc(pl, (unsigned char**)&pl->spec_g, (size_t)std::max<int64_t>(in->n_atoms, 1) * 4 * real_bytes));
     PCK(dalloc(pl, &pl->spec_flag, 1));
   }
   if (real_bytes == 4) PCK(dalloc(pl, &pl->sub_spheres, PB * 8));
@@ -3167,11 +2358,13 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     PCK(cudaMemcpyAsync(pl->host_pose_last.data(), pl->pose_last, sizeof(int) * P,
                         cudaMemcpyDeviceToHost, st));
   // compact atom types: the types the block types use, in index order
-  std::vector<int> h_types(term == kTermLJLK ? (size_t)nbt * A : 0), h_nat(std::max(nbt, 1));
+  std::vector<int> h_types(term == kTermLJLK ? (size_t)nbt * A : 0), h_flags(h_types.size()), h_nat(std::max(nbt, 1));
   if (nbt > 0) {
-    if (term == kTermLJLK)
+    if (term == kTermLJLK) {
       PCK(cudaMemcpyAsync(h_types.data(), in->bt_atom_types, sizeof(int) * h_types.size(),
                           cudaMemcpyDeviceToHost, st));
+      PCK(cudaMemcpyAsync(h_flags.data(), pl->bt_flags, sizeof(int) * h_flags.size(), cudaMemcpyDeviceToHost, st));
+    }
     PCK(cudaMemcpyAsync(h_nat.data(), in->bt_n_atoms, sizeof(int) * nbt, cudaMemcpyDeviceToHost, st));
   }
   PCK(cudaStreamSynchronize(st));
@@ -3180,19 +2373,33 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     free_plan(pl);
     return rc;
   }
-  std::vector<int> type_map(std::max(T, 1), -1), compact;
+  // heavy atoms and hydrogens of one type are two compact types (so that the
+  // far class reads LK's part of a pair, or zero, from one table), unless
+  // that takes more than the 255 a record can hold
+  std::vector<int> type_map(2 * (size_t)std::max(T, 1), -1), compact;
   for (int bt = 0; term == kTermLJLK && bt < nbt; ++bt) {
     int n = std::min(std::max(h_nat[bt], 0), A);
     for (int k = 0; k < n; ++k) {
       int t = h_types[(size_t)bt * A + k];
-      if (t >= 0 && t < T) type_map[t] = 0;
+      if (t >= 0 && t < T) type_map[2 * (size_t)t + (h_flags[(size_t)bt * A + k] == kHeavy ? 1 : 0)] = 0;
     }
   }
-  for (int t = 0; t < T; ++t)
-    if (type_map[t] == 0) {
-      type_map[t] = (int)compact.size();
+  int n_split = 0;
+  for (int v : type_map) n_split += v == 0;
+  const bool split = n_split <= 255;
+  for (int t = 0; t < T; ++t) {
+    int* m = &type_map[2 * (size_t)t];
+    if (!split && (m[0] == 0 || m[1] == 0)) {
+      m[0] = m[1] = (int)compact.size();
       compact.push_back(t);
+      continue;
     }
+    for (int h = 0; h < 2; ++h)
+      if (m[h] == 0) {
+        m[h] = (int)compact.size();
+        compact.push_back(h ? t : t | kTypeLight);
+      }
+  }
   pl->ntp = (int)compact.size();
   if (pl->ntp > 255) {
     free_plan(pl);
@@ -3201,11 +2408,12 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   size_t ntp2 = (size_t)std::max(pl->ntp, 1) * std::max(pl->ntp, 1);
   PCK(dalloc(pl, &pl->compact_types, std::max(pl->ntp, 1)));
   PCK(dalloc(pl, (unsigned char**)&pl->ljtab,
-             ntp2 * (real_bytes == 4 ? sizeof(LJRecord<float>) : sizeof(LJRecord<double>))));
+             2 * ntp2 * (real_bytes == 4 ? sizeof(Quad<float>) : sizeof(Quad<double>))));
+  PCK(dalloc(pl, (unsigned char**)&pl->fartab,
+             ntp2 * (real_bytes == 4 ? sizeof(Quad<float>) : sizeof(Quad<double>))));
   PCK(dalloc(pl, (unsigned char**)&pl->lktab,
              ntp2 * (real_bytes == 4 ? sizeof(LKRecord<float>) : sizeof(LKRecord<double>))));
-  PCK(cudaMemcpyAsync(pl->type_map, type_map.data(), sizeof(int) * std::max(T, 1),
-                      cudaMemcpyHostToDevice, st));
+  PCK(cudaMemcpyAsync(pl->type_map, type_map.data(), sizeof(int) * type_map.size(), cudaMemcpyHostToDevice, st));
   if (pl->ntp > 0)
     PCK(cudaMemcpyAsync(pl->compact_types, compact.data(), sizeof(int) * pl->ntp,
                         cudaMemcpyHostToDevice, st));
@@ -3213,6 +2421,22 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     int gb = std::max(1, std::min(((nbt * A) + 255) / 256, pl->n_sm * 8));
     plan_block_types_kernel<<<gb, 256, 0, st>>>(a, pl->type_map, pl->bt_tf);
     PCK(cudaGetLastError());
+    if (term != kTermLKBall) {
+      const int64_t n_im = (int64_t)nbt * A * pl->n_iwords;
+      const int gi = (int)std::max<int64_t>(1, std::min<int64_t>((n_im + 255) / 256, (int64_t)pl->n_sm * 8));
+      plan_intra_masks_kernel<<<gi, 256, 0, st>>>(pl->bt_pd, pl->bt_n_atoms, nbt, A, pl->n_iwords, pl->imask);
+      PCK(cudaGetLastError());
+      plan_heavy_count_kernel<<<(nbt + 127) / 128, 128, 0, st>>>(pl->bt_tf, pl->bt_n_atoms, nbt, A, pl->bt_n_heavy);
+      PCK(cudaGetLastError());
+    }
+  }
+  if (term != kTermLKBall) {
+    const int n = rotamers ? pl->R : (int)PB;
+    if (n > 0) {
+      plan_real_atoms_kernel<<<std::max(1, std::min((n + 127) / 128, pl->n_sm * 8)), 128, 0, st>>>(
+          rotamers ? pl->rot_bt : pl->blk_bt, rotamers ? pl->rot_off : pl->blk_off, n, pl->bt_n_atoms, pl->real_atom);
+      PCK(cudaGetLastError());
+    }
   }
   if (term == kTermElec) {
     // the potential's constants from the five global parameters, which the
@@ -3244,19 +2468,34 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     if (real_bytes == 4)
       plan_tables_kernel<float><<<gt, 128, 0, st>>>(
           (const float*)in->type_params, (const float*)in->global_params, pl->compact_types,
-          pl->ntp, (LJRecord<float>*)pl->ljtab, (LKRecord<float>*)pl->lktab);
+          pl->ntp, (Quad<float>*)pl->ljtab, (LKRecord<float>*)pl->lktab, (Quad<float>*)pl->fartab, pl->counters + 3);
     else
       plan_tables_kernel<double><<<gt, 128, 0, st>>>(
           (const double*)in->type_params, (const double*)in->global_params, pl->compact_types,
-          pl->ntp, (LJRecord<double>*)pl->ljtab, (LKRecord<double>*)pl->lktab);
+          pl->ntp, (Quad<double>*)pl->ljtab, (LKRecord<double>*)pl->lktab, (Quad<double>*)pl->fartab, pl->counters + 3);
     PCK(cudaGetLastError());
   }
+  int mixed = 0;
   PCK(cudaMemcpyAsync(&status_bits, pl->counters + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+  PCK(cudaMemcpyAsync(&mixed, pl->counters + 3, sizeof(int), cudaMemcpyDeviceToHost, st));
   PCK(cudaStreamSynchronize(st));
   rc = status_from_bits(status_bits);
   if (rc != TMOL_B200_OK) {
     free_plan(pl);
     return rc;
+  }
+  // where the far class starts: LJ/LK where both potentials fade, for every
+  // pair of types (LK's close cubics end by sqrt(405 / 20) = 4.5 A); elec
+  // where its fade starts, beyond the low spline
+  if (term == kTermLJLK && split && !mixed) {
+    const double dmax = real_bytes == 4 ? ((const float*)pl->global_params)[0] : ((const double*)pl->global_params)[0];
+    pl->far_d = std::max(dmax - 1.5, 4.5);
+  } else if (term == kTermElec) {
+    ElecK<double> k;
+    double* v = reinterpret_cast<double*>(&k);
+    for (int i = 0; i < N_ELEC_K; ++i)
+      v[i] = real_bytes == 4 ? ((const float*)pl->elec_k_host)[i] : ((const double*)pl->elec_k_host)[i];
+    pl->far_d = k.hi_start >= k.lo_end && k.hi_start > 0 ? k.hi_start : 0;
   }
   rc = (rotamers || !scoring) ? TMOL_B200_OK : build_work(pl, st);
   if (rc != TMOL_B200_OK) {

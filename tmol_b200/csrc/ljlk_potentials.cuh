@@ -343,15 +343,6 @@ namespace tmol_b200 {
 // cubic is evaluated for the pair.
 
 template <typename Real>
-struct alignas(4 * sizeof(Real)) LJRecord {  // 8 values, two groups of four
-  Real sigma, eps, d_lin, dmin;
-  Real inv_h;   // 1 / (max_dis - dmin), the fade-out interval
-  Real spl_V;   // 12-6 value at dmin (start of the fade)
-  Real spl_dp;  // 12-6 slope at dmin times the fade-out interval
-  Real pad;
-};
-
-template <typename Real>
 struct alignas(4 * sizeof(Real)) LKRecord {  // 16 values (13 used), four groups of four
   Real close_dmin, close_dmax;
   Real flat_V;                // both directions at d_min
@@ -370,24 +361,29 @@ struct alignas(4 * sizeof(Real)) Quad {
   Real a, b, c, d;
 };
 
+// LJ's values for one type pair, two groups in tables of their own:
+//   base (sigma, eps, d_lin, dmin)
+//   fade (1 / (max_dis - dmin), the fade-out interval; the 12-6 value at dmin,
+//         where the fade starts; the 12-6 slope there times the interval)
+
 template <typename Real>
 __device__ __forceinline__ void build_records(const AtomParams<Real>& i,
                                               const AtomParams<Real>& j,
                                               const GlobalParams<Real>& g,
-                                              LJRecord<Real>& lj,
+                                              Quad<Real>& base, Quad<Real>& fade,
                                               LKRecord<Real>& lk) {
   LJPair<Real> q = lj_pair(i, j, g);
-  lj.sigma = q.sigma;
-  lj.eps = q.eps;
-  lj.d_lin = q.d_lin;
-  lj.dmin = q.dmin;
+  base.a = q.sigma;
+  base.b = q.eps;
+  base.c = q.d_lin;
+  base.d = q.dmin;
   {
     Real spl_dV;
-    vdw_V_dV(q.dmin, q.sigma, q.eps, lj.spl_V, spl_dV);
+    vdw_V_dV(q.dmin, q.sigma, q.eps, fade.b, spl_dV);
     const Real h = g.max_dis - q.dmin;
-    lj.inv_h = Real(1) / h;
-    lj.spl_dp = spl_dV * h;
-    lj.pad = Real(0);
+    fade.a = Real(1) / h;
+    fade.c = spl_dV * h;
+    fade.d = Real(0);
   }
 
   bool cc = (i.flags & kCarbonLK) && (j.flags & kCarbonLK);
@@ -418,15 +414,13 @@ __device__ __forceinline__ void build_records(const AtomParams<Real>& i,
 
 // Unweighted LJ (atr, rep) and, with DERIV, their distance derivatives;
 // inv = 1 / d.  The fade-out cubic runs on t = (d - dmin) / (max_dis - dmin)
-// with the record's stored reciprocal and pre-scaled slope; the linear
+// with the stored reciprocal and pre-scaled slope; the linear
 // extension's knot value and slope (clashes only) are the 12-6 form's at
-// d_lin, computed here.  The record's second group of four is read only in
-// the fade-out region.
+// d_lin, computed here.  `fade` is read only in the fade-out region.
 template <typename Real, bool DERIV>
-__device__ __forceinline__ void lj_eval(Real d, Real inv, const LJRecord<Real>* rp,
-                                        Real& atr, Real& rep, Real& datr, Real& drep) {
-  const Quad<Real>* q = reinterpret_cast<const Quad<Real>*>(rp);
-  const Quad<Real> r = q[0];  // sigma, eps, d_lin, dmin
+__device__ __forceinline__ void lj_eval(Real d, Real inv, const Quad<Real>* base,
+                                        const Quad<Real>* fade, Real& atr, Real& rep, Real& datr, Real& drep) {
+  const Quad<Real> r = *base;  // sigma, eps, d_lin, dmin
   Real lj, dlj = 0;
   if (d < r.c) {
     Real lin_V, lin_dV;
@@ -441,7 +435,7 @@ __device__ __forceinline__ void lj_eval(Real d, Real inv, const LJRecord<Real>* 
     lj = r.b * (sd12 - Real(2) * sd6);
     if (DERIV) dlj = r.b * (Real(12) * (sd6 - sd12)) * inv;
   } else {
-    const Quad<Real> f = q[1];  // 1 / interval, value, interval-scaled slope
+    const Quad<Real> f = *fade;  // 1 / interval, value, interval-scaled slope
     Real t = (d - r.d) * f.a;
     Real p0 = f.b, dp0 = f.c;
     lj = p0 + t * (dp0 + t * (-2 * dp0 - 3 * p0 + t * (dp0 + 2 * p0)));

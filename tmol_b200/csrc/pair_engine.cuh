@@ -1,0 +1,788 @@
+// The atom-pair engine of the LJ/LK and elec kernels: one warp scores the
+// atoms of one block (or rotamer) against those of its neighbours.
+// Included by ljlk.cu inside namespace tmol_b200, after ScoreArgs.
+//
+// A warp works in groups.  The rows are up to 32 atoms of block b1, one per
+// lane, in registers; side 1 is a list of up to M1 neighbouring atoms in the
+// warp's shared-memory slab.  A group goes through three phases:
+//   1. screening: side 1 comes in words of up to 32 atoms.  Every lane tests
+//      its row against a word's atoms (broadcast, four at a time, packed
+//      pairs of float32 operations) and shifts the sign bits of d^2 - max^2
+//      and d^2 - far^2 into two masks: no compare, vote or branch per pair.
+//      Bonded neighbours and b1 itself have exclusion masks beside them.
+//   2. emission: each (row, word) writes its surviving pairs into a queue of
+//      16-bit entries, in three classes: far (both potentials are the cubic
+//      fade to zero), near without a heavy pair (LJ alone) and near heavy.
+//   3. evaluation, class by class: every lane takes an equal stretch of
+//      consecutive entries.  Lanes of a step run the same code, a stretch
+//      stays on one or two rows (their atom, force and, in pair mode,
+//      energies stay in registers), and the side-1 forces go out as one
+//      16-byte vector reduction per pair into a padded gradient buffer.
+//
+// What bounds it: instruction issue.  Shared-memory float atomics are
+// compare-and-swap loops here (three per pair and side measured 13-33
+// cycles of an SM and about 25 issue slots); one red.global.add.v4.f32 is a
+// single instruction and 44 cycles of an SM's path to L2, off the critical
+// path, which is why forces leave the SM at once instead of being summed in
+// shared memory.
+
+constexpr int M1 = 224;       // side-1 atoms of a group (< 256: 8-bit index)
+constexpr int MAXW = 12;      // words of a group
+constexpr int MAXW_PAD = 13;  // odd row stride of the mask arrays: no bank conflicts
+constexpr int MAXSP = 4;      // words with exclusion masks
+constexpr int kTfHeavy = 256;
+
+// One atom: coordinates and either the compact atom type | heavy << 8
+// (LJ/LK) or the partial charge (elec).
+template <typename Real>
+struct alignas(16) AtomRec {
+  Real x, y, z;
+  union {
+    int tf;
+    Real q;
+  };
+};
+
+// Queue entry: side-1 atom (bits 0-7), row (8-12), count-pair weight 0.2 (13).
+// The queue lives where the screening coordinates were: they are read out
+// before the first entry is written.  A single word (32 x 32 pairs) always
+// fits; a group with more pairs than the queue holds goes word by word.
+template <typename Real>
+struct Slab {
+  static constexpr int QCAP = 3 * M1 * sizeof(Real) / 2;
+  static_assert(QCAP >= 1024, "the queue holds any single word");
+  AtomRec<Real> at[M1];
+  int gidx[M1];  // global atom index
+  union {
+    struct {
+      Real x[M1], y[M1], z[M1];
+    } c;
+    uint16_t queue[QCAP];
+  };
+  uint32_t far[32 * MAXW_PAD], near[32 * MAXW_PAD];  // [row][word]
+  uint2 smask[MAXSP][32];                            // per row: excluded, weight 0.2
+  AtomRec<Real> row[32];
+  long long out[MAXW];  // pair mode: the word's energy entry
+  int desc[MAXW];       // base | atoms << 8 | (mask + 1) << 16
+  uint32_t heavy[MAXW];
+  int hoff[32];
+  uint8_t slot[M1];  // pair mode: the atom's word
+};
+
+template <typename Real>
+__device__ __forceinline__ Real warp_sum(Real v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+template <typename Real>
+struct E3 {
+  Real atr, rep, lk;
+};
+
+// What evaluating a pair needs beside the slab.
+template <typename Real>
+struct EvalCtx {
+  const Quad<Real>* lj;   // [2][ntp * ntp] LJ groups
+  const LKRecord<Real>* lk;
+  const Quad<Real>* far;  // [ntp * ntp] fade-out knots of both potentials
+  const Real* elec_k;
+  int ntp;
+  Real max2, far2;        // squares of the cutoff and of the far class's start
+  Real far_dmin, far_first, inv_hf;
+  Real wt0, wt1, wt2;     // gradient weights of the three terms (elec: wt0)
+  Real* g;                // padded gradient [n_atoms][4]
+  int64_t row0;           // global atom index of row 0
+  Real* energies;         // pair mode: [n_terms][stride]
+  const Real* dTdV;       // pair mode: the same shape
+  int64_t stride;
+};
+
+__device__ __forceinline__ void add_force(float* g, float x, float y, float z) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g), "f"(x), "f"(y), "f"(z), "f"(0.0f)
+               : "memory");
+}
+__device__ __forceinline__ void add_force(double* g, double x, double y, double z) {
+  atomicAdd(g, x);
+  atomicAdd(g + 1, y);
+  atomicAdd(g + 2, z);
+}
+
+// Packed pairs of float32 operations.
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
+                                                   unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// Screens one row against side-1 atoms [base, base + cnt): bit k of `in`
+// (d^2 < max2) and `near` (d^2 < far2).  Bits at and above cnt are undefined.
+struct RowTest {
+  unsigned in, near;
+};
+
+__device__ __forceinline__ RowTest test_row(const Slab<float>& w, int base, int cnt, float x, float y, float z,
+                                            float max2, float far2) {
+  const unsigned long long nx = pack2(-x, -x), ny = pack2(-y, -y), nz = pack2(-z, -z);
+  const unsigned long long cm = pack2(-max2, -max2), gap = pack2(max2 - far2, max2 - far2);
+  unsigned in = 0, near = 0;
+  for (int j = (cnt - 1) & ~3; j >= 0; j -= 4) {
+    const float4 X = *reinterpret_cast<const float4*>(w.c.x + base + j);
+    const float4 Y = *reinterpret_cast<const float4*>(w.c.y + base + j);
+    const float4 Z = *reinterpret_cast<const float4*>(w.c.z + base + j);
+    const unsigned long long dxa = add2(pack2(X.x, X.y), nx), dxb = add2(pack2(X.z, X.w), nx);
+    const unsigned long long dya = add2(pack2(Y.x, Y.y), ny), dyb = add2(pack2(Y.z, Y.w), ny);
+    const unsigned long long dza = add2(pack2(Z.x, Z.y), nz), dzb = add2(pack2(Z.z, Z.w), nz);
+    const unsigned long long ta = fma2(dza, dza, fma2(dya, dya, fma2(dxa, dxa, cm)));
+    const unsigned long long tb = fma2(dzb, dzb, fma2(dyb, dyb, fma2(dxb, dxb, cm)));
+    const unsigned long long ga = add2(ta, gap), gb = add2(tb, gap);
+    float t0, t1, t2, t3, g0, g1, g2, g3;
+    unpack2(ta, t0, t1);
+    unpack2(tb, t2, t3);
+    unpack2(ga, g0, g1);
+    unpack2(gb, g2, g3);
+    // the last atom first: after the loop atom k's sign is bit k
+    in = __funnelshift_l(__float_as_uint(t3), in, 1);
+    in = __funnelshift_l(__float_as_uint(t2), in, 1);
+    in = __funnelshift_l(__float_as_uint(t1), in, 1);
+    in = __funnelshift_l(__float_as_uint(t0), in, 1);
+    near = __funnelshift_l(__float_as_uint(g3), near, 1);
+    near = __funnelshift_l(__float_as_uint(g2), near, 1);
+    near = __funnelshift_l(__float_as_uint(g1), near, 1);
+    near = __funnelshift_l(__float_as_uint(g0), near, 1);
+  }
+  return RowTest{in, near};
+}
+
+__device__ __forceinline__ RowTest test_row(const Slab<double>& w, int base, int cnt, double x, double y, double z,
+                                            double max2, double far2) {
+  unsigned in = 0, near = 0;
+  for (int j = cnt - 1; j >= 0; --j) {
+    const double dx = w.c.x[base + j] - x, dy = w.c.y[base + j] - y, dz = w.c.z[base + j] - z;
+    const double d2 = dx * dx + dy * dy + dz * dz;
+    in = (in << 1) | (d2 < max2 ? 1u : 0u);
+    near = (near << 1) | (d2 < far2 ? 1u : 0u);
+  }
+  return RowTest{in, near};
+}
+
+enum PairClass : int { kFar = 0, kNear = 1, kNearHeavy = 2 };
+
+// Evaluates queue entries [q0, q0 + n) of one class.  Every lane takes a
+// stretch of S consecutive entries (S kept off multiples of four, whose
+// 16-bit stride would put the lanes' reads on the same banks).
+template <typename Real, bool GRAD, bool PAIR, int TERM, int CLS>
+__device__ __forceinline__ void eval_class(const EvalCtx<Real>& c, const Slab<Real>& w, int q0, int n, int lane,
+                                           E3<Real>& acc) {
+  if (n == 0) return;
+  int S = (n + 31) >> 5;
+  if ((S & 3) == 0) ++S;
+  const int cnt = min(S, n - lane * S);
+  const uint16_t* q = w.queue + q0 + lane * S;
+  int row = -1, slot = -1;
+  AtomRec<Real> a;
+  a.x = a.y = a.z = Real(0);
+  a.tf = 0;
+  Real fx = 0, fy = 0, fz = 0;
+  Real e0 = 0, e1 = 0, e2 = 0;
+  Real wt0 = c.wt0, wt1 = c.wt1, wt2 = c.wt2;
+  ElecK<Real> K;
+  if (TERM == kTermElec) K = load_elec_k(c.elec_k);
+  for (int s = 0; s < cnt; ++s) {
+    const int e = q[s];
+    const int j = e & 255, r = (e >> 8) & 31;
+    if (r != row) {
+      if (GRAD && row >= 0) {
+        add_force(c.g + 4 * (c.row0 + row), fx, fy, fz);
+        fx = fy = fz = 0;
+      }
+      row = r;
+      a = w.row[r];
+    }
+    if (PAIR) {
+      const int sl = w.slot[j];
+      if (sl != slot) {
+        if (slot >= 0 && c.energies) {
+          Real* o = c.energies + w.out[slot];
+          if (e0 != Real(0)) atomicAdd(o, e0);
+          if (TERM == kTermLJLK) {
+            if (e1 != Real(0)) atomicAdd(o + c.stride, e1);
+            if (CLS != kNear && e2 != Real(0)) atomicAdd(o + 2 * c.stride, e2);
+          }
+        }
+        e0 = e1 = e2 = 0;
+        slot = sl;
+        if (GRAD) {
+          const Real* wt = c.dTdV + w.out[sl];
+          wt0 = wt[0];
+          if (TERM == kTermLJLK) {
+            wt1 = wt[c.stride];
+            wt2 = wt[2 * c.stride];
+          }
+        }
+      }
+    }
+    const AtomRec<Real> b = w.at[j];
+    const Real dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+    const Real d2 = dx * dx + dy * dy + dz * dz;
+    const Real wcp = (e >> 13) ? Real(0.2) : Real(1);
+    // coincident atoms (d2 = 0) take the linear LJ, flat LK and flat elec
+    // regions, which never use inv_d, and add no force
+    const Real inv_d = inv_sqrt(d2);
+    const Real d = CLS == kFar || d2 > Real(0) ? d2 * inv_d : Real(0);
+    Real f;  // weighted dE/dd / d
+    if (TERM == kTermElec) {
+      const Real wq = wcp * a.q * b.q;
+      Real v, dv = 0;
+      if (CLS == kFar) {
+        const Real t = (d - K.hi_start) * K.inv_hi_w;
+        v = K.hi[0] + t * (K.hi[1] + t * (K.hi[2] + t * K.hi[3]));
+        if (GRAD) dv = (K.hi[1] + t * (Real(2) * K.hi[2] + Real(3) * t * K.hi[3])) * K.inv_hi_w;
+      } else {
+        elec_eval<Real, GRAD>(d, K, v, dv);
+      }
+      e0 += wq * v;
+      f = wq * wt0 * dv * inv_d;
+    } else {
+      const int tp = (a.tf & 0xff) * c.ntp + (b.tf & 0xff);
+      if (CLS == kFar) {
+        // both potentials fade on the same interval: a cubic from value V
+        // and (interval-scaled) slope D to zero is V A(t) + D B(t), with
+        // A = (1 - t)^2 (1 + 2 t), B = t (1 - t)^2
+        const Quad<Real> k = c.far[tp];  // LJ value, slope; LK value, slope
+        const Real t = (d - c.far_dmin) * c.inv_hf;
+        const Real u = Real(1) - t;
+        const Real uu = u * u;
+        const Real A = uu + Real(2) * t * uu, B = t * uu;
+        e0 += wcp * (k.a * A + k.b * B);
+        e2 += wcp * (k.c * A + k.d * B);
+        if (GRAD) {
+          const Real dA = Real(-6) * t * u, dB = u - Real(3) * t * u;
+          const Real V = wt0 * k.a + wt2 * k.c, D = wt0 * k.b + wt2 * k.d;
+          f = wcp * c.inv_hf * inv_d * (V * dA + D * dB);
+        }
+      } else {
+        Real atr, rep, datr, drep;
+        lj_eval<Real, GRAD>(d, inv_d, c.lj + tp, c.lj + c.ntp * c.ntp + tp, atr, rep, datr, drep);
+        e0 += wcp * atr;
+        e1 += wcp * rep;
+        Real dE = wt0 * datr + wt1 * drep;
+        if (CLS == kNearHeavy) {
+          Real lk, dlk;
+          lk_eval<Real, GRAD>(d, inv_d, c.lk + tp, c.far_dmin, c.far_first, c.inv_hf, lk, dlk);
+          e2 += wcp * lk;
+          dE += wt2 * dlk;
+        }
+        if (GRAD) f = wcp * dE * inv_d;
+      }
+    }
+    if (GRAD) {
+      if (CLS != kFar && d == Real(0)) f = 0;
+      const Real px = f * dx, py = f * dy, pz = f * dz;
+      fx += px;
+      fy += py;
+      fz += pz;
+      add_force(c.g + 4 * (int64_t)w.gidx[j], -px, -py, -pz);
+    }
+  }
+  if (GRAD && row >= 0) add_force(c.g + 4 * (c.row0 + row), fx, fy, fz);
+  if (PAIR) {
+    if (slot >= 0 && c.energies) {
+      Real* o = c.energies + w.out[slot];
+      if (e0 != Real(0)) atomicAdd(o, e0);
+      if (TERM == kTermLJLK) {
+        if (e1 != Real(0)) atomicAdd(o + c.stride, e1);
+        if (CLS != kNear && e2 != Real(0)) atomicAdd(o + 2 * c.stride, e2);
+      }
+    }
+  } else {
+    acc.atr += e0;
+    acc.rep += e1;
+    acc.lk += e2;
+  }
+}
+
+// Screens, queues and evaluates the group's words [0, nw) against rows
+// [0, c1) (this lane's row at (rx, ry, rz)).  counts: pairs in reach, and
+// heavy ones among them.
+template <typename Real, bool GRAD, bool PAIR, int TERM, bool COUNT>
+__device__ __forceinline__ void process_group(const EvalCtx<Real>& c, Slab<Real>& w, int nw, int c1, Real rx,
+                                              Real ry, Real rz, unsigned heavy_rows, int lane, E3<Real>& acc,
+                                              long long* counts) {
+  __syncwarp();
+  const bool hrow = (heavy_rows >> lane) & 1u;
+  int n_far = 0, n_near = 0, n_heavy = 0;
+  for (int k = 0; k < nw; ++k) {
+    const int d = w.desc[k];
+    const int base = d & 255, cnt = (d >> 8) & 63, sp = (d >> 16) - 1;
+    const RowTest t = test_row(w, base, cnt, rx, ry, rz, c.max2, c.far2);
+    unsigned live = lane < c1 ? 0xffffffffu >> (32 - cnt) : 0u;
+    if (sp >= 0) live &= ~w.smask[sp][lane].x;
+    const unsigned in = t.in & live;
+    const unsigned fm = in & ~t.near, nm = in & t.near;
+    w.far[lane * MAXW_PAD + k] = fm;
+    w.near[lane * MAXW_PAD + k] = nm;
+    n_far += __popc(fm);
+    n_near += __popc(nm);
+    if (TERM == kTermLJLK) {
+      const unsigned hw = __ballot_sync(0xffffffffu, lane < cnt && (w.at[base + (lane < cnt ? lane : 0)].tf & kTfHeavy));
+      if (lane == 0) w.heavy[k] = hw;
+      if (hrow) n_heavy += __popc(nm & hw);
+      if (COUNT && hrow) counts[1] += __popc(in & hw);
+    }
+  }
+  __syncwarp();
+  n_far = __reduce_add_sync(0xffffffffu, n_far);
+  n_near = __reduce_add_sync(0xffffffffu, n_near);
+  n_heavy = TERM == kTermLJLK ? __reduce_add_sync(0xffffffffu, n_heavy) : 0;
+  if (COUNT && lane == 0) counts[0] += n_far + n_near;
+  const bool whole = n_far + n_near <= Slab<Real>::QCAP;
+  for (int ka = 0; ka < nw;) {
+    int kb = nw;
+    if (!whole) {
+      kb = ka + 1;
+      const unsigned nm = w.near[lane * MAXW_PAD + ka];
+      n_far = __reduce_add_sync(0xffffffffu, __popc(w.far[lane * MAXW_PAD + ka]));
+      n_near = __reduce_add_sync(0xffffffffu, __popc(nm));
+      n_heavy = TERM == kTermLJLK ? __reduce_add_sync(0xffffffffu, hrow ? __popc(nm & w.heavy[ka]) : 0) : 0;
+    }
+    const int n_light = n_near - n_heavy;
+    // emission: unit u is one (row, word); rows outermost, or words in pair
+    // mode, so that a lane's stretch keeps its row (or energy entry)
+    const int nwr = kb - ka, nu = nwr * c1;
+    const int div = PAIR ? c1 : nwr;
+    const int inv = 65536 / div + 1;  // u / div is exact for u <= 12 * 32
+    int of = 0, ol = n_far, oh = n_far + n_light;
+    for (int u0 = 0; u0 < nu; u0 += 32) {
+      const int u = u0 + lane;
+      unsigned F = 0, L = 0, H = 0, w02 = 0;
+      int eb = 0;
+      if (u < nu) {
+        const int qd = (u * inv) >> 16, rem = u - qd * div;
+        const int r = PAIR ? rem : qd, k = ka + (PAIR ? qd : rem);
+        F = w.far[r * MAXW_PAD + k];
+        L = w.near[r * MAXW_PAD + k];
+        if (TERM == kTermLJLK && ((heavy_rows >> r) & 1u)) {
+          H = L & w.heavy[k];
+          L &= ~H;
+        }
+        const int d = w.desc[k];
+        eb = (r << 8) | (d & 255);
+        const int sp = (d >> 16) - 1;
+        if (sp >= 0) w02 = w.smask[sp][r].y;
+      }
+      const int mine = __popc(F) | (__popc(L) << 16), mine_h = __popc(H);
+      int inc = mine, inc_h = mine_h;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, inc, o);
+        const int th = TERM == kTermLJLK ? __shfl_up_sync(0xffffffffu, inc_h, o) : 0;
+        if (lane >= o) {
+          inc += t;
+          inc_h += th;
+        }
+      }
+      const int tot = __shfl_sync(0xffffffffu, inc, 31);
+      const int tot_h = TERM == kTermLJLK ? __shfl_sync(0xffffffffu, inc_h, 31) : 0;
+      uint16_t* qf = w.queue + of + ((inc - mine) & 0xffff);
+      uint16_t* ql = w.queue + ol + ((inc - mine) >> 16);
+      uint16_t* qh = w.queue + oh + (inc_h - mine_h);
+      for (; F; F &= F - 1) {
+        const int b = __ffs(F) - 1;
+        *qf++ = (uint16_t)(eb + b + (((w02 >> b) & 1u) << 13));
+      }
+      for (; L; L &= L - 1) {
+        const int b = __ffs(L) - 1;
+        *ql++ = (uint16_t)(eb + b + (((w02 >> b) & 1u) << 13));
+      }
+      if (TERM == kTermLJLK)
+        for (; H; H &= H - 1) {
+          const int b = __ffs(H) - 1;
+          *qh++ = (uint16_t)(eb + b + (((w02 >> b) & 1u) << 13));
+        }
+      of += tot & 0xffff;
+      ol += tot >> 16;
+      oh += tot_h;
+    }
+    __syncwarp();
+    eval_class<Real, GRAD, PAIR, TERM, kFar>(c, w, 0, n_far, lane, acc);
+    eval_class<Real, GRAD, PAIR, TERM, kNear>(c, w, n_far, n_light, lane, acc);
+    if (TERM == kTermLJLK)
+      eval_class<Real, GRAD, PAIR, TERM, kNearHeavy>(c, w, n_far + n_light, n_heavy, lane, acc);
+    __syncwarp();
+    ka = kb;
+  }
+}
+
+template <typename Real>
+__device__ __forceinline__ uint32_t load_cpd(const ScoreArgs<Real>& s, int bt, int nconn, int at) {
+  uint32_t v = 0x06060606u;
+  for (int k = 0; k < nconn; ++k) {
+    uint32_t d = s.bt_conn_pd[((int64_t)bt * s.C + k) * s.A + at];
+    v = (v & ~(0xffu << (8 * k))) | (d << (8 * k));
+  }
+  return v;
+}
+
+template <typename Real>
+__device__ __forceinline__ void put_atom(Slab<Real>& w, int j, const AtomRec<Real>& a, int64_t gi) {
+  w.at[j] = a;
+  w.c.x[j] = a.x;
+  w.c.y[j] = a.y;
+  w.c.z[j] = a.z;
+  w.gidx[j] = (int)gi;
+}
+
+// The rows: block type, first connection count, tile start and atoms.
+struct RowSide {
+  int bt, nc, lig, st, c1;
+};
+
+// Stages atoms [at0, at0 + cnt) (cnt <= 32) of a block with exclusions
+// against the rows at side-1 atoms [base, ...) and their masks as mask
+// `sp`: b1 itself (`self`: pairs of later atoms only, weights from the
+// intra-block table) or a count-pair partner (the smallest separation over
+// the connections, ljlk_pose_score.impl.hh:47-67; `seps` its 16 connection
+// separations).  Only partner atoms that lie within four bonds of some atom
+// of b1 are compared row by row.
+template <typename Real>
+__device__ __forceinline__ void stage_special(const ScoreArgs<Real>& s, Slab<Real>& w, const RowSide& r, int base,
+                                              int sp, int bt2, int64_t off2, int at0, int cnt, bool self,
+                                              const uint8_t* seps, int nc2, bool lig, int lane) {
+  const int at = at0 + lane;
+  if (lane < cnt) put_atom(w, base + lane, s.packed[off2 + at], off2 + at);
+  uint2 m = make_uint2(0u, 0u);
+  if (self) {
+    if (lane < r.c1)
+      m = s.imask[((int64_t)bt2 * s.A + r.st + lane) * s.n_iwords + (at0 >> 5)];
+  } else {
+    unsigned bb = 0xffffffffu;  // per connection of b1: the separation from it, a byte each
+    bool rel = false;
+    if (lane < cnt) {
+      const uint32_t cj = load_cpd(s, bt2, nc2, at);
+      for (int u = 0; u < r.nc; ++u) {
+        int best = 63;
+        for (int v = 0; v < nc2; ++v) best = min(best, (int)seps[u * 4 + v] + (int)((cj >> (8 * v)) & 0xff));
+        bb = (bb & ~(0xffu << (8 * u))) | ((unsigned)best << (8 * u));
+        rel |= best <= 4;
+      }
+    }
+    const uint32_t c0 = lane < r.c1 ? load_cpd(s, r.bt, r.nc, r.st + lane) : 0x3f3f3f3fu;
+    for (unsigned rm = __ballot_sync(0xffffffffu, rel); rm; rm &= rm - 1) {
+      const int k = __ffs(rm) - 1;
+      const unsigned bk = __shfl_sync(0xffffffffu, bb, k);
+      int sep = 5;
+      for (int u = 0; u < r.nc; ++u) sep = min(sep, (int)((c0 >> (8 * u)) & 0xff) + (int)((bk >> (8 * u)) & 0xff));
+      if (lig && (sep == 3 || sep == 4)) sep = 5;
+      m.x |= (unsigned)(sep < 4) << k;
+      m.y |= (unsigned)(sep == 4) << k;
+    }
+  }
+  w.smask[sp][lane] = m;
+}
+
+// Keeps, of up to 32 atoms (one per lane), those that can reach b1 (within
+// r1 + max_dis of its centre: the cull is exact) and appends them to side 1
+// at m; returns how many.
+template <typename Real>
+__device__ __forceinline__ int stage_culled(Slab<Real>& w, int m, bool valid, const AtomRec<Real>& a, int64_t gi,
+                                            Real cx, Real cy, Real cz, Real reach2, int slot, int lane) {
+  const Real dx = a.x - cx, dy = a.y - cy, dz = a.z - cz;
+  const bool keep = valid && dx * dx + dy * dy + dz * dz < reach2;
+  const unsigned km = __ballot_sync(0xffffffffu, keep);
+  if (keep) {
+    const int j = m + __popc(km & ((1u << lane) - 1u));
+    put_atom(w, j, a, gi);
+    if (slot >= 0) w.slot[j] = (uint8_t)slot;
+  }
+  return __popc(km);
+}
+
+template <typename Real>
+__device__ __forceinline__ EvalCtx<Real> eval_ctx(const ScoreArgs<Real>& s) {
+  EvalCtx<Real> c;
+  c.lj = s.ljtab;
+  c.lk = s.lktab;
+  c.far = s.fartab;
+  c.elec_k = s.elec_k;
+  c.ntp = s.ntp;
+  c.max2 = s.g.max_dis * s.g.max_dis;
+  c.far2 = s.far_d > Real(0) ? s.far_d * s.far_d : Real(4) * c.max2;
+  c.far_dmin = s.g.max_dis - Real(1.5);
+  c.far_first = c.far_dmin > Real(4.5) ? c.far_dmin : Real(4.5);
+  c.inv_hf = Real(1) / (s.g.max_dis - c.far_dmin);
+  c.wt0 = c.wt1 = c.wt2 = 0;
+  c.g = s.g4;
+  c.row0 = 0;
+  c.energies = nullptr;
+  c.dTdV = nullptr;
+  c.stride = 0;
+  return c;
+}
+
+// The fused kernel.  A work item is (pose p, block b1, candidate range
+// [c0, c1) of later blocks b2 >= b1).  Every warp takes items from a global
+// ticket, tests b1 against each candidate with the bounding-sphere rule of
+// tmol/score/common/sphere_overlap.impl.hh:287-351 (32 per ballot) and
+// scores the hits: b1 itself and its count-pair partners with exclusion
+// masks, the others as one flat list of atoms (every lane loads one, however
+// the blocks' atom counts fall), culled against b1's sphere.  GRAD selects
+// the adjoint (which also yields the energies when s.energies is set);
+// BLOCK_PAIR selects per-block-pair energies / weights instead of per-pose
+// ones: every block then has words of its own.
+template <typename Real, bool GRAD, bool BLOCK_PAIR, int TERM, bool COUNT>
+__global__ void __launch_bounds__(sizeof(Real) == 4 ? 512 : 256, 1)
+    score_kernel(ScoreArgs<Real> s, int items_per_ticket) {
+  if (s.done && *s.done) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  Slab<Real>& w = reinterpret_cast<Slab<Real>*>(smem_raw)[warp];
+  const unsigned lemask = 0xffffffffu >> (31 - lane);
+  const bool want_E = !GRAD || s.energies != nullptr;
+  EvalCtx<Real> ec = eval_ctx(s);
+  if (BLOCK_PAIR) {
+    ec.energies = want_E ? s.energies : nullptr;
+    ec.dTdV = s.dTdV;
+    ec.stride = (int64_t)s.P * s.B * s.B;
+  }
+  const int max_words = BLOCK_PAIR ? min(MAXW, s.max_slots) : MAXW;
+  long long n_bp = 0, n_ap = 0, n_hp = 0, n_in[2] = {0, 0};
+
+  const int n_work = s.ticket[2];
+  for (;;) {
+    int t = 0;
+    if (lane == 0) t = atomicAdd(s.ticket, 1);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    const int it0 = t * items_per_ticket;
+    if (it0 >= n_work) break;
+    const int it1 = min(it0 + items_per_ticket, n_work);
+    for (int item = it0; item < it1; ++item) {
+      // item costs for plan_rebalance: measured by the counting instantiation
+      const long long t_item = COUNT ? clock64() : 0;
+      const int4 wi = s.work[item];
+      const int p = wi.x, b1 = wi.y, cand0 = wi.z, cand1 = wi.w;
+      const int i1 = p * s.B + b1;
+      const int4 bi1 = s.blk_info[i1];
+      if (bi1.x < 0) continue;
+      const int n1 = bi1.z;
+      RowSide r;
+      r.bt = bi1.x;
+      r.nc = bi1.w & 0xff;
+      r.lig = bi1.w >> 8;
+      if (GRAD && !BLOCK_PAIR) {
+        ec.wt0 = s.dTdV[p];
+        if (TERM == kTermLJLK) {
+          ec.wt1 = s.dTdV[s.P + p];
+          ec.wt2 = s.dTdV[2 * s.P + p];
+        }
+      }
+      const Quad<Real> sph1 = reinterpret_cast<const Quad<Real>*>(s.spheres)[i1];
+      const Real reach1 = sph1.d + s.g.max_dis;
+      const Real reach1_2 = reach1 * reach1 * Real(1.0001);
+      // the row's count-pair partners, one per lane
+      const int ncp = s.cp_count[i1];
+      const int cp_b2 = lane < ncp ? s.cp_b2[(int64_t)i1 * CP_CAP + lane] : -1;
+      E3<Real> acc = {0, 0, 0};
+      for (int ti = 0; ti * TILE < n1; ++ti) {
+        r.st = ti * TILE;
+        r.c1 = min(TILE, n1 - r.st);
+        ec.row0 = (int64_t)bi1.y + r.st;
+        AtomRec<Real> ra;
+        ra.x = ra.y = ra.z = Real(0);
+        ra.tf = 0;
+        if (lane < r.c1) ra = s.packed[ec.row0 + lane];
+        w.row[lane] = ra;
+        const unsigned heavy_rows =
+            TERM == kTermLJLK ? __ballot_sync(0xffffffffu, lane < r.c1 && (ra.tf & kTfHeavy)) : 0u;
+        // what is left to stage: candidate batches, the current batch's
+        // blocks with masks (one of them being staged), its other hits
+        int next_c = cand0, batch = cand0;
+        unsigned spec = 0, hits = 0;
+        int sp_n = 0, sp_at = 0, sp_b2 = 0, sp_cp = 0;
+        int4 bi2 = make_int4(-1, 0, 0, 0);
+        int T = 0, k0 = 0, owned = 0, start = 0;  // pose mode: the flat list of the batch's hits
+        bool done = false;
+        while (!done) {
+          int m = 0, top = M1, nw = 0, nsp = 0;
+          for (;;) {
+            if (sp_n > 0) {
+              // the next word of the block being staged with masks
+              const int cnt = min(32, sp_n - sp_at), need = (cnt + 3) & ~3;
+              if (nsp == MAXSP || nw >= max_words || m + need > top) break;
+              const int src = sp_b2 - batch;
+              const int bt2 = __shfl_sync(0xffffffffu, bi2.x, src), off2 = __shfl_sync(0xffffffffu, bi2.y, src);
+              const int cl2 = __shfl_sync(0xffffffffu, bi2.w, src);
+              int base = m;
+              if (BLOCK_PAIR)
+                m += need;
+              else
+                base = top -= need;
+              stage_special(s, w, r, base, nsp, bt2, (int64_t)off2, sp_at, cnt, sp_b2 == b1,
+                            s.cp_seps + ((int64_t)i1 * CP_CAP + sp_cp) * 16, cl2 & 0xff, r.lig && (cl2 >> 8), lane);
+              if (lane == 0) {
+                w.desc[nw] = base | (cnt << 8) | ((nsp + 1) << 16);
+                w.out[nw] = (int64_t)i1 * s.B + sp_b2;
+              }
+              if (BLOCK_PAIR && lane < cnt) w.slot[base + lane] = (uint8_t)nw;
+              ++nsp;
+              ++nw;
+              sp_at += 32;
+              if (sp_at >= sp_n) sp_n = 0;
+            } else if (spec) {
+              const int src = __ffs(spec) - 1;
+              spec &= spec - 1;
+              sp_b2 = batch + src;
+              sp_n = __shfl_sync(0xffffffffu, bi2.z, src);
+              sp_at = sp_b2 == b1 ? r.st : 0;
+              const unsigned pm = __ballot_sync(0xffffffffu, cp_b2 == sp_b2);
+              sp_cp = pm ? __ffs(pm) - 1 : 0;
+              if (sp_at >= sp_n) sp_n = 0;
+            } else if (!BLOCK_PAIR && k0 < T) {
+              // 32 atoms of the flat list: bit b of `word` set where a hit's
+              // atoms begin at list position k0 + b
+              if (m + 32 > top || nw + (m + 63) / 32 > MAXW) break;
+              const unsigned pos = (unsigned)(start - k0);
+              const unsigned word = __reduce_or_sync(0xffffffffu, pos < 32u ? 1u << pos : 0u);
+              const int own = owned + __popc(word & lemask) - 1;
+              owned += __popc(word);
+              const int f = k0 + lane;
+              const bool valid = f < T;
+              const int64_t gi = (int64_t)w.hoff[own] + f;
+              AtomRec<Real> a;
+              a.x = a.y = a.z = Real(0);
+              a.tf = 0;
+              if (valid) a = s.packed[gi];
+              m += stage_culled(w, m, valid, a, gi, sph1.a, sph1.b, sph1.c, reach1_2, -1, lane);
+              k0 += 32;
+            } else if (BLOCK_PAIR && hits) {
+              // 32 atoms of the next hit: a word of their own
+              if (m + 32 > top || nw >= max_words) break;
+              const int src = __ffs(hits) - 1;
+              const int off2 = __shfl_sync(0xffffffffu, bi2.y, src), n2 = __shfl_sync(0xffffffffu, bi2.z, src);
+              const bool valid = k0 + lane < n2;
+              const int64_t gi = (int64_t)off2 + k0 + lane;
+              AtomRec<Real> a;
+              a.x = a.y = a.z = Real(0);
+              a.tf = 0;
+              if (valid) a = s.packed[gi];
+              const int kept = stage_culled(w, m, valid, a, gi, sph1.a, sph1.b, sph1.c, reach1_2, nw, lane);
+              if (kept > 0) {
+                if (lane == 0) {
+                  w.desc[nw] = m | (kept << 8);
+                  w.out[nw] = (int64_t)i1 * s.B + batch + src;
+                }
+                m += (kept + 3) & ~3;
+                ++nw;
+              }
+              k0 += 32;
+              if (k0 >= n2) {
+                k0 = 0;
+                hits &= hits - 1;
+              }
+            } else if (next_c < cand1) {
+              // the next 32 candidates
+              batch = next_c;
+              next_c += 32;
+              const int b2 = batch + lane;
+              bool hit = false;
+              bi2 = make_int4(-1, 0, 0, 0);
+              if (b2 < cand1) {
+                const int i2 = p * s.B + b2;
+                bi2 = s.blk_info[i2];
+                if (bi2.x >= 0) {
+                  const Quad<Real> s2 = reinterpret_cast<const Quad<Real>*>(s.spheres)[i2];
+                  const Real dx = sub_rn(sph1.a, s2.a), dy = sub_rn(sph1.b, s2.b), dz = sub_rn(sph1.c, s2.c);
+                  const Real d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
+                  const Real thr = add_rn(add_rn(sph1.d, s2.d), s.reach);
+                  hit = d2 < mul_rn(thr, thr);
+                }
+                if (s.nbr) s.nbr[(int64_t)i1 * s.B + b2] = hit ? 1 : 0;
+              }
+              bool masked = b2 == b1;
+              for (int k = 0; k < ncp; ++k) masked |= __shfl_sync(0xffffffffu, cp_b2, k) == b2;
+              // a screened-out pair is dropped unless it is b1 itself or one
+              // of its count-pair partners (bond separation <= 4)
+              if (s.skip && hit && !masked &&
+                  ((s.skip[(int64_t)i1 * s.skip_words + (b2 >> 5)] >> (b2 & 31)) & 1u))
+                hit = false;
+              if (COUNT && ti == 0 && hit) {
+                const long long n2 = bi2.z;
+                n_bp += 1;
+                n_ap += b2 == b1 ? n2 * (n2 - 1) / 2 : (long long)n1 * n2;
+                if (TERM == kTermLJLK) {
+                  const long long h1 = s.bt_n_heavy[r.bt], h2 = s.bt_n_heavy[bi2.x];
+                  n_hp += b2 == b1 ? h2 * (h2 - 1) / 2 : h1 * h2;
+                }
+              }
+              spec = __ballot_sync(0xffffffffu, hit && masked);
+              hits = __ballot_sync(0xffffffffu, hit && !masked);
+              if (!BLOCK_PAIR) {
+                // where each hit's atoms begin in the flat list
+                const int n = hit && !masked ? bi2.z : 0;
+                int inc = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                  const int v = __shfl_up_sync(0xffffffffu, inc, o);
+                  if (lane >= o) inc += v;
+                }
+                T = __shfl_sync(0xffffffffu, inc, 31);
+                start = n > 0 ? inc - n : 0x7fffffff;
+                __syncwarp();
+                const unsigned hm = __ballot_sync(0xffffffffu, n > 0);
+                if (n > 0) w.hoff[__popc(hm & (lemask >> 1))] = bi2.y - start;
+                __syncwarp();
+                owned = 0;
+              }
+              k0 = 0;
+            } else {
+              done = true;
+              break;
+            }
+          }
+          if (!BLOCK_PAIR) {
+            // the flat list's words
+            const int nf = (m + 31) >> 5;
+            if (lane < nf) w.desc[nw + lane] = 32 * lane | (min(32, m - 32 * lane) << 8);
+            nw += nf;
+          }
+          if (nw > 0)
+            process_group<Real, GRAD, BLOCK_PAIR, TERM, COUNT>(ec, w, nw, r.c1, ra.x, ra.y, ra.z, heavy_rows, lane,
+                                                               acc, n_in);
+        }
+        __syncwarp();
+      }
+      if (!BLOCK_PAIR && want_E) {
+        const Real v0 = warp_sum(acc.atr);
+        const Real v1 = TERM == kTermLJLK ? warp_sum(acc.rep) : Real(0);
+        const Real v2 = TERM == kTermLJLK ? warp_sum(acc.lk) : Real(0);
+        if (lane == 0) {
+          if (v0 != Real(0)) atomicAdd(&s.energies[p], v0);
+          if (v1 != Real(0)) atomicAdd(&s.energies[s.P + p], v1);
+          if (v2 != Real(0)) atomicAdd(&s.energies[2 * s.P + p], v2);
+        }
+      }
+      if (COUNT && s.item_cost && lane == 0)
+        s.item_cost[item] = (int)min((clock64() - t_item) >> 4, (long long)0x7fffffff);
+    }
+  }
+  if (COUNT && s.counts) {
+    const long long v[N_COUNTS] = {warp_sum(n_bp), warp_sum(n_ap), warp_sum(n_hp), warp_sum(n_in[0]), warp_sum(n_in[1])};
+    if (lane == 0)
+      for (int k = 0; k < N_COUNTS; ++k)
+        if (v[k]) atomicAdd(&s.counts[k], (unsigned long long)v[k]);
+  }
+}
