@@ -87,16 +87,17 @@ typedef struct {
 /* Launch shape of the scoring kernel; zeros select the built-in defaults.
  * A work item is (pose, block b1, a range of later blocks b2 >= b1).
  *   rows_per_item        work items a warp takes per atomic ticket
- *   warps_per_cta        warps per CTA (at most 16; 8 for float64 plans and
- *                        the rotamer and LK-ball kernels); every warp works
- *                        alone
+ *   warps_per_cta        warps per CTA (at most 20; 8 for float64 plans and
+ *                        the LK-ball kernels); every warp works alone, and a
+ *                        call with little work runs fewer per CTA on more SMs
  *   ctas_per_sm          resident CTAs per SM of the persistent grid
- *                        (defaults: 16 x 1 for float pose plans of LJ/LK
- *                        and elec, else 8 x 2)
- *   candidates_per_item  candidate blocks b2 per work item (at most 1024)
- *   slots_per_group      neighbouring blocks whose atoms share one pass of
- *                        the warp's 32 lanes (1-12, default 12): how many
- *                        block pairs a warp screens at once */
+ *                        (defaults: 20 x 1 for float plans of LJ/LK and elec,
+ *                        else 8 x 2)
+ *   candidates_per_item  candidate blocks b2 per work item (at most 1024;
+ *                        default 4-256, longer with more work)
+ *   slots_per_group      block (or rotamer) pairs whose energies are kept
+ *                        apart that a warp screens at once (1-9, default 9;
+ *                        whole-pose calls have no such limit) */
 typedef struct {
   int32_t rows_per_item;
   int32_t warps_per_cta;

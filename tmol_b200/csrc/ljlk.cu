@@ -52,7 +52,6 @@ constexpr int MAX_CONN = 4;
 constexpr int N_COUNTS = 5;
 constexpr int CP_CAP = 16;
 constexpr int MAX_ROWS_PER_ITEM = 64;
-constexpr int MAX_WARPS = 16;
 
 // The energy term a plan scores: LJ + LK (fa_ljatr, fa_ljrep, fa_lk) or
 // elec (fa_elec).  Both share the neighbour detection, count-pair tables,
@@ -178,15 +177,17 @@ __global__ void plan_blocks_kernel(PlanBuildArgs a) {
 // must be in range and the rotamer must lie in its block's range.
 // One record per block slot for the scoring kernel's row and neighbour
 // loads: {block type or -1, first atom, atom count, connections | ligand
-// flag << 8}, from the validated block tables.
+// flag << 8}, from the validated block tables; counts are held to the tables'
+// sizes (a block type beyond them fails the plan, but only after the plan's
+// other kernels have read these records).
 __global__ void plan_block_info_kernel(int64_t n, const int* blk_bt, const int* blk_off, const int* bt_n_atoms,
-                                       const int* bt_n_conn, const int* bt_is_ligand, int4* out) {
+                                       const int* bt_n_conn, const int* bt_is_ligand, int A, int C, int4* out) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int bt = blk_bt[i];
     int4 r = make_int4(bt, blk_off[i], 0, 0);
     if (bt >= 0) {
-      r.z = bt_n_atoms[bt];
-      r.w = (bt_n_conn[bt] & 0xff) | ((bt_is_ligand[bt] ? 1 : 0) << 8);
+      r.z = min(max(bt_n_atoms[bt], 0), A);
+      r.w = min(max(bt_n_conn[bt], 0), C) | ((bt_is_ligand[bt] ? 1 : 0) << 8);
     }
     out[i] = r;
   }
@@ -282,7 +283,7 @@ __global__ void plan_intra_masks_kernel(const uint8_t* bt_pd, const int* bt_n_at
        i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t row = i / n_words;
     const int word = (int)(i - row * n_words), bt = (int)(row / A), at = (int)(row - (int64_t)bt * A);
-    const int n = bt_n_atoms[bt];
+    const int n = min(bt_n_atoms[bt], A);
     uint2 m = make_uint2(0xffffffffu, 0u);
     for (int k = 0; k < 32; ++k) {
       const int j = 32 * word + k;
@@ -300,7 +301,7 @@ __global__ void plan_intra_masks_kernel(const uint8_t* bt_pd, const int* bt_n_at
 __global__ void plan_heavy_count_kernel(const uint16_t* bt_tf, const int* bt_n_atoms, int nbt, int A, int* out) {
   for (int bt = blockIdx.x * blockDim.x + threadIdx.x; bt < nbt; bt += gridDim.x * blockDim.x) {
     int n = 0;
-    for (int k = 0; k < bt_n_atoms[bt]; ++k) n += bt_tf[(int64_t)bt * A + k] >> 8;
+    for (int k = 0; k < min(bt_n_atoms[bt], A); ++k) n += bt_tf[(int64_t)bt * A + k] >> 8;
     out[bt] = n;
   }
 }
@@ -310,6 +311,22 @@ __global__ void plan_real_atoms_kernel(const int* bt_of, const int* off_of, int 
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     if (bt_of[i] < 0) continue;
     for (int k = 0; k < bt_n_atoms[bt_of[i]]; ++k) real[(int64_t)off_of[i] + k] = 1;
+  }
+}
+
+// Where each count-pair partner's masks begin (one per atom of the block and
+// word of the partner) and, in *total, how many there are.
+__global__ void plan_mask_offsets_kernel(const int4* blk_info, const int* cp_count, const int* cp_b2, int64_t n_rows,
+                                         int B, unsigned long long* total, uint32_t* moff) {
+  for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < n_rows;
+       row += (int64_t)gridDim.x * blockDim.x) {
+    const int4 b1 = blk_info[row];
+    if (b1.x < 0) continue;
+    for (int e = 0; e < cp_count[row]; ++e) {
+      const int4 b2 = blk_info[row - row % B + cp_b2[row * CP_CAP + e]];
+      moff[row * CP_CAP + e] =
+          (uint32_t)atomicAdd(total, (unsigned long long)b1.z * (unsigned long long)((b2.z + 31) / 32));
+    }
   }
 }
 
@@ -524,6 +541,10 @@ struct ScoreArgs {
   // excluded within the block and which have weight 0.2
   const uint2* imask;
   int n_iwords;
+  // pose plans: the same between each block and its count-pair partners,
+  // [word of the partner][atom of the block] from cp_moff[row * CP_CAP + e]
+  const uint2* pmask;
+  const uint32_t* cp_moff;
   const int* bt_n_heavy;  // heavy atoms per block type (work counters)
   // LJ/LK and elec: the gradient as [n_atoms][4], zeroed by the sphere pass
   // and copied out by grad_out_kernel
@@ -873,7 +894,7 @@ __global__ void rot_row_fill_kernel(ScoreArgs<Real> s, RotArgs ra) {
 // Energies go to the item's pairs (energies[t * n_pairs + d]), the adjoint
 // weights come from dTdV[t * n_pairs + d].
 template <typename Real, bool GRAD, int TERM, bool COUNT>
-__global__ void __launch_bounds__(sizeof(Real) == 4 ? 512 : 256, 1)
+__global__ void __launch_bounds__(sizeof(Real) == 4 ? 32 * PAIR_WARPS : 256, 1)
     rotamer_kernel(ScoreArgs<Real> s, RotArgs ra, const Real* rs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -939,8 +960,13 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 512 : 256, 1)
             int used = cnt;
             if (cnt > 0 && masked) {
               const int bt = __shfl_sync(0xffffffffu, bt2, src);
-              stage_special(s, w, r, m, nsp, bt, (int64_t)off, at, cnt, diag, seps, diag ? 0 : s.bt_n_conn[bt],
-                            !diag && r.lig && s.bt_is_ligand[bt], lane);
+              uint2 mk = make_uint2(0u, 0u);
+              if (!diag)
+                mk = partner_masks(s, r.bt, r.nc, r.st, r.c1, bt, s.bt_n_conn[bt], at, cnt, seps,
+                                   r.lig && s.bt_is_ligand[bt], lane);
+              else if (lane < r.c1)
+                mk = s.imask[((int64_t)bt * s.A + r.st + lane) * s.n_iwords + (at >> 5)];
+              stage_masked(s, w, m, nsp, (int64_t)off, at, cnt, mk, lane);
               if (lane < cnt) w.slot[m + lane] = (uint8_t)nw;
               ++nsp;
             } else if (cnt > 0) {
@@ -1210,6 +1236,8 @@ struct tmol_b200_ljlk_plan {
   uint8_t* real_atom = nullptr;  // [n_atoms] 1 where a block (or rotamer) has the atom
   uint2* imask = nullptr;        // [nbt * A][n_iwords] pairs within a block type
   int n_iwords = 0;
+  uint2* pmask = nullptr;        // pose plans: pairs with count-pair partners
+  uint32_t* cp_moff = nullptr;   // [P*B*CP_CAP] where each partner's masks begin
   int* bt_n_heavy = nullptr;
   void* fartab = nullptr;
   double far_d = 0;  // where far pairs start, 0: none
@@ -1312,7 +1340,7 @@ void free_plan(tmol_b200_ljlk_plan* pl) {
                   pl->lkb_npol,  pl->lkb_occ,     pl->lkb_nocc,    pl->lkb_par,
                   pl->lkb_waters, pl->lkb_dwaters, pl->lkb_nbocc, pl->lkb_active,
                   pl->blk_info,  pl->packed,      pl->g4,          pl->real_atom,  pl->imask,
-                  pl->bt_n_heavy, pl->fartab,      pl->spec_next,   pl->spec_used, pl->spec_g,
+                  pl->pmask,     pl->cp_moff,     pl->bt_n_heavy, pl->fartab,      pl->spec_next,   pl->spec_used, pl->spec_g,
                   pl->spec_dw,   pl->spec_flag};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -1320,21 +1348,36 @@ void free_plan(tmol_b200_ljlk_plan* pl) {
   delete pl;
 }
 
-void default_launch(tmol_b200_ljlk_launch& l) {
+// Candidate blocks per work item where the caller does not choose.  An item
+// costs its set-up, partly filled words and queue steps, so ranges are long
+// (up to 256: the uneven batch of 256 poses takes 996 us at 256, 1144 us at
+// 64); but every warp should get an item or two, so small calls are cut finer
+// (one pose of 100 residues: 50 us at 8, 99 us at 64).
+int auto_candidates(const tmol_b200_ljlk_plan* pl) {
+  if (pl->term == kTermLKBall) return 64;
+  const int64_t warps = (int64_t)pl->n_sm * pl->launch.ctas_per_sm * pl->launch.warps_per_cta;
+  int64_t pairs = 0;
+  for (int64_t nb : pl->host_pose_last) pairs += nb * (nb + 1) / 2;
+  int c = 4;
+  while (c < 256 && 2 * c * warps <= pairs) c *= 2;
+  return c;
+}
+
+void default_launch(const tmol_b200_ljlk_plan* pl, tmol_b200_ljlk_launch& l) {
   if (l.rows_per_item <= 0) l.rows_per_item = 1;
   if (l.warps_per_cta <= 0) l.warps_per_cta = 8;
   if (l.ctas_per_sm <= 0) l.ctas_per_sm = 2;
-  if (l.candidates_per_item <= 0) l.candidates_per_item = 64;
+  if (l.candidates_per_item <= 0) l.candidates_per_item = auto_candidates(pl);
   if (l.slots_per_group <= 0) l.slots_per_group = MAXW;
   l.slots_per_group = std::min(l.slots_per_group, MAXW);
   l.rows_per_item = std::min(l.rows_per_item, MAX_ROWS_PER_ITEM);
-  l.warps_per_cta = std::min(l.warps_per_cta, MAX_WARPS);
+  l.warps_per_cta = std::min(l.warps_per_cta, PAIR_WARPS);
   l.candidates_per_item = std::min(l.candidates_per_item, 32 * 32);
 }
 
 template <typename Real, int TERM>
 cudaError_t set_smem_limits_term() {
-  const int smem = (int)std::min<size_t>(MAX_WARPS * sizeof(Slab<Real>), 227 * 1024);
+  const int smem = (int)std::min<size_t>(PAIR_WARPS * sizeof(Slab<Real>), 227 * 1024);
   const void* kernels[] = {
       (const void*)score_kernel<Real, false, false, TERM, false>,
       (const void*)score_kernel<Real, false, true, TERM, false>,
@@ -1406,6 +1449,8 @@ ScoreArgs<Real> score_args(tmol_b200_ljlk_plan* pl, const void* coords) {
   s.far_d = (Real)pl->far_d;
   s.imask = pl->imask;
   s.n_iwords = pl->n_iwords;
+  s.pmask = pl->pmask;
+  s.cp_moff = pl->cp_moff;
   s.bt_n_heavy = pl->bt_n_heavy;
   s.g4 = (Real*)pl->g4;
   s.ntp = pl->ntp;
@@ -1480,7 +1525,7 @@ int launch_score(tmol_b200_ljlk_plan* pl, ScoreArgs<Real> s, cudaStream_t st) {
   if (pl->n_work == 0) return TMOL_B200_OK;
   const int R = pl->launch.rows_per_item;
   // the float64 kernel: at most 256 threads
-  const GridShape gs = grid_shape(pl, (pl->n_work + R - 1) / R, sizeof(Real) == 8 ? 8 : MAX_WARPS);
+  const GridShape gs = grid_shape(pl, (pl->n_work + R - 1) / R, sizeof(Real) == 8 ? 8 : PAIR_WARPS);
   size_t smem = gs.warps * sizeof(Slab<Real>);
   // the work counters cost registers and instructions in the item loop:
   // they are compiled into a separate instantiation, used on request
@@ -1717,7 +1762,7 @@ int rotamer_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const int32_
   }
   CK(cudaMemsetAsync(pl->counters, 0, sizeof(int), st));
   // the float64 kernel: at most 256 threads
-  const GridShape gs = grid_shape(pl, n_items, sizeof(Real) == 8 ? 8 : MAX_WARPS);
+  const GridShape gs = grid_shape(pl, n_items, sizeof(Real) == 8 ? 8 : PAIR_WARPS);
   const size_t smem = gs.warps * sizeof(Slab<Real>);
   auto kern = pl->term == kTermElec
                   ? (pl->counting ? rotamer_kernel<Real, GRAD, kTermElec, true> : rotamer_kernel<Real, GRAD, kTermElec, false>)
@@ -2199,14 +2244,15 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   pl->N = in->n_atoms;
   pl->reach = in->max_dis;
   pl->launch = launch ? *launch : tmol_b200_ljlk_launch{0, 0, 0, 0};
-  // float plans of LJ/LK and elec: one CTA of 16 warps per SM unless the
-  // caller chose
+  // float plans of LJ/LK and elec: one CTA of PAIR_WARPS warps per SM unless
+  // the caller chose
   if (real_bytes == 4 && term != kTermLKBall && pl->launch.warps_per_cta <= 0 &&
       pl->launch.ctas_per_sm <= 0) {
-    pl->launch.warps_per_cta = 16;
+    pl->launch.warps_per_cta = PAIR_WARPS;
     pl->launch.ctas_per_sm = 1;
   }
-  default_launch(pl->launch);
+  const bool chose_candidates = pl->launch.candidates_per_item > 0;
+  default_launch(pl, pl->launch);
   int dev = 0;
   int rc = TMOL_B200_OK;
 #define PCK(x)                         \
@@ -2331,7 +2377,7 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     PCK(cudaGetLastError());
     if (pl->blk_info) {
       plan_block_info_kernel<<<g, 256, 0, st>>>(PB, pl->blk_bt, pl->blk_off, pl->bt_n_atoms, pl->bt_n_conn,
-                                                pl->bt_is_ligand, pl->blk_info);
+                                                pl->bt_is_ligand, A, C, pl->blk_info);
       PCK(cudaGetLastError());
     }
   }
@@ -2350,6 +2396,14 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     int gc = std::max(1, std::min<int>((int)((PB * 32 + 255) / 256), pl->n_sm * 16));
     plan_count_pair_kernel<<<gc, 256, 0, st>>>(a);
     PCK(cudaGetLastError());
+  }
+  unsigned long long n_masks = 0;
+  if (pl->blk_info && PB > 0) {
+    PCK(dalloc(pl, &pl->cp_moff, PB * CP_CAP));
+    PCK(cudaMemsetAsync(pl->counts, 0, sizeof(unsigned long long), st));
+    plan_mask_offsets_kernel<<<g, 256, 0, st>>>(pl->blk_info, pl->cp_count, pl->cp_b2, PB, B, pl->counts, pl->cp_moff);
+    PCK(cudaGetLastError());
+    PCK(cudaMemcpyAsync(&n_masks, pl->counts, sizeof(n_masks), cudaMemcpyDeviceToHost, st));
   }
   int status_bits = 0;
   pl->host_pose_last.assign(std::max(P, 1), 0);
@@ -2426,6 +2480,19 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
       const int gi = (int)std::max<int64_t>(1, std::min<int64_t>((n_im + 255) / 256, (int64_t)pl->n_sm * 8));
       plan_intra_masks_kernel<<<gi, 256, 0, st>>>(pl->bt_pd, pl->bt_n_atoms, nbt, A, pl->n_iwords, pl->imask);
       PCK(cudaGetLastError());
+      if (n_masks >= (1ull << 32)) {  // 32 GB of masks
+        free_plan(pl);
+        return TMOL_B200_ERR_CAPACITY;
+      }
+      if (n_masks > 0) {
+        PCK(dalloc(pl, &pl->pmask, n_masks));
+        const int gm = std::max(1, std::min<int>((int)((PB + 7) / 8), pl->n_sm * 16));
+        if (real_bytes == 4)
+          plan_partner_masks_kernel<float><<<gm, 256, 0, st>>>(score_args<float>(pl, nullptr), pl->pmask);
+        else
+          plan_partner_masks_kernel<double><<<gm, 256, 0, st>>>(score_args<double>(pl, nullptr), pl->pmask);
+        PCK(cudaGetLastError());
+      }
       plan_heavy_count_kernel<<<(nbt + 127) / 128, 128, 0, st>>>(pl->bt_tf, pl->bt_n_atoms, nbt, A, pl->bt_n_heavy);
       PCK(cudaGetLastError());
     }
@@ -2497,6 +2564,7 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
       v[i] = real_bytes == 4 ? ((const float*)pl->elec_k_host)[i] : ((const double*)pl->elec_k_host)[i];
     pl->far_d = k.hi_start >= k.lo_end && k.hi_start > 0 ? k.hi_start : 0;
   }
+  if (!chose_candidates) pl->launch.candidates_per_item = auto_candidates(pl);
   rc = (rotamers || !scoring) ? TMOL_B200_OK : build_work(pl, st);
   if (rc != TMOL_B200_OK) {
     free_plan(pl);
@@ -2748,7 +2816,7 @@ int tmol_b200_ljlk_plan_set_launch(tmol_b200_ljlk_plan* plan,
   if (!plan || !launch) return TMOL_B200_ERR_INVALID_ARGUMENT;
   int old_cpi = plan->launch.candidates_per_item;
   plan->launch = *launch;
-  default_launch(plan->launch);
+  default_launch(plan, plan->launch);
   if (plan->launch.candidates_per_item != old_cpi) return build_work(plan, 0);
   return TMOL_B200_OK;
 }

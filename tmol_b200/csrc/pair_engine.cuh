@@ -19,17 +19,27 @@
 //      energies stay in registers), and the side-1 forces go out as one
 //      16-byte vector reduction per pair into a padded gradient buffer.
 //
-// What bounds it: instruction issue.  Shared-memory float atomics are
-// compare-and-swap loops here (three per pair and side measured 13-33
-// cycles of an SM and about 25 issue slots); one red.global.add.v4.f32 is a
-// single instruction and 44 cycles of an SM's path to L2, off the critical
-// path, which is why forces leave the SM at once instead of being summed in
-// shared memory.
+// What bounds it: latency, at 20 warps per SM (about half of the issue slots
+// are used; DRAM and FP32 pipes stay below a fifth).  So the loads an item
+// starts from go out together, a whole list of neighbouring atoms is in flight
+// at once (cp.async into side 1, culled in place), and forces leave the SM
+// without being waited for: shared-memory float atomics are compare-and-swap
+// loops here (three per pair and side measured 13-33 cycles of an SM and
+// about 25 issue slots); one red.global.add.v4.f32 is a single instruction
+// and 44 cycles of an SM's path to L2.  64 x 150 residues, energy + gradient
+// with the sphere pass and the gradient's copy, L2 flushed: 320 us with the
+// shared-memory accumulators and per-block staging this replaces, 157 us with
+// the three phases, 130 us with the loads in flight and 20 warps.
 
-constexpr int M1 = 224;       // side-1 atoms of a group (< 256: 8-bit index)
-constexpr int MAXW = 12;      // words of a group
-constexpr int MAXW_PAD = 13;  // odd row stride of the mask arrays: no bank conflicts
-constexpr int MAXSP = 4;      // words with exclusion masks
+constexpr int M1 = 160;  // side-1 atoms of a group (< 256: 8-bit index)
+constexpr int MAXW = 9;  // words of a group; odd: the mask arrays' row stride has no bank conflicts
+constexpr int MAXSP = 4; // words with exclusion masks
+// Warps per CTA and SM.  The engine waits on memory more than it issues, so
+// warps count for more than registers or a longer side 1: 64 x 150 residues,
+// energy + gradient, 16 warps of 128 registers and M1 = 224 take 144 us, 16
+// and M1 = 160 142 us, 20 warps of 96 registers (two spilled words) and
+// M1 = 160 130 us.
+constexpr int PAIR_WARPS = 20;
 constexpr int kTfHeavy = 256;
 
 // One atom: coordinates and either the compact atom type | heavy << 8
@@ -49,8 +59,7 @@ struct alignas(16) AtomRec {
 // fits; a group with more pairs than the queue holds goes word by word.
 template <typename Real>
 struct Slab {
-  static constexpr int QCAP = 3 * M1 * sizeof(Real) / 2;
-  static_assert(QCAP >= 1024, "the queue holds any single word");
+  static constexpr int QCAP = 3 * M1 * sizeof(Real) / 2 < 1024 ? 1024 : 3 * M1 * sizeof(Real) / 2;
   AtomRec<Real> at[M1];
   int gidx[M1];  // global atom index
   union {
@@ -59,7 +68,7 @@ struct Slab {
     } c;
     uint16_t queue[QCAP];
   };
-  uint32_t far[32 * MAXW_PAD], near[32 * MAXW_PAD];  // [row][word]
+  uint32_t far[32 * MAXW], near[32 * MAXW];  // [row][word]
   uint2 smask[MAXSP][32];                            // per row: excluded, weight 0.2
   AtomRec<Real> row[32];
   long long out[MAXW];  // pair mode: the word's energy entry
@@ -107,6 +116,16 @@ __device__ __forceinline__ void add_force(double* g, double x, double y, double 
   atomicAdd(g + 1, y);
   atomicAdd(g + 2, z);
 }
+
+// One atom record from global to shared memory, without a register.
+template <typename Real>
+__device__ __forceinline__ void copy_async(AtomRec<Real>* dst, const AtomRec<Real>* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+#pragma unroll
+  for (int k = 0; k < (int)sizeof(AtomRec<Real>); k += 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + k), "l"((const char*)src + k) : "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Packed pairs of float32 operations.
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {
@@ -334,8 +353,8 @@ __device__ __forceinline__ void process_group(const EvalCtx<Real>& c, Slab<Real>
     if (sp >= 0) live &= ~w.smask[sp][lane].x;
     const unsigned in = t.in & live;
     const unsigned fm = in & ~t.near, nm = in & t.near;
-    w.far[lane * MAXW_PAD + k] = fm;
-    w.near[lane * MAXW_PAD + k] = nm;
+    w.far[lane * MAXW + k] = fm;
+    w.near[lane * MAXW + k] = nm;
     n_far += __popc(fm);
     n_near += __popc(nm);
     if (TERM == kTermLJLK) {
@@ -355,8 +374,8 @@ __device__ __forceinline__ void process_group(const EvalCtx<Real>& c, Slab<Real>
     int kb = nw;
     if (!whole) {
       kb = ka + 1;
-      const unsigned nm = w.near[lane * MAXW_PAD + ka];
-      n_far = __reduce_add_sync(0xffffffffu, __popc(w.far[lane * MAXW_PAD + ka]));
+      const unsigned nm = w.near[lane * MAXW + ka];
+      n_far = __reduce_add_sync(0xffffffffu, __popc(w.far[lane * MAXW + ka]));
       n_near = __reduce_add_sync(0xffffffffu, __popc(nm));
       n_heavy = TERM == kTermLJLK ? __reduce_add_sync(0xffffffffu, hrow ? __popc(nm & w.heavy[ka]) : 0) : 0;
     }
@@ -365,7 +384,7 @@ __device__ __forceinline__ void process_group(const EvalCtx<Real>& c, Slab<Real>
     // mode, so that a lane's stretch keeps its row (or energy entry)
     const int nwr = kb - ka, nu = nwr * c1;
     const int div = PAIR ? c1 : nwr;
-    const int inv = 65536 / div + 1;  // u / div is exact for u <= 12 * 32
+    const int inv = 65536 / div + 1;  // u / div is exact for u <= 9 * 32
     int of = 0, ol = n_far, oh = n_far + n_light;
     for (int u0 = 0; u0 < nu; u0 += 32) {
       const int u = u0 + lane;
@@ -374,8 +393,8 @@ __device__ __forceinline__ void process_group(const EvalCtx<Real>& c, Slab<Real>
       if (u < nu) {
         const int qd = (u * inv) >> 16, rem = u - qd * div;
         const int r = PAIR ? rem : qd, k = ka + (PAIR ? qd : rem);
-        F = w.far[r * MAXW_PAD + k];
-        L = w.near[r * MAXW_PAD + k];
+        F = w.far[r * MAXW + k];
+        L = w.near[r * MAXW + k];
         if (TERM == kTermLJLK && ((heavy_rows >> r) & 1u)) {
           H = L & w.heavy[k];
           L &= ~H;
@@ -447,52 +466,80 @@ __device__ __forceinline__ void put_atom(Slab<Real>& w, int j, const AtomRec<Rea
   w.gidx[j] = (int)gi;
 }
 
-// The rows: block type, first connection count, tile start and atoms.
+// Exclusions between a tile of rows (atoms [st, st + c1) of block type bt1,
+// one per lane) and atoms [at0, at0 + cnt) of a count-pair partner of type
+// bt2: bit k of x set where the smallest separation over the connections
+// (ljlk_pose_score.impl.hh:47-67; seps[u * 4 + v]) is below four bonds, of y
+// where it is four.  Only partner atoms within four bonds of some connection
+// of b1 are compared row by row.
+template <typename Real>
+__device__ __forceinline__ uint2 partner_masks(const ScoreArgs<Real>& s, int bt1, int nc1, int st, int c1, int bt2,
+                                               int nc2, int at0, int cnt, const uint8_t* seps, bool lig, int lane) {
+  uint2 m = make_uint2(0u, 0u);
+  unsigned bb = 0xffffffffu;  // per connection of b1: the separation from it, a byte each
+  bool rel = false;
+  if (lane < cnt) {
+    const uint32_t cj = load_cpd(s, bt2, nc2, at0 + lane);
+    for (int u = 0; u < nc1; ++u) {
+      int best = 63;
+      for (int v = 0; v < nc2; ++v) best = min(best, (int)seps[u * 4 + v] + (int)((cj >> (8 * v)) & 0xff));
+      bb = (bb & ~(0xffu << (8 * u))) | ((unsigned)best << (8 * u));
+      rel |= best <= 4;
+    }
+  }
+  const uint32_t c0 = lane < c1 ? load_cpd(s, bt1, nc1, st + lane) : 0x3f3f3f3fu;
+  for (unsigned rm = __ballot_sync(0xffffffffu, rel); rm; rm &= rm - 1) {
+    const int k = __ffs(rm) - 1;
+    const unsigned bk = __shfl_sync(0xffffffffu, bb, k);
+    int sep = 5;
+    for (int u = 0; u < nc1; ++u) sep = min(sep, (int)((c0 >> (8 * u)) & 0xff) + (int)((bk >> (8 * u)) & 0xff));
+    if (lig && (sep == 3 || sep == 4)) sep = 5;
+    m.x |= (unsigned)(sep < 4) << k;
+    m.y |= (unsigned)(sep == 4) << k;
+  }
+  return m;
+}
+
+// Plan time: the masks of every (block, count-pair partner), one warp each,
+// as [word of the partner][atom of the block] from cp_moff on.
+template <typename Real>
+__global__ void plan_partner_masks_kernel(ScoreArgs<Real> s, uint2* out) {
+  const int lane = threadIdx.x & 31;
+  const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; row < (int64_t)s.P * s.B;
+       row += n_warps) {
+    const int4 b1 = s.blk_info[row];
+    if (b1.x < 0) continue;
+    const int64_t pose0 = row - row % s.B;
+    for (int e = 0; e < s.cp_count[row]; ++e) {
+      const int64_t k = row * CP_CAP + e;
+      const int4 b2 = s.blk_info[pose0 + s.cp_b2[k]];
+      const bool lig = (b1.w >> 8) && (b2.w >> 8);
+      for (int at0 = 0; at0 < b2.z; at0 += 32)
+        for (int st = 0; st < b1.z; st += TILE) {
+          const int c1 = min(TILE, b1.z - st);
+          const uint2 m = partner_masks(s, b1.x, b1.w & 0xff, st, c1, b2.x, b2.w & 0xff, at0, min(32, b2.z - at0),
+                                        s.cp_seps + k * 16, lig, lane);
+          if (lane < c1) out[(int64_t)s.cp_moff[k] + (int64_t)(at0 >> 5) * b1.z + st + lane] = m;
+        }
+    }
+  }
+}
+
+// The rows: block type, connection count, ligand flag, tile start and atoms.
 struct RowSide {
   int bt, nc, lig, st, c1;
 };
 
 // Stages atoms [at0, at0 + cnt) (cnt <= 32) of a block with exclusions
-// against the rows at side-1 atoms [base, ...) and their masks as mask
-// `sp`: b1 itself (`self`: pairs of later atoms only, weights from the
-// intra-block table) or a count-pair partner (the smallest separation over
-// the connections, ljlk_pose_score.impl.hh:47-67; `seps` its 16 connection
-// separations).  Only partner atoms that lie within four bonds of some atom
-// of b1 are compared row by row.
+// against the rows (b1 itself or a count-pair partner) at side-1 atoms
+// [base, ...), with the lanes' masks (excluded, weight 0.2) as mask `sp`.
 template <typename Real>
-__device__ __forceinline__ void stage_special(const ScoreArgs<Real>& s, Slab<Real>& w, const RowSide& r, int base,
-                                              int sp, int bt2, int64_t off2, int at0, int cnt, bool self,
-                                              const uint8_t* seps, int nc2, bool lig, int lane) {
-  const int at = at0 + lane;
-  if (lane < cnt) put_atom(w, base + lane, s.packed[off2 + at], off2 + at);
-  uint2 m = make_uint2(0u, 0u);
-  if (self) {
-    if (lane < r.c1)
-      m = s.imask[((int64_t)bt2 * s.A + r.st + lane) * s.n_iwords + (at0 >> 5)];
-  } else {
-    unsigned bb = 0xffffffffu;  // per connection of b1: the separation from it, a byte each
-    bool rel = false;
-    if (lane < cnt) {
-      const uint32_t cj = load_cpd(s, bt2, nc2, at);
-      for (int u = 0; u < r.nc; ++u) {
-        int best = 63;
-        for (int v = 0; v < nc2; ++v) best = min(best, (int)seps[u * 4 + v] + (int)((cj >> (8 * v)) & 0xff));
-        bb = (bb & ~(0xffu << (8 * u))) | ((unsigned)best << (8 * u));
-        rel |= best <= 4;
-      }
-    }
-    const uint32_t c0 = lane < r.c1 ? load_cpd(s, r.bt, r.nc, r.st + lane) : 0x3f3f3f3fu;
-    for (unsigned rm = __ballot_sync(0xffffffffu, rel); rm; rm &= rm - 1) {
-      const int k = __ffs(rm) - 1;
-      const unsigned bk = __shfl_sync(0xffffffffu, bb, k);
-      int sep = 5;
-      for (int u = 0; u < r.nc; ++u) sep = min(sep, (int)((c0 >> (8 * u)) & 0xff) + (int)((bk >> (8 * u)) & 0xff));
-      if (lig && (sep == 3 || sep == 4)) sep = 5;
-      m.x |= (unsigned)(sep < 4) << k;
-      m.y |= (unsigned)(sep == 4) << k;
-    }
-  }
-  w.smask[sp][lane] = m;
+__device__ __forceinline__ void stage_masked(const ScoreArgs<Real>& s, Slab<Real>& w, int base, int sp, int64_t off2,
+                                             int at0, int cnt, uint2 mask, int lane) {
+  const int64_t gi = off2 + at0 + lane;
+  if (lane < cnt) put_atom(w, base + lane, s.packed[gi], gi);
+  w.smask[sp][lane] = mask;
 }
 
 // Keeps, of up to 32 atoms (one per lane), those that can reach b1 (within
@@ -545,7 +592,7 @@ __device__ __forceinline__ EvalCtx<Real> eval_ctx(const ScoreArgs<Real>& s) {
 // BLOCK_PAIR selects per-block-pair energies / weights instead of per-pose
 // ones: every block then has words of its own.
 template <typename Real, bool GRAD, bool BLOCK_PAIR, int TERM, bool COUNT>
-__global__ void __launch_bounds__(sizeof(Real) == 4 ? 512 : 256, 1)
+__global__ void __launch_bounds__(sizeof(Real) == 4 ? 32 * PAIR_WARPS : 256, 1)
     score_kernel(ScoreArgs<Real> s, int items_per_ticket) {
   if (s.done && *s.done) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -566,8 +613,7 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 512 : 256, 1)
   for (;;) {
     int t = 0;
     if (lane == 0) t = atomicAdd(s.ticket, 1);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    const int it0 = t * items_per_ticket;
+    const int it0 = __shfl_sync(0xffffffffu, t, 0) * items_per_ticket;
     if (it0 >= n_work) break;
     const int it1 = min(it0 + items_per_ticket, n_work);
     for (int item = it0; item < it1; ++item) {
@@ -576,8 +622,21 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 512 : 256, 1)
       const int4 wi = s.work[item];
       const int p = wi.x, b1 = wi.y, cand0 = wi.z, cand1 = wi.w;
       const int i1 = p * s.B + b1;
+      // what the item starts from, all loaded before the first use: the row's
+      // block, sphere and count-pair partners (one per lane, beside their
+      // count) and the first 32 candidates
       const int4 bi1 = s.blk_info[i1];
+      const Quad<Real> sph1 = reinterpret_cast<const Quad<Real>*>(s.spheres)[i1];
+      const int ncp = s.cp_count[i1];
+      int cp_b2 = lane < CP_CAP ? s.cp_b2[(int64_t)i1 * CP_CAP + lane] : -1;
+      int4 pre_bi = make_int4(-1, 0, 0, 0);
+      Quad<Real> pre_s = {0, 0, 0, 0};
+      if (cand0 + lane < cand1) {
+        pre_bi = s.blk_info[p * s.B + cand0 + lane];
+        pre_s = reinterpret_cast<const Quad<Real>*>(s.spheres)[p * s.B + cand0 + lane];
+      }
       if (bi1.x < 0) continue;
+      if (lane >= ncp) cp_b2 = -1;
       const int n1 = bi1.z;
       RowSide r;
       r.bt = bi1.x;
@@ -590,12 +649,8 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 512 : 256, 1)
           ec.wt2 = s.dTdV[2 * s.P + p];
         }
       }
-      const Quad<Real> sph1 = reinterpret_cast<const Quad<Real>*>(s.spheres)[i1];
       const Real reach1 = sph1.d + s.g.max_dis;
       const Real reach1_2 = reach1 * reach1 * Real(1.0001);
-      // the row's count-pair partners, one per lane
-      const int ncp = s.cp_count[i1];
-      const int cp_b2 = lane < ncp ? s.cp_b2[(int64_t)i1 * CP_CAP + lane] : -1;
       E3<Real> acc = {0, 0, 0};
       for (int ti = 0; ti * TILE < n1; ++ti) {
         r.st = ti * TILE;
@@ -624,15 +679,22 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 512 : 256, 1)
               const int cnt = min(32, sp_n - sp_at), need = (cnt + 3) & ~3;
               if (nsp == MAXSP || nw >= max_words || m + need > top) break;
               const int src = sp_b2 - batch;
-              const int bt2 = __shfl_sync(0xffffffffu, bi2.x, src), off2 = __shfl_sync(0xffffffffu, bi2.y, src);
-              const int cl2 = __shfl_sync(0xffffffffu, bi2.w, src);
+              const int off2 = __shfl_sync(0xffffffffu, bi2.y, src);
               int base = m;
               if (BLOCK_PAIR)
                 m += need;
               else
                 base = top -= need;
-              stage_special(s, w, r, base, nsp, bt2, (int64_t)off2, sp_at, cnt, sp_b2 == b1,
-                            s.cp_seps + ((int64_t)i1 * CP_CAP + sp_cp) * 16, cl2 & 0xff, r.lig && (cl2 >> 8), lane);
+              const int64_t cpe = (int64_t)i1 * CP_CAP + sp_cp;
+              // b1 itself: [atom][word] of its block type; a partner: [word][atom]
+              uint2 mk = make_uint2(0u, 0u);
+              if (lane < r.c1) {
+                if (sp_b2 == b1)
+                  mk = s.imask[((int64_t)r.bt * s.A + r.st + lane) * s.n_iwords + (sp_at >> 5)];
+                else
+                  mk = s.pmask[(int64_t)s.cp_moff[cpe] + (int64_t)(sp_at >> 5) * n1 + r.st + lane];
+              }
+              stage_masked(s, w, base, nsp, (int64_t)off2, sp_at, cnt, mk, lane);
               if (lane == 0) {
                 w.desc[nw] = base | (cnt << 8) | ((nsp + 1) << 16);
                 w.out[nw] = (int64_t)i1 * s.B + sp_b2;
@@ -652,22 +714,43 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 512 : 256, 1)
               sp_cp = pm ? __ffs(pm) - 1 : 0;
               if (sp_at >= sp_n) sp_n = 0;
             } else if (!BLOCK_PAIR && k0 < T) {
-              // 32 atoms of the flat list: bit b of `word` set where a hit's
-              // atoms begin at list position k0 + b
-              if (m + 32 > top || nw + (m + 63) / 32 > MAXW) break;
-              const unsigned pos = (unsigned)(start - k0);
-              const unsigned word = __reduce_or_sync(0xffffffffu, pos < 32u ? 1u << pos : 0u);
-              const int own = owned + __popc(word & lemask) - 1;
-              owned += __popc(word);
-              const int f = k0 + lane;
-              const bool valid = f < T;
-              const int64_t gi = (int64_t)w.hoff[own] + f;
-              AtomRec<Real> a;
-              a.x = a.y = a.z = Real(0);
-              a.tf = 0;
-              if (valid) a = s.packed[gi];
-              m += stage_culled(w, m, valid, a, gi, sph1.a, sph1.b, sph1.c, reach1_2, -1, lane);
-              k0 += 32;
+              // as many of the list's atoms as side 1 has room for: all of
+              // their loads in flight at once, uncompacted behind m, then
+              // culled and moved up in place, 32 at a time
+              const int room = min((top - m) & ~31, 32 * (MAXW - nw - ((m + 31) >> 5)));
+              if (room <= 0) break;
+              const int n = min(room, T - k0);
+              for (int q = 0; q < n; q += 32) {
+                // bit b of `word` is set where a hit's atoms begin at list
+                // position k0 + q + b
+                const unsigned pos = (unsigned)(start - k0 - q);
+                const unsigned word = __reduce_or_sync(0xffffffffu, pos < 32u ? 1u << pos : 0u);
+                const int own = owned + __popc(word & lemask) - 1;
+                owned += __popc(word);
+                if (q + lane < n) {
+                  const int gi = w.hoff[own] + k0 + q + lane;
+                  w.gidx[m + q + lane] = gi;
+                  copy_async(&w.at[m + q + lane], s.packed + gi);
+                }
+              }
+              copy_wait();
+              __syncwarp();
+              int src = m;
+              for (int q = 0; q < n; q += 32, src += 32) {
+                const bool valid = q + lane < n;
+                AtomRec<Real> a;
+                a.x = a.y = a.z = Real(0);
+                a.tf = 0;
+                int gi = 0;
+                if (valid) {
+                  a = w.at[src + lane];
+                  gi = w.gidx[src + lane];
+                }
+                __syncwarp();
+                m += stage_culled(w, m, valid, a, gi, sph1.a, sph1.b, sph1.c, reach1_2, -1, lane);
+              }
+              k0 += n;
+              __syncwarp();
             } else if (BLOCK_PAIR && hits) {
               // 32 atoms of the next hit: a word of their own
               if (m + 32 > top || nw >= max_words) break;
@@ -694,17 +777,25 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 512 : 256, 1)
                 hits &= hits - 1;
               }
             } else if (next_c < cand1) {
-              // the next 32 candidates
+              // the next 32 candidates, loaded while the ones before were
+              // processed
               batch = next_c;
               next_c += 32;
               const int b2 = batch + lane;
               bool hit = false;
-              bi2 = make_int4(-1, 0, 0, 0);
+              bi2 = pre_bi;
+              const Quad<Real> s2 = pre_s;
+              pre_bi = make_int4(-1, 0, 0, 0);
+              {
+                // after the last batch: the first again, for the next tile
+                const int nx = (next_c < cand1 ? next_c : cand0) + lane;
+                if (nx < cand1) {
+                  pre_bi = s.blk_info[p * s.B + nx];
+                  pre_s = reinterpret_cast<const Quad<Real>*>(s.spheres)[p * s.B + nx];
+                }
+              }
               if (b2 < cand1) {
-                const int i2 = p * s.B + b2;
-                bi2 = s.blk_info[i2];
                 if (bi2.x >= 0) {
-                  const Quad<Real> s2 = reinterpret_cast<const Quad<Real>*>(s.spheres)[i2];
                   const Real dx = sub_rn(sph1.a, s2.a), dy = sub_rn(sph1.b, s2.b), dz = sub_rn(sph1.c, s2.c);
                   const Real d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
                   const Real thr = add_rn(add_rn(sph1.d, s2.d), s.reach);

@@ -23,12 +23,11 @@ import torch
 
 DEFAULT_GRID = {
     "rows_per_item": (1, 2),
-    # (warps per CTA, CTAs per SM): 16 warps per SM, the register limit at
-    # 128 registers a thread (the LK-ball and rotamer kernels take at most
-    # 8 warps per CTA)
-    "cta_shape": ((4, 4), (8, 2), (16, 1)),
-    "candidates_per_item": (32, 64, 128),
-    "slots_per_group": (8, 12),
+    # (warps per CTA, CTAs per SM): up to 20 warps per SM, the register limit
+    # at 96 registers a thread (LK-ball: 16, at most 8 warps per CTA)
+    "cta_shape": ((4, 4), (8, 2), (10, 2), (20, 1)),
+    "candidates_per_item": (32, 64, 128, 256),
+    "slots_per_group": (9,),
 }
 
 
