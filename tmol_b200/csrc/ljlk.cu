@@ -17,7 +17,7 @@
 //                                  to each pose's last real block
 //   spheres[P*B][4]                centroid + radius, rebuilt every call
 //
-//   packed[n_atoms], g4[n_atoms][4]  staged atoms and padded gradient, per call
+//   packed[n_atoms], g4[n_atoms][8]  staged atoms and padded gradient, per call
 //
 // Scoring is one persistent launch per call after the sphere kernel (every
 // warp takes work items from an atomic ticket; pair_engine.cuh), and a copy
@@ -515,9 +515,9 @@ struct ScoreArgs {
   // taken from a speculative pass (pose_backward_speculative)
   const int* done;
   // what the sphere pass zeroes before the scoring launch adds to it (no
-  // separate memsets in a step): reals of dcoords, of energies and of
+  // separate memsets in a step): reals of energies and of
   // zero_aux (LK-ball: the waters' gradient), and the work counters
-  int64_t zero_dcoords, zero_energies, zero_aux_n;
+  int64_t zero_energies, zero_aux_n;
   Real* zero_aux;
   int zero_counts;
   // pose plans of the LJ/LK and elec terms: per block {block type, first
@@ -546,7 +546,7 @@ struct ScoreArgs {
   const uint2* pmask;
   const uint32_t* cp_moff;
   const int* bt_n_heavy;  // heavy atoms per block type (work counters)
-  // LJ/LK and elec: the gradient as [n_atoms][4], zeroed by the sphere pass
+  // the gradient as [n_atoms][GRAD_STRIDE], zeroed by the sphere pass
   // and copied out by grad_out_kernel
   Real* g4;
   const uint8_t* bt_pd;
@@ -567,7 +567,6 @@ struct ScoreArgs {
   Real* energies;
   int32_t* nbr;
   const Real* dTdV;
-  Real* dcoords;
   int* ticket;
   unsigned long long* counts;
   // optional skip mask: bit b2 of row (p, b1) set = do not score the block
@@ -647,7 +646,6 @@ __global__ void spheres_kernel(ScoreArgs<Real> s) {
   if (s.done && *s.done) return;  // the scoring launch that follows does no work
   const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t n_threads = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = tid; i < s.zero_dcoords; i += n_threads) s.dcoords[i] = Real(0);
   for (int64_t i = tid; i < s.zero_energies; i += n_threads) s.energies[i] = Real(0);
   for (int64_t i = tid; i < s.zero_aux_n; i += n_threads) s.zero_aux[i] = Real(0);
   if (s.zero_counts && s.counts && tid < N_COUNTS) s.counts[tid] = 0;
@@ -681,7 +679,11 @@ __device__ __forceinline__ void pack_block(const ScoreArgs<Real>& s, int bt, int
     else
       a.tf = s.bt_tf[(int64_t)bt * s.A + k];
     s.packed[(int64_t)off + k] = a;
-    if (s.g4) reinterpret_cast<Quad<Real>*>(s.g4)[(int64_t)off + k] = Quad<Real>{0, 0, 0, 0};
+    if (s.g4) {
+      Quad<Real>* g = reinterpret_cast<Quad<Real>*>(s.g4 + GRAD_STRIDE * ((int64_t)off + k));
+      g[0] = Quad<Real>{0, 0, 0, 0};
+      g[1] = Quad<Real>{0, 0, 0, 0};
+    }
   }
 }
 
@@ -1034,7 +1036,7 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 32 * PAIR_WARPS : 256, 1)
 }
 
 // The gradient from its padded form: out [n_atoms][3] = hit or miss
-// [n_atoms][4] (hit when *flag is set; a null flag: miss), 0 for atoms that
+// [n_atoms][GRAD_STRIDE] (hit when *flag is set; a null flag: miss), 0 for atoms that
 // belong to no block.
 template <typename Real>
 __global__ void grad_out_kernel(const int* flag, const Real* hit, const Real* miss, const uint8_t* real, Real* out,
@@ -1043,7 +1045,8 @@ __global__ void grad_out_kernel(const int* flag, const Real* hit, const Real* mi
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * n_atoms;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t a = i / 3;
-    out[i] = real[a] ? src[4 * a + (i - 3 * a)] : Real(0);
+    const Real* g = src + GRAD_STRIDE * a + (i - 3 * a);
+    out[i] = real[a] ? g[0] + g[4] : Real(0);
   }
 }
 
@@ -1232,7 +1235,7 @@ struct tmol_b200_ljlk_plan {
   int* blk_off = nullptr;
   int4* blk_info = nullptr;  // pose plans of LJ/LK and elec: {bt, off, n_atoms, n_conn | ligand << 8}
   void* packed = nullptr;    // LJ/LK and elec: atoms as staged records [n_atoms], rewritten every call
-  void* g4 = nullptr;        // and the gradient as [n_atoms][4]
+  void* g4 = nullptr;        // and the gradient as [n_atoms][GRAD_STRIDE]
   uint8_t* real_atom = nullptr;  // [n_atoms] 1 where a block (or rotamer) has the atom
   uint2* imask = nullptr;        // [nbt * A][n_iwords] pairs within a block type
   int n_iwords = 0;
@@ -1272,7 +1275,7 @@ struct tmol_b200_ljlk_plan {
   // device flag a backward sets when its weights match those
   void* spec_next = nullptr;  // [n_terms, P]
   void* spec_used = nullptr;  // [n_terms, P]
-  void* spec_g = nullptr;     // [N, 4] (LK-ball: [N, 3])
+  void* spec_g = nullptr;     // [N, GRAD_STRIDE]
   void* spec_dw = nullptr;    // LK-ball: [N, 4, 3], the waters' gradient
   int* spec_flag = nullptr;
   bool spec_ready = false;  // spec_next holds a backward's weights
@@ -1827,7 +1830,7 @@ int lkb_waters_backward_impl(tmol_b200_ljlk_plan* pl, const void* coords, const 
 
 template <typename Real, bool GRAD, bool BLOCK_PAIR>
 int lkb_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const void* waters, void* energies, int32_t* nbr,
-                   const void* dTdV, void* dcoords, void* dwaters, cudaStream_t st, const int* done = nullptr) {
+                   const void* dTdV, void* g4, void* dwaters, cudaStream_t st, const int* done = nullptr) {
   ScoreArgs<Real> s = score_args<Real>(pl, coords);
   s.done = done;
   LkbArgs<Real> k = lkb_args<Real>(pl);
@@ -1837,7 +1840,7 @@ int lkb_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const void* wate
   s.energies = (Real*)energies;
   s.nbr = nbr;
   s.dTdV = (const Real*)dTdV;
-  s.dcoords = (Real*)dcoords;
+  s.g4 = (Real*)g4;  // the padded gradient, or null (zeroed by the sphere pass)
   const size_t PBB = (size_t)pl->P * pl->B * pl->B;
   // block-pair energies and weights are addressed by an int block-pair index
   if (BLOCK_PAIR && PBB >= ((size_t)1 << 31)) return TMOL_B200_ERR_CAPACITY;
@@ -1847,7 +1850,6 @@ int lkb_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const void* wate
   // ticket: by the sphere pass (which a taken speculative gradient skips:
   // its outputs are then copied whole)
   if (energies && !BLOCK_PAIR) s.zero_energies = (int64_t)pl->P * 4;
-  if (dcoords) s.zero_dcoords = (int64_t)pl->N * 3;
   if (dwaters) {
     s.zero_aux = (Real*)dwaters;
     s.zero_aux_n = (int64_t)pl->N * LKB_NW * 3;
@@ -1904,14 +1906,14 @@ int lkb_backward_speculative_impl(tmol_b200_ljlk_plan* pl, const void* coords, c
     CK(cudaMemsetAsync(pl->spec_flag, 0, sizeof(int), st));
   }
   // zeroes the outputs; its scoring launch does no work when the flag is set
-  const int rc = lkb_score_impl<Real, true, false>(pl, coords, waters, nullptr, nullptr, dTdV, dcoords, dwaters,
-                                                   st, pl->spec_flag);
+  int rc = lkb_score_impl<Real, true, false>(pl, coords, waters, nullptr, nullptr, dTdV, pl->g4, dwaters, st,
+                                             pl->spec_flag);
   if (rc != TMOL_B200_OK) return rc;
-  const int64_t n_g = (int64_t)pl->N * 3, n_dw = (int64_t)pl->N * LKB_NW * 3;
-  if (n_g > 0) {
+  rc = grad_out<Real>(pl, pl->spec_flag, pl->spec_g, dcoords, st);
+  if (rc != TMOL_B200_OK) return rc;
+  const int64_t n_dw = (int64_t)pl->N * LKB_NW * 3;
+  if (n_dw > 0) {
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n_dw + 255) / 256, (int64_t)pl->n_sm * 8));
-    spec_copy_kernel<Real><<<grid, 256, 0, st>>>(pl->spec_flag, (const Real*)pl->spec_g, (Real*)dcoords, n_g);
-    CK(cudaGetLastError());
     spec_copy_kernel<Real><<<grid, 256, 0, st>>>(pl->spec_flag, (const Real*)pl->spec_dw, (Real*)dwaters, n_dw);
     CK(cudaGetLastError());
   }
@@ -1935,14 +1937,16 @@ int lkb_rotamer_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const vo
   ra.n_pairs = n_pairs;
   s.energies = (Real*)energies;
   s.dTdV = (const Real*)dTdV;
-  s.dcoords = (Real*)dcoords;
+  if (!GRAD) s.g4 = nullptr;
   s.nbr = nullptr;
   s.counts = pl->counts;
   CK(cudaMemsetAsync(pl->counts, 0, N_COUNTS * sizeof(unsigned long long), st));
   if (energies) CK(cudaMemsetAsync(energies, 0, (size_t)4 * n_pairs * sizeof(Real), st));
-  if (dcoords) CK(cudaMemsetAsync(dcoords, 0, (size_t)pl->N * 3 * sizeof(Real), st));
   if (dwaters) CK(cudaMemsetAsync(dwaters, 0, (size_t)pl->N * LKB_NW * 3 * sizeof(Real), st));
-  if (n_items == 0) return TMOL_B200_OK;
+  if (n_items == 0) {
+    if (dcoords) CK(cudaMemsetAsync(dcoords, 0, (size_t)pl->N * 3 * sizeof(Real), st));
+    return TMOL_B200_OK;
+  }
   if (pl->R > 0) {
     const int gr = std::max(1, std::min((pl->R + 7) / 8, pl->n_sm * 16));
     rot_spheres_kernel<Real><<<gr, 256, 0, st>>>(s, ra, (Real*)pl->rot_spheres);
@@ -1957,7 +1961,7 @@ int lkb_rotamer_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const vo
   else
     lkb_rotamer_kernel<Real, GRAD, false><<<grid, 32 * warps, 0, st>>>(s, k, ra, (const Real*)pl->rot_spheres);
   CK(cudaGetLastError());
-  return TMOL_B200_OK;
+  return GRAD ? grad_out<Real>(pl, nullptr, nullptr, dcoords, st) : TMOL_B200_OK;
 }
 
 }  // namespace
@@ -2014,7 +2018,7 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
     CK(cudaMemcpyAsync(wg, k->water_gen_global_params, sizeof(wg), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   std::vector<std::vector<int>> pol(nbt), occ(nbt);
-  std::vector<Real> par((size_t)std::max(nbt * A, 1) * LKB_NPAR, Real(0));
+  std::vector<Real> par((size_t)std::max(nbt * A, 1) * LKB_PAR_PAD, Real(0));
   for (int bt = 0; scoring && bt < nbt; ++bt)
     for (int t = 0; t < NT; ++t) {
       const size_t tb = (size_t)bt * NT + t;
@@ -2025,7 +2029,7 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
         if (i < 0 || i >= TILE || a >= h_nat[bt] || a >= A) return TMOL_B200_ERR_INDEX_RANGE;
         if (q < npol[tb]) pol[bt].push_back(a);
         occ[bt].push_back(a);
-        std::copy_n(&tpar[(tb * TILE + q) * LKB_NPAR], LKB_NPAR, &par[((size_t)bt * A + a) * LKB_NPAR]);
+        std::copy_n(&tpar[(tb * TILE + q) * LKB_NPAR], LKB_NPAR, &par[((size_t)bt * A + a) * LKB_PAR_PAD]);
       }
     }
   // occluders that are donors or acceptors (parameters 4 and 7) first: the
@@ -2033,7 +2037,7 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
   std::vector<int> hnbocc(std::max(nbt, 1), 0);
   for (int bt = 0; bt < nbt; ++bt) {
     auto bridges = [&](int a) {
-      const Real* q = &par[((size_t)bt * A + a) * LKB_NPAR];
+      const Real* q = &par[((size_t)bt * A + a) * LKB_PAR_PAD];
       return q[4] != Real(0) || q[7] != Real(0);
     };
     std::stable_partition(occ[bt].begin(), occ[bt].end(), bridges);
@@ -2073,7 +2077,7 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
     // the score op's speculative gradient (lkb_backward_speculative)
     CK(dalloc(pl, (Real**)&pl->spec_next, (size_t)4 * std::max(pl->P, 1)));
     CK(dalloc(pl, (Real**)&pl->spec_used, (size_t)4 * std::max(pl->P, 1)));
-    CK(dalloc(pl, (Real**)&pl->spec_g, (size_t)std::max<int64_t>(pl->N, 1) * 3));
+    CK(dalloc(pl, (Real**)&pl->spec_g, (size_t)std::max<int64_t>(pl->N, 1) * GRAD_STRIDE));
     CK(dalloc(pl, (Real**)&pl->spec_dw, (size_t)std::max<int64_t>(pl->N, 1) * LKB_NW * 3));
     CK(dalloc(pl, &pl->spec_flag, 1));
   }
@@ -2282,13 +2286,15 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   PCK(dalloc(pl, &pl->cp_minsep, PB * CP_CAP));
   PCK(dalloc(pl, &pl->cp_seps, PB * CP_CAP * 16));
   PCK(dalloc(pl, (unsigned char**)&pl->spheres, PB * 4 * real_bytes));
-  if (term != kTermLKBall) {
+  if (scoring) {
     const int64_t n_at = std::max<int64_t>(in->n_atoms, 1);
     PCK(dalloc(pl, (unsigned char**)&pl->packed,
                n_at * (real_bytes == 4 ? sizeof(AtomRec<float>) : sizeof(AtomRec<double>))));
-    PCK(dalloc(pl, (unsigned char**)&pl->g4, (size_t)n_at * 4 * real_bytes));
+    PCK(dalloc(pl, (unsigned char**)&pl->g4, (size_t)n_at * GRAD_STRIDE * real_bytes));
     PCK(dalloc(pl, &pl->real_atom, n_at));
     PCK(cudaMemsetAsync(pl->real_atom, 0, n_at, st));
+  }
+  if (term != kTermLKBall) {
     pl->n_iwords = (A + 31) / 32;
     PCK(dalloc(pl, &pl->imask, (size_t)nbt * A * pl->n_iwords));
     PCK(dalloc(pl, &pl->bt_n_heavy, nbt));
@@ -2297,7 +2303,7 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     PCK(dalloc(pl, &pl->blk_info, PB));
     PCK(dalloc(pl, (unsigned char**)&pl->spec_next, (size_t)n_terms(term) * std::max(P, 1) * real_bytes));
     PCK(dalloc(pl, (unsigned char**)&pl->spec_used, (size_t)n_terms(term) * std::max(P, 1) * real_bytes));
-    PCK(dalloc(pl, (unsigned char**)&pl->spec_g, (size_t)std::max<int64_t>(in->n_atoms, 1) * 4 * real_bytes));
+    PCK(dalloc(pl, (unsigned char**)&pl->spec_g, (size_t)std::max<int64_t>(in->n_atoms, 1) * GRAD_STRIDE * real_bytes));
     PCK(dalloc(pl, &pl->spec_flag, 1));
   }
   if (real_bytes == 4) PCK(dalloc(pl, &pl->sub_spheres, PB * 8));
@@ -2497,7 +2503,7 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
       PCK(cudaGetLastError());
     }
   }
-  if (term != kTermLKBall) {
+  if (scoring) {
     const int n = rotamers ? pl->R : (int)PB;
     if (n > 0) {
       plan_real_atoms_kernel<<<std::max(1, std::min((n + 127) / 128, pl->n_sm * 8)), 128, 0, st>>>(
@@ -3273,14 +3279,16 @@ int tmol_b200_lkball_energy_and_gradient(tmol_b200_lkball_plan* plan, const void
   if (plan->real_bytes == 4) {
     if ((rc = lkb_waters_impl<float>(plan, coords, plan->lkb_waters, st, true))) return rc;
     if ((rc = lkb_score_impl<float, true, false>(plan, coords, plan->lkb_waters, energies, nullptr, weights,
-                                                 dcoords, plan->lkb_dwaters, st)))
+                                                 plan->g4, plan->lkb_dwaters, st)))
       return rc;
+    if ((rc = grad_out<float>(plan, nullptr, nullptr, dcoords, st))) return rc;
     return lkb_waters_backward_impl<float>(plan, coords, plan->lkb_dwaters, dcoords, st);
   }
   if ((rc = lkb_waters_impl<double>(plan, coords, plan->lkb_waters, st, true))) return rc;
   if ((rc = lkb_score_impl<double, true, false>(plan, coords, plan->lkb_waters, energies, nullptr, weights,
-                                                dcoords, plan->lkb_dwaters, st)))
+                                                plan->g4, plan->lkb_dwaters, st)))
     return rc;
+  if ((rc = grad_out<double>(plan, nullptr, nullptr, dcoords, st))) return rc;
   return lkb_waters_backward_impl<double>(plan, coords, plan->lkb_dwaters, dcoords, st);
 }
 
@@ -3291,15 +3299,19 @@ int tmol_b200_lkball_backward(tmol_b200_lkball_plan* plan, const void* coords, c
   if (!plan || plan->term != kTermLKBall || !plan->lkb_pol || !dTdV) return TMOL_B200_ERR_INVALID_ARGUMENT;
   if (plan->N > 0 && (!coords || !waters || !dcoords || !dwaters)) return TMOL_B200_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
-  if (plan->real_bytes == 4)
-    return block_pair ? lkb_score_impl<float, true, true>(plan, coords, waters, nullptr, nullptr, dTdV, dcoords,
-                                                          dwaters, st)
-                      : lkb_score_impl<float, true, false>(plan, coords, waters, nullptr, nullptr, dTdV, dcoords,
-                                                           dwaters, st);
-  return block_pair ? lkb_score_impl<double, true, true>(plan, coords, waters, nullptr, nullptr, dTdV, dcoords,
-                                                         dwaters, st)
-                    : lkb_score_impl<double, true, false>(plan, coords, waters, nullptr, nullptr, dTdV, dcoords,
-                                                          dwaters, st);
+  int rc;
+  if (plan->real_bytes == 4) {
+    rc = block_pair ? lkb_score_impl<float, true, true>(plan, coords, waters, nullptr, nullptr, dTdV, plan->g4,
+                                                        dwaters, st)
+                    : lkb_score_impl<float, true, false>(plan, coords, waters, nullptr, nullptr, dTdV, plan->g4,
+                                                         dwaters, st);
+    return rc ? rc : grad_out<float>(plan, nullptr, nullptr, dcoords, st);
+  }
+  rc = block_pair ? lkb_score_impl<double, true, true>(plan, coords, waters, nullptr, nullptr, dTdV, plan->g4,
+                                                       dwaters, st)
+                  : lkb_score_impl<double, true, false>(plan, coords, waters, nullptr, nullptr, dTdV, plan->g4,
+                                                        dwaters, st);
+  return rc ? rc : grad_out<double>(plan, nullptr, nullptr, dcoords, st);
 }
 
 int64_t tmol_b200_ljlk_plan_device_bytes(const tmol_b200_ljlk_plan* plan) {

@@ -17,6 +17,7 @@
 
 constexpr int LKB_NW = 4;    // waters per polar atom
 constexpr int LKB_NPAR = 9;  // per-atom parameters
+constexpr int LKB_PAR_PAD = 12;  // their stride in the kernels' table: three vector loads
 
 enum LkbSiteKind : int { kLkbNone = 0, kLkbDonor = 1, kLkbSp2 = 2, kLkbSp3 = 3, kLkbRing = 4 };
 
@@ -43,7 +44,7 @@ struct LkbArgs {
   const int* nocc;
   const int* nbocc;     // [nbt] leading occluders that are donors or acceptors (the bridge term)
   int maxpol, maxocc;
-  const Real* par;      // [nbt][A][9]
+  const Real* par;      // [nbt][A][12], 9 used
   Real water_dist, hbond_dis, hbond_oh, hbond_h, max_dis;
 };
 
@@ -669,20 +670,65 @@ __device__ __forceinline__ int lkb_inter_sep(const ScoreArgs<Real>& s, int bt1, 
   return sep;
 }
 
-template <typename Real, typename K>
-__device__ __forceinline__ LkbParams<Real> lkb_params(const K& k, int A, int bt, int atom) {
-  const Real* q = k.par + ((int64_t)bt * A + atom) * LKB_NPAR;
+template <typename Real>
+__device__ __forceinline__ LkbParams<Real> lkb_params(const Real* par, int row) {
+  const Quad<Real>* q = reinterpret_cast<const Quad<Real>*>(par) + 3 * (int64_t)row;
+  const Quad<Real> u = q[0], v = q[1];
   LkbParams<Real> r;
-  r.lj_radius = q[0];
-  r.lk_dgfree = q[1];
-  r.lk_lambda = q[2];
-  r.lk_volume = q[3];
-  r.is_donor = q[4];
-  r.is_hydroxyl = q[5];
-  r.is_polarh = q[6];
-  r.is_acceptor = q[7];
-  r.is_carbon_lk = q[8];
+  r.lj_radius = u.a;
+  r.lk_dgfree = u.b;
+  r.lk_lambda = u.c;
+  r.lk_volume = u.d;
+  r.is_donor = v.a;
+  r.is_hydroxyl = v.b;
+  r.is_polarh = v.c;
+  r.is_acceptor = v.d;
+  r.is_carbon_lk = q[2].a;
   return r;
+}
+
+// An atom's four waters: twelve values, 16-byte aligned where the whole array
+// is (`vec`; torch's allocations are).
+template <typename Real>
+__device__ __forceinline__ void lkb_load_waters(const Real* waters, int64_t row, bool vec, Real* W) {
+  const Real* p = waters + row * (LKB_NW * 3);
+  if (vec) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const Quad<Real> q = reinterpret_cast<const Quad<Real>*>(p)[k];
+      W[4 * k] = q.a;
+      W[4 * k + 1] = q.b;
+      W[4 * k + 2] = q.c;
+      W[4 * k + 3] = q.d;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < LKB_NW * 3; ++k) W[k] = p[k];
+  }
+}
+
+// Adds the gradient on an atom's waters, four values a reduction.
+__device__ __forceinline__ void lkb_add_waters(float* dwaters, int64_t row, bool vec, const float* g) {
+  float* p = dwaters + row * (LKB_NW * 3);
+  if (vec) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float a = g[4 * k], b = g[4 * k + 1], c = g[4 * k + 2], d = g[4 * k + 3];
+      if (a != 0.0f || b != 0.0f || c != 0.0f || d != 0.0f)
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + 4 * k), "f"(a), "f"(b), "f"(c), "f"(d)
+                     : "memory");
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < LKB_NW * 3; ++k)
+      if (g[k] != 0.0f) atomicAdd(p + k, g[k]);
+  }
+}
+__device__ __forceinline__ void lkb_add_waters(double* dwaters, int64_t row, bool, const double* g) {
+  double* p = dwaters + row * (LKB_NW * 3);
+#pragma unroll
+  for (int k = 0; k < LKB_NW * 3; ++k)
+    if (g[k] != 0.0) atomicAdd(p + k, g[k]);
 }
 
 // Pairs in reach wait in two per-warp queues, those whose occluder bridges
@@ -702,12 +748,12 @@ struct LkbQueue {
 // What evaluating a queued pair needs (a compact by-value context).
 template <typename Real>
 struct LkbEval {
-  const Real* coords;
+  const AtomRec<Real>* packed;
   const Real* waters;
   const Real* par;
-  Real* dcoords;
-  Real* dwaters;
-  int A;
+  Real* g4;       // padded gradient [n_atoms][GRAD_STRIDE]
+  Real* dwaters;  // [n_atoms][4][3]
+  bool vec_w, vec_dw;  // 16-byte aligned
   Real water_dist, hbond_dis, hbond_oh, hbond_h, max_dis;
 };
 
@@ -736,32 +782,25 @@ __device__ TMOL_B200_LKB_DRAIN_ATTR Lkb4<Real> lkb_drain(const LkbEval<Real> ev,
   if (lane >= n) return out;
   const int64_t rp = q.rp[lane], ro = q.ro[lane];
   const int pidx = q.pi[lane], oidx = q.oi[lane], sep = q.sep[lane];
-  Real I[3], J[3], WI[LKB_NW * 3], WJ[LKB_NW * 3];
-  lkb_load3(ev.coords, rp, I);
-  lkb_load3(ev.coords, ro, J);
-#pragma unroll
-  for (int c = 0; c < LKB_NW * 3; ++c) {
-    WI[c] = ev.waters[rp * LKB_NW * 3 + c];
-    WJ[c] = ev.waters[ro * LKB_NW * 3 + c];
-  }
-  const LkbParams<Real> pp = lkb_params<Real>(ev, 0, 0, pidx);  // row bt * A + atom
-  const LkbParams<Real> po = lkb_params<Real>(ev, 0, 0, oidx);
+  Real WI[LKB_NW * 3], WJ[LKB_NW * 3];
+  const AtomRec<Real> ai = ev.packed[rp], aj = ev.packed[ro];
+  const Real I[3] = {ai.x, ai.y, ai.z}, J[3] = {aj.x, aj.y, aj.z};
+  lkb_load_waters(ev.waters, rp, ev.vec_w, WI);
+  lkb_load_waters(ev.waters, ro, ev.vec_w, WJ);
+  const LkbParams<Real> pp = lkb_params(ev.par, pidx);  // row bt * A + atom
+  const LkbParams<Real> po = lkb_params(ev.par, oidx);
   Real gI[3] = {0, 0, 0}, gJ[3] = {0, 0, 0}, gWI[LKB_NW * 3], gWJ[LKB_NW * 3];
   if (GRAD)
 #pragma unroll
     for (int c = 0; c < LKB_NW * 3; ++c) gWI[c] = gWJ[c] = 0;
   lkb_pair<Real, GRAD>(I, J, WI, WJ, sep, pp, po, ev, out.v, w.v, gI, gJ, gWI, gWJ);
   if (GRAD) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      if (gI[c] != Real(0)) atomicAdd(&ev.dcoords[3 * rp + c], gI[c]);
-      if (gJ[c] != Real(0)) atomicAdd(&ev.dcoords[3 * ro + c], gJ[c]);
-    }
-#pragma unroll
-    for (int c = 0; c < LKB_NW * 3; ++c) {
-      if (gWI[c] != Real(0)) atomicAdd(&ev.dwaters[rp * LKB_NW * 3 + c], gWI[c]);
-      if (gWJ[c] != Real(0)) atomicAdd(&ev.dwaters[ro * LKB_NW * 3 + c], gWJ[c]);
-    }
+    // vector reductions: the thirty values of a pair as scalar ones took the
+    // path to L2 longer than the pair's arithmetic
+    if (gI[0] != Real(0) || gI[1] != Real(0) || gI[2] != Real(0)) add_force(ev.g4 + GRAD_STRIDE * rp, gI[0], gI[1], gI[2]);
+    if (gJ[0] != Real(0) || gJ[1] != Real(0) || gJ[2] != Real(0)) add_force(ev.g4 + GRAD_STRIDE * ro, gJ[0], gJ[1], gJ[2]);
+    lkb_add_waters(ev.dwaters, rp, ev.vec_dw, gWI);
+    lkb_add_waters(ev.dwaters, ro, ev.vec_dw, gWJ);
   }
   return out;
 }
@@ -909,10 +948,8 @@ __device__ __forceinline__ void lkb_enqueue_pairs(const ScoreArgs<Real>& s, cons
       if (sep > 3) {
         rp = offp + ap;
         ro = offo + ao;
-        Real I[3], J[3];
-        lkb_load3(s.coords, rp, I);
-        lkb_load3(s.coords, ro, J);
-        const Real dv[3] = {I[0] - J[0], I[1] - J[1], I[2] - J[2]};
+        const AtomRec<Real> ai = s.packed[rp], aj = s.packed[ro];
+        const Real dv[3] = {ai.x - aj.x, ai.y - aj.y, ai.z - aj.z};
         const Real dist = lkb_sqrt(lkb_dot(dv, dv));
         in_reach = dist < k.max_dis && !isnan(k.waters[(int64_t)rp * LKB_NW * 3]);
         pidx = btp * s.A + ap;
@@ -963,12 +1000,13 @@ __device__ __forceinline__ bool lkb_striking(const ScoreArgs<Real>& s, int64_t i
 template <typename Real>
 __device__ __forceinline__ LkbEval<Real> lkb_eval_of(const ScoreArgs<Real>& s, const LkbArgs<Real>& k) {
   LkbEval<Real> ev;
-  ev.coords = s.coords;
+  ev.packed = s.packed;
   ev.waters = k.waters;
   ev.par = k.par;
-  ev.dcoords = s.dcoords;
+  ev.g4 = s.g4;
   ev.dwaters = k.dwaters_out;
-  ev.A = s.A;
+  ev.vec_w = (reinterpret_cast<uintptr_t>(k.waters) & (4 * sizeof(Real) - 1)) == 0;
+  ev.vec_dw = (reinterpret_cast<uintptr_t>(k.dwaters_out) & (4 * sizeof(Real) - 1)) == 0;
   ev.water_dist = k.water_dist;
   ev.hbond_dis = k.hbond_dis;
   ev.hbond_oh = k.hbond_oh;

@@ -16,29 +16,26 @@
 //   3. evaluation, class by class: every lane takes an equal stretch of
 //      consecutive entries.  Lanes of a step run the same code, a stretch
 //      stays on one or two rows (their atom, force and, in pair mode,
-//      energies stay in registers), and the side-1 forces go out as one
-//      16-byte vector reduction per pair into a padded gradient buffer.
+//      energies stay in registers), and the side-1 forces go out as 16-byte
+//      vector reductions into a padded gradient buffer.
 //
 // What bounds it: latency, at 20 warps per SM (about half of the issue slots
 // are used; DRAM and FP32 pipes stay below a fifth).  So the loads an item
 // starts from go out together, a whole list of neighbouring atoms is in flight
 // at once (cp.async into side 1, culled in place), and forces leave the SM
 // without being waited for: shared-memory float atomics are compare-and-swap
-// loops here (three per pair and side measured 13-33 cycles of an SM and
-// about 25 issue slots); one red.global.add.v4.f32 is a single instruction
-// and 44 cycles of an SM's path to L2.  64 x 150 residues, energy + gradient
-// with the sphere pass and the gradient's copy, L2 flushed: 320 us with the
-// shared-memory accumulators and per-block staging this replaces, 157 us with
-// the three phases, 130 us with the loads in flight and 20 warps.
+// loops here (64 x 150 residues, energy + gradient: 185 us with the side-1
+// forces summed in shared memory, 138 us without); one red.global.add.v4.f32 is
+// a single instruction and 44 cycles of an SM's path to L2.
 
 constexpr int M1 = 160;  // side-1 atoms of a group (< 256: 8-bit index)
 constexpr int MAXW = 9;  // words of a group; odd: the mask arrays' row stride has no bank conflicts
 constexpr int MAXSP = 4; // words with exclusion masks
 // Warps per CTA and SM.  The engine waits on memory more than it issues, so
 // warps count for more than registers or a longer side 1: 64 x 150 residues,
-// energy + gradient, 16 warps of 128 registers and M1 = 224 take 144 us, 16
-// and M1 = 160 142 us, 20 warps of 96 registers (two spilled words) and
-// M1 = 160 130 us.
+// energy + gradient, 16 warps of 128 registers take 144 us with M1 = 224 and
+// 142 us with 160; 20 warps of 96 registers 130 us with 160 and with 128
+// (before forces were split).
 constexpr int PAIR_WARPS = 20;
 constexpr int kTfHeavy = 256;
 
@@ -100,17 +97,41 @@ struct EvalCtx {
   Real max2, far2;        // squares of the cutoff and of the far class's start
   Real far_dmin, far_first, inv_hf;
   Real wt0, wt1, wt2;     // gradient weights of the three terms (elec: wt0)
-  Real* g;                // padded gradient [n_atoms][4]
+  Real* g;                // padded gradient [n_atoms][GRAD_STRIDE]
   int64_t row0;           // global atom index of row 0
   Real* energies;         // pair mode: [n_terms][stride]
   const Real* dTdV;       // pair mode: the same shape
   int64_t stride;
 };
 
-__device__ __forceinline__ void add_force(float* g, float x, float y, float z) {
+// Adds a force to an atom's padded gradient: GRAD_STRIDE values, two groups
+// (x, y, z, -) whose sum is the gradient.  The first group takes multiples of
+// 2^-6 kcal/mol/A, whose float32 sums are exact (below 2^18) and so the same
+// in any order; what remains of a force goes to the second, whose sums stay
+// small.  A single float32 sum of forty signed terms in no fixed order, where
+// clashes of 10^3 kcal/mol/A nearly cancel, differs by 3e-4 from call to call.
+// SMALL: a force of the far class (well below one), to the second group alone.
+constexpr int GRAD_STRIDE = 8;
+
+__device__ __forceinline__ void red4(float* g, float x, float y, float z) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g), "f"(x), "f"(y), "f"(z), "f"(0.0f)
                : "memory");
 }
+__device__ __forceinline__ float force_grid(float x) {
+  const float c = 1.5f * 131072.0f;  // 1.5 x 2^17: float32 spacing 2^-6
+  return __fsub_rn(__fadd_rn(x, c), c);
+}
+template <bool SMALL = false>
+__device__ __forceinline__ void add_force(float* g, float x, float y, float z) {
+  if (SMALL) {
+    red4(g + 4, x, y, z);
+    return;
+  }
+  const float hx = force_grid(x), hy = force_grid(y), hz = force_grid(z);
+  if (hx != 0.0f || hy != 0.0f || hz != 0.0f) red4(g, hx, hy, hz);
+  red4(g + 4, __fsub_rn(x, hx), __fsub_rn(y, hy), __fsub_rn(z, hz));
+}
+template <bool SMALL = false>
 __device__ __forceinline__ void add_force(double* g, double x, double y, double z) {
   atomicAdd(g, x);
   atomicAdd(g + 1, y);
@@ -226,7 +247,7 @@ __device__ __forceinline__ void eval_class(const EvalCtx<Real>& c, const Slab<Re
     const int j = e & 255, r = (e >> 8) & 31;
     if (r != row) {
       if (GRAD && row >= 0) {
-        add_force(c.g + 4 * (c.row0 + row), fx, fy, fz);
+        add_force<CLS == kFar>(c.g + GRAD_STRIDE * (c.row0 + row), fx, fy, fz);
         fx = fy = fz = 0;
       }
       row = r;
@@ -315,10 +336,10 @@ __device__ __forceinline__ void eval_class(const EvalCtx<Real>& c, const Slab<Re
       fx += px;
       fy += py;
       fz += pz;
-      add_force(c.g + 4 * (int64_t)w.gidx[j], -px, -py, -pz);
+      add_force<CLS == kFar>(c.g + GRAD_STRIDE * (int64_t)w.gidx[j], -px, -py, -pz);
     }
   }
-  if (GRAD && row >= 0) add_force(c.g + 4 * (c.row0 + row), fx, fy, fz);
+  if (GRAD && row >= 0) add_force<CLS == kFar>(c.g + GRAD_STRIDE * (c.row0 + row), fx, fy, fz);
   if (PAIR) {
     if (slot >= 0 && c.energies) {
       Real* o = c.energies + w.out[slot];
