@@ -520,6 +520,15 @@ struct ScoreArgs {
   int64_t zero_energies, zero_aux_n;
   Real* zero_aux;
   int zero_counts;
+  int64_t zero_nbr;  // entries of nbr
+  // speculative gradients: the sphere pass copies the last backward's weights
+  // (a forward: spec_from to spec_to, spec_n values), or compares a backward's
+  // weights with them (spec_flag set where all are equal; the launches then
+  // have nothing to do)
+  const Real* spec_from;
+  Real* spec_to;
+  int spec_n;
+  int* spec_flag;
   // pose plans of the LJ/LK and elec terms: per block {block type, first
   // atom, atom count, connections | ligand << 8} and every atom as a
   // staged record (coordinates with its type or charge), written by the
@@ -643,11 +652,26 @@ __device__ __forceinline__ void pack_block(const ScoreArgs<Real>& s, int bt, int
 
 template <typename Real>
 __global__ void spheres_kernel(ScoreArgs<Real> s) {
-  if (s.done && *s.done) return;  // the scoring launch that follows does no work
+  if (s.spec_flag) {
+    // every block compares for itself: a few hundred values that L2 holds
+    int differ = 0;
+    for (int i = threadIdx.x; i < s.spec_n; i += blockDim.x) differ |= !(s.spec_from[i] == s.spec_to[i]);
+    differ = __syncthreads_or(differ);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *s.spec_flag = differ ? 0 : 1;
+    if (!differ) return;
+  } else if (s.done && *s.done) {
+    return;  // the scoring launch that follows does no work
+  }
   const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t n_threads = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = tid; i < s.zero_energies; i += n_threads) s.energies[i] = Real(0);
   for (int64_t i = tid; i < s.zero_aux_n; i += n_threads) s.zero_aux[i] = Real(0);
+  if (!s.spec_flag)
+    for (int64_t i = tid; i < s.spec_n; i += n_threads) s.spec_to[i] = s.spec_from[i];
+  // the neighbour matrix, four entries a store where it is aligned
+  const int64_t n4 = (reinterpret_cast<uintptr_t>(s.nbr) & 15) == 0 ? s.zero_nbr / 4 : 0;
+  for (int64_t i = tid; i < n4; i += n_threads) reinterpret_cast<int4*>(s.nbr)[i] = make_int4(0, 0, 0, 0);
+  for (int64_t i = 4 * n4 + tid; i < s.zero_nbr; i += n_threads) s.nbr[i] = 0;
   if (s.zero_counts && s.counts && tid < N_COUNTS) s.counts[tid] = 0;
   if (tid == 0 && s.ticket) *s.ticket = 0;  // the scoring launch's work ticket
   const int lane = threadIdx.x & 31;
@@ -1037,10 +1061,13 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 32 * PAIR_WARPS : 256, 1)
 
 // The gradient from its padded form: out [n_atoms][3] = hit or miss
 // [n_atoms][GRAD_STRIDE] (hit when *flag is set; a null flag: miss), 0 for atoms that
-// belong to no block.
+// belong to no block.  keep = weights: those of a backward, for the next
+// speculative forward.
 template <typename Real>
 __global__ void grad_out_kernel(const int* flag, const Real* hit, const Real* miss, const uint8_t* real, Real* out,
-                                int64_t n_atoms) {
+                                int64_t n_atoms, const Real* weights, Real* keep, int n_weights) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_weights; i += (int64_t)gridDim.x * blockDim.x)
+    keep[i] = weights[i];
   const Real* src = flag && *flag ? hit : miss;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * n_atoms;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -1550,13 +1577,25 @@ int launch_score(tmol_b200_ljlk_plan* pl, ScoreArgs<Real> s, cudaStream_t st) {
 
 // dcoords [N, 3] from the padded gradient (`hit` instead when *flag is set).
 template <typename Real>
-int grad_out(tmol_b200_ljlk_plan* pl, const int* flag, const void* hit, void* dcoords, cudaStream_t st) {
-  if (pl->N == 0) return TMOL_B200_OK;
+int grad_out(tmol_b200_ljlk_plan* pl, const int* flag, const void* hit, void* dcoords, cudaStream_t st,
+             const void* weights = nullptr, void* keep = nullptr, int n_weights = 0) {
+  if (pl->N == 0 && n_weights == 0) return TMOL_B200_OK;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((3 * pl->N + 255) / 256, (int64_t)pl->n_sm * 16));
   grad_out_kernel<Real><<<grid, 256, 0, st>>>(flag, (const Real*)hit, (const Real*)pl->g4, pl->real_atom,
-                                              (Real*)dcoords, pl->N);
+                                              (Real*)dcoords, pl->N, (const Real*)weights, (Real*)keep, n_weights);
   CK(cudaGetLastError());
   return TMOL_B200_OK;
+}
+
+// Zeroes the neighbour matrix: in the sphere pass, or where that would take
+// it longer than a launch costs (from 32 MB on, some 10 us), by a memset.
+template <typename Real>
+cudaError_t clear_neighbors(const tmol_b200_ljlk_plan* pl, ScoreArgs<Real>& s, cudaStream_t st) {
+  if (!s.nbr) return cudaSuccess;
+  const int64_t n = (int64_t)pl->P * pl->B * pl->B;
+  if (n > ((int64_t)1 << 23)) return cudaMemsetAsync(s.nbr, 0, (size_t)n * sizeof(int32_t), st);
+  s.zero_nbr = n;
+  return cudaSuccess;
 }
 
 template <typename Real>
@@ -1571,7 +1610,7 @@ int forward_impl(tmol_b200_ljlk_plan* pl, const void* coords, int block_pair,
     CK(cudaMemsetAsync(energies, 0, n_e * sizeof(Real), st));
   else
     s.zero_energies = (int64_t)n_e;  // by the sphere pass
-  if (nbr) CK(cudaMemsetAsync(nbr, 0, (size_t)pl->P * pl->B * pl->B * sizeof(int32_t), st));
+  CK(clear_neighbors(pl, s, st));
   s.zero_counts = 1;
   if (block_pair) return launch_score<Real, false, true>(pl, s, st);
   return launch_score<Real, false, false>(pl, s, st);
@@ -1611,6 +1650,24 @@ __global__ void __launch_bounds__(1024) spec_match_kernel(const Real* a, const R
   if (threadIdx.x == 0) *flag = differ ? 0 : 1;
 }
 
+// Has a backward's weights compared with those its speculative forward used:
+// by every block of the sphere pass (a launch less; a minimiser's call is a
+// few launches long), or, above 2048 values (500 poses), where those reads
+// would cost more than a launch, by a kernel of its own.
+template <typename Real>
+cudaError_t spec_compare(tmol_b200_ljlk_plan* pl, ScoreArgs<Real>& s, const void* dTdV, int n, cudaStream_t st) {
+  s.done = pl->spec_flag;
+  if (n > 2048) {
+    spec_match_kernel<Real><<<1, 1024, 0, st>>>((const Real*)dTdV, (const Real*)pl->spec_used, n, pl->spec_flag);
+    return cudaGetLastError();
+  }
+  s.spec_from = (const Real*)dTdV;
+  s.spec_to = (Real*)pl->spec_used;
+  s.spec_n = n;
+  s.spec_flag = pl->spec_flag;
+  return cudaSuccess;
+}
+
 // dst[0, n) = src[0, n) when *flag is set.
 template <typename Real>
 __global__ void spec_copy_kernel(const int* flag, const Real* src, Real* dst, int64_t n) {
@@ -1628,14 +1685,15 @@ int forward_speculative_impl(tmol_b200_ljlk_plan* pl, const void* coords, void* 
   pl->spec_taken = false;
   if (!pl->spec_ready) return forward_impl<Real>(pl, coords, 0, energies, nbr, st);
   pl->spec_taken = true;
-  const size_t w_bytes = (size_t)n_terms(pl->term) * pl->P * sizeof(Real);
-  if (w_bytes) CK(cudaMemcpyAsync(pl->spec_used, pl->spec_next, w_bytes, cudaMemcpyDeviceToDevice, st));
   ScoreArgs<Real> s = score_args<Real>(pl, coords);
+  s.spec_from = (const Real*)pl->spec_next;
+  s.spec_to = (Real*)pl->spec_used;
+  s.spec_n = n_terms(pl->term) * pl->P;
   s.energies = (Real*)energies;
   s.nbr = nbr;
   s.dTdV = (const Real*)pl->spec_used;
   s.g4 = (Real*)pl->spec_g;
-  if (nbr) CK(cudaMemsetAsync(nbr, 0, (size_t)pl->P * pl->B * pl->B * sizeof(int32_t), st));
+  CK(clear_neighbors(pl, s, st));
   // energies, the kept gradient and the counters: by the sphere pass
   s.zero_energies = (int64_t)n_terms(pl->term) * pl->P;
   s.zero_counts = 1;
@@ -1652,22 +1710,19 @@ template <typename Real>
 int backward_speculative_impl(tmol_b200_ljlk_plan* pl, const void* coords, const void* dTdV, void* dcoords,
                               int speculated, cudaStream_t st) {
   const int n_w = n_terms(pl->term) * pl->P;
-  if (speculated && pl->spec_taken && n_w > 0) {
-    spec_match_kernel<Real><<<1, 1024, 0, st>>>((const Real*)dTdV, (const Real*)pl->spec_used, n_w, pl->spec_flag);
-    CK(cudaGetLastError());
-  } else {
-    CK(cudaMemsetAsync(pl->spec_flag, 0, sizeof(int), st));
-  }
   ScoreArgs<Real> s = score_args<Real>(pl, coords);
   s.dTdV = (const Real*)dTdV;
   s.counts = nullptr;
-  s.done = pl->spec_flag;
+  const int* hit = nullptr;
+  if (speculated && pl->spec_taken && n_w > 0) {
+    CK(spec_compare(pl, s, dTdV, n_w, st));
+    hit = pl->spec_flag;
+  }
   int rc = launch_score<Real, true, false>(pl, s, st);
   if (rc != TMOL_B200_OK) return rc;
   // a hit takes the kept gradient, a miss the one just recomputed
-  rc = grad_out<Real>(pl, pl->spec_flag, pl->spec_g, dcoords, st);
+  rc = grad_out<Real>(pl, hit, pl->spec_g, dcoords, st, dTdV, pl->spec_next, n_w);
   if (rc != TMOL_B200_OK) return rc;
-  if (n_w > 0) CK(cudaMemcpyAsync(pl->spec_next, dTdV, (size_t)n_w * sizeof(Real), cudaMemcpyDeviceToDevice, st));
   pl->spec_ready = true;
   return TMOL_B200_OK;
 }
@@ -1830,9 +1885,15 @@ int lkb_waters_backward_impl(tmol_b200_ljlk_plan* pl, const void* coords, const 
 
 template <typename Real, bool GRAD, bool BLOCK_PAIR>
 int lkb_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const void* waters, void* energies, int32_t* nbr,
-                   const void* dTdV, void* g4, void* dwaters, cudaStream_t st, const int* done = nullptr) {
+                   const void* dTdV, void* g4, void* dwaters, cudaStream_t st, bool spec_forward = false,
+                   bool spec_backward = false) {
   ScoreArgs<Real> s = score_args<Real>(pl, coords);
-  s.done = done;
+  if (spec_forward) {
+    s.spec_from = (const Real*)pl->spec_next;
+    s.spec_to = (Real*)pl->spec_used;
+    s.spec_n = 4 * pl->P;
+  }
+  if (spec_backward) CK(spec_compare(pl, s, dTdV, 4 * pl->P, st));
   LkbArgs<Real> k = lkb_args<Real>(pl);
   k.water_dist = ((const Real*)pl->global_params)[3];  // the score op's own copy
   k.waters = (const Real*)waters;
@@ -1845,7 +1906,7 @@ int lkb_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const void* wate
   // block-pair energies and weights are addressed by an int block-pair index
   if (BLOCK_PAIR && PBB >= ((size_t)1 << 31)) return TMOL_B200_ERR_CAPACITY;
   if (energies && BLOCK_PAIR) CK(cudaMemsetAsync(energies, 0, PBB * 4 * sizeof(Real), st));
-  if (nbr) CK(cudaMemsetAsync(nbr, 0, PBB * sizeof(int32_t), st));
+  CK(clear_neighbors(pl, s, st));
   // the whole-pose energies, the gradients, the counters and the work
   // ticket: by the sphere pass (which a taken speculative gradient skips:
   // its outputs are then copied whole)
@@ -1888,10 +1949,8 @@ int lkb_forward_speculative_impl(tmol_b200_ljlk_plan* pl, const void* coords, co
   if (!pl->spec_ready)
     return lkb_score_impl<Real, false, false>(pl, coords, waters, energies, nbr, nullptr, nullptr, nullptr, st);
   pl->spec_taken = true;
-  const size_t w_bytes = (size_t)4 * pl->P * sizeof(Real);
-  if (w_bytes) CK(cudaMemcpyAsync(pl->spec_used, pl->spec_next, w_bytes, cudaMemcpyDeviceToDevice, st));
   return lkb_score_impl<Real, true, false>(pl, coords, waters, energies, nbr, pl->spec_used, pl->spec_g,
-                                           pl->spec_dw, st);
+                                           pl->spec_dw, st, true);
 }
 
 template <typename Real>
@@ -1899,25 +1958,21 @@ int lkb_backward_speculative_impl(tmol_b200_ljlk_plan* pl, const void* coords, c
                                   const void* dTdV, void* dcoords, void* dwaters, int speculated,
                                   cudaStream_t st) {
   const int n_w = 4 * pl->P;
-  if (speculated && pl->spec_taken && n_w > 0) {
-    spec_match_kernel<Real><<<1, 1024, 0, st>>>((const Real*)dTdV, (const Real*)pl->spec_used, n_w, pl->spec_flag);
-    CK(cudaGetLastError());
-  } else {
-    CK(cudaMemsetAsync(pl->spec_flag, 0, sizeof(int), st));
-  }
-  // zeroes the outputs; its scoring launch does no work when the flag is set
+  // when the weights are equal the launches do no work and the kept gradients
+  // are copied out
+  const bool compare = speculated && pl->spec_taken && n_w > 0;
+  const int* hit = compare ? pl->spec_flag : nullptr;
   int rc = lkb_score_impl<Real, true, false>(pl, coords, waters, nullptr, nullptr, dTdV, pl->g4, dwaters, st,
-                                             pl->spec_flag);
+                                             false, compare);
   if (rc != TMOL_B200_OK) return rc;
-  rc = grad_out<Real>(pl, pl->spec_flag, pl->spec_g, dcoords, st);
+  rc = grad_out<Real>(pl, hit, pl->spec_g, dcoords, st, dTdV, pl->spec_next, n_w);
   if (rc != TMOL_B200_OK) return rc;
   const int64_t n_dw = (int64_t)pl->N * LKB_NW * 3;
-  if (n_dw > 0) {
+  if (hit && n_dw > 0) {
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n_dw + 255) / 256, (int64_t)pl->n_sm * 8));
-    spec_copy_kernel<Real><<<grid, 256, 0, st>>>(pl->spec_flag, (const Real*)pl->spec_dw, (Real*)dwaters, n_dw);
+    spec_copy_kernel<Real><<<grid, 256, 0, st>>>(hit, (const Real*)pl->spec_dw, (Real*)dwaters, n_dw);
     CK(cudaGetLastError());
   }
-  if (n_w > 0) CK(cudaMemcpyAsync(pl->spec_next, dTdV, (size_t)n_w * sizeof(Real), cudaMemcpyDeviceToDevice, st));
   pl->spec_ready = true;
   return TMOL_B200_OK;
 }

@@ -346,8 +346,17 @@ def check(func, status):
 
 
 def call(name, *args):
-    lib = load()
-    check(name, getattr(lib, name)(*args))
+    status = getattr(_lib or load(), name)(*args)
+    if status != 0:
+        check(name, status)
+
+
+def raw_stream(device):
+    """The current CUDA stream of ``device`` as an address, without building
+    torch's stream object for it (2 us of a small call's 200)."""
+    import torch
+
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 def measure_fp32_peak_tflops(stream_handle=0):

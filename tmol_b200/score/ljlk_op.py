@@ -243,7 +243,7 @@ class LJLKPlan:
         return native.load().tmol_b200_ljlk_plan_device_bytes(self.ptr)
 
     def _stream(self):
-        return ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return ctypes.c_void_p(native.raw_stream(self.device))
 
     def _check_coords(self, coords):
         if coords.device != self.device or coords.dtype != self.dtype:
@@ -531,13 +531,10 @@ _PLAN_CACHE_SIZE = 8
 
 
 def _plan_key(coords, static):
-    parts = [coords.device, coords.dtype]
-    for t in static:
-        if isinstance(t, torch.Tensor):
-            parts.append((t.data_ptr(), tuple(t.shape), t.dtype, t._version))
-        else:
-            parts.append(t)
-    return tuple(parts)
+    tensor = torch.Tensor
+    return (coords.device, coords.dtype) + tuple(
+        [(t.data_ptr(), t.shape, t.dtype, t._version) if isinstance(t, tensor) else t for t in static]
+    )
 
 
 def get_plan(coords, static, rotamers=False, plan_class=None):
