@@ -1,8 +1,8 @@
 """The atom-pair engine at the sizes where its groups can go wrong: one-atom
 rows to several groups per block, a group with more pairs than the queue
 holds (a pose squeezed until nearly every pair is in reach), block pairs and
-rotamer pairs of such poses, and type parameters without a common fade
-interval (no far class).
+rotamer pairs of such poses, type parameters without a common fade interval
+(no far class), and the LK-ball walk over such poses.
 
 float64 energies and gradients against the oracle.  A gradient component is
 a sum of at most a few thousand signed terms, each no larger than the largest
@@ -93,3 +93,26 @@ def test_no_common_fade_interval():
     Eo, _, _ = O.OracleCall(x, args, f64=True).pose_scores()
     close(E, Eo, 1e-11)
     clear_plan_cache()
+
+
+@pytest.mark.parametrize("scale", [1.0, 0.6])
+@pytest.mark.parametrize("block_pair", [False, True])
+def test_lkball_lists(block_pair, scale):
+    """The LK-ball walk over the neighbours' heavy atoms: lists of less than
+    one and of many windows of 32 atoms, windows that begin inside a
+    neighbour, and (poses drawn together) rows that meet every one of them.
+    Energies and gradient as in the docstring above, with three more digits
+    for the waters' frames and the ramps' quotients between."""
+    from tests.test_gpu_lkball import gpu_run
+    from tests.test_lkball_oracle import oracle_run
+    from tmol_b200.score.lkball_energy_term import LKBallEnergyTerm
+
+    ps = synthetic_pose_stack([30, 1, 2, 9, 75], [5, 6, 7, 8, 9], spacing=0.0)
+    ps.coords = ps.coords * scale
+    _, E, dx, nbr = gpu_run(ps, LKBallEnergyTerm(), torch.float64, block_pair)
+    _, Eo, dxo, nbro = oracle_run(ps, True)
+    if block_pair:
+        E = E.sum((2, 3))
+    close(E, numpy.asarray(Eo).reshape(E.shape), 1e-9)
+    assert numpy.array_equal(nbr.cpu().numpy(), nbro)
+    close(dx, dxo, 1e-9)

@@ -306,6 +306,13 @@ __global__ void plan_heavy_count_kernel(const uint16_t* bt_tf, const int* bt_n_a
   }
 }
 
+// LK-ball: where each block's (rotamer's) heavy atoms go, *total of them.
+__global__ void plan_heavy_bases_kernel(const int* bt_of, const int* nocc, int n, unsigned long long* total,
+                                        int* base) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    base[i] = bt_of[i] < 0 ? 0 : (int)atomicAdd(total, (unsigned long long)nocc[bt_of[i]]);
+}
+
 __global__ void plan_real_atoms_kernel(const int* bt_of, const int* off_of, int n, const int* bt_n_atoms,
                                        uint8_t* real) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -578,6 +585,15 @@ struct ScoreArgs {
   const Real* dTdV;
   int* ticket;
   unsigned long long* counts;
+  // LK-ball: the heavy atoms of every block (or rotamer) as records (flags:
+  // atom | polar with waters << 16 | bridges << 17), from hbase[i] on, written
+  // by the sphere pass from each block type's list hmeta [nbt][maxocc]
+  AtomRec<Real>* hpacked;
+  const int* hbase;
+  const int* hmeta;
+  const int* nocc;
+  int maxocc;
+  const Real* waters;
   // optional skip mask: bit b2 of row (p, b1) set = do not score the block
   // pair (never honoured for b1 == b2 or count-pair partners)
   const uint32_t* skip;
@@ -649,6 +665,8 @@ __device__ __forceinline__ void warp_sphere(const Real* coords, const int* bt_n_
 
 template <typename Real>
 __device__ __forceinline__ void pack_block(const ScoreArgs<Real>& s, int bt, int off, int lane);
+template <typename Real>
+__device__ __forceinline__ void pack_heavy(const ScoreArgs<Real>& s, int bt, int off, int hb, int lane);
 
 template <typename Real>
 __global__ void spheres_kernel(ScoreArgs<Real> s) {
@@ -680,6 +698,7 @@ __global__ void spheres_kernel(ScoreArgs<Real> s) {
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n_blocks; i += warps) {
     warp_sphere(s.coords, s.bt_n_atoms, s.blk_bt[i], s.blk_off[i], lane, s.spheres + 4 * (int64_t)i);
     if (s.packed) pack_block(s, s.blk_bt[i], s.blk_off[i], lane);
+    if (s.hpacked) pack_heavy(s, s.blk_bt[i], s.blk_off[i], s.hbase[i], lane);
   }
 }
 
@@ -708,6 +727,24 @@ __device__ __forceinline__ void pack_block(const ScoreArgs<Real>& s, int bt, int
       g[0] = Quad<Real>{0, 0, 0, 0};
       g[1] = Quad<Real>{0, 0, 0, 0};
     }
+  }
+}
+
+// LK-ball: block (bt, off)'s heavy atoms as records from hb on.  A polar atom
+// without a first water (a NaN) takes no part as one.
+template <typename Real>
+__device__ __forceinline__ void pack_heavy(const ScoreArgs<Real>& s, int bt, int off, int hb, int lane) {
+  if (bt < 0) return;
+  for (int k = lane; k < s.nocc[bt]; k += 32) {
+    int meta = s.hmeta[(int64_t)bt * s.maxocc + k];
+    const int64_t row = (int64_t)off + (meta & 0xffff);
+    if ((meta & (1 << 16)) && isnan(s.waters[row * 12])) meta &= ~(1 << 16);
+    AtomRec<Real> a;
+    a.x = s.coords[3 * row];
+    a.y = s.coords[3 * row + 1];
+    a.z = s.coords[3 * row + 2];
+    a.tf = meta;
+    s.hpacked[(int64_t)hb + k] = a;
   }
 }
 
@@ -743,6 +780,7 @@ __global__ void rot_spheres_kernel(ScoreArgs<Real> s, RotArgs ra, Real* rs) {
   for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < ra.R; r += warps) {
     warp_sphere(s.coords, s.bt_n_atoms, ra.rot_bt[r], ra.rot_off[r], lane, rs + 4 * (int64_t)r);
     if (s.packed) pack_block(s, ra.rot_bt[r], ra.rot_off[r], lane);
+    if (s.hpacked) pack_heavy(s, ra.rot_bt[r], ra.rot_off[r], s.hbase[r], lane);
   }
 }
 
@@ -1249,6 +1287,9 @@ struct tmol_b200_ljlk_plan {
   int* lkb_nbocc = nullptr;
   int lkb_maxpol = 0, lkb_maxocc = 0;
   void* lkb_par = nullptr;
+  void* hpacked = nullptr;  // heavy atoms as records
+  int* hbase = nullptr;     // [P*B] (rotamer plans: [R])
+  int* hmeta = nullptr;     // [nbt][lkb_maxocc]
   double lkb_water_dist = 0;
   int* lkb_active = nullptr;    // occupied water sites, ascending
   int64_t lkb_n_active = 0;
@@ -1367,6 +1408,7 @@ void free_plan(tmol_b200_ljlk_plan* pl) {
                   pl->rot_off,   pl->rot_block,  pl->rot_pose,    pl->nrb,
                   pl->rob,       pl->rot_spheres, pl->row_pairs,  pl->row_items,
                   pl->bt_q,      pl->elec_k,      pl->lkb_sites,   pl->lkb_pol,
+                  pl->hpacked,   pl->hbase,       pl->hmeta,
                   pl->lkb_npol,  pl->lkb_occ,     pl->lkb_nocc,    pl->lkb_par,
                   pl->lkb_waters, pl->lkb_dwaters, pl->lkb_nbocc, pl->lkb_active,
                   pl->blk_info,  pl->packed,      pl->g4,          pl->real_atom,  pl->imask,
@@ -1845,6 +1887,7 @@ LkbArgs<Real> lkb_args(tmol_b200_ljlk_plan* pl) {
   k.maxpol = pl->lkb_maxpol;
   k.maxocc = pl->lkb_maxocc;
   k.par = (const Real*)pl->lkb_par;
+  k.hbase = pl->hbase;
   const Real* gp = (const Real*)pl->global_params;
   k.hbond_dis = gp[0];
   k.hbond_oh = gp[1];
@@ -1883,6 +1926,17 @@ int lkb_waters_backward_impl(tmol_b200_ljlk_plan* pl, const void* coords, const 
   return TMOL_B200_OK;
 }
 
+// What the sphere pass needs to write the heavy atoms' records.
+template <typename Real>
+void heavy_args(const tmol_b200_ljlk_plan* pl, ScoreArgs<Real>& s, const void* waters) {
+  s.hpacked = (AtomRec<Real>*)pl->hpacked;
+  s.hbase = pl->hbase;
+  s.hmeta = pl->hmeta;
+  s.nocc = pl->lkb_nocc;
+  s.maxocc = pl->lkb_maxocc;
+  s.waters = (const Real*)waters;
+}
+
 template <typename Real, bool GRAD, bool BLOCK_PAIR>
 int lkb_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const void* waters, void* energies, int32_t* nbr,
                    const void* dTdV, void* g4, void* dwaters, cudaStream_t st, bool spec_forward = false,
@@ -1902,6 +1956,7 @@ int lkb_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const void* wate
   s.nbr = nbr;
   s.dTdV = (const Real*)dTdV;
   s.g4 = (Real*)g4;  // the padded gradient, or null (zeroed by the sphere pass)
+  heavy_args(pl, s, waters);
   const size_t PBB = (size_t)pl->P * pl->B * pl->B;
   // block-pair energies and weights are addressed by an int block-pair index
   if (BLOCK_PAIR && PBB >= ((size_t)1 << 31)) return TMOL_B200_ERR_CAPACITY;
@@ -1993,6 +2048,7 @@ int lkb_rotamer_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const vo
   s.energies = (Real*)energies;
   s.dTdV = (const Real*)dTdV;
   if (!GRAD) s.g4 = nullptr;
+  heavy_args(pl, s, waters);
   s.nbr = nullptr;
   s.counts = pl->counts;
   CK(cudaMemsetAsync(pl->counts, 0, N_COUNTS * sizeof(unsigned long long), st));
@@ -2127,6 +2183,33 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
     CK(cudaMemcpyAsync(pl->lkb_npol, hnpol.data(), sizeof(int) * hnpol.size(), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(pl->lkb_nocc, hnocc.data(), sizeof(int) * hnocc.size(), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(pl->lkb_par, par.data(), sizeof(Real) * par.size(), cudaMemcpyHostToDevice, st));
+  }
+  if (scoring) {
+    // every block's (rotamer's) heavy atoms: which of its atoms they are, and
+    // where their records go
+    std::vector<int> hmeta((size_t)std::max(nbt, 1) * maxocc, 0);
+    for (int bt = 0; bt < nbt; ++bt)
+      for (size_t y = 0; y < occ[bt].size(); ++y) {
+        const int a = occ[bt][y];
+        if (a >= (1 << 16)) return TMOL_B200_ERR_SHAPE;
+        const bool polar = std::find(pol[bt].begin(), pol[bt].end(), a) != pol[bt].end();
+        hmeta[(size_t)bt * maxocc + y] = a | (polar ? 1 << 16 : 0) | ((int)y < hnbocc[bt] ? 1 << 17 : 0);
+      }
+    CK(dalloc(pl, &pl->hmeta, hmeta.size()));
+    CK(cudaMemcpyAsync(pl->hmeta, hmeta.data(), sizeof(int) * hmeta.size(), cudaMemcpyHostToDevice, st));
+    const int n = pl->rotamers ? pl->R : pl->P * pl->B;
+    CK(dalloc(pl, &pl->hbase, n));
+    unsigned long long n_heavy = 0;
+    if (n > 0) {
+      CK(cudaMemsetAsync(pl->counts, 0, sizeof(unsigned long long), st));
+      plan_heavy_bases_kernel<<<std::max(1, std::min((n + 255) / 256, pl->n_sm * 8)), 256, 0, st>>>(
+          pl->rotamers ? pl->rot_bt : pl->blk_bt, pl->lkb_nocc, n, pl->counts, pl->hbase);
+      CK(cudaGetLastError());
+      CK(cudaMemcpyAsync(&n_heavy, pl->counts, sizeof(n_heavy), cudaMemcpyDeviceToHost, st));
+    }
+    CK(cudaStreamSynchronize(st));
+    if (n_heavy >= (1ull << 31)) return TMOL_B200_ERR_SHAPE;  // record indices are int
+    CK(dalloc(pl, (AtomRec<Real>**)&pl->hpacked, (size_t)n_heavy));
   }
   if (scoring && !pl->rotamers) {
     // the score op's speculative gradient (lkb_backward_speculative)
@@ -2349,13 +2432,13 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     PCK(dalloc(pl, &pl->real_atom, n_at));
     PCK(cudaMemsetAsync(pl->real_atom, 0, n_at, st));
   }
-  if (term != kTermLKBall) {
+  if (scoring) {
     pl->n_iwords = (A + 31) / 32;
     PCK(dalloc(pl, &pl->imask, (size_t)nbt * A * pl->n_iwords));
     PCK(dalloc(pl, &pl->bt_n_heavy, nbt));
   }
+  if (!rotamers && scoring) PCK(dalloc(pl, &pl->blk_info, PB));
   if (!rotamers && term != kTermLKBall) {
-    PCK(dalloc(pl, &pl->blk_info, PB));
     PCK(dalloc(pl, (unsigned char**)&pl->spec_next, (size_t)n_terms(term) * std::max(P, 1) * real_bytes));
     PCK(dalloc(pl, (unsigned char**)&pl->spec_used, (size_t)n_terms(term) * std::max(P, 1) * real_bytes));
     PCK(dalloc(pl, (unsigned char**)&pl->spec_g, (size_t)std::max<int64_t>(in->n_atoms, 1) * GRAD_STRIDE * real_bytes));
@@ -2536,7 +2619,7 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     int gb = std::max(1, std::min(((nbt * A) + 255) / 256, pl->n_sm * 8));
     plan_block_types_kernel<<<gb, 256, 0, st>>>(a, pl->type_map, pl->bt_tf);
     PCK(cudaGetLastError());
-    if (term != kTermLKBall) {
+    {
       const int64_t n_im = (int64_t)nbt * A * pl->n_iwords;
       const int gi = (int)std::max<int64_t>(1, std::min<int64_t>((n_im + 255) / 256, (int64_t)pl->n_sm * 8));
       plan_intra_masks_kernel<<<gi, 256, 0, st>>>(pl->bt_pd, pl->bt_n_atoms, nbt, A, pl->n_iwords, pl->imask);

@@ -44,6 +44,7 @@ struct LkbArgs {
   const int* nocc;
   const int* nbocc;     // [nbt] leading occluders that are donors or acceptors (the bridge term)
   int maxpol, maxocc;
+  const int* hbase;     // [P*B] (rotamer plans: [R]) first heavy record of each block (rotamer)
   const Real* par;      // [nbt][A][12], 9 used
   Real water_dist, hbond_dis, hbond_oh, hbond_h, max_dis;
 };
@@ -878,123 +879,191 @@ __device__ __forceinline__ void lkb_pump(const LkbEval<Real>& ev, LkbWarp<Real, 
   }
 }
 
-// One side of a pair of blocks (or rotamers): block type, first coordinate
-// row, polar / occluder counts.
-struct LkbSide {
-  int bt, off, npol, nocc, nbr;
+// The rows of a walk: a block (or rotamer), its heavy records and atoms.
+struct LkbRows {
+  int bt, off, hb, nocc, npol, n_atoms;
 };
 
-template <typename Real>
-__device__ __forceinline__ LkbSide lkb_side(const LkbArgs<Real>& k, int bt, int off) {
-  return LkbSide{bt, off, k.npol[bt], k.nocc[bt], k.nbocc[bt]};
-}
+// One neighbour (a block or rotamer) as a lane sees it.
+struct LkbHit {
+  bool hit;
+  int entry;        // its count-pair table entry; -1: the rows themselves; -2: bond separations do not matter
+  int bt, off, hb;  // block type, first coordinate row, first heavy record
+  int tag;          // output row (tagged queues)
+};
 
-// Every polar / occluder pair of sides 1 and 2 (intra: ordered pairs of
-// distinct atoms of side 1; else both directions): filtered on bond
-// separation (intra: the block type's path distances; inter: through the
-// connections when `striking`), distance and the polar atom's waters, and
-// queued; full queues are evaluated under w into e4.
-template <typename Real, bool GRAD, bool TAGGED, bool COUNT = true>
-__device__ __forceinline__ void lkb_enqueue_pairs(const ScoreArgs<Real>& s, const LkbArgs<Real>& k,
-                                                  const LkbEval<Real>& ev, LkbWarp<Real, TAGGED>& q, const LkbSide& a,
-                                                  const LkbSide& b, bool intra, bool striking, int nc1, int nc2,
-                                                  const uint8_t* seps, const Lkb4<Real> w, Real* e4, int tag,
-                                                  const LkbTagged<Real> tg) {
+// Heavy atoms of a list of neighbours, a few dozen at a time, and where the
+// current 32 neighbours' atoms come from.
+constexpr int LKB_LIST = 64;
+template <typename Real, bool TAGGED>
+struct LkbList {
+  Real x[LKB_LIST], y[LKB_LIST], z[LKB_LIST];
+  int tf[LKB_LIST];  // atom | polar with waters << 16 | bridges << 17
+  int row[LKB_LIST], par[LKB_LIST], entry[LKB_LIST];
+  int tag[TAGGED ? LKB_LIST : 1];
+  int hoff[32], off[32], bt[32], ent[32], htag[TAGGED ? 32 : 1];
+};
+
+// Queues every polar / occluder pair between the rows and the n_cand
+// neighbours that `next(first)` yields 32 at a time (each lane one), and
+// evaluates full queues under w into e4.  The neighbours' heavy atoms are one
+// flat list: each is loaded once with its flags (polar with waters, bridges)
+// and culled against the rows' sphere (centre c, reach2 the squared reach),
+// and every row meets 32 of them at a time, in both directions.  Pairs of the
+// rows' own block and of count-pair partners have their exclusions from the
+// plan's masks, a rotamer's partners (PMASK false) their bond separations.
+// What bounds it: latency and issue of the evaluation (49% of the issue slots
+// used).  Pairs enumerated one by one, with index arithmetic and eight loads
+// each, were half of the kernel's instructions: 64 x 150 residues, energies +
+// gradients, 196 -> 164 us; rotamers of 8 x 100 residues 2.55 -> 2.12 ms.
+template <typename Real, bool GRAD, bool TAGGED, bool COUNT, bool PMASK, typename Next>
+__device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs<Real>& k, const LkbEval<Real>& ev,
+                                         LkbWarp<Real, TAGGED>& q, LkbList<Real, TAGGED>& L, const LkbRows& a,
+                                         Real cx, Real cy, Real cz, Real reach2, int n_cand, Next next,
+                                         const Lkb4<Real> w, Real* e4, const LkbTagged<Real> tg) {
   const int lane = q.lane;
-  const int no = intra ? a.nocc : b.nocc;
-  const int n01 = a.npol * no;
-  const int total = intra ? n01 : n01 + a.nocc * b.npol;
-  // idx / no in float: exact for these sizes (idx < 2^16, no <= 256: the
-  // error is far below 0.5 / no)
-  const float inv_no = no > 0 ? 1.0f / float(no) : 0.0f;
-  const float inv_nocc1 = a.nocc > 0 ? 1.0f / float(a.nocc) : 0.0f;
-  if (COUNT) {
-    q.n_bp += 1;
-    q.n_pairs += total;
-  }
-  for (int base = 0; base < total; base += 32) {
-    const int idx = base + lane;
-    bool in_reach = false, bridged = false;
-    int rp = 0, ro = 0, pidx = 0, oidx = 0, sep = 0;
-    if (idx < total) {
-      int ap, ao, btp, bto, offp, offo, y;
-      if (idx < n01) {
-        const int x = (int)((float(idx) + 0.5f) * inv_no);
-        y = idx - x * no;
-        btp = a.bt;
-        bto = intra ? a.bt : b.bt;
-        ap = k.pol[(int64_t)btp * k.maxpol + x];
-        ao = k.occ[(int64_t)bto * k.maxocc + y];
-        offp = a.off;
-        offo = intra ? a.off : b.off;
-        if (intra)
-          sep = ap == ao ? 0 : s.bt_pd[((int64_t)a.bt * s.A + ap) * s.A + ao];
-        else
-          sep = striking ? lkb_inter_sep(s, a.bt, b.bt, nc1, nc2, seps, ap, ao) : 6;
-        bridged = y < (intra ? a.nbr : b.nbr);
-      } else {
-        const int j = idx - n01;
-        const int x = (int)((float(j) + 0.5f) * inv_nocc1);
-        y = j - x * a.nocc;
-        btp = b.bt;
-        bto = a.bt;
-        ap = k.pol[(int64_t)btp * k.maxpol + x];
-        ao = k.occ[(int64_t)bto * k.maxocc + y];
-        offp = b.off;
-        offo = a.off;
-        sep = striking ? lkb_inter_sep(s, a.bt, b.bt, nc1, nc2, seps, ao, ap) : 6;
-        bridged = y < a.nbr;
-      }
-      if (sep > 3) {
-        rp = offp + ap;
-        ro = offo + ao;
-        const AtomRec<Real> ai = s.packed[rp], aj = s.packed[ro];
-        const Real dv[3] = {ai.x - aj.x, ai.y - aj.y, ai.z - aj.z};
-        const Real dist = lkb_sqrt(lkb_dot(dv, dv));
-        in_reach = dist < k.max_dis && !isnan(k.waters[(int64_t)rp * LKB_NW * 3]);
-        pidx = btp * s.A + ap;
-        oidx = bto * s.A + ao;
-      }
-    }
-    const unsigned m1 = __ballot_sync(0xffffffffu, in_reach && bridged);
-    const unsigned m0 = __ballot_sync(0xffffffffu, in_reach && !bridged);
-    if (in_reach) {
-      const int which = bridged ? 1 : 0;
-      LkbQueue<TAGGED>& Q = q.qs[which];
-      const int pos = (bridged ? q.nq[1] : q.nq[0]) + __popc((bridged ? m1 : m0) & q.lt_mask);
-      Q.rp[pos] = rp;
-      Q.ro[pos] = ro;
-      Q.pi[pos] = pidx;
-      Q.oi[pos] = oidx;
-      Q.sep[pos] = (uint8_t)(sep > 255 ? 255 : sep);
-      if (TAGGED) Q.tag[pos] = tag;
-    }
-    q.nq[0] += __popc(m0);
-    q.nq[1] += __popc(m1);
+  const unsigned lemask = q.lt_mask | (1u << lane);
+  const int nc1 = PMASK ? 0 : s.bt_n_conn[a.bt];
+  int m = 0;  // atoms in the list
+  for (int c0 = 0; c0 < n_cand; c0 += 32) {
+    const LkbHit h = next(c0);
     if (COUNT) {
-      q.n_eval += __popc(m0 | m1);
-      q.n_bridge += __popc(m1);
+      q.n_bp += __popc(__ballot_sync(0xffffffffu, h.hit));
+      const int pairs = !h.hit ? 0 : h.entry == -1 ? a.npol * a.nocc : a.npol * k.nocc[h.bt] + a.nocc * k.npol[h.bt];
+      q.n_pairs += __reduce_add_sync(0xffffffffu, pairs);
     }
-    lkb_pump<Real, GRAD, TAGGED>(ev, q, false, w, e4, tg);
+    const int n = h.hit ? k.nocc[h.bt] : 0;
+    int inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    const int T = __shfl_sync(0xffffffffu, inc, 31);
+    const int start = n > 0 ? inc - n : 0x7fffffff;
+    const unsigned hm = __ballot_sync(0xffffffffu, n > 0);
+    __syncwarp();
+    if (n > 0) {
+      const int slot = __popc(hm & q.lt_mask);
+      L.hoff[slot] = h.hb - start;
+      L.off[slot] = h.off;
+      L.bt[slot] = h.bt;
+      L.ent[slot] = h.entry;
+      if (TAGGED) L.htag[slot] = h.tag;
+    }
+    __syncwarp();
+    const bool final = c0 + 32 >= n_cand;
+    int owned = 0;
+    for (int k0 = 0; k0 < T || (final && m > 0); k0 += 32) {
+      if (k0 < T) {
+        // 32 atoms of the flat list: bit p of `word` set where a neighbour's
+        // atoms begin at list position k0 + p
+        const unsigned pos = (unsigned)(start - k0);
+        const unsigned word = __reduce_or_sync(0xffffffffu, pos < 32u ? 1u << pos : 0u);
+        const int own = max(owned + __popc(word & lemask) - 1, 0);
+        owned += __popc(word);
+        AtomRec<Real> o;
+        o.x = o.y = o.z = Real(0);
+        o.tf = 0;
+        const bool valid = k0 + lane < T;
+        if (valid) o = s.hpacked[L.hoff[own] + k0 + lane];
+        const Real dx = o.x - cx, dy = o.y - cy, dz = o.z - cz;
+        const bool keep = valid && dx * dx + dy * dy + dz * dz < reach2;
+        const unsigned km = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          const int j = m + __popc(km & q.lt_mask);
+          L.x[j] = o.x;
+          L.y[j] = o.y;
+          L.z[j] = o.z;
+          L.tf[j] = o.tf;
+          L.row[j] = L.off[own] + (o.tf & 0xffff);
+          L.par[j] = L.bt[own] * s.A + (o.tf & 0xffff);
+          L.entry[j] = L.ent[own];
+          if (TAGGED) L.tag[j] = L.htag[own];
+        }
+        m += __popc(km);
+        __syncwarp();
+      }
+      if (m < 32 && !(final && k0 + 32 >= T && m > 0)) continue;
+      // the list's first 32 atoms against every row: the row polar and the
+      // list's atom occluding, then the other way round
+      AtomRec<Real> o;
+      o.x = L.x[lane];
+      o.y = L.y[lane];
+      o.z = L.z[lane];
+      o.tf = L.tf[lane];
+      const int orow = L.row[lane], opar = L.par[lane], entry = L.entry[lane], ja = o.tf & 0xffff;
+      const int otag = TAGGED ? L.tag[lane] : 0;
+      const bool valid = lane < m;
+      int64_t moff = 0;
+      if (PMASK && valid && entry >= 0) moff = (int64_t)s.cp_moff[entry] + (int64_t)(ja >> 5) * a.n_atoms;
+      for (int step = 0; step < 2 * a.nocc; ++step) {
+        const AtomRec<Real> r = s.hpacked[a.hb + (step >> 1)];
+        const bool back = step & 1;
+        const int ra = r.tf & 0xffff;
+        const Real dv[3] = {r.x - o.x, r.y - o.y, r.z - o.z};
+        bool in_reach = valid && lkb_sqrt(lkb_dot(dv, dv)) < k.max_dis && (((back ? o.tf : r.tf) >> 16) & 1);
+        int sep = 6;
+        if (in_reach && entry != -2) {
+          if (PMASK || entry == -1) {
+            const uint2 mk = entry == -1 ? s.imask[((int64_t)a.bt * s.A + ra) * s.n_iwords + (ja >> 5)]
+                                         : s.pmask[moff + ra];
+            sep = (mk.x >> (ja & 31)) & 1u ? 0 : ((mk.y >> (ja & 31)) & 1u ? 4 : 6);
+          } else {
+            const int bt2 = (opar - ja) / s.A;
+            sep = lkb_inter_sep(s, a.bt, bt2, nc1, s.bt_n_conn[bt2], s.cp_seps + (int64_t)entry * 16, ra, ja);
+          }
+          in_reach = sep > 3;
+        }
+        const bool bridged = ((back ? r.tf : o.tf) >> 17) & 1;
+        const unsigned m1 = __ballot_sync(0xffffffffu, in_reach && bridged);
+        const unsigned m0 = __ballot_sync(0xffffffffu, in_reach && !bridged);
+        if (in_reach) {
+          const int rr = a.off + ra, rpar = a.bt * s.A + ra;
+          LkbQueue<TAGGED>& Q = q.qs[bridged ? 1 : 0];
+          const int at = (bridged ? q.nq[1] : q.nq[0]) + __popc((bridged ? m1 : m0) & q.lt_mask);
+          Q.rp[at] = back ? orow : rr;
+          Q.ro[at] = back ? rr : orow;
+          Q.pi[at] = back ? opar : rpar;
+          Q.oi[at] = back ? rpar : opar;
+          Q.sep[at] = (uint8_t)sep;
+          if (TAGGED) Q.tag[at] = otag;
+        }
+        q.nq[0] += __popc(m0);
+        q.nq[1] += __popc(m1);
+        if (COUNT) {
+          q.n_eval += __popc(m0 | m1);
+          q.n_bridge += __popc(m1);
+        }
+        lkb_pump<Real, GRAD, TAGGED>(ev, q, false, w, e4, tg);
+      }
+      // the rest of the list to its front
+      const int rest = m > 32 ? m - 32 : 0;
+      __syncwarp();
+      if (lane < rest) {
+        L.x[lane] = L.x[32 + lane];
+        L.y[lane] = L.y[32 + lane];
+        L.z[lane] = L.z[32 + lane];
+        L.tf[lane] = L.tf[32 + lane];
+        L.row[lane] = L.row[32 + lane];
+        L.par[lane] = L.par[32 + lane];
+        L.entry[lane] = L.entry[32 + lane];
+        if (TAGGED) L.tag[lane] = L.tag[32 + lane];
+      }
+      m = rest;
+      __syncwarp();
+    }
   }
 }
 
-// The count-pair data of block pair (row i1, block b2): whether any atom
-// pair is within 4 bonds and, if so, the connection-to-connection
-// separations.
+// The count-pair table entry of block b2 in row i1 (cp_b2: the row's
+// partners, one per lane), or -2.
 template <typename Real>
-__device__ __forceinline__ bool lkb_striking(const ScoreArgs<Real>& s, int64_t i1, int b2, int cp_b2, int cp_min,
-                                             uint8_t* seps) {
-  const unsigned pm = __ballot_sync(0xffffffffu, cp_b2 == b2);
-  bool striking = false;
-  if (pm) {
-    const int src = __ffs(pm) - 1;
-    striking = __shfl_sync(0xffffffffu, cp_min, src) <= 4;
-    const int64_t e = i1 * CP_CAP + src;
-    if (striking)
-      for (int c = 0; c < 16; ++c) seps[c] = s.cp_seps[e * 16 + c];
-  }
-  return striking;
+__device__ __forceinline__ int lkb_entry(const ScoreArgs<Real>& s, int64_t i1, int ncp, int cp_b2, int b2) {
+  int e = -2;
+  for (int p = 0; p < ncp; ++p)
+    if (__shfl_sync(0xffffffffu, cp_b2, p) == b2) e = (int)(i1 * CP_CAP + p);
+  return e;
 }
 
 template <typename Real>
@@ -1036,6 +1105,7 @@ __global__ void __launch_bounds__(256, TMOL_B200_LKB_MIN_CTAS) lkb_score_kernel(
   // [warp][plain, bridged]; block-pair mode tags queued pairs with their
   // block pair (p * B + b1) * B + b2
   __shared__ LkbQueue<BLOCK_PAIR> queues[LKB_MAX_WARPS][2];
+  __shared__ LkbList<Real, BLOCK_PAIR> lists[LKB_MAX_WARPS];
   LkbWarp<Real, BLOCK_PAIR> q;
   q.lane = threadIdx.x & 31;
   q.qs = queues[threadIdx.x >> 5];
@@ -1068,53 +1138,42 @@ __global__ void __launch_bounds__(256, TMOL_B200_LKB_MIN_CTAS) lkb_score_kernel(
         if (s.item_cost && lane == 0) s.item_cost[item] = 0;
         continue;
       }
-      const Real* sph1 = s.spheres + 4 * (int64_t)i1;
-      const Real c1x = sph1[0], c1y = sph1[1], c1z = sph1[2], rad1 = sph1[3];
-      unsigned my_mask = 0;
-      const int n_batches = (cand1 - cand0 + 31) / 32;
-      for (int bi = 0; bi < n_batches; ++bi) {
-        const int b2 = cand0 + bi * 32 + lane;
-        bool hit = false;
-        if (b2 < cand1) {
-          const int i2 = p * s.B + b2;
-          if (s.blk_bt[i2] >= 0) {
-            const Real* s2 = s.spheres + 4 * (int64_t)i2;
-            const Real dx = sub_rn(c1x, s2[0]), dy = sub_rn(c1y, s2[1]), dz = sub_rn(c1z, s2[2]);
-            const Real d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
-            const Real thr = add_rn(add_rn(rad1, s2[3]), s.reach);
-            hit = d2 < mul_rn(thr, thr);
-          }
-          if (s.nbr) s.nbr[(int64_t)i1 * s.B + b2] = hit ? 1 : 0;
-        }
-        const unsigned mk = __ballot_sync(0xffffffffu, hit);
-        if (lane == bi) my_mask = mk;
-      }
+      const Quad<Real> sph1 = reinterpret_cast<const Quad<Real>*>(s.spheres)[i1];
       // the row's count-pair partners, one per lane
       const int ncp = s.cp_count[i1];
-      const int cp_b2 = lane < ncp ? s.cp_b2[i1 * CP_CAP + lane] : -1;
-      const int cp_min = lane < ncp ? s.cp_minsep[i1 * CP_CAP + lane] : 6;
+      const int cp_b2 = lane < ncp ? s.cp_b2[(int64_t)i1 * CP_CAP + lane] : -1;
       Lkb4<Real> w = {{0, 0, 0, 0}};
       if (GRAD && !BLOCK_PAIR)
         for (int c = 0; c < 4; ++c) w.v[c] = s.dTdV[(int64_t)c * s.P + p];
       Real acc[4] = {0, 0, 0, 0};
-      const LkbSide side1 = lkb_side(k, bt1, s.blk_off[i1]);
-      for (int bi = 0; bi < n_batches; ++bi) {
-        unsigned mask = __shfl_sync(0xffffffffu, my_mask, bi);
-        while (mask) {
-          const int kk = __ffs(mask) - 1;
-          mask &= mask - 1;
-          const int b2 = cand0 + bi * 32 + kk;
+      const LkbRows rows = {bt1, s.blk_off[i1], k.hbase[i1], k.nocc[bt1], k.npol[bt1], s.bt_n_atoms[bt1]};
+      const Real reach1 = sph1.d + k.max_dis;
+      auto next = [&](int first) {
+        const int b2 = cand0 + first + lane;
+        LkbHit h = {false, -2, 0, 0, 0, 0};
+        h.entry = lkb_entry(s, i1, ncp, cp_b2, b2);
+        if (b2 < cand1) {
           const int i2 = p * s.B + b2;
-          const bool intra = b2 == b1;
-          uint8_t seps[16];
-          const bool striking = !intra && lkb_striking(s, i1, b2, cp_b2, cp_min, seps);
-          const LkbSide side2 = lkb_side(k, s.blk_bt[i2], s.blk_off[i2]);
-          const int nc1 = striking ? s.bt_n_conn[bt1] : 0, nc2 = striking ? s.bt_n_conn[side2.bt] : 0;
-          lkb_enqueue_pairs<Real, GRAD, BLOCK_PAIR, COUNT>(s, k, ev, q, side1, side2, intra, striking, nc1, nc2, seps,
-                                                    BLOCK_PAIR ? none : w, acc,
-                                                    BLOCK_PAIR ? (int)((int64_t)i1 * s.B + b2) : 0, tg);
+          const int bt2 = s.blk_bt[i2];
+          if (bt2 >= 0) {
+            const Quad<Real> s2 = reinterpret_cast<const Quad<Real>*>(s.spheres)[i2];
+            const Real dx = sub_rn(sph1.a, s2.a), dy = sub_rn(sph1.b, s2.b), dz = sub_rn(sph1.c, s2.c);
+            const Real d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
+            const Real thr = add_rn(add_rn(sph1.d, s2.d), s.reach);
+            h.hit = d2 < mul_rn(thr, thr);
+            h.bt = bt2;
+            h.off = s.blk_off[i2];
+            h.hb = k.hbase[i2];
+            if (BLOCK_PAIR) h.tag = (int)((int64_t)i1 * s.B + b2);
+            if (b2 == b1) h.entry = -1;
+          }
+          if (s.nbr) s.nbr[(int64_t)i1 * s.B + b2] = h.hit ? 1 : 0;
         }
-      }
+        return h;
+      };
+      lkb_walk<Real, GRAD, BLOCK_PAIR, COUNT, true>(s, k, ev, q, lists[threadIdx.x >> 5], rows, sph1.a, sph1.b,
+                                                    sph1.c, reach1 * reach1 * Real(1.0001), cand1 - cand0, next,
+                                                    BLOCK_PAIR ? none : w, acc, tg);
       if (!BLOCK_PAIR) lkb_pump<Real, GRAD, BLOCK_PAIR>(ev, q, true, w, acc, tg);
       // whole-pose energies (also in the adjoint when asked for: one pass
       // for energy and gradient)
@@ -1145,6 +1204,7 @@ template <typename Real, bool GRAD, bool COUNT>
 __global__ void __launch_bounds__(256, TMOL_B200_LKB_MIN_CTAS)
     lkb_rotamer_kernel(ScoreArgs<Real> s, LkbArgs<Real> k, RotArgs ra, const Real* rot_spheres) {
   __shared__ LkbQueue<true> queues[LKB_MAX_WARPS][2];
+  __shared__ LkbList<Real, true> lists[LKB_MAX_WARPS];
   LkbWarp<Real, true> q;
   q.lane = threadIdx.x & 31;
   q.qs = queues[threadIdx.x >> 5];
@@ -1169,33 +1229,38 @@ __global__ void __launch_bounds__(256, TMOL_B200_LKB_MIN_CTAS)
     const long long pair_first = item.w;
     const int p = ra.rot_pose[rot1], b1 = ra.rot_block[rot1];
     const int64_t i1 = (int64_t)p * s.B + b1;
-    const LkbSide side1 = lkb_side(k, ra.rot_bt[rot1], ra.rot_off[rot1]);
+    const int bt1 = ra.rot_bt[rot1];
+    const LkbRows rows = {bt1, ra.rot_off[rot1], k.hbase[rot1], k.nocc[bt1], k.npol[bt1], s.bt_n_atoms[bt1]};
+    // b2 and its count-pair entry are the same for every rot2 of the item
     const int ncp = s.cp_count[i1];
     const int cp_b2 = lane < ncp ? s.cp_b2[i1 * CP_CAP + lane] : -1;
-    const int cp_min = lane < ncp ? s.cp_minsep[i1 * CP_CAP + lane] : 6;
-    // b2 and its count-pair data are the same for every rot2 of the item
     const int b2 = n_rot2 > 0 ? ra.rot_block[rot2_first] : b1;
-    uint8_t seps[16];
-    const bool striking = b2 != b1 && lkb_striking(s, i1, b2, cp_b2, cp_min, seps);
-    const Real* sp1 = rot_spheres + 4 * (int64_t)rot1;
-    const Real c1x = sp1[0], c1y = sp1[1], c1z = sp1[2], r1 = sp1[3];
-    for (int j = 0; j < n_rot2; ++j) {
-      const int rot2 = rot2_first + j;
-      const bool intra = rot2 == rot1;
-      if (!intra) {
+    const int entry = lkb_entry(s, i1, b2 != b1 ? ncp : 0, cp_b2, b2);
+    const Quad<Real> sp1 = reinterpret_cast<const Quad<Real>*>(rot_spheres)[rot1];
+    const Real reach1 = sp1.d + k.max_dis;
+    auto next = [&](int first) {
+      const int j = first + lane;
+      LkbHit h = {false, entry, 0, 0, 0, 0};
+      if (j < n_rot2) {
+        const int rot2 = rot2_first + j;
+        const bool self = rot2 == rot1;
         // no atom pair of two rotamers whose bounding spheres are farther
-        // apart than max_dis (with a margin far above rounding) is in
-        // reach: their energies are zero
-        const Real* sp2 = rot_spheres + 4 * (int64_t)rot2;
-        const Real dx = c1x - sp2[0], dy = c1y - sp2[1], dz = c1z - sp2[2];
-        const Real thr = r1 + sp2[3] + k.max_dis + Real(0.01);
-        if (dx * dx + dy * dy + dz * dz > thr * thr) continue;
+        // apart than max_dis (with a margin far above rounding) is in reach:
+        // their energies are zero
+        const Quad<Real> q2 = reinterpret_cast<const Quad<Real>*>(rot_spheres)[rot2];
+        const Real dx = sp1.a - q2.a, dy = sp1.b - q2.b, dz = sp1.c - q2.c;
+        const Real thr = sp1.d + q2.d + k.max_dis + Real(0.01);
+        h.hit = self || !(dx * dx + dy * dy + dz * dz > thr * thr);
+        if (self) h.entry = -1;
+        h.bt = ra.rot_bt[rot2];
+        h.off = ra.rot_off[rot2];
+        h.hb = k.hbase[rot2];
+        h.tag = (int)(pair_first + j);
       }
-      const LkbSide side2 = lkb_side(k, ra.rot_bt[rot2], ra.rot_off[rot2]);
-      const int nc1 = striking ? s.bt_n_conn[side1.bt] : 0, nc2 = striking ? s.bt_n_conn[side2.bt] : 0;
-      lkb_enqueue_pairs<Real, GRAD, true, COUNT>(s, k, ev, q, side1, side2, intra, striking, nc1, nc2, seps, none, unused,
-                                          (int)(pair_first + j), tg);
-    }
+      return h;
+    };
+    lkb_walk<Real, GRAD, true, COUNT, false>(s, k, ev, q, lists[threadIdx.x >> 5], rows, sp1.a, sp1.b, sp1.c,
+                                             reach1 * reach1 * Real(1.0001), n_rot2, next, none, unused, tg);
   }
   // entries carry their pair: the queues drain across items, once at the end
   lkb_pump<Real, GRAD, true>(ev, q, true, none, unused, tg);
