@@ -905,15 +905,14 @@ __global__ void __launch_bounds__(1024) scan2_kernel(long long* a, long long* b,
   }
 }
 
-// Writes the dispatch indices (pose, rot1, rot2) in the reference's order
-// (pose, b1, b2, rotamer of b1, rotamer of b2) and the work items, row by
-// row from the scanned offsets.
+// Writes the work items (rot1, first rot2, n rot2, first pair) in the
+// reference's order of their pairs (pose, b1, b2, rotamer of b1, rotamer of
+// b2), row by row from the scanned offsets.
 template <typename Real>
 __global__ void rot_row_fill_kernel(ScoreArgs<Real> s, RotArgs ra) {
   const int lane = threadIdx.x & 31;
   const int n_rows = s.P * s.B;
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  const long long np = ra.n_pairs;
   for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < n_rows; row += warps) {
     if (s.blk_bt[row] < 0) continue;
     const int p = row / s.B, b1 = row - p * s.B;
@@ -936,18 +935,30 @@ __global__ void rot_row_fill_kernel(ScoreArgs<Real> s, RotArgs ra) {
           if (item_off + i < ra.n_items)
             ra.items[item_off + i] = make_int4(o1 + i, diag ? o1 + i : o2, n2, (int)first);
         }
-        const long long cnt = (long long)n1 * n2;
-        for (long long q = lane; q < cnt; q += 32) {
-          const long long d = pair_off + q;
-          if (d >= np) break;
-          const int i = (int)(q / n2), j = (int)(q - (long long)i * n2);
-          ra.indices[d] = p;
-          ra.indices[np + d] = o1 + i;
-          ra.indices[2 * np + d] = diag ? o1 + i : o2 + j;
-        }
-        pair_off += cnt;
+        pair_off += (long long)n1 * n2;
         item_off += n1;
       }
+    }
+  }
+}
+
+// The dispatch indices (pose, rot1, rot2) of every work item's pairs, one warp
+// an item: consecutive pairs, written with no division.  Bound by the stores:
+// 13 M pairs (156 MB) took 220 us inside the row-by-row pass above, whose one
+// warp per row left most of the chip idle.
+__global__ void rot_indices_kernel(RotArgs ra) {
+  const int lane = threadIdx.x & 31;
+  const long long np = ra.n_pairs;
+  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long it = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; it < ra.n_items; it += warps) {
+    const int4 item = ra.items[it];
+    const int p = ra.rot_pose[item.x];
+    for (int j = lane; j < item.z; j += 32) {
+      const long long d = (long long)item.w + j;
+      if (d >= np) break;
+      ra.indices[d] = p;
+      ra.indices[np + d] = item.x;
+      ra.indices[2 * np + d] = item.y + j;
     }
   }
 }
@@ -1832,6 +1843,9 @@ int rotamer_fill_impl(tmol_b200_ljlk_plan* pl, int32_t* indices, int32_t* items,
   if (n_rows == 0 || (pl->n_pairs == 0 && pl->n_items == 0)) return TMOL_B200_OK;
   int gw = std::max(1, std::min((n_rows + 7) / 8, pl->n_sm * 16));
   rot_row_fill_kernel<Real><<<gw, 256, 0, st>>>(s, ra);
+  CK(cudaGetLastError());
+  const int gi = (int)std::max<int64_t>(1, std::min<int64_t>((pl->n_items + 7) / 8, (int64_t)pl->n_sm * 16));
+  rot_indices_kernel<<<gi, 256, 0, st>>>(ra);
   CK(cudaGetLastError());
   return TMOL_B200_OK;
 }
