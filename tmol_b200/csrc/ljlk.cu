@@ -1291,12 +1291,9 @@ struct tmol_b200_ljlk_plan {
   // LK-ball plans: water sites [N * 4], per block type polar / occluder
   // atom lists and per-atom parameters [nbt * A * 9] reals
   void* lkb_sites = nullptr;
-  int* lkb_pol = nullptr;
   int* lkb_npol = nullptr;
-  int* lkb_occ = nullptr;
   int* lkb_nocc = nullptr;
-  int* lkb_nbocc = nullptr;
-  int lkb_maxpol = 0, lkb_maxocc = 0;
+  int lkb_maxocc = 0;
   void* lkb_par = nullptr;
   void* hpacked = nullptr;  // heavy atoms as records
   int* hbase = nullptr;     // [P*B] (rotamer plans: [R])
@@ -1362,6 +1359,8 @@ struct tmol_b200_ljlk_plan {
   unsigned char global_params[5 * sizeof(double)];
   // kernel timing: event pairs around each scoring-kernel launch
   bool profiling = false;
+  std::vector<std::pair<void**, size_t>> to_place;  // buffers asked for and not yet placed
+  std::vector<void*> blocks;                        // the device allocations they lie in
   std::vector<cudaEvent_t> prof_events;
   int prof_n = 0;
   tmol_b200_ljlk_launch launch;
@@ -1394,11 +1393,34 @@ namespace {
     if (e_ != cudaSuccess) return TMOL_B200_ERR_CUDA; \
   } while (0)
 
+// A plan's buffers are asked for with dalloc and placed, all that are asked
+// for since the last time, in one device allocation by dplace: each allocation
+// that needs new pages, or whose end leaves one empty, maps or unmaps them.
+// First call with a new LJ/LK topology, 64 x 150 residues: 4.0 ms with an
+// allocation per buffer (also with blocks of 64 KB to 2 MB), 2.6 ms with one;
+// an LK-ball plan of that size 8.9 and 6.3 ms.
 template <typename T>
-cudaError_t dalloc(tmol_b200_ljlk_plan* pl, T** p, size_t n) {
-  size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
+void dalloc(tmol_b200_ljlk_plan* pl, T** p, size_t n) {
+  const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
   pl->device_bytes += bytes;
-  return cudaMalloc((void**)p, bytes);
+  pl->to_place.push_back({(void**)p, bytes});
+}
+
+cudaError_t dplace(tmol_b200_ljlk_plan* pl) {
+  size_t total = 0;
+  for (const auto& r : pl->to_place) total += (r.second + 255) / 256 * 256;
+  if (total == 0) return cudaSuccess;
+  void* base = nullptr;
+  const cudaError_t e = cudaMalloc(&base, total);
+  if (e != cudaSuccess) return e;
+  pl->blocks.push_back(base);
+  char* at = (char*)base;
+  for (const auto& r : pl->to_place) {
+    *r.first = at;
+    at += (r.second + 255) / 256 * 256;
+  }
+  pl->to_place.clear();
+  return cudaSuccess;
 }
 
 int status_from_bits(int bits) {
@@ -1409,24 +1431,9 @@ int status_from_bits(int bits) {
 }
 
 void free_plan(tmol_b200_ljlk_plan* pl) {
-  void* ptrs[] = {pl->blk_bt,    pl->blk_off,    pl->pose_last,  pl->bt_tf,
-                  pl->type_map,  pl->compact_types, pl->ljtab,   pl->lktab,
-                  pl->bt_pd,     pl->bt_conn_pd, pl->bt_flags,   pl->bt_n_atoms,
-                  pl->bt_n_conn, pl->bt_is_ligand, pl->cp_count, pl->cp_b2,
-                  pl->cp_minsep, pl->cp_seps,    pl->work,       pl->spheres,
-                  pl->item_cost,
-                  pl->counters,  pl->counts,     pl->sub_spheres, pl->rot_bt,
-                  pl->rot_off,   pl->rot_block,  pl->rot_pose,    pl->nrb,
-                  pl->rob,       pl->rot_spheres, pl->row_pairs,  pl->row_items,
-                  pl->bt_q,      pl->elec_k,      pl->lkb_sites,   pl->lkb_pol,
-                  pl->hpacked,   pl->hbase,       pl->hmeta,
-                  pl->lkb_npol,  pl->lkb_occ,     pl->lkb_nocc,    pl->lkb_par,
-                  pl->lkb_waters, pl->lkb_dwaters, pl->lkb_nbocc, pl->lkb_active,
-                  pl->blk_info,  pl->packed,      pl->g4,          pl->real_atom,  pl->imask,
-                  pl->pmask,     pl->cp_moff,     pl->bt_n_heavy, pl->fartab,      pl->spec_next,   pl->spec_used, pl->spec_g,
-                  pl->spec_dw,   pl->spec_flag};
-  for (void* p : ptrs)
-    if (p) cudaFree(p);
+  for (void* p : pl->blocks) cudaFree(p);
+  if (pl->work) cudaFree(pl->work);
+  if (pl->item_cost) cudaFree(pl->item_cost);
   for (cudaEvent_t e : pl->prof_events) cudaEventDestroy(e);
   delete pl;
 }
@@ -1893,13 +1900,8 @@ LkbArgs<Real> lkb_args(tmol_b200_ljlk_plan* pl) {
   k.n_sites = pl->N * LKB_NW;
   k.active = pl->lkb_active;
   k.n_active = pl->lkb_n_active;
-  k.pol = pl->lkb_pol;
   k.npol = pl->lkb_npol;
-  k.occ = pl->lkb_occ;
   k.nocc = pl->lkb_nocc;
-  k.nbocc = pl->lkb_nbocc;
-  k.maxpol = pl->lkb_maxpol;
-  k.maxocc = pl->lkb_maxocc;
   k.par = (const Real*)pl->lkb_par;
   k.hbase = pl->hbase;
   const Real* gp = (const Real*)pl->global_params;
@@ -2168,32 +2170,23 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
     std::stable_partition(occ[bt].begin(), occ[bt].end(), bridges);
     for (int a : occ[bt]) hnbocc[bt] += bridges(a) ? 1 : 0;
   }
-  int maxpol = 1, maxocc = 1;
-  for (int bt = 0; bt < nbt; ++bt) {
-    maxpol = std::max(maxpol, (int)pol[bt].size());
-    maxocc = std::max(maxocc, (int)occ[bt].size());
-  }
-  std::vector<int> hpol((size_t)std::max(nbt, 1) * maxpol, 0), hocc((size_t)std::max(nbt, 1) * maxocc, 0);
+  int maxocc = 1;
+  for (int bt = 0; bt < nbt; ++bt) maxocc = std::max(maxocc, (int)occ[bt].size());
   std::vector<int> hnpol(std::max(nbt, 1), 0), hnocc(std::max(nbt, 1), 0);
   for (int bt = 0; bt < nbt; ++bt) {
     hnpol[bt] = (int)pol[bt].size();
     hnocc[bt] = (int)occ[bt].size();
-    std::copy(pol[bt].begin(), pol[bt].end(), &hpol[(size_t)bt * maxpol]);
-    std::copy(occ[bt].begin(), occ[bt].end(), &hocc[(size_t)bt * maxocc]);
   }
-  pl->lkb_maxpol = maxpol;
   pl->lkb_maxocc = maxocc;
   pl->lkb_water_dist = (double)wg[0];
   if (scoring) {
-    CK(dalloc(pl, &pl->lkb_pol, hpol.size()));
-    CK(dalloc(pl, &pl->lkb_occ, hocc.size()));
-    CK(dalloc(pl, &pl->lkb_npol, hnpol.size()));
-    CK(dalloc(pl, &pl->lkb_nocc, hnocc.size()));
-    CK(dalloc(pl, &pl->lkb_nbocc, hnbocc.size()));
-    CK(cudaMemcpyAsync(pl->lkb_nbocc, hnbocc.data(), sizeof(int) * hnbocc.size(), cudaMemcpyHostToDevice, st));
-    CK(dalloc(pl, (Real**)&pl->lkb_par, par.size()));
-    CK(cudaMemcpyAsync(pl->lkb_pol, hpol.data(), sizeof(int) * hpol.size(), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(pl->lkb_occ, hocc.data(), sizeof(int) * hocc.size(), cudaMemcpyHostToDevice, st));
+    dalloc(pl, &pl->lkb_npol, hnpol.size());
+    dalloc(pl, &pl->lkb_nocc, hnocc.size());
+    dalloc(pl, (Real**)&pl->lkb_par, par.size());
+    const int n_blocks = pl->rotamers ? pl->R : pl->P * pl->B;
+    dalloc(pl, &pl->hmeta, (size_t)std::max(nbt, 1) * maxocc);
+    dalloc(pl, &pl->hbase, n_blocks);
+    CK(dplace(pl));
     CK(cudaMemcpyAsync(pl->lkb_npol, hnpol.data(), sizeof(int) * hnpol.size(), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(pl->lkb_nocc, hnocc.data(), sizeof(int) * hnocc.size(), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(pl->lkb_par, par.data(), sizeof(Real) * par.size(), cudaMemcpyHostToDevice, st));
@@ -2209,10 +2202,8 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
         const bool polar = std::find(pol[bt].begin(), pol[bt].end(), a) != pol[bt].end();
         hmeta[(size_t)bt * maxocc + y] = a | (polar ? 1 << 16 : 0) | ((int)y < hnbocc[bt] ? 1 << 17 : 0);
       }
-    CK(dalloc(pl, &pl->hmeta, hmeta.size()));
     CK(cudaMemcpyAsync(pl->hmeta, hmeta.data(), sizeof(int) * hmeta.size(), cudaMemcpyHostToDevice, st));
     const int n = pl->rotamers ? pl->R : pl->P * pl->B;
-    CK(dalloc(pl, &pl->hbase, n));
     unsigned long long n_heavy = 0;
     if (n > 0) {
       CK(cudaMemsetAsync(pl->counts, 0, sizeof(unsigned long long), st));
@@ -2223,24 +2214,28 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
     }
     CK(cudaStreamSynchronize(st));
     if (n_heavy >= (1ull << 31)) return TMOL_B200_ERR_SHAPE;  // record indices are int
-    CK(dalloc(pl, (AtomRec<Real>**)&pl->hpacked, (size_t)n_heavy));
+    dalloc(pl, (AtomRec<Real>**)&pl->hpacked, (size_t)n_heavy);
   }
   if (scoring && !pl->rotamers) {
     // the score op's speculative gradient (lkb_backward_speculative)
-    CK(dalloc(pl, (Real**)&pl->spec_next, (size_t)4 * std::max(pl->P, 1)));
-    CK(dalloc(pl, (Real**)&pl->spec_used, (size_t)4 * std::max(pl->P, 1)));
-    CK(dalloc(pl, (Real**)&pl->spec_g, (size_t)std::max<int64_t>(pl->N, 1) * GRAD_STRIDE));
-    CK(dalloc(pl, (Real**)&pl->spec_dw, (size_t)std::max<int64_t>(pl->N, 1) * LKB_NW * 3));
-    CK(dalloc(pl, &pl->spec_flag, 1));
+    dalloc(pl, (Real**)&pl->spec_next, (size_t)4 * std::max(pl->P, 1));
+    dalloc(pl, (Real**)&pl->spec_used, (size_t)4 * std::max(pl->P, 1));
+    dalloc(pl, (Real**)&pl->spec_g, (size_t)std::max<int64_t>(pl->N, 1) * GRAD_STRIDE);
+    dalloc(pl, (Real**)&pl->spec_dw, (size_t)std::max<int64_t>(pl->N, 1) * LKB_NW * 3);
+    dalloc(pl, &pl->spec_flag, 1);
   }
-  if (!waters) return TMOL_B200_OK;
+  if (!waters) {
+    CK(dplace(pl));
+    return TMOL_B200_OK;
+  }
   const int64_t n_sites = pl->N * LKB_NW;
   if (n_sites >= ((int64_t)1 << 31)) return TMOL_B200_ERR_SHAPE;  // site indices are int
   if (scoring) {
-    CK(dalloc(pl, (Real**)&pl->lkb_waters, (size_t)n_sites * 3));
-    CK(dalloc(pl, (Real**)&pl->lkb_dwaters, (size_t)n_sites * 3));
+    dalloc(pl, (Real**)&pl->lkb_waters, (size_t)n_sites * 3);
+    dalloc(pl, (Real**)&pl->lkb_dwaters, (size_t)n_sites * 3);
   }
-  CK(dalloc(pl, (LkbSite<Real>**)&pl->lkb_sites, (size_t)n_sites));
+  dalloc(pl, (LkbSite<Real>**)&pl->lkb_sites, (size_t)n_sites);
+  CK(dplace(pl));
   CK(cudaMemsetAsync(pl->lkb_sites, 0, sizeof(LkbSite<Real>) * std::max<int64_t>(n_sites, 1), st));
   const int64_t PB = (int64_t)pl->P * pl->B;
   if (PB > 0 && nbt > 0 && k->n_rots > 0) {
@@ -2289,7 +2284,8 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
   for (int64_t i = 0; i < n_sites; ++i)
     if (h_sites[i].kind != kLkbNone) active.push_back((int)i);
   pl->lkb_n_active = (int64_t)active.size();
-  CK(dalloc(pl, &pl->lkb_active, active.size()));
+  dalloc(pl, &pl->lkb_active, active.size());
+  CK(dplace(pl));
   if (!active.empty())
     CK(cudaMemcpyAsync(pl->lkb_active, active.data(), sizeof(int) * active.size(), cudaMemcpyHostToDevice, st));
   if (scoring && n_sites > 0)
@@ -2422,53 +2418,68 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   PCK(cudaDeviceGetAttribute(&pl->n_sm, cudaDevAttrMultiProcessorCount, dev));
   PCK(real_bytes == 4 ? set_smem_limits<float>(term) : set_smem_limits<double>(term));
   const int64_t PB = (int64_t)P * B;
-  PCK(dalloc(pl, &pl->blk_bt, PB));
-  PCK(dalloc(pl, &pl->blk_off, PB));
-  PCK(dalloc(pl, &pl->pose_last, P));
-  PCK(dalloc(pl, &pl->bt_tf, (size_t)nbt * A));
-  PCK(dalloc(pl, &pl->type_map, 2 * (size_t)std::max(T, 1)));
-  PCK(dalloc(pl, &pl->bt_pd, (size_t)nbt * A * A));
-  PCK(dalloc(pl, &pl->bt_conn_pd, (size_t)nbt * C * A));
-  PCK(dalloc(pl, &pl->bt_flags, (size_t)nbt * A));
-  PCK(dalloc(pl, &pl->bt_n_atoms, nbt));
-  PCK(dalloc(pl, &pl->bt_n_conn, nbt));
-  PCK(dalloc(pl, &pl->bt_is_ligand, nbt));
-  PCK(dalloc(pl, &pl->cp_count, PB));
-  PCK(dalloc(pl, &pl->cp_b2, PB * CP_CAP));
-  PCK(dalloc(pl, &pl->cp_minsep, PB * CP_CAP));
-  PCK(dalloc(pl, &pl->cp_seps, PB * CP_CAP * 16));
-  PCK(dalloc(pl, (unsigned char**)&pl->spheres, PB * 4 * real_bytes));
+  dalloc(pl, &pl->blk_bt, PB);
+  dalloc(pl, &pl->blk_off, PB);
+  dalloc(pl, &pl->pose_last, P);
+  dalloc(pl, &pl->bt_tf, (size_t)nbt * A);
+  dalloc(pl, &pl->type_map, 2 * (size_t)std::max(T, 1));
+  dalloc(pl, &pl->bt_pd, (size_t)nbt * A * A);
+  dalloc(pl, &pl->bt_conn_pd, (size_t)nbt * C * A);
+  dalloc(pl, &pl->bt_flags, (size_t)nbt * A);
+  dalloc(pl, &pl->bt_n_atoms, nbt);
+  dalloc(pl, &pl->bt_n_conn, nbt);
+  dalloc(pl, &pl->bt_is_ligand, nbt);
+  dalloc(pl, &pl->cp_count, PB);
+  dalloc(pl, &pl->cp_b2, PB * CP_CAP);
+  dalloc(pl, &pl->cp_minsep, PB * CP_CAP);
+  dalloc(pl, &pl->cp_seps, PB * CP_CAP * 16);
+  dalloc(pl, (unsigned char**)&pl->spheres, PB * 4 * real_bytes);
   if (scoring) {
     const int64_t n_at = std::max<int64_t>(in->n_atoms, 1);
-    PCK(dalloc(pl, (unsigned char**)&pl->packed,
-               n_at * (real_bytes == 4 ? sizeof(AtomRec<float>) : sizeof(AtomRec<double>))));
-    PCK(dalloc(pl, (unsigned char**)&pl->g4, (size_t)n_at * GRAD_STRIDE * real_bytes));
-    PCK(dalloc(pl, &pl->real_atom, n_at));
-    PCK(cudaMemsetAsync(pl->real_atom, 0, n_at, st));
+    dalloc(pl, (unsigned char**)&pl->packed,
+               n_at * (real_bytes == 4 ? sizeof(AtomRec<float>) : sizeof(AtomRec<double>)));
+    dalloc(pl, (unsigned char**)&pl->g4, (size_t)n_at * GRAD_STRIDE * real_bytes);
+    dalloc(pl, &pl->real_atom, n_at);
   }
   if (scoring) {
     pl->n_iwords = (A + 31) / 32;
-    PCK(dalloc(pl, &pl->imask, (size_t)nbt * A * pl->n_iwords));
-    PCK(dalloc(pl, &pl->bt_n_heavy, nbt));
+    dalloc(pl, &pl->imask, (size_t)nbt * A * pl->n_iwords);
+    dalloc(pl, &pl->bt_n_heavy, nbt);
   }
-  if (!rotamers && scoring) PCK(dalloc(pl, &pl->blk_info, PB));
+  if (!rotamers && scoring) dalloc(pl, &pl->blk_info, PB);
   if (!rotamers && term != kTermLKBall) {
-    PCK(dalloc(pl, (unsigned char**)&pl->spec_next, (size_t)n_terms(term) * std::max(P, 1) * real_bytes));
-    PCK(dalloc(pl, (unsigned char**)&pl->spec_used, (size_t)n_terms(term) * std::max(P, 1) * real_bytes));
-    PCK(dalloc(pl, (unsigned char**)&pl->spec_g, (size_t)std::max<int64_t>(in->n_atoms, 1) * GRAD_STRIDE * real_bytes));
-    PCK(dalloc(pl, &pl->spec_flag, 1));
+    dalloc(pl, (unsigned char**)&pl->spec_next, (size_t)n_terms(term) * std::max(P, 1) * real_bytes);
+    dalloc(pl, (unsigned char**)&pl->spec_used, (size_t)n_terms(term) * std::max(P, 1) * real_bytes);
+    dalloc(pl, (unsigned char**)&pl->spec_g, (size_t)std::max<int64_t>(in->n_atoms, 1) * GRAD_STRIDE * real_bytes);
+    dalloc(pl, &pl->spec_flag, 1);
   }
-  if (real_bytes == 4) PCK(dalloc(pl, &pl->sub_spheres, PB * 8));
-  PCK(dalloc(pl, &pl->counters, 4));
-  PCK(dalloc(pl, &pl->counts, N_COUNTS));
+  if (real_bytes == 4) dalloc(pl, &pl->sub_spheres, PB * 8);
+  dalloc(pl, &pl->counters, 4);
+  dalloc(pl, &pl->counts, N_COUNTS);
   if (term == kTermElec) {
-    PCK(dalloc(pl, (unsigned char**)&pl->bt_q, (size_t)nbt * A * real_bytes));
-    PCK(dalloc(pl, (unsigned char**)&pl->elec_k, (size_t)N_ELEC_K * real_bytes));
-    if (nbt > 0 && A > 0)
-      PCK(cudaMemcpyAsync(pl->bt_q, elec->partial_charge, (size_t)nbt * A * real_bytes,
-                          cudaMemcpyDeviceToDevice, st));
+    dalloc(pl, (unsigned char**)&pl->bt_q, (size_t)nbt * A * real_bytes);
+    dalloc(pl, (unsigned char**)&pl->elec_k, (size_t)N_ELEC_K * real_bytes);
   }
+  if (!rotamers && scoring) dalloc(pl, &pl->cp_moff, PB * CP_CAP);
+  if (rotamers) {
+    const int R = in->n_rots;
+    pl->rotamers = true;
+    pl->R = R;
+    dalloc(pl, &pl->rot_bt, R);
+    dalloc(pl, &pl->rot_off, R);
+    dalloc(pl, &pl->rot_block, R);
+    dalloc(pl, &pl->rot_pose, R);
+    dalloc(pl, &pl->nrb, PB);
+    dalloc(pl, &pl->rob, PB);
+    dalloc(pl, (unsigned char**)&pl->rot_spheres, (size_t)R * 4 * real_bytes);
+    dalloc(pl, &pl->row_pairs, PB + 2);
+    dalloc(pl, &pl->row_items, PB);
+  }
+  PCK(dplace(pl));
 
+  if (scoring) PCK(cudaMemsetAsync(pl->real_atom, 0, std::max<int64_t>(in->n_atoms, 1), st));
+  if (term == kTermElec && nbt > 0 && A > 0)
+    PCK(cudaMemcpyAsync(pl->bt_q, elec->partial_charge, (size_t)nbt * A * real_bytes, cudaMemcpyDeviceToDevice, st));
   PCK(cudaMemsetAsync(pl->pose_last, 0, sizeof(int) * std::max(P, 1), st));
   PCK(cudaMemsetAsync(pl->counters, 0, sizeof(int) * 4, st));
   PCK(cudaMemsetAsync(pl->bt_flags, 0, sizeof(int) * std::max<int64_t>((int64_t)nbt * A, 1), st));
@@ -2504,17 +2515,6 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   a.rot_bt = a.rot_off = a.rot_block = a.rot_pose = nullptr;
   if (rotamers) {
     const int R = in->n_rots;
-    pl->rotamers = true;
-    pl->R = R;
-    PCK(dalloc(pl, &pl->rot_bt, R));
-    PCK(dalloc(pl, &pl->rot_off, R));
-    PCK(dalloc(pl, &pl->rot_block, R));
-    PCK(dalloc(pl, &pl->rot_pose, R));
-    PCK(dalloc(pl, &pl->nrb, PB));
-    PCK(dalloc(pl, &pl->rob, PB));
-    PCK(dalloc(pl, (unsigned char**)&pl->rot_spheres, (size_t)R * 4 * real_bytes));
-    PCK(dalloc(pl, &pl->row_pairs, PB + 2));
-    PCK(dalloc(pl, &pl->row_items, PB));
     if (PB > 0) {
       PCK(cudaMemcpyAsync(pl->nrb, in->n_rots_for_block, sizeof(int) * PB, cudaMemcpyDeviceToDevice, st));
       PCK(cudaMemcpyAsync(pl->rob, in->rot_offset_for_block, sizeof(int) * PB, cudaMemcpyDeviceToDevice, st));
@@ -2557,7 +2557,6 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   }
   unsigned long long n_masks = 0;
   if (pl->blk_info && PB > 0) {
-    PCK(dalloc(pl, &pl->cp_moff, PB * CP_CAP));
     PCK(cudaMemsetAsync(pl->counts, 0, sizeof(unsigned long long), st));
     plan_mask_offsets_kernel<<<g, 256, 0, st>>>(pl->blk_info, pl->cp_count, pl->cp_b2, PB, B, pl->counts, pl->cp_moff);
     PCK(cudaGetLastError());
@@ -2618,13 +2617,19 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     return TMOL_B200_ERR_SHAPE;
   }
   size_t ntp2 = (size_t)std::max(pl->ntp, 1) * std::max(pl->ntp, 1);
-  PCK(dalloc(pl, &pl->compact_types, std::max(pl->ntp, 1)));
-  PCK(dalloc(pl, (unsigned char**)&pl->ljtab,
-             2 * ntp2 * (real_bytes == 4 ? sizeof(Quad<float>) : sizeof(Quad<double>))));
-  PCK(dalloc(pl, (unsigned char**)&pl->fartab,
-             ntp2 * (real_bytes == 4 ? sizeof(Quad<float>) : sizeof(Quad<double>))));
-  PCK(dalloc(pl, (unsigned char**)&pl->lktab,
-             ntp2 * (real_bytes == 4 ? sizeof(LKRecord<float>) : sizeof(LKRecord<double>))));
+  dalloc(pl, &pl->compact_types, std::max(pl->ntp, 1));
+  dalloc(pl, (unsigned char**)&pl->ljtab,
+             2 * ntp2 * (real_bytes == 4 ? sizeof(Quad<float>) : sizeof(Quad<double>)));
+  dalloc(pl, (unsigned char**)&pl->fartab,
+             ntp2 * (real_bytes == 4 ? sizeof(Quad<float>) : sizeof(Quad<double>)));
+  dalloc(pl, (unsigned char**)&pl->lktab,
+             ntp2 * (real_bytes == 4 ? sizeof(LKRecord<float>) : sizeof(LKRecord<double>)));
+  if (n_masks >= (1ull << 32)) {  // 32 GB of masks
+    free_plan(pl);
+    return TMOL_B200_ERR_CAPACITY;
+  }
+  if (nbt > 0 && n_masks > 0) dalloc(pl, &pl->pmask, n_masks);
+  PCK(dplace(pl));
   PCK(cudaMemcpyAsync(pl->type_map, type_map.data(), sizeof(int) * type_map.size(), cudaMemcpyHostToDevice, st));
   if (pl->ntp > 0)
     PCK(cudaMemcpyAsync(pl->compact_types, compact.data(), sizeof(int) * pl->ntp,
@@ -2638,12 +2643,7 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
       const int gi = (int)std::max<int64_t>(1, std::min<int64_t>((n_im + 255) / 256, (int64_t)pl->n_sm * 8));
       plan_intra_masks_kernel<<<gi, 256, 0, st>>>(pl->bt_pd, pl->bt_n_atoms, nbt, A, pl->n_iwords, pl->imask);
       PCK(cudaGetLastError());
-      if (n_masks >= (1ull << 32)) {  // 32 GB of masks
-        free_plan(pl);
-        return TMOL_B200_ERR_CAPACITY;
-      }
       if (n_masks > 0) {
-        PCK(dalloc(pl, &pl->pmask, n_masks));
         const int gm = std::max(1, std::min<int>((int)((PB + 7) / 8), pl->n_sm * 16));
         if (real_bytes == 4)
           plan_partner_masks_kernel<float><<<gm, 256, 0, st>>>(score_args<float>(pl, nullptr), pl->pmask);
@@ -3310,13 +3310,13 @@ int tmol_b200_lkball_rotamer_plan_create(const tmol_b200_lkball_inputs* inputs, 
 int tmol_b200_lkball_rotamer_count(tmol_b200_lkball_plan* plan, const void* coords, int64_t* n_pairs,
                                    int64_t* n_items, void* stream) {
   NvtxRange nvtx_range("tmol_b200_lkball_rotamer_count");
-  if (!plan || !plan->lkb_pol) return TMOL_B200_ERR_INVALID_ARGUMENT;
+  if (!plan || !plan->lkb_nocc) return TMOL_B200_ERR_INVALID_ARGUMENT;
   return rotamer_count(plan, kTermLKBall, coords, n_pairs, n_items, stream);
 }
 
 int tmol_b200_lkball_rotamer_fill(tmol_b200_lkball_plan* plan, int32_t* indices, int32_t* items, void* stream) {
   NvtxRange nvtx_range("tmol_b200_lkball_rotamer_fill");
-  if (!plan || !plan->lkb_pol) return TMOL_B200_ERR_INVALID_ARGUMENT;
+  if (!plan || !plan->lkb_nocc) return TMOL_B200_ERR_INVALID_ARGUMENT;
   return rotamer_fill(plan, kTermLKBall, indices, items, stream);
 }
 
@@ -3324,7 +3324,7 @@ int tmol_b200_lkball_rotamer_forward(tmol_b200_lkball_plan* plan, const void* co
                                      const int32_t* items, int64_t n_items, int64_t n_pairs, void* energies,
                                      void* stream) {
   NvtxRange nvtx_range("tmol_b200_lkball_rotamer_forward");
-  if (!rotamer_plan_of(plan, kTermLKBall) || !plan->lkb_pol || !energies || n_items < 0 || n_pairs < 0 ||
+  if (!rotamer_plan_of(plan, kTermLKBall) || !plan->lkb_nocc || !energies || n_items < 0 || n_pairs < 0 ||
       (n_items > 0 && !items) || (plan->N > 0 && (!coords || !waters)))
     return TMOL_B200_ERR_INVALID_ARGUMENT;
   if (n_items >= ((int64_t)1 << 31) || n_pairs >= ((int64_t)1 << 31)) return TMOL_B200_ERR_CAPACITY;
@@ -3340,7 +3340,7 @@ int tmol_b200_lkball_rotamer_backward(tmol_b200_lkball_plan* plan, const void* c
                                       const int32_t* items, int64_t n_items, int64_t n_pairs, const void* dTdV,
                                       void* dcoords, void* dwaters, void* stream) {
   NvtxRange nvtx_range("tmol_b200_lkball_rotamer_backward");
-  if (!rotamer_plan_of(plan, kTermLKBall) || !plan->lkb_pol || !dTdV || !dcoords || !dwaters || n_items < 0 ||
+  if (!rotamer_plan_of(plan, kTermLKBall) || !plan->lkb_nocc || !dTdV || !dcoords || !dwaters || n_items < 0 ||
       n_pairs < 0 || (n_items > 0 && !items) || (plan->N > 0 && (!coords || !waters)))
     return TMOL_B200_ERR_INVALID_ARGUMENT;
   if (n_items >= ((int64_t)1 << 31) || n_pairs >= ((int64_t)1 << 31)) return TMOL_B200_ERR_CAPACITY;
@@ -3380,7 +3380,7 @@ int tmol_b200_lkball_waters_backward(tmol_b200_lkball_plan* plan, const void* co
 int tmol_b200_lkball_forward(tmol_b200_lkball_plan* plan, const void* coords, const void* waters,
                              int block_pair, void* energies, int32_t* block_neighbors, void* stream) {
   NvtxRange nvtx_range("tmol_b200_lkball_forward");
-  if (!plan || plan->term != kTermLKBall || !plan->lkb_pol || !energies) return TMOL_B200_ERR_INVALID_ARGUMENT;
+  if (!plan || plan->term != kTermLKBall || !plan->lkb_nocc || !energies) return TMOL_B200_ERR_INVALID_ARGUMENT;
   if (plan->N > 0 && (!coords || !waters)) return TMOL_B200_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   if (plan->real_bytes == 4)
@@ -3397,7 +3397,7 @@ int tmol_b200_lkball_forward(tmol_b200_lkball_plan* plan, const void* coords, co
 int tmol_b200_lkball_forward_speculative(tmol_b200_lkball_plan* plan, const void* coords, const void* waters,
                                          void* energies, int32_t* block_neighbors, void* stream) {
   NvtxRange nvtx_range("tmol_b200_lkball_forward_speculative");
-  if (!plan || plan->term != kTermLKBall || plan->rotamers || !plan->lkb_pol || !plan->spec_g || !energies)
+  if (!plan || plan->term != kTermLKBall || plan->rotamers || !plan->lkb_nocc || !plan->spec_g || !energies)
     return TMOL_B200_ERR_INVALID_ARGUMENT;
   if (plan->N > 0 && (!coords || !waters)) return TMOL_B200_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
@@ -3410,7 +3410,7 @@ int tmol_b200_lkball_backward_speculative(tmol_b200_lkball_plan* plan, const voi
                                           const void* dTdV, void* dcoords, void* dwaters, int speculated,
                                           void* stream) {
   NvtxRange nvtx_range("tmol_b200_lkball_backward_speculative");
-  if (!plan || plan->term != kTermLKBall || plan->rotamers || !plan->lkb_pol || !plan->spec_g || !dTdV)
+  if (!plan || plan->term != kTermLKBall || plan->rotamers || !plan->lkb_nocc || !plan->spec_g || !dTdV)
     return TMOL_B200_ERR_INVALID_ARGUMENT;
   if (plan->N > 0 && (!coords || !waters || !dcoords || !dwaters)) return TMOL_B200_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
@@ -3422,7 +3422,7 @@ int tmol_b200_lkball_backward_speculative(tmol_b200_lkball_plan* plan, const voi
 int tmol_b200_lkball_energy_and_gradient(tmol_b200_lkball_plan* plan, const void* coords, const void* weights,
                                          void* energies, void* dcoords, void* stream) {
   NvtxRange nvtx_range("tmol_b200_lkball_energy_and_gradient");
-  if (!plan || plan->term != kTermLKBall || !plan->lkb_pol || !plan->lkb_sites || !weights || !energies ||
+  if (!plan || plan->term != kTermLKBall || !plan->lkb_nocc || !plan->lkb_sites || !weights || !energies ||
       !dcoords)
     return TMOL_B200_ERR_INVALID_ARGUMENT;
   if (plan->N > 0 && !coords) return TMOL_B200_ERR_INVALID_ARGUMENT;
@@ -3448,7 +3448,7 @@ int tmol_b200_lkball_backward(tmol_b200_lkball_plan* plan, const void* coords, c
                               int block_pair, const void* dTdV, void* dcoords, void* dwaters,
                               void* stream) {
   NvtxRange nvtx_range("tmol_b200_lkball_backward");
-  if (!plan || plan->term != kTermLKBall || !plan->lkb_pol || !dTdV) return TMOL_B200_ERR_INVALID_ARGUMENT;
+  if (!plan || plan->term != kTermLKBall || !plan->lkb_nocc || !dTdV) return TMOL_B200_ERR_INVALID_ARGUMENT;
   if (plan->N > 0 && (!coords || !waters || !dcoords || !dwaters)) return TMOL_B200_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   int rc;

@@ -38,12 +38,8 @@ struct LkbArgs {
   Real* waters_out;
   const Real* dwaters;  // adjoint in
   Real* dwaters_out;    // adjoint out
-  const int* pol;       // [nbt][maxpol] polar atoms of each block type
   const int* npol;      // [nbt]
-  const int* occ;       // [nbt][maxocc] heavy atoms (polar ones included), donors / acceptors first
   const int* nocc;
-  const int* nbocc;     // [nbt] leading occluders that are donors or acceptors (the bridge term)
-  int maxpol, maxocc;
   const int* hbase;     // [P*B] (rotamer plans: [R]) first heavy record of each block (rotamer)
   const Real* par;      // [nbt][A][12], 9 used
   Real water_dist, hbond_dis, hbond_oh, hbond_h, max_dis;
