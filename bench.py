@@ -750,7 +750,7 @@ def run_rotamers(args, world, rank, local):
             "atom_pairs_per_s": counts["atom_pairs"] * args.steps * world / (ms / 1e3),
             "energies_only_ms_per_step": e_ms,
             "work_per_step": counts,
-            "gpu_launches": 7 * args.steps,
+            "gpu_launches": 8 * args.steps,
             "clocks": clk.summary(),
             "roofline": {
                 "bound": "fp32",
@@ -911,9 +911,9 @@ def run_lkball_rotamers(args, world, rank, local):
             "scoring_only_ms_per_step": e_ms,
             "work_per_step": counts,
             # waters, 4 dispatch kernels (rotamer and block spheres, row
-            # counts, scan), the fill, the rotamer spheres and the scoring
+            # counts, scan), the fill and the indices, the rotamer spheres and the scoring
             # kernel
-            "gpu_launches": 8 * args.steps,
+            "gpu_launches": 9 * args.steps,
             "clocks": clk.summary(),
             "roofline": {
                 "bound": "fp32",
@@ -1367,14 +1367,14 @@ def run_elec(args, world, rank, local):
                 "poses_per_gpu": P,
                 "atoms_per_gpu": int(coords.shape[0]),
                 "l2": "flushed (256 MiB write) before every timed step",
-                "launch": "CUDA graph replay: 2 kernels per step",
+                "launch": "CUDA graph replay: 3 kernels per step",
                 "launch_shape": dict(
                     zip(LAUNCH_FIELDS, launch)
                 ),
                 "parallelism": f"weak, {world} independent batch(es)",
             },
             "work_per_step": m["work_per_step"],
-            "gpu_launches": 2 * args.steps,
+            "gpu_launches": 3 * args.steps,
             "clocks": clk.summary(),
             "roofline": {
                 "bound": "fp32",
@@ -1652,15 +1652,15 @@ def run_lkball(args, world, rank, local):
                 "poses_per_gpu": P,
                 "atoms_per_gpu": int(coords.shape[0]),
                 "l2": "flushed (256 MiB write) before every timed step",
-                "launch": "CUDA graph replay: 4 kernels per step (waters, block spheres, scoring with its "
-                "adjoint, waters adjoint) and 5 memsets",
+                "launch": "CUDA graph replay: 5 kernels per step (waters, block spheres, scoring with its "
+                "adjoint, gradient out, waters adjoint)",
                 "launch_shape": dict(
                     zip(LAUNCH_FIELDS, launch)
                 ),
                 "parallelism": f"weak, {world} independent batch(es)",
             },
             "work_per_step": m["work_per_step"],
-            "gpu_launches": 4 * args.steps,
+            "gpu_launches": 5 * args.steps,
             "clocks": clk.summary(),
             "roofline": {
                 "bound": "fp32",
@@ -1858,11 +1858,11 @@ def run_sfxn(args, world, rank, local):
                 "poses_per_gpu": P,
                 "atoms_per_gpu": int(coords.shape[0]),
                 "l2": "flushed (256 MiB write) before every timed step",
-                "launch": "CUDA graph replay: 10 kernels per step (LJ/LK 2, elec 2, LK-ball 4 on three concurrent "
+                "launch": "CUDA graph replay: 13 kernels per step (LJ/LK 3, elec 3, LK-ball 5 on three concurrent "
                 "streams, gradient sum 2)",
                 "parallelism": f"weak, {world} independent batch(es)",
             },
-            "gpu_launches": 10 * args.steps,
+            "gpu_launches": 13 * args.steps,
             "clocks": clk.summary(),
             "roofline": {
                 "bound": "fp32",
@@ -2399,7 +2399,7 @@ def measure_pose_batch(args, workload_name, world, rank, local, steps, extras=Tr
                 "residues_per_gpu": n_residues,
                 "atoms_per_gpu": int(coords.shape[0]),
                 "l2": "flushed (256 MiB write) before every timed step",
-                "launch": "CUDA graph replay: 2 kernels per step" + (" + perturbation" if perturb else ""),
+                "launch": "CUDA graph replay: 3 kernels per step" + (" + perturbation" if perturb else ""),
                 "launch_shape": dict(
                     zip(LAUNCH_FIELDS, launch_shape)
                 ),
@@ -2407,7 +2407,7 @@ def measure_pose_batch(args, workload_name, world, rank, local, steps, extras=Tr
             },
             "atom_pairs_per_s": counts["atom_pairs"] * steps * world / (ms_max / 1e3),
             "work_per_step": counts,
-            "gpu_launches": 2 * steps,
+            "gpu_launches": 3 * steps,
             "clocks": clk.summary(),
             "roofline": {
                 "bound": "fp32",
