@@ -78,6 +78,53 @@ def test_rotamer_groups(scale):
     clear_plan_cache()
 
 
+def pair_plan(name, rotamers, dtype, scale):
+    """A plan over squeezed poses (or their rotamers) and its coordinates."""
+    from tmol_b200.score.elec_energy_term import elec_rotamer_score_args
+    from tmol_b200.score.elec_op import ElecPlan
+    from tmol_b200.score.ljlk_op import LJLKPlan
+
+    ps = synthetic_pose_stack([30, 1, 2, 9, 75], [5, 6, 7, 8, 9], spacing=0.0)
+    term = {"ljlk": LJLKEnergyTerm, "elec": ElecEnergyTerm}[name]()
+    if rotamers:
+        ps = synthetic_pose_stack([12, 3], [15, 16], spacing=0.0)
+        rs = synthetic_rotamer_set(ps, max_rots=40, seed=3)
+        args = {"ljlk": rotamer_score_args, "elec": elec_rotamer_score_args}[name](ps, rs, term)
+        x = rs.coords
+    else:
+        args = {"ljlk": pose_score_args, "elec": elec_pose_score_args}[name](ps, term, True)
+        x = ps.coords.flatten(0, 1)
+    x = (x * scale).to(DEV, dtype).contiguous()
+    plan = {"ljlk": LJLKPlan, "elec": ElecPlan}[name](x, on_gpu(args, dtype)[:-1], rotamers=rotamers)
+    return plan, x
+
+
+@pytest.mark.parametrize("scale", [1.0, 0.5])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("rotamers", [False, True])
+@pytest.mark.parametrize("name", ["ljlk", "elec"])
+def test_pair_energies_repeat(name, rotamers, dtype, scale):
+    """A pair's energy is the same bits in every call, whichever other pairs
+    its warp scores beside it: across repeated calls, work items split anew
+    by their measured costs or cut to other lengths, and groups of one and of
+    nine pairs."""
+    plan, x = pair_plan(name, rotamers, dtype, scale)
+    if rotamers:
+        indices, items = plan.rotamer_dispatch(x)
+        run = lambda: plan.rotamer_forward(x, items, indices.shape[1])
+    else:
+        run = lambda: plan.forward(x, block_pair=True)[0]
+    first = run()
+    for _ in range(4):
+        assert torch.equal(run(), first)
+    for launch in (dict(slots_per_group=1), dict(slots_per_group=3, candidates_per_item=4), dict(warps_per_cta=2)):
+        plan.set_launch(**launch)
+        assert torch.equal(run(), first), launch
+    if not rotamers:
+        plan.balance(run)
+        assert torch.equal(run(), first)
+
+
 def test_no_common_fade_interval():
     """A type whose LJ minimum lies inside the fade interval fades on an
     interval of its own: the general path serves every pair.  (Energies, from

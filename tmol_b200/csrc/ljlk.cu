@@ -973,7 +973,7 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 32 * PAIR_WARPS : 256, 1)
     rotamer_kernel(ScoreArgs<Real> s, RotArgs ra, const Real* rs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  Slab<Real>& w = reinterpret_cast<Slab<Real>*>(smem_raw)[warp];
+  Slab<Real>& w = *reinterpret_cast<Slab<Real>*>(smem_raw + warp * slab_bytes<Real>(!GRAD));
   EvalCtx<Real> ec = eval_ctx(s);
   ec.energies = s.energies;
   ec.dTdV = s.dTdV;
@@ -1467,7 +1467,7 @@ void default_launch(const tmol_b200_ljlk_plan* pl, tmol_b200_ljlk_launch& l) {
 
 template <typename Real, int TERM>
 cudaError_t set_smem_limits_term() {
-  const int smem = (int)std::min<size_t>(PAIR_WARPS * sizeof(Slab<Real>), 227 * 1024);
+  const int smem = (int)std::min<size_t>(PAIR_WARPS * slab_bytes<Real>(true), 227 * 1024);
   const void* kernels[] = {
       (const void*)score_kernel<Real, false, false, TERM, false>,
       (const void*)score_kernel<Real, false, true, TERM, false>,
@@ -1616,7 +1616,7 @@ int launch_score(tmol_b200_ljlk_plan* pl, ScoreArgs<Real> s, cudaStream_t st) {
   const int R = pl->launch.rows_per_item;
   // the float64 kernel: at most 256 threads
   const GridShape gs = grid_shape(pl, (pl->n_work + R - 1) / R, sizeof(Real) == 8 ? 8 : PAIR_WARPS);
-  size_t smem = gs.warps * sizeof(Slab<Real>);
+  size_t smem = gs.warps * slab_bytes<Real>(BLOCK_PAIR && !GRAD);
   // the work counters cost registers and instructions in the item loop:
   // they are compiled into a separate instantiation, used on request
   auto kern = pl->term == kTermElec
@@ -1884,7 +1884,7 @@ int rotamer_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const int32_
   CK(cudaMemsetAsync(pl->counters, 0, sizeof(int), st));
   // the float64 kernel: at most 256 threads
   const GridShape gs = grid_shape(pl, n_items, sizeof(Real) == 8 ? 8 : PAIR_WARPS);
-  const size_t smem = gs.warps * sizeof(Slab<Real>);
+  const size_t smem = gs.warps * slab_bytes<Real>(!GRAD);
   auto kern = pl->term == kTermElec
                   ? (pl->counting ? rotamer_kernel<Real, GRAD, kTermElec, true> : rotamer_kernel<Real, GRAD, kTermElec, false>)
                   : (pl->counting ? rotamer_kernel<Real, GRAD, kTermLJLK, true> : rotamer_kernel<Real, GRAD, kTermLJLK, false>);

@@ -60,7 +60,6 @@ template <typename Real>
 struct Slab {
   static constexpr int QCAP = 3 * M1 * sizeof(Real) / 2 < 1024 ? 1024 : 3 * M1 * sizeof(Real) / 2;
   AtomRec<Real> at[M1];
-  int gidx[M1];  // global atom index
   union {
     struct {
       Real x[M1], y[M1], z[M1];
@@ -73,9 +72,40 @@ struct Slab {
   long long out[MAXW];  // pair mode: the word's energy entry
   int desc[MAXW];       // base | atoms << 8 | (mask + 1) << 16
   uint32_t heavy[MAXW];
-  int hoff[32];
   uint8_t slot[M1];  // pair mode: the atom's word
+  // last, and next to each other: pair energies use their place (PairSums)
+  int gidx[M1];  // global atom index (gradients)
+  int hoff[32];  // pose mode: the flat list's hits
 };
+
+// Pair energies (no gradient): the energies of up to EWIN queue entries, from
+// which each word's are added in the order of its entries, and where each
+// word's entries begin in each class.  In float the window lies on the index
+// lists that only gradients and pose mode have; with the 448 bytes that it
+// takes beyond the slab, 20 warps stay within 196 KB of shared memory, which
+// leaves L1 60 KB.
+constexpr int EWIN = 96;
+template <typename Real>
+struct PairSums {
+  static constexpr size_t at = sizeof(Real) == 4 ? offsetof(Slab<Real>, gidx) : sizeof(Slab<Real>);
+  Real e[3][EWIN];
+  uint16_t first[3][MAXW + 1];
+  uint16_t pad[2];
+};
+static_assert(PairSums<float>::at % 16 == 0 && sizeof(PairSums<float>) % 16 == 0 && sizeof(PairSums<double>) % 16 == 0,
+              "a warp's slab keeps its alignment");
+static_assert(offsetof(Slab<float>, gidx) + (M1 + 32) * sizeof(int) == sizeof(Slab<float>),
+              "the float sums lie on the slab's last members");
+
+// Bytes of a warp's slab; sums: of one that adds up pair energies.
+template <typename Real>
+__host__ __device__ constexpr size_t slab_bytes(bool sums) {
+  return sums ? PairSums<Real>::at + sizeof(PairSums<Real>) : sizeof(Slab<Real>);
+}
+template <typename Real>
+__device__ __forceinline__ PairSums<Real>& pair_sums(Slab<Real>& w) {
+  return *reinterpret_cast<PairSums<Real>*>(reinterpret_cast<char*>(&w) + PairSums<Real>::at);
+}
 
 template <typename Real>
 __device__ __forceinline__ Real warp_sum(Real v) {
@@ -224,12 +254,79 @@ __device__ __forceinline__ RowTest test_row(const Slab<double>& w, int base, int
 
 enum PairClass : int { kFar = 0, kNear = 1, kNearHeavy = 2 };
 
+// One pair of a class: its energies, weighted by its count-pair weight wcp,
+// and the force f (a - b) on a, (weighted dE/dd) / d.
+template <typename Real>
+struct PairTerms {
+  Real e0, e1, e2, f;
+};
+
+template <typename Real, bool GRAD, int TERM, int CLS>
+__device__ __forceinline__ PairTerms<Real> eval_pair(const EvalCtx<Real>& c, const ElecK<Real>& K,
+                                                     const AtomRec<Real>& a, const AtomRec<Real>& b, Real dx, Real dy,
+                                                     Real dz, Real wcp, Real wt0, Real wt1, Real wt2) {
+  PairTerms<Real> p = {0, 0, 0, 0};
+  const Real d2 = dx * dx + dy * dy + dz * dz;
+  // coincident atoms (d2 = 0) take the linear LJ, flat LK and flat elec
+  // regions, which never use inv_d, and add no force
+  const Real inv_d = inv_sqrt(d2);
+  const Real d = CLS == kFar || d2 > Real(0) ? d2 * inv_d : Real(0);
+  if (TERM == kTermElec) {
+    const Real wq = wcp * a.q * b.q;
+    Real v, dv = 0;
+    if (CLS == kFar) {
+      const Real t = (d - K.hi_start) * K.inv_hi_w;
+      v = K.hi[0] + t * (K.hi[1] + t * (K.hi[2] + t * K.hi[3]));
+      if (GRAD) dv = (K.hi[1] + t * (Real(2) * K.hi[2] + Real(3) * t * K.hi[3])) * K.inv_hi_w;
+    } else {
+      elec_eval<Real, GRAD>(d, K, v, dv);
+    }
+    p.e0 = wq * v;
+    if (GRAD) p.f = wq * wt0 * dv * inv_d;
+  } else {
+    const int tp = (a.tf & 0xff) * c.ntp + (b.tf & 0xff);
+    if (CLS == kFar) {
+      // both potentials fade on the same interval: a cubic from value V
+      // and (interval-scaled) slope D to zero is V A(t) + D B(t), with
+      // A = (1 - t)^2 (1 + 2 t), B = t (1 - t)^2
+      const Quad<Real> k = c.far[tp];  // LJ value, slope; LK value, slope
+      const Real t = (d - c.far_dmin) * c.inv_hf;
+      const Real u = Real(1) - t;
+      const Real uu = u * u;
+      const Real A = uu + Real(2) * t * uu, B = t * uu;
+      p.e0 = wcp * (k.a * A + k.b * B);
+      p.e2 = wcp * (k.c * A + k.d * B);
+      if (GRAD) {
+        const Real dA = Real(-6) * t * u, dB = u - Real(3) * t * u;
+        const Real V = wt0 * k.a + wt2 * k.c, D = wt0 * k.b + wt2 * k.d;
+        p.f = wcp * c.inv_hf * inv_d * (V * dA + D * dB);
+      }
+    } else {
+      Real atr, rep, datr, drep;
+      lj_eval<Real, GRAD>(d, inv_d, c.lj + tp, c.lj + c.ntp * c.ntp + tp, atr, rep, datr, drep);
+      p.e0 = wcp * atr;
+      p.e1 = wcp * rep;
+      Real dE = wt0 * datr + wt1 * drep;
+      if (CLS == kNearHeavy) {
+        Real lk, dlk;
+        lk_eval<Real, GRAD>(d, inv_d, c.lk + tp, c.far_dmin, c.far_first, c.inv_hf, lk, dlk);
+        p.e2 = wcp * lk;
+        dE += wt2 * dlk;
+      }
+      if (GRAD) p.f = wcp * dE * inv_d;
+    }
+  }
+  if (GRAD && CLS != kFar && d == Real(0)) p.f = 0;
+  return p;
+}
+
 // Evaluates queue entries [q0, q0 + n) of one class.  Every lane takes a
 // stretch of S consecutive entries (S kept off multiples of four, whose
 // 16-bit stride would put the lanes' reads on the same banks).
 template <typename Real, bool GRAD, bool PAIR, int TERM, int CLS>
 __device__ __forceinline__ void eval_class(const EvalCtx<Real>& c, const Slab<Real>& w, int q0, int n, int lane,
                                            E3<Real>& acc) {
+  static_assert(GRAD || !PAIR, "pair energies: sum_class");
   if (n == 0) return;
   int S = (n + 31) >> 5;
   if ((S & 3) == 0) ++S;
@@ -240,7 +337,6 @@ __device__ __forceinline__ void eval_class(const EvalCtx<Real>& c, const Slab<Re
   a.x = a.y = a.z = Real(0);
   a.tf = 0;
   Real fx = 0, fy = 0, fz = 0;
-  Real e0 = 0, e1 = 0, e2 = 0;
   Real wt0 = c.wt0, wt1 = c.wt1, wt2 = c.wt2;
   ElecK<Real> K;
   if (TERM == kTermElec) K = load_elec_k(c.elec_k);
@@ -258,83 +354,26 @@ __device__ __forceinline__ void eval_class(const EvalCtx<Real>& c, const Slab<Re
     if (PAIR) {
       const int sl = w.slot[j];
       if (sl != slot) {
-        if (slot >= 0 && c.energies) {
-          Real* o = c.energies + w.out[slot];
-          if (e0 != Real(0)) atomicAdd(o, e0);
-          if (TERM == kTermLJLK) {
-            if (e1 != Real(0)) atomicAdd(o + c.stride, e1);
-            if (CLS != kNear && e2 != Real(0)) atomicAdd(o + 2 * c.stride, e2);
-          }
-        }
-        e0 = e1 = e2 = 0;
         slot = sl;
-        if (GRAD) {
-          const Real* wt = c.dTdV + w.out[sl];
-          wt0 = wt[0];
-          if (TERM == kTermLJLK) {
-            wt1 = wt[c.stride];
-            wt2 = wt[2 * c.stride];
-          }
+        const Real* wt = c.dTdV + w.out[sl];
+        wt0 = wt[0];
+        if (TERM == kTermLJLK) {
+          wt1 = wt[c.stride];
+          wt2 = wt[2 * c.stride];
         }
       }
     }
     const AtomRec<Real> b = w.at[j];
     const Real dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
-    const Real d2 = dx * dx + dy * dy + dz * dz;
     const Real wcp = (e >> 13) ? Real(0.2) : Real(1);
-    // coincident atoms (d2 = 0) take the linear LJ, flat LK and flat elec
-    // regions, which never use inv_d, and add no force
-    const Real inv_d = inv_sqrt(d2);
-    const Real d = CLS == kFar || d2 > Real(0) ? d2 * inv_d : Real(0);
-    Real f;  // weighted dE/dd / d
-    if (TERM == kTermElec) {
-      const Real wq = wcp * a.q * b.q;
-      Real v, dv = 0;
-      if (CLS == kFar) {
-        const Real t = (d - K.hi_start) * K.inv_hi_w;
-        v = K.hi[0] + t * (K.hi[1] + t * (K.hi[2] + t * K.hi[3]));
-        if (GRAD) dv = (K.hi[1] + t * (Real(2) * K.hi[2] + Real(3) * t * K.hi[3])) * K.inv_hi_w;
-      } else {
-        elec_eval<Real, GRAD>(d, K, v, dv);
-      }
-      e0 += wq * v;
-      f = wq * wt0 * dv * inv_d;
-    } else {
-      const int tp = (a.tf & 0xff) * c.ntp + (b.tf & 0xff);
-      if (CLS == kFar) {
-        // both potentials fade on the same interval: a cubic from value V
-        // and (interval-scaled) slope D to zero is V A(t) + D B(t), with
-        // A = (1 - t)^2 (1 + 2 t), B = t (1 - t)^2
-        const Quad<Real> k = c.far[tp];  // LJ value, slope; LK value, slope
-        const Real t = (d - c.far_dmin) * c.inv_hf;
-        const Real u = Real(1) - t;
-        const Real uu = u * u;
-        const Real A = uu + Real(2) * t * uu, B = t * uu;
-        e0 += wcp * (k.a * A + k.b * B);
-        e2 += wcp * (k.c * A + k.d * B);
-        if (GRAD) {
-          const Real dA = Real(-6) * t * u, dB = u - Real(3) * t * u;
-          const Real V = wt0 * k.a + wt2 * k.c, D = wt0 * k.b + wt2 * k.d;
-          f = wcp * c.inv_hf * inv_d * (V * dA + D * dB);
-        }
-      } else {
-        Real atr, rep, datr, drep;
-        lj_eval<Real, GRAD>(d, inv_d, c.lj + tp, c.lj + c.ntp * c.ntp + tp, atr, rep, datr, drep);
-        e0 += wcp * atr;
-        e1 += wcp * rep;
-        Real dE = wt0 * datr + wt1 * drep;
-        if (CLS == kNearHeavy) {
-          Real lk, dlk;
-          lk_eval<Real, GRAD>(d, inv_d, c.lk + tp, c.far_dmin, c.far_first, c.inv_hf, lk, dlk);
-          e2 += wcp * lk;
-          dE += wt2 * dlk;
-        }
-        if (GRAD) f = wcp * dE * inv_d;
-      }
+    const PairTerms<Real> p = eval_pair<Real, GRAD, TERM, CLS>(c, K, a, b, dx, dy, dz, wcp, wt0, wt1, wt2);
+    if (!PAIR) {
+      acc.atr += p.e0;
+      acc.rep += p.e1;
+      acc.lk += p.e2;
     }
     if (GRAD) {
-      if (CLS != kFar && d == Real(0)) f = 0;
-      const Real px = f * dx, py = f * dy, pz = f * dz;
+      const Real px = p.f * dx, py = p.f * dy, pz = p.f * dz;
       fx += px;
       fy += py;
       fz += pz;
@@ -342,19 +381,39 @@ __device__ __forceinline__ void eval_class(const EvalCtx<Real>& c, const Slab<Re
     }
   }
   if (GRAD && row >= 0) add_force<CLS == kFar>(c.g + GRAD_STRIDE * (c.row0 + row), fx, fy, fz);
-  if (PAIR) {
-    if (slot >= 0 && c.energies) {
-      Real* o = c.energies + w.out[slot];
-      if (e0 != Real(0)) atomicAdd(o, e0);
-      if (TERM == kTermLJLK) {
-        if (e1 != Real(0)) atomicAdd(o + c.stride, e1);
-        if (CLS != kNear && e2 != Real(0)) atomicAdd(o + 2 * c.stride, e2);
-      }
+}
+
+// Pair energies: the lanes evaluate a window of a class's entries, then the
+// lane of each word (k) and term (t) adds up the word's, one after the other,
+// to v.  So a pair's energy is the same bits in every call, whichever pairs
+// share its group.  (A sum per lane, added by an atomic a lane, is not;
+// rotamers of 16 x 150 residues take 8.54 ms so and 8.44 ms with the window.
+// A sum per row and word, each held by one lane, is, but takes 12.1 ms: a class
+// of a group has two or three entries a lane, and whole rows balance badly.)
+template <typename Real, int TERM, int CLS>
+__device__ __forceinline__ void sum_class(const EvalCtx<Real>& c, Slab<Real>& w, int q0, int n, int lane, int k, int t,
+                                          Real& v) {
+  PairSums<Real>& ps = pair_sums(w);
+  ElecK<Real> K;
+  if (TERM == kTermElec) K = load_elec_k(c.elec_k);
+  const bool adds = k >= 0 && !(CLS == kFar && t == 1) && !(CLS == kNear && t == 2);
+  const int first = adds ? ps.first[CLS][k] : 0, last = adds ? ps.first[CLS][k + 1] : 0;
+  for (int base = 0; base < n; base += EWIN) {
+    const int m = min(EWIN, n - base);
+    for (int i = lane; i < m; i += 32) {
+      const int e = w.queue[q0 + base + i];
+      const AtomRec<Real> a = w.row[(e >> 8) & 31], b = w.at[e & 255];
+      const Real wcp = (e >> 13) ? Real(0.2) : Real(1);
+      const PairTerms<Real> p = eval_pair<Real, false, TERM, CLS>(c, K, a, b, a.x - b.x, a.y - b.y, a.z - b.z, wcp,
+                                                                  Real(0), Real(0), Real(0));
+      ps.e[0][i] = p.e0;
+      if (TERM == kTermLJLK && CLS != kFar) ps.e[1][i] = p.e1;
+      if (TERM == kTermLJLK && CLS != kNear) ps.e[2][i] = p.e2;
     }
-  } else {
-    acc.atr += e0;
-    acc.rep += e1;
-    acc.lk += e2;
+    __syncwarp();
+    const int end = min(last - base, m);
+    for (int i = max(first - base, 0); i < end; ++i) v += ps.e[t][i];
+    __syncwarp();
   }
 }
 
@@ -412,10 +471,11 @@ __device__ __forceinline__ void process_group(const EvalCtx<Real>& c, Slab<Real>
     for (int u0 = 0; u0 < nu; u0 += 32) {
       const int u = u0 + lane;
       unsigned F = 0, L = 0, H = 0, w02 = 0;
-      int eb = 0;
+      int eb = 0, begins = -1;
       if (u < nu) {
         const int qd = (u * inv) >> 16, rem = u - qd * div;
         const int r = PAIR ? rem : qd, k = ka + (PAIR ? qd : rem);
+        if (PAIR && rem == 0) begins = qd;
         F = w.far[r * MAXW + k];
         L = w.near[r * MAXW + k];
         if (TERM == kTermLJLK && ((heavy_rows >> r) & 1u)) {
@@ -440,6 +500,12 @@ __device__ __forceinline__ void process_group(const EvalCtx<Real>& c, Slab<Real>
       }
       const int tot = __shfl_sync(0xffffffffu, inc, 31);
       const int tot_h = TERM == kTermLJLK ? __shfl_sync(0xffffffffu, inc_h, 31) : 0;
+      if (PAIR && !GRAD && begins >= 0) {
+        PairSums<Real>& ps = pair_sums(w);
+        ps.first[kFar][begins] = (uint16_t)(of + ((inc - mine) & 0xffff));
+        ps.first[kNear][begins] = (uint16_t)(ol - n_far + ((inc - mine) >> 16));
+        ps.first[kNearHeavy][begins] = (uint16_t)(oh - n_far - n_light + inc_h - mine_h);
+      }
       uint16_t* qf = w.queue + of + ((inc - mine) & 0xffff);
       uint16_t* ql = w.queue + ol + ((inc - mine) >> 16);
       uint16_t* qh = w.queue + oh + (inc_h - mine_h);
@@ -460,11 +526,34 @@ __device__ __forceinline__ void process_group(const EvalCtx<Real>& c, Slab<Real>
       ol += tot >> 16;
       oh += tot_h;
     }
+    if (PAIR && !GRAD && lane == 0) {
+      PairSums<Real>& ps = pair_sums(w);
+      ps.first[kFar][nwr] = (uint16_t)n_far;
+      ps.first[kNear][nwr] = (uint16_t)n_light;
+      ps.first[kNearHeavy][nwr] = (uint16_t)n_heavy;
+    }
     __syncwarp();
-    eval_class<Real, GRAD, PAIR, TERM, kFar>(c, w, 0, n_far, lane, acc);
-    eval_class<Real, GRAD, PAIR, TERM, kNear>(c, w, n_far, n_light, lane, acc);
-    if (TERM == kTermLJLK)
-      eval_class<Real, GRAD, PAIR, TERM, kNearHeavy>(c, w, n_far + n_light, n_heavy, lane, acc);
+    if constexpr (PAIR && !GRAD) {
+      const int t = lane / MAXW, kw = lane % MAXW, k = kw < nwr && t < (TERM == kTermLJLK ? 3 : 1) ? kw : -1;
+      Real v = 0;
+      sum_class<Real, TERM, kFar>(c, w, 0, n_far, lane, k, t, v);
+      sum_class<Real, TERM, kNear>(c, w, n_far, n_light, lane, k, t, v);
+      if (TERM == kTermLJLK) sum_class<Real, TERM, kNearHeavy>(c, w, n_far + n_light, n_heavy, lane, k, t, v);
+      // a pair's words are next to each other and go out one after the other
+      const long long o = k >= 0 ? w.out[ka + k] : 0;
+      int nth = 0;
+      while (nth < k && w.out[ka + k - nth - 1] == o) ++nth;
+      const int most = __reduce_max_sync(0xffffffffu, nth);
+      for (int p = 0; p <= most; ++p) {
+        if (p == nth && v != Real(0)) atomicAdd(c.energies + t * c.stride + o, v);
+        __syncwarp();
+      }
+    } else {
+      eval_class<Real, GRAD, PAIR, TERM, kFar>(c, w, 0, n_far, lane, acc);
+      eval_class<Real, GRAD, PAIR, TERM, kNear>(c, w, n_far, n_light, lane, acc);
+      if (TERM == kTermLJLK)
+        eval_class<Real, GRAD, PAIR, TERM, kNearHeavy>(c, w, n_far + n_light, n_heavy, lane, acc);
+    }
     __syncwarp();
     ka = kb;
   }
@@ -620,12 +709,12 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 32 * PAIR_WARPS : 256, 1)
   if (s.done && *s.done) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  Slab<Real>& w = reinterpret_cast<Slab<Real>*>(smem_raw)[warp];
+  Slab<Real>& w = *reinterpret_cast<Slab<Real>*>(smem_raw + warp * slab_bytes<Real>(BLOCK_PAIR && !GRAD));
   const unsigned lemask = 0xffffffffu >> (31 - lane);
   const bool want_E = !GRAD || s.energies != nullptr;
   EvalCtx<Real> ec = eval_ctx(s);
   if (BLOCK_PAIR) {
-    ec.energies = want_E ? s.energies : nullptr;
+    ec.energies = s.energies;
     ec.dTdV = s.dTdV;
     ec.stride = (int64_t)s.P * s.B * s.B;
   }
