@@ -125,6 +125,68 @@ def test_pair_energies_repeat(name, rotamers, dtype, scale):
         assert torch.equal(run(), first)
 
 
+@pytest.mark.parametrize("scale", [1e-8, 1e-4, 0.3, 1.0, 1e4, 1e8])
+@pytest.mark.parametrize("name", ["ljlk", "lkball"])
+def test_gradient_spread(name, scale):
+    """Two calls' float32 gradients differ in the order of their sums alone,
+    and in the small part only: clashes' forces are summed exactly.  What is
+    left adds some 300 terms of less than one under unit weights, each sum
+    rounded by at most 2^-25: sqrt(300) x 3e-8 = 5e-7 a component, three times
+    that between the extremes of ten calls, and as much again where the last
+    addition rounds the other way: below 4e-6 of the weights' size as a root
+    mean square (one plain sum: 1.5e-5).  The scale of the loss does not
+    matter."""
+    from tmol_b200.score.lkball_energy_term import LKBallEnergyTerm, score_args, water_gen_args
+    from tmol_b200.score.lkball_op import LKBallPlan
+    from tmol_b200.score.ljlk_op import LJLKPlan
+
+    ps = synthetic_pose_stack([150] * 4, [0, 1, 2, 3], device=DEV, extra_chi_sd=30.0)
+    x = ps.coords.flatten(0, 1).contiguous()
+    if name == "ljlk":
+        plan = LJLKPlan(x, pose_score_args(ps, LJLKEnergyTerm(device=DEV))[:-1])
+        weights = torch.tensor([1.0, 0.55, 1.0], device=DEV)
+    else:
+        term = LKBallEnergyTerm(device=DEV)
+        plan = LKBallPlan(x, water_gen_args(ps, term), score_args(ps, term, None)[:-2])
+        weights = torch.tensor([-0.38, 0.92, -0.33, -0.33], device=DEV)
+    weights = (weights[:, None] * scale).expand(-1, 4).contiguous()
+    if name == "ljlk":
+        run = lambda: plan.backward(x, weights)
+    else:
+        W = plan.waters(x)
+        run = lambda: plan.backward(x, W, weights)[0]
+    G = torch.stack([run().clone() for _ in range(10)])
+    spread = (G.max(0)[0] - G.min(0)[0]).double()
+    assert float(spread.pow(2).mean().sqrt()) < 4e-6 * scale
+
+
+def test_infinite_force():
+    """A force beyond float32's range is an infinite gradient, not a NaN: one
+    atom pair of two residues brought to 1.2 A, the others farther apart."""
+    from tmol_b200.score.ljlk_op import LJLKPlan
+
+    ps = synthetic_pose_stack([4], [6], spacing=0.0)
+    args = pose_score_args(ps, LJLKEnergyTerm())
+    first = args[0].tolist() + [ps.coords.shape[1]]
+    x = ps.coords.flatten(0, 1).double()
+    u = torch.tensor([0.5, 0.8, 0.7], dtype=torch.float64)
+    a = int((x[: first[1]] @ u).argmax())
+    b = first[3] + int((x[first[3] :] @ u).argmin())
+    x[first[1] : first[3]] += torch.tensor([500.0, -500.0, 0.0], dtype=torch.float64)
+    x[first[3] :] += x[a] - x[b] + 1.2 * u / u.norm()
+    apart = x.clone()
+    apart[first[3] :] += 100.0
+    rep = torch.tensor([[0.0], [1.0], [0.0]], dtype=torch.float64, device=DEV)
+    plan64 = LJLKPlan(x.to(DEV), on_gpu(args, torch.float64)[:-1])
+    g, rest = plan64.backward(x.to(DEV), rep)[[a, b]], plan64.backward(apart.to(DEV), rep)[[a, b]]
+    top = torch.finfo(torch.float32).max
+    w = 1.5 * top / float(g.abs().min())
+    assert float(rest.abs().max()) * w < top / 4 and w < top
+    plan = LJLKPlan(x.float().to(DEV), on_gpu(args, torch.float32)[:-1])
+    got = plan.backward(x.float().to(DEV), rep * w)[[a, b]]
+    assert torch.equal(got, torch.sign(g).float() * float("inf"))
+
+
 def test_no_common_fade_interval():
     """A type whose LJ minimum lies inside the fade interval fades on an
     interval of its own: the general path serves every pair.  (Energies, from

@@ -794,8 +794,11 @@ __device__ TMOL_B200_LKB_DRAIN_ATTR Lkb4<Real> lkb_drain(const LkbEval<Real> ev,
   if (GRAD) {
     // vector reductions: the thirty values of a pair as scalar ones took the
     // path to L2 longer than the pair's arithmetic
-    if (gI[0] != Real(0) || gI[1] != Real(0) || gI[2] != Real(0)) add_force(ev.g4 + GRAD_STRIDE * rp, gI[0], gI[1], gI[2]);
-    if (gJ[0] != Real(0) || gJ[1] != Real(0) || gJ[2] != Real(0)) add_force(ev.g4 + GRAD_STRIDE * ro, gJ[0], gJ[1], gJ[2]);
+    const Real grid = force_grid_of(fmax(fmax(fabs(w.v[0]), fabs(w.v[1])), fmax(fabs(w.v[2]), fabs(w.v[3]))));
+    if (gI[0] != Real(0) || gI[1] != Real(0) || gI[2] != Real(0))
+      add_force(ev.g4 + GRAD_STRIDE * rp, grid, gI[0], gI[1], gI[2]);
+    if (gJ[0] != Real(0) || gJ[1] != Real(0) || gJ[2] != Real(0))
+      add_force(ev.g4 + GRAD_STRIDE * ro, grid, gJ[0], gJ[1], gJ[2]);
     lkb_add_waters(ev.dwaters, rp, ev.vec_dw, gWI);
     lkb_add_waters(ev.dwaters, ro, ev.vec_dw, gWJ);
   }

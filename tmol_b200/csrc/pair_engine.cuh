@@ -129,6 +129,7 @@ struct EvalCtx {
   Real max2, far2;        // squares of the cutoff and of the far class's start
   Real far_dmin, far_first, inv_hf;
   Real wt0, wt1, wt2;     // gradient weights of the three terms (elec: wt0)
+  Real grid;              // force_grid_of them
   Real* g;                // padded gradient [n_atoms][GRAD_STRIDE]
   int64_t row0;           // global atom index of row 0
   Real* energies;         // pair mode: [n_terms][stride]
@@ -142,29 +143,43 @@ struct EvalCtx {
 // in any order; what remains of a force goes to the second, whose sums stay
 // small.  A single float32 sum of forty signed terms in no fixed order, where
 // clashes of 10^3 kcal/mol/A nearly cancel, differs by 3e-4 from call to call.
-// SMALL: a force of the far class (well below one), to the second group alone.
+// These figures are for forces of up to 2^16 under weights of about one; the
+// grid scales with the power of two of the largest weight, so that they hold
+// relative to the weights whatever the caller's loss is multiplied by.
+// (Larger forces, and weights of unlike size on one atom, are summed right but
+// on coarser or several grids.)
+// SMALL: a force of the far class (about one, weighted alike), to the second
+// group alone.
 constexpr int GRAD_STRIDE = 8;
+
+// What force_grid rounds with: 1.5 x 2^17 (float32 spacing 2^-6) times the
+// power of two at or below the largest weight's magnitude m.
+__device__ __forceinline__ float force_grid_of(float m) {
+  return 1.5f * 131072.0f * __uint_as_float(__float_as_uint(fminf(m, 0x1p100f)) & 0x7f800000u);
+}
+__device__ __forceinline__ double force_grid_of(double) { return 0.0; }  // not split
 
 __device__ __forceinline__ void red4(float* g, float x, float y, float z) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g), "f"(x), "f"(y), "f"(z), "f"(0.0f)
                : "memory");
 }
-__device__ __forceinline__ float force_grid(float x) {
-  const float c = 1.5f * 131072.0f;  // 1.5 x 2^17: float32 spacing 2^-6
-  return __fsub_rn(__fadd_rn(x, c), c);
+// The part of x on the grid; none of an infinite x, whose remainder would be a NaN.
+__device__ __forceinline__ float on_grid(float x, float grid) {
+  const float h = __fsub_rn(__fadd_rn(x, grid), grid);
+  return fabsf(x) < 0x1p127f ? h : 0.0f;
 }
 template <bool SMALL = false>
-__device__ __forceinline__ void add_force(float* g, float x, float y, float z) {
+__device__ __forceinline__ void add_force(float* g, float grid, float x, float y, float z) {
   if (SMALL) {
     red4(g + 4, x, y, z);
     return;
   }
-  const float hx = force_grid(x), hy = force_grid(y), hz = force_grid(z);
+  const float hx = on_grid(x, grid), hy = on_grid(y, grid), hz = on_grid(z, grid);
   if (hx != 0.0f || hy != 0.0f || hz != 0.0f) red4(g, hx, hy, hz);
   red4(g + 4, __fsub_rn(x, hx), __fsub_rn(y, hy), __fsub_rn(z, hz));
 }
 template <bool SMALL = false>
-__device__ __forceinline__ void add_force(double* g, double x, double y, double z) {
+__device__ __forceinline__ void add_force(double* g, double, double x, double y, double z) {
   atomicAdd(g, x);
   atomicAdd(g + 1, y);
   atomicAdd(g + 2, z);
@@ -254,6 +269,11 @@ __device__ __forceinline__ RowTest test_row(const Slab<double>& w, int base, int
 
 enum PairClass : int { kFar = 0, kNear = 1, kNearHeavy = 2 };
 
+template <typename Real, int TERM>
+__device__ __forceinline__ Real grid_of_weights(Real wt0, Real wt1, Real wt2) {
+  return force_grid_of(TERM == kTermElec ? fabs(wt0) : fmax(fabs(wt0), fmax(fabs(wt1), fabs(wt2))));
+}
+
 // One pair of a class: its energies, weighted by its count-pair weight wcp,
 // and the force f (a - b) on a, (weighted dE/dd) / d.
 template <typename Real>
@@ -337,7 +357,7 @@ __device__ __forceinline__ void eval_class(const EvalCtx<Real>& c, const Slab<Re
   a.x = a.y = a.z = Real(0);
   a.tf = 0;
   Real fx = 0, fy = 0, fz = 0;
-  Real wt0 = c.wt0, wt1 = c.wt1, wt2 = c.wt2;
+  Real wt0 = c.wt0, wt1 = c.wt1, wt2 = c.wt2, grid = c.grid;
   ElecK<Real> K;
   if (TERM == kTermElec) K = load_elec_k(c.elec_k);
   for (int s = 0; s < cnt; ++s) {
@@ -345,7 +365,7 @@ __device__ __forceinline__ void eval_class(const EvalCtx<Real>& c, const Slab<Re
     const int j = e & 255, r = (e >> 8) & 31;
     if (r != row) {
       if (GRAD && row >= 0) {
-        add_force<CLS == kFar>(c.g + GRAD_STRIDE * (c.row0 + row), fx, fy, fz);
+        add_force<CLS == kFar>(c.g + GRAD_STRIDE * (c.row0 + row), grid, fx, fy, fz);
         fx = fy = fz = 0;
       }
       row = r;
@@ -361,6 +381,7 @@ __device__ __forceinline__ void eval_class(const EvalCtx<Real>& c, const Slab<Re
           wt1 = wt[c.stride];
           wt2 = wt[2 * c.stride];
         }
+        grid = grid_of_weights<Real, TERM>(wt0, wt1, wt2);
       }
     }
     const AtomRec<Real> b = w.at[j];
@@ -377,10 +398,10 @@ __device__ __forceinline__ void eval_class(const EvalCtx<Real>& c, const Slab<Re
       fx += px;
       fy += py;
       fz += pz;
-      add_force<CLS == kFar>(c.g + GRAD_STRIDE * (int64_t)w.gidx[j], -px, -py, -pz);
+      add_force<CLS == kFar>(c.g + GRAD_STRIDE * (int64_t)w.gidx[j], grid, -px, -py, -pz);
     }
   }
-  if (GRAD && row >= 0) add_force<CLS == kFar>(c.g + GRAD_STRIDE * (c.row0 + row), fx, fy, fz);
+  if (GRAD && row >= 0) add_force<CLS == kFar>(c.g + GRAD_STRIDE * (c.row0 + row), grid, fx, fy, fz);
 }
 
 // Pair energies: the lanes evaluate a window of a class's entries, then the
@@ -684,7 +705,7 @@ __device__ __forceinline__ EvalCtx<Real> eval_ctx(const ScoreArgs<Real>& s) {
   c.far_dmin = s.g.max_dis - Real(1.5);
   c.far_first = c.far_dmin > Real(4.5) ? c.far_dmin : Real(4.5);
   c.inv_hf = Real(1) / (s.g.max_dis - c.far_dmin);
-  c.wt0 = c.wt1 = c.wt2 = 0;
+  c.wt0 = c.wt1 = c.wt2 = c.grid = 0;
   c.g = s.g4;
   c.row0 = 0;
   c.energies = nullptr;
@@ -760,6 +781,7 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 32 * PAIR_WARPS : 256, 1)
           ec.wt1 = s.dTdV[s.P + p];
           ec.wt2 = s.dTdV[2 * s.P + p];
         }
+        ec.grid = grid_of_weights<Real, TERM>(ec.wt0, ec.wt1, ec.wt2);
       }
       const Real reach1 = sph1.d + s.g.max_dis;
       const Real reach1_2 = reach1 * reach1 * Real(1.0001);
