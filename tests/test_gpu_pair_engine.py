@@ -187,6 +187,55 @@ def test_infinite_force():
     assert torch.equal(got, torch.sign(g).float() * float("inf"))
 
 
+def test_plan_memory():
+    """Plans of one size after another, some alive, map no device memory; a
+    plan freed with its call still queued hands its memory on only after it;
+    what plans gave back beyond 64 MB, and all of it after the last plan, goes
+    back to the device (which the pool does in pieces of 32 MB)."""
+    import gc
+
+    from tmol_b200.score.ljlk_op import LJLKPlan
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info(DEV)[0]
+
+    clear_plan_cache()
+    gc.collect()
+    ps = synthetic_pose_stack([100] * 8, list(range(8)), device=DEV)
+    x = ps.coords.flatten(0, 1).contiguous()
+    args = pose_score_args(ps, LJLKEnergyTerm(device=DEV))[:-1]
+    weights = torch.ones(3, 8, device=DEV)
+    warm = LJLKPlan(x, args)
+    E, g = warm.energy_and_gradient(x, weights)
+    del warm
+    plans = [LJLKPlan(x, args) for _ in range(3)]
+    held = free()
+    for k in range(12):
+        plans[k % 3] = None
+        assert free() == held
+        plans[k % 3] = LJLKPlan(x, args)
+        assert free() == held
+    out, dx = torch.empty_like(E), torch.empty_like(g)
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(other):
+        torch.cuda._sleep(20_000_000)
+        plans[0].energy_and_gradient(x, weights, out, dx)
+    plans[0] = None
+    plans[0] = LJLKPlan(x + 1.0, args)
+    plans[0].energy_and_gradient(x + 1.0, weights * 0.5)
+    torch.cuda.synchronize()
+    assert torch.allclose(out, E, rtol=1e-5) and torch.allclose(dx, g, rtol=1e-4, atol=1e-4)
+    held = free()  # some of it torch's for the second stream
+    many = [LJLKPlan(x, args) for _ in range(100)]
+    assert many[0].device_bytes() * 100 > 3 * (64 << 20)
+    del many
+    assert held - free() <= 64 << 20
+    plans.clear()
+    assert free() - held >= 32 << 20
+
+
 def test_no_common_fade_interval():
     """A type whose LJ minimum lies inside the fade interval fades on an
     interval of its own: the general path serves every pair.  (Energies, from

@@ -29,6 +29,8 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <vector>
 
 #include "../../include/tmol_b200_elec.h"
@@ -1282,6 +1284,12 @@ __global__ void fp32_peak_kernel(float* out, int iters, float a, float b) {
 
 using namespace tmol_b200;
 
+// A buffer from its device's pool of plan memory.
+struct PoolBlock {
+  void* p = nullptr;
+  size_t bytes = 0;
+};
+
 struct tmol_b200_ljlk_plan {
   int real_bytes;
   int term = kTermLJLK;
@@ -1360,7 +1368,11 @@ struct tmol_b200_ljlk_plan {
   // kernel timing: event pairs around each scoring-kernel launch
   bool profiling = false;
   std::vector<std::pair<void**, size_t>> to_place;  // buffers asked for and not yet placed
-  std::vector<void*> blocks;                        // the device allocations they lie in
+  std::vector<PoolBlock> blocks;                    // the device allocations they lie in
+  PoolBlock work_blocks[2];                         // of work and item_cost
+  cudaMemPool_t pool = nullptr;                     // which come from here
+  void* fence = nullptr;                            // a small one of its own
+  int device = 0;
   std::vector<cudaEvent_t> prof_events;
   int prof_n = 0;
   tmol_b200_ljlk_launch launch;
@@ -1393,12 +1405,104 @@ namespace {
     if (e_ != cudaSuccess) return TMOL_B200_ERR_CUDA; \
   } while (0)
 
+// Plans' memory: a pool of each device, shared by its plans.  Mapping and
+// unmapping device pages costs a few hundred microseconds a plan, more than
+// the other work of a small one, and every new topology or rotamer set is a
+// new plan.  First call with a new topology, plan cache full, with a plan's
+// blocks from cudaMalloc and from the pool: LK-ball, 8 x 100 residues 4.6 and
+// 2.8 ms; LJ/LK block pairs, 16 x 150 4.1 and 3.0 ms; LJ/LK, 64 x 150 5.5 and
+// 3.6 ms.  What plans give back is kept for the next ones, up to POOL_KEEP
+// bytes (the driver maps 32 MB at a time), and not at all once the last plan is
+// gone.
+struct PlanPool {
+  cudaMemPool_t pool = nullptr;
+  int plans = 0;
+  size_t used = 0;  // bytes that plans hold
+  void* page = nullptr;  // keeps the page of the plans' fences mapped
+};
+constexpr size_t POOL_KEEP = (size_t)64 << 20;
+constexpr size_t FENCE_BYTES = 256;
+// by device; never destroyed, since plans may outlive the library's statics
+std::mutex& plan_pools_lock = *new std::mutex;
+std::map<int, PlanPool>& plan_pools = *new std::map<int, PlanPool>;
+
+cudaError_t join_pool(tmol_b200_ljlk_plan* pl, int dev) {
+  std::lock_guard<std::mutex> hold(plan_pools_lock);
+  PlanPool& pp = plan_pools[dev];
+  if (!pp.pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool;
+    cudaError_t e = cudaMemPoolCreate(&pool, &props);
+    if (e != cudaSuccess) return e;
+    // given back by leave_pool, not at whichever synchronisation comes next
+    uint64_t all = UINT64_MAX;
+    e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &all);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return e;
+    }
+    pp.pool = pool;
+  }
+  if (!pp.page) {
+    const cudaError_t e = cudaMalloc(&pp.page, FENCE_BYTES);
+    if (e != cudaSuccess) return e;
+  }
+  ++pp.plans;
+  pl->pool = pp.pool;
+  pl->device = dev;
+  return cudaSuccess;
+}
+
+// trim: give back what the pool need not keep.
+void leave_pool(const tmol_b200_ljlk_plan* pl, bool trim) {
+  std::lock_guard<std::mutex> hold(plan_pools_lock);
+  PlanPool& pp = plan_pools[pl->device];
+  --pp.plans;
+  if (!trim) return;
+  cudaMemPoolTrimTo(pp.pool, pp.plans > 0 ? pp.used + POOL_KEEP : 0);
+  if (pp.plans == 0) {
+    cudaFree(pp.page);
+    pp.page = nullptr;
+  }
+}
+
+cudaError_t pool_alloc(tmol_b200_ljlk_plan* pl, PoolBlock* b, size_t bytes, cudaStream_t st) {
+  const cudaError_t e = cudaMallocFromPoolAsync(&b->p, bytes, pl->pool, st);
+  if (e != cudaSuccess) return e;
+  b->bytes = bytes;
+  std::lock_guard<std::mutex> hold(plan_pools_lock);
+  plan_pools[pl->device].used += bytes;
+  return cudaSuccess;
+}
+
+// Waits until the device has done what was asked of it, as the pool, which
+// hands freed buffers out again to whichever stream comes next, does not:
+// cudaFree of an allocation that is not the pool's waits, and is allowed or
+// refused beside a stream capture as the plan's own frees would be.
+cudaError_t fence(tmol_b200_ljlk_plan* pl) {
+  if (!pl->fence) return cudaSuccess;
+  const cudaError_t e = cudaFree(pl->fence);
+  if (e == cudaSuccess) pl->fence = nullptr;
+  return e;
+}
+
+// Frees buffers of a plan, after a fence.
+void pool_free(const tmol_b200_ljlk_plan* pl, PoolBlock* b, size_t n) {
+  size_t bytes = 0;
+  for (size_t k = 0; k < n; ++k) {
+    if (b[k].p) cudaFree(b[k].p);
+    bytes += b[k].bytes;
+    b[k] = PoolBlock{};
+  }
+  std::lock_guard<std::mutex> hold(plan_pools_lock);
+  plan_pools[pl->device].used -= bytes;
+}
+
 // A plan's buffers are asked for with dalloc and placed, all that are asked
-// for since the last time, in one device allocation by dplace: each allocation
-// that needs new pages, or whose end leaves one empty, maps or unmaps them.
-// First call with a new LJ/LK topology, 64 x 150 residues: 4.0 ms with an
-// allocation per buffer (also with blocks of 64 KB to 2 MB), 2.6 ms with one;
-// an LK-ball plan of that size 8.9 and 6.3 ms.
+// for since the last time, in one allocation by dplace.
 template <typename T>
 void dalloc(tmol_b200_ljlk_plan* pl, T** p, size_t n) {
   const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
@@ -1406,15 +1510,15 @@ void dalloc(tmol_b200_ljlk_plan* pl, T** p, size_t n) {
   pl->to_place.push_back({(void**)p, bytes});
 }
 
-cudaError_t dplace(tmol_b200_ljlk_plan* pl) {
+cudaError_t dplace(tmol_b200_ljlk_plan* pl, cudaStream_t st) {
   size_t total = 0;
   for (const auto& r : pl->to_place) total += (r.second + 255) / 256 * 256;
   if (total == 0) return cudaSuccess;
-  void* base = nullptr;
-  const cudaError_t e = cudaMalloc(&base, total);
+  PoolBlock block;
+  const cudaError_t e = pool_alloc(pl, &block, total, st);
   if (e != cudaSuccess) return e;
-  pl->blocks.push_back(base);
-  char* at = (char*)base;
+  pl->blocks.push_back(block);
+  char* at = (char*)block.p;
   for (const auto& r : pl->to_place) {
     *r.first = at;
     at += (r.second + 255) / 256 * 256;
@@ -1431,9 +1535,15 @@ int status_from_bits(int bits) {
 }
 
 void free_plan(tmol_b200_ljlk_plan* pl) {
-  for (void* p : pl->blocks) cudaFree(p);
-  if (pl->work) cudaFree(pl->work);
-  if (pl->item_cost) cudaFree(pl->item_cost);
+  if (pl->pool) {
+    // refused beside a capture: the buffers stay where they are
+    const bool done = fence(pl) == cudaSuccess;
+    if (done) {
+      pool_free(pl, pl->work_blocks, 2);
+      pool_free(pl, pl->blocks.data(), pl->blocks.size());
+    }
+    leave_pool(pl, done);
+  }
   for (cudaEvent_t e : pl->prof_events) cudaEventDestroy(e);
   delete pl;
 }
@@ -1503,15 +1613,20 @@ int build_work(tmol_b200_ljlk_plan* pl, cudaStream_t st) {
       for (int c = r; c < nb; c += pl->launch.candidates_per_item)
         work.push_back(make_int4(p, r, c, std::min(nb, c + pl->launch.candidates_per_item)));
   }
-  if (pl->work) cudaFree(pl->work);
-  if (pl->item_cost) cudaFree(pl->item_cost);
+  if (pl->work) {
+    CK(fence(pl));
+    pool_free(pl, pl->work_blocks, 2);
+  }
   pl->work = nullptr;
   pl->item_cost = nullptr;
   pl->n_work = (int)work.size();
   // room for the items plan_rebalance splits off the heaviest ones
   pl->work_cap = pl->n_work + pl->n_work / 2 + 64;
-  CK(cudaMalloc((void**)&pl->work, (size_t)pl->work_cap * sizeof(int4)));
-  CK(cudaMalloc((void**)&pl->item_cost, (size_t)pl->work_cap * sizeof(int)));
+  if (!pl->fence) CK(cudaMalloc(&pl->fence, FENCE_BYTES));
+  CK(pool_alloc(pl, &pl->work_blocks[0], (size_t)pl->work_cap * sizeof(int4), st));
+  CK(pool_alloc(pl, &pl->work_blocks[1], (size_t)pl->work_cap * sizeof(int), st));
+  pl->work = (int4*)pl->work_blocks[0].p;
+  pl->item_cost = (int*)pl->work_blocks[1].p;
   CK(cudaMemsetAsync(pl->item_cost, 0, (size_t)pl->work_cap * sizeof(int), st));
   if (!work.empty())
     CK(cudaMemcpyAsync(pl->work, work.data(), work.size() * sizeof(int4),
@@ -2186,7 +2301,7 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
     const int n_blocks = pl->rotamers ? pl->R : pl->P * pl->B;
     dalloc(pl, &pl->hmeta, (size_t)std::max(nbt, 1) * maxocc);
     dalloc(pl, &pl->hbase, n_blocks);
-    CK(dplace(pl));
+    CK(dplace(pl, st));
     CK(cudaMemcpyAsync(pl->lkb_npol, hnpol.data(), sizeof(int) * hnpol.size(), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(pl->lkb_nocc, hnocc.data(), sizeof(int) * hnocc.size(), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(pl->lkb_par, par.data(), sizeof(Real) * par.size(), cudaMemcpyHostToDevice, st));
@@ -2225,7 +2340,7 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
     dalloc(pl, &pl->spec_flag, 1);
   }
   if (!waters) {
-    CK(dplace(pl));
+    CK(dplace(pl, st));
     return TMOL_B200_OK;
   }
   const int64_t n_sites = pl->N * LKB_NW;
@@ -2235,7 +2350,7 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
     dalloc(pl, (Real**)&pl->lkb_dwaters, (size_t)n_sites * 3);
   }
   dalloc(pl, (LkbSite<Real>**)&pl->lkb_sites, (size_t)n_sites);
-  CK(dplace(pl));
+  CK(dplace(pl, st));
   CK(cudaMemsetAsync(pl->lkb_sites, 0, sizeof(LkbSite<Real>) * std::max<int64_t>(n_sites, 1), st));
   const int64_t PB = (int64_t)pl->P * pl->B;
   if (PB > 0 && nbt > 0 && k->n_rots > 0) {
@@ -2285,7 +2400,7 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
     if (h_sites[i].kind != kLkbNone) active.push_back((int)i);
   pl->lkb_n_active = (int64_t)active.size();
   dalloc(pl, &pl->lkb_active, active.size());
-  CK(dplace(pl));
+  CK(dplace(pl, st));
   if (!active.empty())
     CK(cudaMemcpyAsync(pl->lkb_active, active.data(), sizeof(int) * active.size(), cudaMemcpyHostToDevice, st));
   if (scoring && n_sites > 0)
@@ -2415,6 +2530,8 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     }                                  \
   } while (0)
   PCK(cudaGetDevice(&dev));
+  PCK(join_pool(pl, dev));
+  PCK(cudaMalloc(&pl->fence, FENCE_BYTES));
   PCK(cudaDeviceGetAttribute(&pl->n_sm, cudaDevAttrMultiProcessorCount, dev));
   PCK(real_bytes == 4 ? set_smem_limits<float>(term) : set_smem_limits<double>(term));
   const int64_t PB = (int64_t)P * B;
@@ -2475,7 +2592,7 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     dalloc(pl, &pl->row_pairs, PB + 2);
     dalloc(pl, &pl->row_items, PB);
   }
-  PCK(dplace(pl));
+  PCK(dplace(pl, st));
 
   if (scoring) PCK(cudaMemsetAsync(pl->real_atom, 0, std::max<int64_t>(in->n_atoms, 1), st));
   if (term == kTermElec && nbt > 0 && A > 0)
@@ -2629,7 +2746,7 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
     return TMOL_B200_ERR_CAPACITY;
   }
   if (nbt > 0 && n_masks > 0) dalloc(pl, &pl->pmask, n_masks);
-  PCK(dplace(pl));
+  PCK(dplace(pl, st));
   PCK(cudaMemcpyAsync(pl->type_map, type_map.data(), sizeof(int) * type_map.size(), cudaMemcpyHostToDevice, st));
   if (pl->ntp > 0)
     PCK(cudaMemcpyAsync(pl->compact_types, compact.data(), sizeof(int) * pl->ntp,
