@@ -31,6 +31,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "../../include/tmol_b200_elec.h"
@@ -3202,6 +3203,37 @@ int tmol_b200_measure_fp32_peak(void* stream, double* tflops) {
   return TMOL_B200_OK;
 }
 
+namespace {
+
+// The items' indices by descending cost (>= 0), equal ones in order: a radix
+// sort, 11 bits a pass, which passes over digits that all items share.  The
+// drop-in ops' first two calls of a plan end with one, and a small batch has
+// many items: with 5 500 of them (8 x 100 residues) a rebalance takes 590 us
+// with std::stable_sort and 280 us with this.
+std::vector<int> costliest_first(const std::vector<int>& cost) {
+  struct Item {
+    unsigned key;
+    int index;
+  };
+  const size_t n = cost.size();
+  std::vector<Item> items(n), next(n);
+  for (size_t i = 0; i < n; ++i) items[i] = Item{0x7fffffffu - (unsigned)cost[i], (int)i};
+  for (int shift = 0; shift < 31; shift += 11) {
+    unsigned at[2048] = {};
+    for (const Item& x : items) ++at[(x.key >> shift) & 2047];
+    if (n == 0 || at[(items[0].key >> shift) & 2047] == n) continue;
+    unsigned sum = 0;
+    for (unsigned& c : at) sum += std::exchange(c, sum);
+    for (const Item& x : items) next[at[(x.key >> shift) & 2047]++] = x;
+    items.swap(next);
+  }
+  std::vector<int> order(n);
+  for (size_t i = 0; i < n; ++i) order[i] = items[i].index;
+  return order;
+}
+
+}  // namespace
+
 int tmol_b200_ljlk_plan_rebalance(tmol_b200_ljlk_plan* plan, void* stream) {
   NvtxRange nvtx_range("tmol_b200_ljlk_plan_rebalance");
   if (!plan) return TMOL_B200_ERR_INVALID_ARGUMENT;
@@ -3235,10 +3267,8 @@ int tmol_b200_ljlk_plan_rebalance(tmol_b200_ljlk_plan* plan, void* stream) {
     }
   }
   n = (int)work.size();
-  std::vector<int> order(n);
-  for (int i = 0; i < n; ++i) order[i] = i;
   // longest items first, so that the last items any warp takes are short
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+  const std::vector<int> order = costliest_first(cost);
   std::vector<int4> sorted(n);
   std::vector<int> sorted_cost(n);
   for (int i = 0; i < n; ++i) {
