@@ -2,15 +2,15 @@
 
 The tunables are the fields of ``tmol_b200_ljlk_launch``: work items per
 ticket, warps per CTA, CTAs per SM, candidate blocks per work item (how a
-row's block pairs are partitioned into work items) and neighbouring blocks
-per screening group (how many block pairs share one pass of a warp's 32
-lanes: the kernel's "threads per block pair"); and the order of the work
-items (longest-first by measured cost, see ``LJLKPlan.rebalance``).  Each
-candidate shape is timed with the library's CUDA events around the scoring
-kernel; the winner is cached in a JSON file keyed by GPU name and a
-signature of the workload (poses, block slots, real blocks per pose and
-the histogram of atoms per block), so a later plan for a similar PoseStack
-starts from it.
+row's block pairs are partitioned into work items) and block pairs per group
+(of calls that keep their energies apart; whole-pose calls have no such
+limit); and the order of the work items (longest-first by measured cost, see
+``LJLKPlan.rebalance``).  Each candidate shape is timed with the library's
+CUDA events around the scoring kernel; the winner is cached in a JSON file
+keyed by GPU name, the kernels the shapes are for (``KERNELS``) and a
+signature of the workload (poses, block slots, real blocks per pose and the
+histogram of atoms per block), so a later plan for a similar PoseStack starts
+from it.
 
 Cache file: ``$TMOL_B200_TUNE_CACHE`` or ``~/.cache/tmol_b200/launch.json``.
 """
@@ -39,6 +39,11 @@ def launch_shapes(grid):
     ):
         yield (rows, warps, ctas, cands, slots)
 
+
+# names the kernels that a cached shape was tuned for: changed with them, or
+# their launch shapes, so that older entries are left alone
+KERNELS = "pair engine"
+
 # atoms per block: histogram bin edges of the signature
 SIZE_BINS = (8, 16, 24, 32)
 
@@ -65,7 +70,7 @@ def block_size_summary(plan):
 
 
 def signature(plan):
-    """The cache key: GPU, term, dtype, poses and block slots, and the
+    """The cache key: GPU, kernels, term, dtype, poses and block slots, and the
     block-size summary (real blocks per pose to the nearest 10, mean atoms
     per block to the nearest atom, the size histogram to the nearest 5 %)."""
     name = torch.cuda.get_device_name(plan.device)
@@ -73,7 +78,7 @@ def signature(plan):
     per_pose, mean_atoms, hist = block_size_summary(plan)
     h = ",".join(f"{round(20 * x) * 5}" for x in hist)
     return (
-        f"{name}|{term}|{plan.dtype}|P={plan.n_poses}|B={plan.max_n_blocks}|"
+        f"{name}|{KERNELS}|{term}|{plan.dtype}|P={plan.n_poses}|B={plan.max_n_blocks}|"
         f"blocks/pose={10 * round(per_pose / 10)}|atoms/block={mean_atoms:.0f}|sizes%={h}"
     )
 
