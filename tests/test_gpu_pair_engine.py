@@ -10,6 +10,8 @@ component's magnitude allows by a factor of ten or so, so its float64 sum is
 good to 1e-12 of the largest component (2.2e-16 x a few thousand); energies
 likewise to 1e-11 relative."""
 
+import json
+
 import numpy
 import pytest
 import torch
@@ -185,6 +187,37 @@ def test_infinite_force():
     plan = LJLKPlan(x.float().to(DEV), on_gpu(args, torch.float32)[:-1])
     got = plan.backward(x.float().to(DEV), rep * w)[[a, b]]
     assert torch.equal(got, torch.sign(g).float() * float("inf"))
+
+
+@pytest.mark.parametrize("name", ["ljlk", "elec"])
+def test_default_launch_again(name, tmp_path):
+    """set_launch with zeros is the launch shape a plan is made with."""
+    from torch.profiler import ProfilerActivity, profile
+
+    from tmol_b200.score.elec_op import ElecPlan
+    from tmol_b200.score.ljlk_op import LJLKPlan
+
+    many = synthetic_pose_stack([200] * 8, list(range(8)))
+    args = {"ljlk": pose_score_args, "elec": elec_pose_score_args}[name](
+        many, {"ljlk": LJLKEnergyTerm, "elec": ElecEnergyTerm}[name]()
+    )
+    x = many.coords.flatten(0, 1).to(DEV).contiguous()
+    plan = {"ljlk": LJLKPlan, "elec": ElecPlan}[name](x, on_gpu(args, torch.float32)[:-1])
+
+    def blocks():
+        plan.forward(x)
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            plan.forward(x)
+            torch.cuda.synchronize()
+        prof.export_chrome_trace(str(tmp_path / "trace.json"))
+        events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
+        return [e["args"]["block"] for e in events if "score_kernel" in e.get("name", "")]
+
+    made = blocks()
+    if not made:
+        pytest.skip("no kernel trace on this machine")
+    plan.set_launch()
+    assert blocks() == made
 
 
 def test_plan_memory():

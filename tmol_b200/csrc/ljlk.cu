@@ -1566,6 +1566,12 @@ int auto_candidates(const tmol_b200_ljlk_plan* pl) {
 
 void default_launch(const tmol_b200_ljlk_plan* pl, tmol_b200_ljlk_launch& l) {
   if (l.rows_per_item <= 0) l.rows_per_item = 1;
+  // float plans of LJ/LK and elec: one CTA of PAIR_WARPS warps per SM unless
+  // the caller chose
+  if (pl->real_bytes == 4 && pl->term != kTermLKBall && l.warps_per_cta <= 0 && l.ctas_per_sm <= 0) {
+    l.warps_per_cta = PAIR_WARPS;
+    l.ctas_per_sm = 1;
+  }
   if (l.warps_per_cta <= 0) l.warps_per_cta = 8;
   if (l.ctas_per_sm <= 0) l.ctas_per_sm = 2;
   if (l.candidates_per_item <= 0) l.candidates_per_item = auto_candidates(pl);
@@ -2512,13 +2518,6 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   pl->N = in->n_atoms;
   pl->reach = in->max_dis;
   pl->launch = launch ? *launch : tmol_b200_ljlk_launch{0, 0, 0, 0};
-  // float plans of LJ/LK and elec: one CTA of PAIR_WARPS warps per SM unless
-  // the caller chose
-  if (real_bytes == 4 && term != kTermLKBall && pl->launch.warps_per_cta <= 0 &&
-      pl->launch.ctas_per_sm <= 0) {
-    pl->launch.warps_per_cta = PAIR_WARPS;
-    pl->launch.ctas_per_sm = 1;
-  }
   const bool chose_candidates = pl->launch.candidates_per_item > 0;
   default_launch(pl, pl->launch);
   int dev = 0;
