@@ -105,7 +105,6 @@ struct PlanBuildArgs {
   int* bt_flags;  // heavy flag per bt-atom (before type flags are merged)
   int* cp_count;
   int* cp_b2;
-  int* cp_minsep;
   uint8_t* cp_seps;
   int* status;
   int rotamers;  // rotamer plan: blocks may own any number of rotamers
@@ -176,8 +175,6 @@ __global__ void plan_blocks_kernel(PlanBuildArgs a) {
   }
 }
 
-// Rotamer plan: per rotamer, its pose, block, block type and coordinates
-// must be in range and the rotamer must lie in its block's range.
 // One record per block slot for the scoring kernel's row and neighbour
 // loads: {block type or -1, first atom, atom count, connections | ligand
 // flag << 8}, from the validated block tables; counts are held to the tables'
@@ -196,6 +193,8 @@ __global__ void plan_block_info_kernel(int64_t n, const int* blk_bt, const int* 
   }
 }
 
+// Rotamer plan: per rotamer, its pose, block, block type and coordinates
+// must be in range and the rotamer must lie in its block's range.
 __global__ void plan_rotamers_kernel(PlanBuildArgs a) {
   const tmol_b200_ljlk_inputs& in = a.in;
   const int P = in.n_poses, B = in.max_n_blocks;
@@ -414,18 +413,13 @@ __global__ void plan_count_pair_kernel(PlanBuildArgs a) {
       for (int base = b1 + 1; base < B; base += 32) {
         int b2 = base + lane;
         bool hit = false;
-        int ms = 0;
-        if (b2 < B && a.blk_bt[p * B + b2] >= 0) {
-          ms = mrow[b2];
-          hit = ms <= 4;
-        }
+        if (b2 < B && a.blk_bt[p * B + b2] >= 0) hit = mrow[b2] <= 4;
         unsigned m = __ballot_sync(0xffffffffu, hit);
         if (hit) {
           int slot = cnt + __popc(m & ((1u << lane) - 1));
           if (slot < CP_CAP) {
             int64_t e = (int64_t)row * CP_CAP + slot;
             a.cp_b2[e] = b2;
-            a.cp_minsep[e] = ms;
             const int32_t* s =
                 in.inter_block_bondsep + (((int64_t)p * B + b1) * B + b2) * C * C;
             for (int c1 = 0; c1 < MAX_CONN; ++c1)
@@ -499,7 +493,6 @@ __global__ void plan_count_pair_conn_kernel(PlanBuildArgs a) {
         if (cnt < CP_CAP) {
           const int64_t e = (int64_t)row * CP_CAP + cnt;
           a.cp_b2[e] = part_b2[best];
-          a.cp_minsep[e] = part_min[best];
           for (int k = 0; k < 16; ++k) a.cp_seps[e * 16 + k] = part_sep[best][k];
         } else {
           atomicOr(a.status, kStCapacity);
@@ -568,14 +561,12 @@ struct ScoreArgs {
   // the gradient as [n_atoms][GRAD_STRIDE], zeroed by the sphere pass
   // and copied out by grad_out_kernel
   Real* g4;
-  const uint8_t* bt_pd;
   const uint8_t* bt_conn_pd;
   const int* bt_n_atoms;
   const int* bt_n_conn;
   const int* bt_is_ligand;
   const int* cp_count;
   const int* cp_b2;
-  const int* cp_minsep;
   const uint8_t* cp_seps;
   Real* spheres;
   GlobalParams<Real> g;
@@ -996,8 +987,8 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 32 * PAIR_WARPS : 256, 1)
     const int64_t i1 = (int64_t)p * s.B + b1;
     RowSide r;
     r.bt = ra.rot_bt[rot1];
-    r.nc = s.bt_n_conn[r.bt];
-    r.lig = s.bt_is_ligand[r.bt];
+    const int nc1 = s.bt_n_conn[r.bt];
+    const bool lig1 = s.bt_is_ligand[r.bt];
     const int n1 = s.bt_n_atoms[r.bt], off1 = ra.rot_off[rot1];
     const Quad<Real> sph1 = reinterpret_cast<const Quad<Real>*>(rs)[rot1];
     const Real reach1 = sph1.d + s.g.max_dis;
@@ -1040,8 +1031,8 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 32 * PAIR_WARPS : 256, 1)
               const int bt = __shfl_sync(0xffffffffu, bt2, src);
               uint2 mk = make_uint2(0u, 0u);
               if (!diag)
-                mk = partner_masks(s, r.bt, r.nc, r.st, r.c1, bt, s.bt_n_conn[bt], at, cnt, seps,
-                                   r.lig && s.bt_is_ligand[bt], lane);
+                mk = partner_masks(s, r.bt, nc1, r.st, r.c1, bt, s.bt_n_conn[bt], at, cnt, seps,
+                                   lig1 && s.bt_is_ligand[bt], lane);
               else if (lane < r.c1)
                 mk = s.imask[((int64_t)bt * s.A + r.st + lane) * s.n_iwords + (at >> 5)];
               stage_masked(s, w, m, nsp, (int64_t)off, at, cnt, mk, lane);
@@ -1344,7 +1335,6 @@ struct tmol_b200_ljlk_plan {
   int* bt_is_ligand = nullptr;
   int* cp_count = nullptr;
   int* cp_b2 = nullptr;
-  int* cp_minsep = nullptr;
   uint8_t* cp_seps = nullptr;
   int4* work = nullptr;
   int* item_cost = nullptr;
@@ -1666,14 +1656,12 @@ ScoreArgs<Real> score_args(tmol_b200_ljlk_plan* pl, const void* coords) {
   s.bt_n_heavy = pl->bt_n_heavy;
   s.g4 = (Real*)pl->g4;
   s.ntp = pl->ntp;
-  s.bt_pd = pl->bt_pd;
   s.bt_conn_pd = pl->bt_conn_pd;
   s.bt_n_atoms = pl->bt_n_atoms;
   s.bt_n_conn = pl->bt_n_conn;
   s.bt_is_ligand = pl->bt_is_ligand;
   s.cp_count = pl->cp_count;
   s.cp_b2 = pl->cp_b2;
-  s.cp_minsep = pl->cp_minsep;
   s.cp_seps = pl->cp_seps;
   s.spheres = (Real*)pl->spheres;
   const Real* gp = (const Real*)pl->global_params;
@@ -2548,7 +2536,6 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   dalloc(pl, &pl->bt_is_ligand, nbt);
   dalloc(pl, &pl->cp_count, PB);
   dalloc(pl, &pl->cp_b2, PB * CP_CAP);
-  dalloc(pl, &pl->cp_minsep, PB * CP_CAP);
   dalloc(pl, &pl->cp_seps, PB * CP_CAP * 16);
   dalloc(pl, (unsigned char**)&pl->spheres, PB * 4 * real_bytes);
   if (scoring) {
@@ -2621,7 +2608,6 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   a.bt_flags = pl->bt_flags;
   a.cp_count = pl->cp_count;
   a.cp_b2 = pl->cp_b2;
-  a.cp_minsep = pl->cp_minsep;
   a.cp_seps = pl->cp_seps;
   a.status = pl->counters + 1;
   a.term = term;

@@ -659,9 +659,9 @@ __global__ void plan_partner_masks_kernel(ScoreArgs<Real> s, uint2* out) {
   }
 }
 
-// The rows: block type, connection count, ligand flag, tile start and atoms.
+// The rows: block type, tile start and atoms.
 struct RowSide {
-  int bt, nc, lig, st, c1;
+  int bt, st, c1;
 };
 
 // Stages atoms [at0, at0 + cnt) (cnt <= 32) of a block with exclusions
@@ -773,8 +773,6 @@ __global__ void __launch_bounds__(sizeof(Real) == 4 ? 32 * PAIR_WARPS : 256, 1)
       const int n1 = bi1.z;
       RowSide r;
       r.bt = bi1.x;
-      r.nc = bi1.w & 0xff;
-      r.lig = bi1.w >> 8;
       if (GRAD && !BLOCK_PAIR) {
         ec.wt0 = s.dTdV[p];
         if (TERM == kTermLJLK) {
