@@ -902,6 +902,10 @@ struct LkbList {
   int tag[TAGGED ? LKB_LIST : 1];
   int hoff[32], off[32], bt[32], ent[32], htag[TAGGED ? 32 : 1];
 };
+// a float64 kernel with tags fills a CTA's static shared memory to the byte:
+// what is added to either struct has to come out of LKB_Q, LKB_LIST or the warps
+static_assert(LKB_MAX_WARPS * (2 * sizeof(LkbQueue<true>) + sizeof(LkbList<double, true>)) <= 48 * 1024,
+              "static shared memory");
 
 // Queues every polar / occluder pair between the rows and the n_cand
 // neighbours that `next(first)` yields 32 at a time (each lane one), and

@@ -39,6 +39,10 @@ constexpr int MAXSP = 4; // words with exclusion masks
 // 142 us with 160; 20 warps of 96 registers 130 us with 160 and with 128
 // (before forces were split).
 constexpr int PAIR_WARPS = 20;
+// A whole-pose group holds up to MAXSP words with masks and the flat list's
+// M1 / 32 beside them (its room test leaves those out), and a queue entry has
+// 8 bits for the atom.
+static_assert(M1 % 32 == 0 && M1 / 32 + MAXSP <= MAXW && M1 < 256, "a group's words and atoms");
 constexpr int kTfHeavy = 256;
 
 // One atom: coordinates and either the compact atom type | heavy << 8
@@ -59,6 +63,7 @@ struct alignas(16) AtomRec {
 template <typename Real>
 struct Slab {
   static constexpr int QCAP = 3 * M1 * sizeof(Real) / 2 < 1024 ? 1024 : 3 * M1 * sizeof(Real) / 2;
+  static_assert(QCAP >= 32 * 32, "a word's pairs");
   AtomRec<Real> at[M1];
   union {
     struct {
