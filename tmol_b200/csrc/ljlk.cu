@@ -1915,6 +1915,10 @@ template <typename Real>
 int rotamer_count_impl(tmol_b200_ljlk_plan* pl, const void* coords, int64_t* n_pairs,
                        int64_t* n_items, cudaStream_t st) {
   ScoreArgs<Real> s = score_args<Real>(pl, coords);
+  // spheres alone: the atoms' records and the gradient are the score's own
+  // (48 bytes an atom that the dispatch does not read)
+  s.packed = nullptr;
+  s.g4 = nullptr;
   RotArgs ra = rot_args(pl);
   const int n_rows = pl->P * pl->B;
   long long totals[2] = {0, 0};
@@ -3294,6 +3298,8 @@ int tmol_b200_ljlk_screen_candidates(tmol_b200_ljlk_plan* plan,
   const int n_blocks = plan->P * plan->B;
   if (n_blocks == 0) return TMOL_B200_OK;
   ScoreArgs<float> s = score_args<float>(plan, coords);
+  s.packed = nullptr;  // spheres alone
+  s.g4 = nullptr;
   const int threads = 256;
   const int grid = std::max(1, std::min((n_blocks + 7) / 8, plan->n_sm * 16));
   spheres_kernel<float><<<grid, threads, 0, st>>>(s);
