@@ -255,7 +255,9 @@ def test_plan_memory():
     with torch.cuda.stream(other):
         torch.cuda._sleep(20_000_000)
         plans[0].energy_and_gradient(x, weights, out, dx)
+    assert not other.query()
     plans[0] = None
+    assert other.query()
     plans[0] = LJLKPlan(x + 1.0, args)
     plans[0].energy_and_gradient(x + 1.0, weights * 0.5)
     torch.cuda.synchronize()

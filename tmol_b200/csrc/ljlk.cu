@@ -1474,7 +1474,7 @@ cudaError_t pool_alloc(tmol_b200_ljlk_plan* pl, PoolBlock* b, size_t bytes, cuda
 // cudaFree of an allocation that is not the pool's waits, and is allowed or
 // refused beside a stream capture as the plan's own frees would be.
 cudaError_t fence(tmol_b200_ljlk_plan* pl) {
-  if (!pl->fence) return cudaSuccess;
+  if (!pl->fence) return cudaDeviceSynchronize();
   const cudaError_t e = cudaFree(pl->fence);
   if (e == cudaSuccess) pl->fence = nullptr;
   return e;
@@ -1610,20 +1610,25 @@ int build_work(tmol_b200_ljlk_plan* pl, cudaStream_t st) {
       for (int c = r; c < nb; c += pl->launch.candidates_per_item)
         work.push_back(make_int4(p, r, c, std::min(nb, c + pl->launch.candidates_per_item)));
   }
-  if (pl->work) {
-    CK(fence(pl));
-    pool_free(pl, pl->work_blocks, 2);
-  }
-  pl->work = nullptr;
-  pl->item_cost = nullptr;
-  pl->n_work = (int)work.size();
   // room for the items plan_rebalance splits off the heaviest ones
-  pl->work_cap = pl->n_work + pl->n_work / 2 + 64;
-  if (!pl->fence) CK(cudaMalloc(&pl->fence, FENCE_BYTES));
-  CK(pool_alloc(pl, &pl->work_blocks[0], (size_t)pl->work_cap * sizeof(int4), st));
-  CK(pool_alloc(pl, &pl->work_blocks[1], (size_t)pl->work_cap * sizeof(int), st));
-  pl->work = (int4*)pl->work_blocks[0].p;
-  pl->item_cost = (int*)pl->work_blocks[1].p;
+  const int n_work = (int)work.size(), cap = n_work + n_work / 2 + 64;
+  // the new buffers before the old ones go: a plan that cannot have them
+  // keeps its items
+  PoolBlock blocks[2];
+  cudaError_t e = pool_alloc(pl, &blocks[0], (size_t)cap * sizeof(int4), st);
+  if (e == cudaSuccess) e = pool_alloc(pl, &blocks[1], (size_t)cap * sizeof(int), st);
+  if (e == cudaSuccess && pl->work) e = fence(pl);
+  if (e == cudaSuccess && !pl->fence) e = cudaMalloc(&pl->fence, FENCE_BYTES);
+  if (e != cudaSuccess) {
+    pool_free(pl, blocks, 2);
+    return TMOL_B200_ERR_CUDA;
+  }
+  pool_free(pl, pl->work_blocks, 2);
+  std::copy_n(blocks, 2, pl->work_blocks);
+  pl->work = (int4*)blocks[0].p;
+  pl->item_cost = (int*)blocks[1].p;
+  pl->n_work = n_work;
+  pl->work_cap = cap;
   CK(cudaMemsetAsync(pl->item_cost, 0, (size_t)pl->work_cap * sizeof(int), st));
   if (!work.empty())
     CK(cudaMemcpyAsync(pl->work, work.data(), work.size() * sizeof(int4),
@@ -3079,11 +3084,13 @@ int tmol_b200_ljlk_plan_destroy(tmol_b200_ljlk_plan* plan) {
 int tmol_b200_ljlk_plan_set_launch(tmol_b200_ljlk_plan* plan,
                                    const tmol_b200_ljlk_launch* launch) {
   if (!plan || !launch) return TMOL_B200_ERR_INVALID_ARGUMENT;
-  int old_cpi = plan->launch.candidates_per_item;
+  const tmol_b200_ljlk_launch before = plan->launch;
   plan->launch = *launch;
   default_launch(plan, plan->launch);
-  if (plan->launch.candidates_per_item != old_cpi) return build_work(plan, 0);
-  return TMOL_B200_OK;
+  if (plan->launch.candidates_per_item == before.candidates_per_item) return TMOL_B200_OK;
+  const int rc = build_work(plan, 0);
+  if (rc != TMOL_B200_OK) plan->launch = before;
+  return rc;
 }
 
 int tmol_b200_ljlk_forward(tmol_b200_ljlk_plan* plan, const void* coords,
