@@ -8,7 +8,10 @@ float64 energies and gradients against the oracle.  A gradient component is
 a sum of at most a few thousand signed terms, each no larger than the largest
 component's magnitude allows by a factor of ten or so, so its float64 sum is
 good to 1e-12 of the largest component (2.2e-16 x a few thousand); energies
-likewise to 1e-11 relative."""
+likewise to 1e-11 relative.  A float32 pair force is good to about 1e-6 of
+itself (some sixteen roundings, steep in the distance), so a component, whose
+terms sum to some tens of the largest component in magnitude, to 2e-5 of the
+largest component."""
 
 import json
 
@@ -78,6 +81,83 @@ def test_rotamer_groups(scale):
     assert numpy.array_equal(indices.cpu().numpy(), ind)
     close(E, Eo, 1e-11)
     clear_plan_cache()
+
+
+def one_atom_pose_stack():
+    """Poses with blocks of a single atom, alone, among residues and as the
+    last of more blocks than a group has words."""
+    from tmol_b200.chem.restypes import ChemicalDatabase, PackedBlockTypes, ResidueType, ResidueTypeSet
+    from tmol_b200.pose.builder import PoseTopology, build_pose_stack
+
+    one = ResidueType(
+        name="ONE", base_name="ONE", atoms=[["A0", "CH3"]], bonds=[], connections=[], icoors=[], chis=[], aliases=[],
+        is_polymer=False, is_ligand_fragment=True,
+    )
+    pbt = PackedBlockTypes(
+        ChemicalDatabase.get_default(), list(ResidueTypeSet.get_default().types.values()) + [one]
+    )
+    rng = numpy.random.default_rng(7)
+    names = [["ONE"], ["GLY"] * 3 + ["ONE"] * 40, (["ONE", "ALA"] * 10) + ["ONE"]]
+    coords = [
+        rng.normal(scale=3.0, size=(sum(pbt.active_block_types[pbt.bt_index[n]].n_atoms for n in pose), 3))
+        for pose in names
+    ]
+    return build_pose_stack([PoseTopology(n, []) for n in names], coords, pbt=pbt)
+
+
+@pytest.mark.parametrize("name, poses", [("ljlk", 1.0), ("ljlk", 0.5), ("ljlk", "one atom"), ("elec", 1.0), ("elec", 0.5)])
+@pytest.mark.parametrize("block_pair", [False, True])
+def test_weighted_gradients(name, block_pair, poses):
+    """Energies and gradients under weights of every pose or block pair's own,
+    in both precisions, of squeezed poses (groups with more pairs than the
+    queue holds) and of blocks of one atom."""
+    from tmol_b200.score.elec_op import ElecPlan
+    from tmol_b200.score.ljlk_op import LJLKPlan
+
+    if poses == "one atom":  # a block type without charges
+        ps, scale = one_atom_pose_stack(), 1.0
+    else:
+        ps, scale = synthetic_pose_stack([30, 1, 2, 9, 75], [5, 6, 7, 8, 9], spacing=0.0), poses
+    x = (ps.coords * scale).flatten(0, 1).float()
+    args_of, term, plan_of, n = {
+        "ljlk": (pose_score_args, LJLKEnergyTerm(), LJLKPlan, 3),
+        "elec": (elec_pose_score_args, ElecEnergyTerm(), ElecPlan, 1),
+    }[name]
+    args = args_of(ps, term, block_pair)
+    oc = O.OracleCall(x.double(), args, f64=True, term=name)
+    Eo, _, nbr = oc.pose_scores(block_pair=block_pair)
+    w = numpy.zeros((3,) + Eo.shape[1:])
+    w[:n] = numpy.random.default_rng(11).normal(size=(n,) + Eo.shape[1:]).astype(numpy.float32)
+    go = oc.backward(nbr, w, per_pose_weights=not block_pair)
+    for dtype, rel in ((torch.float64, 1e-12), (torch.float32, 2e-5)):
+        c = x.to(DEV, dtype).contiguous()
+        plan = plan_of(c, on_gpu(args, dtype)[:-1])
+        E, _ = plan.forward(c, block_pair=block_pair)
+        if dtype == torch.float64:
+            close(E, Eo[:n].reshape(E.shape), 1e-11)
+        else:
+            E_close(E.cpu().numpy(), Eo[:n].reshape(E.shape))
+        close(plan.backward(c, torch.tensor(w[:n], device=DEV), block_pair=block_pair), go, rel)
+
+
+@pytest.mark.parametrize("scale", [1.0, 0.5])
+def test_weighted_rotamer_gradients(scale):
+    from tmol_b200.score.ljlk_op import LJLKPlan
+
+    ps = synthetic_pose_stack([12, 3], [15, 16], spacing=0.0)
+    rs = synthetic_rotamer_set(ps, max_rots=40, seed=3)
+    args = rotamer_score_args(ps, rs, LJLKEnergyTerm())
+    x = (rs.coords * scale).float()
+    oc = O.OracleCall(x.double(), args, f64=True)
+    Eo, ind, nbr = oc.rotamer_scores()
+    w = numpy.random.default_rng(12).normal(size=Eo.shape).astype(numpy.float32).astype(numpy.float64)
+    go = oc.rotamer_backward(nbr, w)
+    for dtype, rel in ((torch.float64, 1e-12), (torch.float32, 2e-5)):
+        c = x.to(DEV, dtype).contiguous()
+        plan = LJLKPlan(c, on_gpu(args, dtype)[:-1], rotamers=True)
+        indices, items = plan.rotamer_dispatch(c)
+        assert numpy.array_equal(indices.cpu().numpy(), ind)
+        close(plan.rotamer_backward(c, items, torch.tensor(w, device=DEV)), go, rel)
 
 
 def pair_plan(name, rotamers, dtype, scale):
