@@ -751,6 +751,7 @@ struct LkbEval {
   Real* g4;       // padded gradient [n_atoms][GRAD_STRIDE]
   Real* dwaters;  // [n_atoms][4][3]
   bool vec_w, vec_dw;  // 16-byte aligned
+  Real grid;           // force_grid_of the item's weights (untagged)
   Real water_dist, hbond_dis, hbond_oh, hbond_h, max_dis;
 };
 
@@ -758,6 +759,11 @@ template <typename Real>
 struct Lkb4 {
   Real v[4];
 };
+
+template <typename Real>
+__device__ __forceinline__ Real lkb_grid(const Lkb4<Real>& w) {
+  return force_grid_of(fmax(fmax(fabs(w.v[0]), fabs(w.v[1])), fmax(fabs(w.v[2]), fabs(w.v[3]))));
+}
 
 // Evaluates entry `lane` of q when lane < n: returns its four energies and,
 // with GRAD, adds the adjoint of w . E to dcoords / dwaters.
@@ -774,7 +780,7 @@ struct Lkb4 {
 
 template <typename Real, bool GRAD, typename Queue>
 __device__ TMOL_B200_LKB_DRAIN_ATTR Lkb4<Real> lkb_drain(const LkbEval<Real> ev, const Queue& q, int n, int lane,
-                                             const Lkb4<Real> w) {
+                                             const Lkb4<Real> w, Real grid) {
   Lkb4<Real> out = {{0, 0, 0, 0}};
   if (lane >= n) return out;
   const int64_t rp = q.rp[lane], ro = q.ro[lane];
@@ -794,7 +800,6 @@ __device__ TMOL_B200_LKB_DRAIN_ATTR Lkb4<Real> lkb_drain(const LkbEval<Real> ev,
   if (GRAD) {
     // vector reductions: the thirty values of a pair as scalar ones took the
     // path to L2 longer than the pair's arithmetic
-    const Real grid = force_grid_of(fmax(fmax(fabs(w.v[0]), fabs(w.v[1])), fmax(fabs(w.v[2]), fabs(w.v[3]))));
     if (gI[0] != Real(0) || gI[1] != Real(0) || gI[2] != Real(0))
       add_force(ev.g4 + GRAD_STRIDE * rp, grid, gI[0], gI[1], gI[2]);
     if (gJ[0] != Real(0) || gJ[1] != Real(0) || gJ[2] != Real(0))
@@ -851,7 +856,7 @@ __device__ __forceinline__ void lkb_pump(const LkbEval<Real>& ev, LkbWarp<Real, 
     const int tag = TAGGED && lane < n ? Q.tag[lane] : 0;
     if (TAGGED && GRAD && lane < n)
       for (int c = 0; c < 4; ++c) wl.v[c] = tg.dTdV[(int64_t)c * tg.n + tag];
-    const Lkb4<Real> got = lkb_drain<Real, GRAD>(ev, Q, n, lane, wl);
+    const Lkb4<Real> got = lkb_drain<Real, GRAD>(ev, Q, n, lane, wl, TAGGED && GRAD ? lkb_grid(wl) : ev.grid);
     if (TAGGED) {
       if (!GRAD && lane < n)
         for (int c = 0; c < 4; ++c)
@@ -1077,6 +1082,7 @@ __device__ __forceinline__ LkbEval<Real> lkb_eval_of(const ScoreArgs<Real>& s, c
   ev.par = k.par;
   ev.g4 = s.g4;
   ev.dwaters = k.dwaters_out;
+  ev.grid = 0;
   ev.vec_w = (reinterpret_cast<uintptr_t>(k.waters) & (4 * sizeof(Real) - 1)) == 0;
   ev.vec_dw = (reinterpret_cast<uintptr_t>(k.dwaters_out) & (4 * sizeof(Real) - 1)) == 0;
   ev.water_dist = k.water_dist;
@@ -1117,7 +1123,7 @@ __global__ void __launch_bounds__(256, TMOL_B200_LKB_MIN_CTAS) lkb_score_kernel(
   q.n_bp = q.n_pairs = q.n_bridge = q.n_eval = 0;
   const int lane = q.lane;
   const int64_t stride = (int64_t)s.P * s.B * s.B;
-  const LkbEval<Real> ev = lkb_eval_of(s, k);
+  LkbEval<Real> ev = lkb_eval_of(s, k);
   LkbTagged<Real> tg;
   tg.energies = s.energies;
   tg.dTdV = s.dTdV;
@@ -1148,6 +1154,7 @@ __global__ void __launch_bounds__(256, TMOL_B200_LKB_MIN_CTAS) lkb_score_kernel(
       Lkb4<Real> w = {{0, 0, 0, 0}};
       if (GRAD && !BLOCK_PAIR)
         for (int c = 0; c < 4; ++c) w.v[c] = s.dTdV[(int64_t)c * s.P + p];
+      ev.grid = lkb_grid(w);
       Real acc[4] = {0, 0, 0, 0};
       const LkbRows rows = {bt1, s.blk_off[i1], k.hbase[i1], k.nocc[bt1], k.npol[bt1], s.bt_n_atoms[bt1]};
       const Real reach1 = sph1.d + k.max_dis;
