@@ -54,6 +54,9 @@ constexpr int MAX_CONN = 4;
 // Per warp they are warp-uniform.
 constexpr int N_COUNTS = 5;
 constexpr int CP_CAP = 16;
+// LK-ball's heavy-atom records: the atom, whether it is polar with waters and
+// whether it bridges (donor or acceptor)
+constexpr int kHeavyAtom = (1 << 24) - 1, kHeavyPolar = 1 << 24, kHeavyBridges = 1 << 25;
 constexpr int MAX_ROWS_PER_ITEM = 64;
 
 // The energy term a plan scores: LJ + LK (fa_ljatr, fa_ljrep, fa_lk) or
@@ -580,7 +583,7 @@ struct ScoreArgs {
   int* ticket;
   unsigned long long* counts;
   // LK-ball: the heavy atoms of every block (or rotamer) as records (flags:
-  // atom | polar with waters << 16 | bridges << 17), from hbase[i] on, written
+  // atom | kHeavyPolar | kHeavyBridges), from hbase[i] on, written
   // by the sphere pass from each block type's list hmeta [nbt][maxocc]
   AtomRec<Real>* hpacked;
   const int* hbase;
@@ -731,8 +734,8 @@ __device__ __forceinline__ void pack_heavy(const ScoreArgs<Real>& s, int bt, int
   if (bt < 0) return;
   for (int k = lane; k < s.nocc[bt]; k += 32) {
     int meta = s.hmeta[(int64_t)bt * s.maxocc + k];
-    const int64_t row = (int64_t)off + (meta & 0xffff);
-    if ((meta & (1 << 16)) && isnan(s.waters[row * 12])) meta &= ~(1 << 16);
+    const int64_t row = (int64_t)off + (meta & kHeavyAtom);
+    if ((meta & kHeavyPolar) && isnan(s.waters[row * 12])) meta &= ~kHeavyPolar;
     AtomRec<Real> a;
     a.x = s.coords[3 * row];
     a.y = s.coords[3 * row + 1];
@@ -2317,9 +2320,9 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
     for (int bt = 0; bt < nbt; ++bt)
       for (size_t y = 0; y < occ[bt].size(); ++y) {
         const int a = occ[bt][y];
-        if (a >= (1 << 16)) return TMOL_B200_ERR_SHAPE;
+        if (a > kHeavyAtom) return TMOL_B200_ERR_SHAPE;  // 2^24 atoms: their path distances are 2^50 bytes
         const bool polar = std::find(pol[bt].begin(), pol[bt].end(), a) != pol[bt].end();
-        hmeta[(size_t)bt * maxocc + y] = a | (polar ? 1 << 16 : 0) | ((int)y < hnbocc[bt] ? 1 << 17 : 0);
+        hmeta[(size_t)bt * maxocc + y] = a | (polar ? kHeavyPolar : 0) | ((int)y < hnbocc[bt] ? kHeavyBridges : 0);
       }
     CK(cudaMemcpyAsync(pl->hmeta, hmeta.data(), sizeof(int) * hmeta.size(), cudaMemcpyHostToDevice, st));
     const int n = pl->rotamers ? pl->R : pl->P * pl->B;

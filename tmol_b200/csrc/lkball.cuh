@@ -902,7 +902,7 @@ constexpr int LKB_LIST = 64;
 template <typename Real, bool TAGGED>
 struct LkbList {
   Real x[LKB_LIST], y[LKB_LIST], z[LKB_LIST];
-  int tf[LKB_LIST];  // atom | polar with waters << 16 | bridges << 17
+  int tf[LKB_LIST];  // atom | kHeavyPolar | kHeavyBridges
   int row[LKB_LIST], par[LKB_LIST], entry[LKB_LIST];
   int tag[TAGGED ? LKB_LIST : 1];
   int hoff[32], off[32], bt[32], ent[32], htag[TAGGED ? 32 : 1];
@@ -984,8 +984,8 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
           L.y[j] = o.y;
           L.z[j] = o.z;
           L.tf[j] = o.tf;
-          L.row[j] = L.off[own] + (o.tf & 0xffff);
-          L.par[j] = L.bt[own] * s.A + (o.tf & 0xffff);
+          L.row[j] = L.off[own] + (o.tf & kHeavyAtom);
+          L.par[j] = L.bt[own] * s.A + (o.tf & kHeavyAtom);
           L.entry[j] = L.ent[own];
           if (TAGGED) L.tag[j] = L.htag[own];
         }
@@ -1000,7 +1000,7 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
       o.y = L.y[lane];
       o.z = L.z[lane];
       o.tf = L.tf[lane];
-      const int orow = L.row[lane], opar = L.par[lane], entry = L.entry[lane], ja = o.tf & 0xffff;
+      const int orow = L.row[lane], opar = L.par[lane], entry = L.entry[lane], ja = o.tf & kHeavyAtom;
       const int otag = TAGGED ? L.tag[lane] : 0;
       const bool valid = lane < m;
       int64_t moff = 0;
@@ -1008,9 +1008,9 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
       for (int step = 0; step < 2 * a.nocc; ++step) {
         const AtomRec<Real> r = s.hpacked[a.hb + (step >> 1)];
         const bool back = step & 1;
-        const int ra = r.tf & 0xffff;
+        const int ra = r.tf & kHeavyAtom;
         const Real dv[3] = {r.x - o.x, r.y - o.y, r.z - o.z};
-        bool in_reach = valid && lkb_sqrt(lkb_dot(dv, dv)) < k.max_dis && (((back ? o.tf : r.tf) >> 16) & 1);
+        bool in_reach = valid && lkb_sqrt(lkb_dot(dv, dv)) < k.max_dis && ((back ? o.tf : r.tf) & kHeavyPolar);
         int sep = 6;
         if (in_reach && entry != -2) {
           if (PMASK || entry == -1) {
@@ -1023,7 +1023,7 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
           }
           in_reach = sep > 3;
         }
-        const bool bridged = ((back ? r.tf : o.tf) >> 17) & 1;
+        const bool bridged = ((back ? r.tf : o.tf) & kHeavyBridges) != 0;
         const unsigned m1 = __ballot_sync(0xffffffffu, in_reach && bridged);
         const unsigned m0 = __ballot_sync(0xffffffffu, in_reach && !bridged);
         if (in_reach) {
