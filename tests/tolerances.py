@@ -16,8 +16,8 @@ loses up to ~1e-3 kcal/mol/A whichever order it is taken in.  The
 reference's own float32 op, measured against its float64 result on eight
 150-residue poses (oracle/ljlk_oracle.c is bit-exact with it), has a largest
 error of 1.4e-3 kcal/mol/A and no component outside this band.  The scoring
-kernels sum in another order (per-atom partial sums in shared memory, then
-one global atomic per atom and work item).
+kernels sum in another order, and in two parts: multiples of 2^-6 of the
+weights' size, whose sums are exact, and the remainders.
 
 Comparing two float32 results of the same sums (the reference op's stored
 float32 output, or the GPU path against itself) doubles both terms, since

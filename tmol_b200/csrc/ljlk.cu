@@ -13,10 +13,13 @@
 //                                  count-pair reach (min bond separation <= 4)
 //                                  with their connection-pair separations;
 //                                  replaces the dense [P,B,B,C,C] tensor
-//   work[n_work] (int4)            rows: (pose, b1) for every block slot up
-//                                  to each pose's last real block
+//   imask, pmask                   bits of the pairs within a block type, and
+//                                  with a count-pair partner, that are left
+//                                  out or weighted 0.2
+//   work[n_work] (int4)            items: (pose, b1, range of later blocks) for
+//                                  every block slot up to each pose's last real
+//                                  block
 //   spheres[P*B][4]                centroid + radius, rebuilt every call
-//
 //   packed[n_atoms], g4[n_atoms][8]  staged atoms and padded gradient, per call
 //
 // Scoring is one persistent launch per call after the sphere kernel (every
@@ -2826,7 +2829,10 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   }
   // where the far class starts: LJ/LK where both potentials fade, for every
   // pair of types (LK's close cubics end by sqrt(405 / 20) = 4.5 A); elec
-  // where its fade starts, beyond the low spline
+  // where its fade starts, if that is beyond the low spline.  One pair of types
+  // whose LJ fades on an interval of its own takes the class from all (the near
+  // class is right for every pair): 64 x 150 residues, energy + gradient 171 us
+  // with the class, 188-201 without; 16 x 300 130 and 154
   if (term == kTermLJLK && split && !mixed) {
     const double dmax = real_bytes == 4 ? ((const float*)pl->global_params)[0] : ((const double*)pl->global_params)[0];
     pl->far_d = std::max(dmax - 1.5, 4.5);

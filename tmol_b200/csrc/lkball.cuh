@@ -10,8 +10,8 @@
 // hydrogen; acceptor: the acceptor and its two base atoms, which may sit in
 // bonded blocks) and its torsion / angle.  Per call, one thread per (atom,
 // slot) builds the waters; the scoring kernel walks the plan's work items
-// like score_kernel and evaluates every polar / occluder pair of each
-// neighbouring block pair, lanes striding over the pairs; the adjoint
+// like score_kernel, lists the neighbours' heavy atoms, queues the polar /
+// occluder pairs in reach and evaluates them 32 at a time; the adjoint
 // accumulates d/dcoords and d/dwaters with atomics, and a second pass moves
 // d/dwaters onto the placing atoms.
 
@@ -651,7 +651,7 @@ __device__ inline int lkb_pair(const Real* I, const Real* J, const Real* WI, con
 // neighbour rule as score_kernel applies it, then every polar / occluder
 // pair of each neighbouring block pair (intra-block: ordered pairs of
 // distinct atoms; inter-block: polars of either block against occluders of
-// the other), lanes striding over the pairs.
+// the other), found by lkb_walk.
 
 template <typename Real>
 __device__ __forceinline__ int lkb_inter_sep(const ScoreArgs<Real>& s, int bt1, int bt2, int nc1, int nc2,

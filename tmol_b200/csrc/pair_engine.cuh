@@ -15,20 +15,21 @@
 //      fade to zero), near without a heavy pair (LJ alone) and near heavy.
 //   3. evaluation, class by class: every lane takes an equal stretch of
 //      consecutive entries.  Lanes of a step run the same code, a stretch
-//      stays on one or two rows (their atom, force and, in pair mode,
-//      energies stay in registers), and the side-1 forces go out as 16-byte
-//      vector reductions into a padded gradient buffer.
+//      stays on one or two rows (their atom and force stay in registers), and
+//      the side-1 forces go out as 16-byte vector reductions into a padded
+//      gradient buffer.  Energies of pairs (blocks, rotamers) are evaluated a
+//      window of entries at a time and added up pair by pair.
 //
 // What bounds it: latency, at 20 warps per SM (59% of the issue slots are
-// used, the FMA pipes 26%, DRAM 1%; 64 x 150 residues, energy + gradient, 128
+// used, the FMA pipes 26%, DRAM 1%; 64 x 150 residues, energy + gradient, 129
 // us and 82 M warp instructions, where warps that listed pairs and summed both
 // atoms' forces in shared memory took 302 us and 137 M).  So the loads an item
 // starts from go out together, a whole list of neighbouring atoms is in flight
 // at once (cp.async into side 1, culled in place), and forces leave the SM
 // without being waited for: shared-memory float atomics are compare-and-swap
 // loops here (64 x 150 residues, energy + gradient: 185 us with the side-1
-// forces summed in shared memory, 138 us without); one red.global.add.v4.f32 is
-// a single instruction and 44 cycles of an SM's path to L2.
+// forces summed in shared memory, 138 us without); a red.global.add.v4.f32 is
+// one instruction that nothing waits for.
 
 constexpr int M1 = 160;  // side-1 atoms of a group (< 256: 8-bit index)
 constexpr int MAXW = 9;  // words of a group; odd: the mask arrays' row stride has no bank conflicts
