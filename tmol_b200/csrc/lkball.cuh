@@ -654,20 +654,6 @@ __device__ inline int lkb_pair(const Real* I, const Real* J, const Real* WI, con
 // the other), found by lkb_walk.
 
 template <typename Real>
-__device__ __forceinline__ int lkb_inter_sep(const ScoreArgs<Real>& s, int bt1, int bt2, int nc1, int nc2,
-                                             const uint8_t* seps, int a1, int a2) {
-  int sep = 5;  // one past the largest separation that matters (4)
-  for (int u = 0; u < nc1; ++u) {
-    const int pd1 = s.bt_conn_pd[((int64_t)bt1 * s.C + u) * s.A + a1];
-    for (int v = 0; v < nc2; ++v) {
-      const int t = pd1 + seps[u * 4 + v] + s.bt_conn_pd[((int64_t)bt2 * s.C + v) * s.A + a2];
-      sep = t < sep ? t : sep;
-    }
-  }
-  return sep;
-}
-
-template <typename Real>
 __device__ __forceinline__ LkbParams<Real> lkb_params(const Real* par, int row) {
   const Quad<Real>* q = reinterpret_cast<const Quad<Real>*>(par) + 3 * (int64_t)row;
   const Quad<Real> u = q[0], v = q[1];
@@ -912,18 +898,33 @@ struct LkbList {
 static_assert(LKB_MAX_WARPS * (2 * sizeof(LkbQueue<true>) + sizeof(LkbList<double, true>)) <= 48 * 1024,
               "static shared memory");
 
+// Whether a squared distance is one below `max`, as the square root decides it
+// (in float64 asked only where it could decide otherwise).
+__device__ __forceinline__ bool lkb_within(float d2, float max) { return lkb_sqrt(d2) < max; }
+__device__ __forceinline__ bool lkb_within(double d2, double max) {
+  const double m2 = max * max;
+  return d2 < m2 * (1 - 1e-12) || (d2 < m2 * (1 + 1e-12) && lkb_sqrt(d2) < max);
+}
+
 // Queues every polar / occluder pair between the rows and the n_cand
 // neighbours that `next(first)` yields 32 at a time (each lane one), and
 // evaluates full queues under w into e4.  The neighbours' heavy atoms are one
 // flat list: each is loaded once with its flags (polar with waters, bridges)
 // and culled against the rows' sphere (centre c, reach2 the squared reach),
-// and every row meets 32 of them at a time, in both directions.  Pairs of the
-// rows' own block and of count-pair partners have their exclusions from the
-// plan's masks, a rotamer's partners (PMASK false) their bond separations.
-// What bounds it: latency and issue of the evaluation (49% of the issue slots
-// used).  Pairs enumerated one by one, with index arithmetic and eight loads
-// each, were half of the kernel's instructions: 64 x 150 residues, energies +
-// gradients, 196 -> 164 us; rotamers of 8 x 100 residues 2.55 -> 2.12 ms.
+// and 32 of them at a time, one a lane, meet the rows: a lane first finds its
+// pairs as bits (in reach, not excluded, weight 0.2), in loops whose loads do
+// not wait for one another, then the warp queues a pair of each lane at a time
+// until none has one left.  Pairs of the rows' own block and of count-pair
+// partners have their exclusions from the plan's masks, a rotamer's partners
+// (PMASK false) their bond separations.
+// What bounds it: latency and issue of the evaluation.  Times of the scoring
+// kernel where pairs were enumerated one by one, with index arithmetic and
+// eight loads each; where every row was voted on and queued in both directions
+// in turn, its record and masks loaded in between; and now: 64 x 150 residues,
+// energies + gradients 196, 164 and 164 us; rotamers of 8 x 100 residues,
+// energies 2.55, 2.12 and 1.42 ms; one pose of 100 residues, energies 37, 35 and
+// 26 us; 4 x 100 in float64, energies 101, 128 and 99 us; of one residue 7.5,
+// 14.7 and 9.2 us.
 template <typename Real, bool GRAD, bool TAGGED, bool COUNT, bool PMASK, typename Next>
 __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs<Real>& k, const LkbEval<Real>& ev,
                                          LkbWarp<Real, TAGGED>& q, LkbList<Real, TAGGED>& L, const LkbRows& a,
@@ -932,6 +933,7 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
   const int lane = q.lane;
   const unsigned lemask = q.lt_mask | (1u << lane);
   const int nc1 = PMASK ? 0 : s.bt_n_conn[a.bt];
+  const int rtf0 = lane < a.nocc ? s.hpacked[a.hb + lane].tf : 0;  // the first 32 rows
   int m = 0;  // atoms in the list
   for (int c0 = 0; c0 < n_cand; c0 += 32) {
     const LkbHit h = next(c0);
@@ -1003,47 +1005,107 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
       const int orow = L.row[lane], opar = L.par[lane], entry = L.entry[lane], ja = o.tf & kHeavyAtom;
       const int otag = TAGGED ? L.tag[lane] : 0;
       const bool valid = lane < m;
-      int64_t moff = 0;
-      if (PMASK && valid && entry >= 0) moff = (int64_t)s.cp_moff[entry] + (int64_t)(ja >> 5) * a.n_atoms;
-      for (int step = 0; step < 2 * a.nocc; ++step) {
-        const AtomRec<Real> r = s.hpacked[a.hb + (step >> 1)];
-        const bool back = step & 1;
-        const int ra = r.tf & kHeavyAtom;
-        const Real dv[3] = {r.x - o.x, r.y - o.y, r.z - o.z};
-        bool in_reach = valid && lkb_sqrt(lkb_dot(dv, dv)) < k.max_dis && ((back ? o.tf : r.tf) & kHeavyPolar);
-        int sep = 6;
-        if (in_reach && entry != -2) {
-          if (PMASK || entry == -1) {
-            const uint2 mk = entry == -1 ? s.imask[((int64_t)a.bt * s.A + ra) * s.n_iwords + (ja >> 5)]
-                                         : s.pmask[moff + ra];
-            sep = (mk.x >> (ja & 31)) & 1u ? 0 : ((mk.y >> (ja & 31)) & 1u ? 4 : 6);
-          } else {
-            const int bt2 = (opar - ja) / s.A;
-            sep = lkb_inter_sep(s, a.bt, bt2, nc1, s.bt_n_conn[bt2], s.cp_seps + (int64_t)entry * 16, ra, ja);
+      const bool special = valid && entry != -2;
+      const bool any_special = __any_sync(0xffffffffu, special);
+      for (int rt = 0; rt < a.nocc; rt += 32) {
+        const int nr = min(32, a.nocc - rt);
+        const int rtf = rt == 0 ? rtf0 : (lane < nr ? s.hpacked[a.hb + rt + lane].tf : 0);
+        // bit i: row rt + i and this lane's atom are a pair in reach (near)
+        // with weight 0.2 (four): no branch or vote in the rows' loads
+        unsigned near = 0, four = 0;
+#pragma unroll 4
+        for (int i = 0; i < nr; ++i) {
+          const AtomRec<Real> r = s.hpacked[a.hb + rt + i];
+          const Real dv[3] = {r.x - o.x, r.y - o.y, r.z - o.z};
+          near |= (lkb_within(lkb_dot(dv, dv), k.max_dis) ? 1u : 0u) << i;
+        }
+        if (!valid) near = 0;
+        if (any_special) {
+          unsigned out = 0;
+          const uint2* masks = nullptr;  // of the word that holds this atom, by row atom
+          int64_t stride = 1;
+          if (special && entry == -1) {
+            masks = s.imask + (int64_t)a.bt * s.A * s.n_iwords + (ja >> 5);
+            stride = s.n_iwords;
+          } else if (PMASK && special) {
+            masks = s.pmask + s.cp_moff[entry] + (int64_t)(ja >> 5) * a.n_atoms;
           }
-          in_reach = sep > 3;
+#pragma unroll 4
+          for (int i = 0; i < nr; ++i) {
+            const int ra = __shfl_sync(0xffffffffu, rtf, i) & kHeavyAtom;
+            uint2 mk = make_uint2(0u, 0u);
+            if (masks) mk = masks[ra * stride];
+            out |= ((mk.x >> (ja & 31)) & 1u) << i;
+            four |= ((mk.y >> (ja & 31)) & 1u) << i;
+          }
+          if (!PMASK) {
+            // a count-pair partner: its atom's separation from each of the
+            // rows' connections, a byte each, then row by row
+            const bool partner = special && entry >= 0;
+            unsigned far = 0x3f3f3f3fu;
+            if (partner) {
+              const int bt2 = (opar - ja) / s.A, nc2 = s.bt_n_conn[bt2];
+              const uint8_t* seps = s.cp_seps + (int64_t)entry * 16;
+              const uint32_t cj = load_cpd(s, bt2, nc2, ja);
+              for (int u = 0; u < nc1; ++u) {
+                int best = 63;
+                for (int v = 0; v < nc2; ++v)
+                  best = min(best, (int)seps[u * 4 + v] + (int)((cj >> (8 * v)) & 0xff));
+                far = (far & ~(0xffu << (8 * u))) | ((unsigned)best << (8 * u));
+              }
+            }
+            if (__any_sync(0xffffffffu, partner)) {
+              const uint32_t c0 = lane < nr ? load_cpd(s, a.bt, nc1, rtf & kHeavyAtom) : 0u;
+              for (int i = 0; i < nr; ++i) {
+                const uint32_t ci = __shfl_sync(0xffffffffu, c0, i);
+                int sep = 5;
+                for (int u = 0; u < nc1; ++u)
+                  sep = min(sep, (int)((ci >> (8 * u)) & 0xff) + (int)((far >> (8 * u)) & 0xff));
+                if (partner) {
+                  out |= (unsigned)(sep < 4) << i;
+                  four |= (unsigned)(sep == 4) << i;
+                }
+              }
+            }
+          }
+          near &= ~out;
         }
-        const bool bridged = ((back ? r.tf : o.tf) & kHeavyBridges) != 0;
-        const unsigned m1 = __ballot_sync(0xffffffffu, in_reach && bridged);
-        const unsigned m0 = __ballot_sync(0xffffffffu, in_reach && !bridged);
-        if (in_reach) {
-          const int rr = a.off + ra, rpar = a.bt * s.A + ra;
-          LkbQueue<TAGGED>& Q = q.qs[bridged ? 1 : 0];
-          const int at = (bridged ? q.nq[1] : q.nq[0]) + __popc((bridged ? m1 : m0) & q.lt_mask);
-          Q.rp[at] = back ? orow : rr;
-          Q.ro[at] = back ? rr : orow;
-          Q.pi[at] = back ? opar : rpar;
-          Q.oi[at] = back ? rpar : opar;
-          Q.sep[at] = (uint8_t)sep;
-          if (TAGGED) Q.tag[at] = otag;
+        // the pairs in either direction: the row polar and the list's atom
+        // occluding, then the other way round; one of each lane at a time
+        const unsigned polar_rows = __ballot_sync(0xffffffffu, rtf & kHeavyPolar);
+        const unsigned bridge_rows = __ballot_sync(0xffffffffu, rtf & kHeavyBridges);
+        unsigned there = near & polar_rows, back = (o.tf & kHeavyPolar) ? near : 0u;
+        for (;;) {
+          const bool act = (there | back) != 0, bk = there == 0;
+          const int i = act ? __ffs(bk ? back : there) - 1 : 0;
+          const bool bridged = bk ? (bridge_rows >> i) & 1u : (o.tf & kHeavyBridges) != 0;
+          const unsigned m1 = __ballot_sync(0xffffffffu, act && bridged);
+          const unsigned m0 = __ballot_sync(0xffffffffu, act && !bridged);
+          if ((m0 | m1) == 0) break;
+          const int ra = __shfl_sync(0xffffffffu, rtf, i) & kHeavyAtom;
+          if (act) {
+            if (bk)
+              back &= back - 1;
+            else
+              there &= there - 1;
+            const int rr = a.off + ra, rpar = a.bt * s.A + ra;
+            LkbQueue<TAGGED>& Q = q.qs[bridged ? 1 : 0];
+            const int at = (bridged ? q.nq[1] : q.nq[0]) + __popc((bridged ? m1 : m0) & q.lt_mask);
+            Q.rp[at] = bk ? orow : rr;
+            Q.ro[at] = bk ? rr : orow;
+            Q.pi[at] = bk ? opar : rpar;
+            Q.oi[at] = bk ? rpar : opar;
+            Q.sep[at] = (four >> i) & 1u ? 4 : 6;
+            if (TAGGED) Q.tag[at] = otag;
+          }
+          q.nq[0] += __popc(m0);
+          q.nq[1] += __popc(m1);
+          if (COUNT) {
+            q.n_eval += __popc(m0 | m1);
+            q.n_bridge += __popc(m1);
+          }
+          lkb_pump<Real, GRAD, TAGGED>(ev, q, false, w, e4, tg);
         }
-        q.nq[0] += __popc(m0);
-        q.nq[1] += __popc(m1);
-        if (COUNT) {
-          q.n_eval += __popc(m0 | m1);
-          q.n_bridge += __popc(m1);
-        }
-        lkb_pump<Real, GRAD, TAGGED>(ev, q, false, w, e4, tg);
       }
       // the rest of the list to its front
       const int rest = m > 32 ? m - 32 : 0;
