@@ -1652,15 +1652,15 @@ def run_lkball(args, world, rank, local):
                 "poses_per_gpu": P,
                 "atoms_per_gpu": int(coords.shape[0]),
                 "l2": "flushed (256 MiB write) before every timed step",
-                "launch": "CUDA graph replay: 5 kernels per step (waters, block spheres, scoring with its "
-                "adjoint, gradient out, waters adjoint)",
+                "launch": "CUDA graph replay: 4 kernels per step (waters, block spheres, scoring with its "
+                "adjoint, waters adjoint)",
                 "launch_shape": dict(
                     zip(LAUNCH_FIELDS, launch)
                 ),
                 "parallelism": f"weak, {world} independent batch(es)",
             },
             "work_per_step": m["work_per_step"],
-            "gpu_launches": 5 * args.steps,
+            "gpu_launches": 4 * args.steps,
             "clocks": clk.summary(),
             "roofline": {
                 "bound": "fp32",
@@ -1858,11 +1858,11 @@ def run_sfxn(args, world, rank, local):
                 "poses_per_gpu": P,
                 "atoms_per_gpu": int(coords.shape[0]),
                 "l2": "flushed (256 MiB write) before every timed step",
-                "launch": "CUDA graph replay: 13 kernels per step (LJ/LK 3, elec 3, LK-ball 5 on three concurrent "
+                "launch": "CUDA graph replay: 12 kernels per step (LJ/LK 3, elec 3, LK-ball 4 on three concurrent "
                 "streams, gradient sum 2)",
                 "parallelism": f"weak, {world} independent batch(es)",
             },
-            "gpu_launches": 13 * args.steps,
+            "gpu_launches": 12 * args.steps,
             "clocks": clk.summary(),
             "roofline": {
                 "bound": "fp32",

@@ -567,6 +567,8 @@ struct ScoreArgs {
   // the gradient as [n_atoms][GRAD_STRIDE], zeroed by the sphere pass
   // and copied out by grad_out_kernel
   Real* g4;
+  Real* dcoords;  // LK-ball: the gradient itself, zero_dcoords reals zeroed by the sphere pass
+  int64_t zero_dcoords;
   const uint8_t* bt_conn_pd;
   const int* bt_n_atoms;
   const int* bt_n_conn;
@@ -684,6 +686,7 @@ __global__ void spheres_kernel(ScoreArgs<Real> s) {
   const int64_t n_threads = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = tid; i < s.zero_energies; i += n_threads) s.energies[i] = Real(0);
   for (int64_t i = tid; i < s.zero_aux_n; i += n_threads) s.zero_aux[i] = Real(0);
+  for (int64_t i = tid; i < s.zero_dcoords; i += n_threads) s.dcoords[i] = Real(0);
   if (!s.spec_flag)
     for (int64_t i = tid; i < s.spec_n; i += n_threads) s.spec_to[i] = s.spec_from[i];
   // the neighbour matrix, four entries a store where it is aligned
@@ -1356,7 +1359,7 @@ struct tmol_b200_ljlk_plan {
   // device flag a backward sets when its weights match those
   void* spec_next = nullptr;  // [n_terms, P]
   void* spec_used = nullptr;  // [n_terms, P]
-  void* spec_g = nullptr;     // [N, GRAD_STRIDE]
+  void* spec_g = nullptr;     // [N, GRAD_STRIDE]; LK-ball: [N, 3]
   void* spec_dw = nullptr;    // LK-ball: [N, 4, 3], the waters' gradient
   int* spec_flag = nullptr;
   bool spec_ready = false;  // spec_next holds a backward's weights
@@ -1849,12 +1852,16 @@ cudaError_t spec_compare(tmol_b200_ljlk_plan* pl, ScoreArgs<Real>& s, const void
   return cudaSuccess;
 }
 
-// dst[0, n) = src[0, n) when *flag is set.
+// LK-ball: copies the kept gradients out when *flag is set (a null flag: not),
+// and keeps a backward's weights for the next speculative forward.
 template <typename Real>
-__global__ void spec_copy_kernel(const int* flag, const Real* src, Real* dst, int64_t n) {
-  if (!*flag) return;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    dst[i] = src[i];
+__global__ void lkb_spec_out_kernel(const int* flag, const Real* dx, Real* dx_out, int64_t n_dx, const Real* dw,
+                                    Real* dw_out, int64_t n_dw, const Real* weights, Real* keep, int n_weights) {
+  const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, n_threads = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = tid; i < n_weights; i += n_threads) keep[i] = weights[i];
+  if (!flag || !*flag) return;
+  for (int64_t i = tid; i < n_dx; i += n_threads) dx_out[i] = dx[i];
+  for (int64_t i = tid; i < n_dw; i += n_threads) dw_out[i] = dw[i];
 }
 
 // The pose op's forward that also takes the gradient with the weights of
@@ -2080,7 +2087,7 @@ void heavy_args(const tmol_b200_ljlk_plan* pl, ScoreArgs<Real>& s, const void* w
 
 template <typename Real, bool GRAD, bool BLOCK_PAIR>
 int lkb_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const void* waters, void* energies, int32_t* nbr,
-                   const void* dTdV, void* g4, void* dwaters, cudaStream_t st, bool spec_forward = false,
+                   const void* dTdV, void* dcoords, void* dwaters, cudaStream_t st, bool spec_forward = false,
                    bool spec_backward = false) {
   ScoreArgs<Real> s = score_args<Real>(pl, coords);
   if (spec_forward) {
@@ -2096,7 +2103,7 @@ int lkb_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const void* wate
   s.energies = (Real*)energies;
   s.nbr = nbr;
   s.dTdV = (const Real*)dTdV;
-  s.g4 = (Real*)g4;  // the padded gradient, or null (zeroed by the sphere pass)
+  s.dcoords = (Real*)dcoords;
   heavy_args(pl, s, waters);
   const size_t PBB = (size_t)pl->P * pl->B * pl->B;
   // block-pair energies and weights are addressed by an int block-pair index
@@ -2107,6 +2114,7 @@ int lkb_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const void* wate
   // ticket: by the sphere pass (which a taken speculative gradient skips:
   // its outputs are then copied whole)
   if (energies && !BLOCK_PAIR) s.zero_energies = (int64_t)pl->P * 4;
+  if (dcoords) s.zero_dcoords = (int64_t)pl->N * 3;
   if (dwaters) {
     s.zero_aux = (Real*)dwaters;
     s.zero_aux_n = (int64_t)pl->N * LKB_NW * 3;
@@ -2158,15 +2166,16 @@ int lkb_backward_speculative_impl(tmol_b200_ljlk_plan* pl, const void* coords, c
   // are copied out
   const bool compare = speculated && pl->spec_taken && n_w > 0;
   const int* hit = compare ? pl->spec_flag : nullptr;
-  int rc = lkb_score_impl<Real, true, false>(pl, coords, waters, nullptr, nullptr, dTdV, pl->g4, dwaters, st,
+  int rc = lkb_score_impl<Real, true, false>(pl, coords, waters, nullptr, nullptr, dTdV, dcoords, dwaters, st,
                                              false, compare);
   if (rc != TMOL_B200_OK) return rc;
-  rc = grad_out<Real>(pl, hit, pl->spec_g, dcoords, st, dTdV, pl->spec_next, n_w);
-  if (rc != TMOL_B200_OK) return rc;
-  const int64_t n_dw = (int64_t)pl->N * LKB_NW * 3;
-  if (hit && n_dw > 0) {
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n_dw + 255) / 256, (int64_t)pl->n_sm * 8));
-    spec_copy_kernel<Real><<<grid, 256, 0, st>>>(hit, (const Real*)pl->spec_dw, (Real*)dwaters, n_dw);
+  const int64_t n_dx = hit ? pl->N * 3 : 0, n_dw = hit ? pl->N * LKB_NW * 3 : 0;
+  const int64_t n = std::max<int64_t>(n_dw, n_w);
+  if (n > 0) {
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)pl->n_sm * 8));
+    lkb_spec_out_kernel<Real><<<grid, 256, 0, st>>>(hit, (const Real*)pl->spec_g, (Real*)dcoords, n_dx,
+                                                    (const Real*)pl->spec_dw, (Real*)dwaters, n_dw, (const Real*)dTdV,
+                                                    (Real*)pl->spec_next, n_w);
     CK(cudaGetLastError());
   }
   pl->spec_ready = true;
@@ -2188,17 +2197,15 @@ int lkb_rotamer_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const vo
   ra.n_pairs = n_pairs;
   s.energies = (Real*)energies;
   s.dTdV = (const Real*)dTdV;
-  if (!GRAD) s.g4 = nullptr;
+  s.dcoords = (Real*)dcoords;
   heavy_args(pl, s, waters);
   s.nbr = nullptr;
   s.counts = pl->counts;
   CK(cudaMemsetAsync(pl->counts, 0, N_COUNTS * sizeof(unsigned long long), st));
   if (energies) CK(cudaMemsetAsync(energies, 0, (size_t)4 * n_pairs * sizeof(Real), st));
   if (dwaters) CK(cudaMemsetAsync(dwaters, 0, (size_t)pl->N * LKB_NW * 3 * sizeof(Real), st));
-  if (n_items == 0) {
-    if (dcoords) CK(cudaMemsetAsync(dcoords, 0, (size_t)pl->N * 3 * sizeof(Real), st));
-    return TMOL_B200_OK;
-  }
+  if (dcoords) CK(cudaMemsetAsync(dcoords, 0, (size_t)pl->N * 3 * sizeof(Real), st));
+  if (n_items == 0) return TMOL_B200_OK;
   if (pl->R > 0) {
     const int gr = std::max(1, std::min((pl->R + 7) / 8, pl->n_sm * 16));
     rot_spheres_kernel<Real><<<gr, 256, 0, st>>>(s, ra, (Real*)pl->rot_spheres);
@@ -2213,7 +2220,7 @@ int lkb_rotamer_score_impl(tmol_b200_ljlk_plan* pl, const void* coords, const vo
   else
     lkb_rotamer_kernel<Real, GRAD, false><<<grid, 32 * warps, 0, st>>>(s, k, ra, (const Real*)pl->rot_spheres);
   CK(cudaGetLastError());
-  return GRAD ? grad_out<Real>(pl, nullptr, nullptr, dcoords, st) : TMOL_B200_OK;
+  return TMOL_B200_OK;
 }
 
 }  // namespace
@@ -2345,7 +2352,7 @@ int build_lkball(tmol_b200_ljlk_plan* pl, const tmol_b200_lkball_inputs* k, cons
     // the score op's speculative gradient (lkb_backward_speculative)
     dalloc(pl, (Real**)&pl->spec_next, (size_t)4 * std::max(pl->P, 1));
     dalloc(pl, (Real**)&pl->spec_used, (size_t)4 * std::max(pl->P, 1));
-    dalloc(pl, (Real**)&pl->spec_g, (size_t)std::max<int64_t>(pl->N, 1) * GRAD_STRIDE);
+    dalloc(pl, (Real**)&pl->spec_g, (size_t)std::max<int64_t>(pl->N, 1) * 3);
     dalloc(pl, (Real**)&pl->spec_dw, (size_t)std::max<int64_t>(pl->N, 1) * LKB_NW * 3);
     dalloc(pl, &pl->spec_flag, 1);
   }
@@ -2555,10 +2562,12 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   dalloc(pl, (unsigned char**)&pl->spheres, PB * 4 * real_bytes);
   if (scoring) {
     const int64_t n_at = std::max<int64_t>(in->n_atoms, 1);
-    dalloc(pl, (unsigned char**)&pl->packed,
-               n_at * (real_bytes == 4 ? sizeof(AtomRec<float>) : sizeof(AtomRec<double>)));
-    dalloc(pl, (unsigned char**)&pl->g4, (size_t)n_at * GRAD_STRIDE * real_bytes);
-    dalloc(pl, &pl->real_atom, n_at);
+    if (term != kTermLKBall) {
+      dalloc(pl, (unsigned char**)&pl->packed,
+             n_at * (real_bytes == 4 ? sizeof(AtomRec<float>) : sizeof(AtomRec<double>)));
+      dalloc(pl, (unsigned char**)&pl->g4, (size_t)n_at * GRAD_STRIDE * real_bytes);
+      dalloc(pl, &pl->real_atom, n_at);
+    }
   }
   if (scoring) {
     pl->n_iwords = (A + 31) / 32;
@@ -2596,7 +2605,7 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
   }
   PCK(dplace(pl, st));
 
-  if (scoring) PCK(cudaMemsetAsync(pl->real_atom, 0, std::max<int64_t>(in->n_atoms, 1), st));
+  if (pl->real_atom) PCK(cudaMemsetAsync(pl->real_atom, 0, std::max<int64_t>(in->n_atoms, 1), st));
   if (term == kTermElec && nbt > 0 && A > 0)
     PCK(cudaMemcpyAsync(pl->bt_q, elec->partial_charge, (size_t)nbt * A * real_bytes, cudaMemcpyDeviceToDevice, st));
   PCK(cudaMemsetAsync(pl->pose_last, 0, sizeof(int) * std::max(P, 1), st));
@@ -2773,7 +2782,7 @@ int create_plan(const tmol_b200_ljlk_inputs* in, int real_bytes,
       PCK(cudaGetLastError());
     }
   }
-  if (scoring) {
+  if (pl->real_atom) {
     const int n = rotamers ? pl->R : (int)PB;
     if (n > 0) {
       plan_real_atoms_kernel<<<std::max(1, std::min((n + 127) / 128, pl->n_sm * 8)), 128, 0, st>>>(
@@ -3585,16 +3594,14 @@ int tmol_b200_lkball_energy_and_gradient(tmol_b200_lkball_plan* plan, const void
   if (plan->real_bytes == 4) {
     if ((rc = lkb_waters_impl<float>(plan, coords, plan->lkb_waters, st, true))) return rc;
     if ((rc = lkb_score_impl<float, true, false>(plan, coords, plan->lkb_waters, energies, nullptr, weights,
-                                                 plan->g4, plan->lkb_dwaters, st)))
+                                                 dcoords, plan->lkb_dwaters, st)))
       return rc;
-    if ((rc = grad_out<float>(plan, nullptr, nullptr, dcoords, st))) return rc;
     return lkb_waters_backward_impl<float>(plan, coords, plan->lkb_dwaters, dcoords, st);
   }
   if ((rc = lkb_waters_impl<double>(plan, coords, plan->lkb_waters, st, true))) return rc;
   if ((rc = lkb_score_impl<double, true, false>(plan, coords, plan->lkb_waters, energies, nullptr, weights,
-                                                plan->g4, plan->lkb_dwaters, st)))
+                                                dcoords, plan->lkb_dwaters, st)))
     return rc;
-  if ((rc = grad_out<double>(plan, nullptr, nullptr, dcoords, st))) return rc;
   return lkb_waters_backward_impl<double>(plan, coords, plan->lkb_dwaters, dcoords, st);
 }
 
@@ -3605,19 +3612,15 @@ int tmol_b200_lkball_backward(tmol_b200_lkball_plan* plan, const void* coords, c
   if (!plan || plan->term != kTermLKBall || !plan->lkb_nocc || !dTdV) return TMOL_B200_ERR_INVALID_ARGUMENT;
   if (plan->N > 0 && (!coords || !waters || !dcoords || !dwaters)) return TMOL_B200_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
-  int rc;
-  if (plan->real_bytes == 4) {
-    rc = block_pair ? lkb_score_impl<float, true, true>(plan, coords, waters, nullptr, nullptr, dTdV, plan->g4,
-                                                        dwaters, st)
-                    : lkb_score_impl<float, true, false>(plan, coords, waters, nullptr, nullptr, dTdV, plan->g4,
-                                                         dwaters, st);
-    return rc ? rc : grad_out<float>(plan, nullptr, nullptr, dcoords, st);
-  }
-  rc = block_pair ? lkb_score_impl<double, true, true>(plan, coords, waters, nullptr, nullptr, dTdV, plan->g4,
-                                                       dwaters, st)
-                  : lkb_score_impl<double, true, false>(plan, coords, waters, nullptr, nullptr, dTdV, plan->g4,
-                                                        dwaters, st);
-  return rc ? rc : grad_out<double>(plan, nullptr, nullptr, dcoords, st);
+  if (plan->real_bytes == 4)
+    return block_pair ? lkb_score_impl<float, true, true>(plan, coords, waters, nullptr, nullptr, dTdV, dcoords,
+                                                          dwaters, st)
+                      : lkb_score_impl<float, true, false>(plan, coords, waters, nullptr, nullptr, dTdV, dcoords,
+                                                           dwaters, st);
+  return block_pair ? lkb_score_impl<double, true, true>(plan, coords, waters, nullptr, nullptr, dTdV, dcoords,
+                                                         dwaters, st)
+                    : lkb_score_impl<double, true, false>(plan, coords, waters, nullptr, nullptr, dTdV, dcoords,
+                                                          dwaters, st);
 }
 
 int64_t tmol_b200_ljlk_plan_device_bytes(const tmol_b200_ljlk_plan* plan) {

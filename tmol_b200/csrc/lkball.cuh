@@ -731,13 +731,12 @@ struct LkbQueue {
 // What evaluating a queued pair needs (a compact by-value context).
 template <typename Real>
 struct LkbEval {
-  const AtomRec<Real>* packed;
+  const Real* coords;
   const Real* waters;
   const Real* par;
-  Real* g4;       // padded gradient [n_atoms][GRAD_STRIDE]
+  Real* dcoords;  // [n_atoms][3]
   Real* dwaters;  // [n_atoms][4][3]
   bool vec_w, vec_dw;  // 16-byte aligned
-  Real grid;           // force_grid_of the item's weights (untagged)
   Real water_dist, hbond_dis, hbond_oh, hbond_h, max_dis;
 };
 
@@ -745,11 +744,6 @@ template <typename Real>
 struct Lkb4 {
   Real v[4];
 };
-
-template <typename Real>
-__device__ __forceinline__ Real lkb_grid(const Lkb4<Real>& w) {
-  return force_grid_of(fmax(fmax(fabs(w.v[0]), fabs(w.v[1])), fmax(fabs(w.v[2]), fabs(w.v[3]))));
-}
 
 // Evaluates entry `lane` of q when lane < n: returns its four energies and,
 // with GRAD, adds the adjoint of w . E to dcoords / dwaters.
@@ -766,14 +760,15 @@ __device__ __forceinline__ Real lkb_grid(const Lkb4<Real>& w) {
 
 template <typename Real, bool GRAD, typename Queue>
 __device__ TMOL_B200_LKB_DRAIN_ATTR Lkb4<Real> lkb_drain(const LkbEval<Real> ev, const Queue& q, int n, int lane,
-                                             const Lkb4<Real> w, Real grid) {
+                                             const Lkb4<Real> w) {
   Lkb4<Real> out = {{0, 0, 0, 0}};
   if (lane >= n) return out;
   const int64_t rp = q.rp[lane], ro = q.ro[lane];
   const int pidx = q.pi[lane], oidx = q.oi[lane], sep = q.sep[lane];
   Real WI[LKB_NW * 3], WJ[LKB_NW * 3];
-  const AtomRec<Real> ai = ev.packed[rp], aj = ev.packed[ro];
-  const Real I[3] = {ai.x, ai.y, ai.z}, J[3] = {aj.x, aj.y, aj.z};
+  Real I[3], J[3];
+  lkb_load3(ev.coords, rp, I);
+  lkb_load3(ev.coords, ro, J);
   lkb_load_waters(ev.waters, rp, ev.vec_w, WI);
   lkb_load_waters(ev.waters, ro, ev.vec_w, WJ);
   const LkbParams<Real> pp = lkb_params(ev.par, pidx);  // row bt * A + atom
@@ -784,12 +779,14 @@ __device__ TMOL_B200_LKB_DRAIN_ATTR Lkb4<Real> lkb_drain(const LkbEval<Real> ev,
     for (int c = 0; c < LKB_NW * 3; ++c) gWI[c] = gWJ[c] = 0;
   lkb_pair<Real, GRAD>(I, J, WI, WJ, sep, pp, po, ev, out.v, w.v, gI, gJ, gWI, gWJ);
   if (GRAD) {
-    // vector reductions: the thirty values of a pair as scalar ones took the
-    // path to L2 longer than the pair's arithmetic
-    if (gI[0] != Real(0) || gI[1] != Real(0) || gI[2] != Real(0))
-      add_force(ev.g4 + GRAD_STRIDE * rp, grid, gI[0], gI[1], gI[2]);
-    if (gJ[0] != Real(0) || gJ[1] != Real(0) || gJ[2] != Real(0))
-      add_force(ev.g4 + GRAD_STRIDE * ro, grid, gJ[0], gJ[1], gJ[2]);
+    // straight into the caller's gradient: with sums in LJ/LK's padded form and
+    // its vector reductions the kernel took 164 us for 64 x 150 residues
+    // instead of 161, and another pass copied them out
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      if (gI[c] != Real(0)) atomicAdd(&ev.dcoords[3 * rp + c], gI[c]);
+      if (gJ[c] != Real(0)) atomicAdd(&ev.dcoords[3 * ro + c], gJ[c]);
+    }
     lkb_add_waters(ev.dwaters, rp, ev.vec_dw, gWI);
     lkb_add_waters(ev.dwaters, ro, ev.vec_dw, gWJ);
   }
@@ -842,7 +839,7 @@ __device__ __forceinline__ void lkb_pump(const LkbEval<Real>& ev, LkbWarp<Real, 
     const int tag = TAGGED && lane < n ? Q.tag[lane] : 0;
     if (TAGGED && GRAD && lane < n)
       for (int c = 0; c < 4; ++c) wl.v[c] = tg.dTdV[(int64_t)c * tg.n + tag];
-    const Lkb4<Real> got = lkb_drain<Real, GRAD>(ev, Q, n, lane, wl, TAGGED && GRAD ? lkb_grid(wl) : ev.grid);
+    const Lkb4<Real> got = lkb_drain<Real, GRAD>(ev, Q, n, lane, wl);
     if (TAGGED) {
       if (!GRAD && lane < n)
         for (int c = 0; c < 4; ++c)
@@ -1139,12 +1136,11 @@ __device__ __forceinline__ int lkb_entry(const ScoreArgs<Real>& s, int64_t i1, i
 template <typename Real>
 __device__ __forceinline__ LkbEval<Real> lkb_eval_of(const ScoreArgs<Real>& s, const LkbArgs<Real>& k) {
   LkbEval<Real> ev;
-  ev.packed = s.packed;
+  ev.coords = s.coords;
   ev.waters = k.waters;
   ev.par = k.par;
-  ev.g4 = s.g4;
+  ev.dcoords = s.dcoords;
   ev.dwaters = k.dwaters_out;
-  ev.grid = 0;
   ev.vec_w = (reinterpret_cast<uintptr_t>(k.waters) & (4 * sizeof(Real) - 1)) == 0;
   ev.vec_dw = (reinterpret_cast<uintptr_t>(k.dwaters_out) & (4 * sizeof(Real) - 1)) == 0;
   ev.water_dist = k.water_dist;
@@ -1185,7 +1181,7 @@ __global__ void __launch_bounds__(256, TMOL_B200_LKB_MIN_CTAS) lkb_score_kernel(
   q.n_bp = q.n_pairs = q.n_bridge = q.n_eval = 0;
   const int lane = q.lane;
   const int64_t stride = (int64_t)s.P * s.B * s.B;
-  LkbEval<Real> ev = lkb_eval_of(s, k);
+  const LkbEval<Real> ev = lkb_eval_of(s, k);
   LkbTagged<Real> tg;
   tg.energies = s.energies;
   tg.dTdV = s.dTdV;
@@ -1216,7 +1212,6 @@ __global__ void __launch_bounds__(256, TMOL_B200_LKB_MIN_CTAS) lkb_score_kernel(
       Lkb4<Real> w = {{0, 0, 0, 0}};
       if (GRAD && !BLOCK_PAIR)
         for (int c = 0; c < 4; ++c) w.v[c] = s.dTdV[(int64_t)c * s.P + p];
-      ev.grid = lkb_grid(w);
       Real acc[4] = {0, 0, 0, 0};
       const LkbRows rows = {bt1, s.blk_off[i1], k.hbase[i1], k.nocc[bt1], k.npol[bt1], s.bt_n_atoms[bt1]};
       const Real reach1 = sph1.d + k.max_dis;
