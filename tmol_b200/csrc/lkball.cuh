@@ -780,8 +780,9 @@ __device__ TMOL_B200_LKB_DRAIN_ATTR Lkb4<Real> lkb_drain(const LkbEval<Real> ev,
   lkb_pair<Real, GRAD>(I, J, WI, WJ, sep, pp, po, ev, out.v, w.v, gI, gJ, gWI, gWJ);
   if (GRAD) {
     // straight into the caller's gradient: with sums in LJ/LK's padded form and
-    // its vector reductions the kernel took 164 us for 64 x 150 residues
-    // instead of 161, and another pass copied them out
+    // its vector reductions the kernel took 164 us for 64 x 150 residues (161
+    // without, before the loops in front were folded), and another pass copied
+    // them out
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       if (gI[c] != Real(0)) atomicAdd(&ev.dcoords[3 * rp + c], gI[c]);
@@ -914,14 +915,16 @@ __device__ __forceinline__ bool lkb_within(double d2, double max) {
 // until none has one left.  Pairs of the rows' own block and of count-pair
 // partners have their exclusions from the plan's masks, a rotamer's partners
 // (PMASK false) their bond separations.
-// What bounds it: latency and issue of the evaluation.  Times of the scoring
-// kernel where pairs were enumerated one by one, with index arithmetic and
-// eight loads each; where every row was voted on and queued in both directions
-// in turn, its record and masks loaded in between; and now: 64 x 150 residues,
-// energies + gradients 196, 164 and 164 us; rotamers of 8 x 100 residues,
-// energies 2.55, 2.12 and 1.42 ms; one pose of 100 residues, energies 37, 35 and
-// 26 us; 4 x 100 in float64, energies 101, 128 and 99 us; of one residue 7.5,
-// 14.7 and 9.2 us.
+// What bounds it: latency and issue of the evaluation, and beside the adjoint
+// the instruction cache: the rows' loops are unrolled for the energies alone
+// (64 x 150 residues, energies + gradients: 157 us with them unrolled by four,
+// 152 by two, 148 not at all).  Times of the scoring kernel where pairs were
+// enumerated one by one, with index arithmetic and eight loads each; where every
+// row was voted on and queued in both directions in turn, its record and masks
+// loaded in between; and now: 64 x 150 residues, energies + gradients 196, 164
+// and 148 us; rotamers of 4 x 100 residues, ten a block, energies 151, 169 and
+// 106 us; one pose of 100 residues, energies 37, 35 and 26 us; 4 x 100 in
+// float64, energies 101, 128 and 102 us; one residue 7.5, 14.7 and 7.8-8.8 us.
 template <typename Real, bool GRAD, bool TAGGED, bool COUNT, bool PMASK, typename Next>
 __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs<Real>& k, const LkbEval<Real>& ev,
                                          LkbWarp<Real, TAGGED>& q, LkbList<Real, TAGGED>& L, const LkbRows& a,
@@ -993,15 +996,18 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
       }
       if (m < 32 && !(final && k0 + 32 >= T && m > 0)) continue;
       // the list's first 32 atoms against every row: the row polar and the
-      // list's atom occluding, then the other way round
+      // list's atom occluding, then the other way round; of a list of 16 or 8
+      // atoms, an item's last, two or four lanes share one, each with every
+      // second or fourth row
+      const int shift = m > 16 ? 0 : (m > 8 ? 1 : 2), rep = 1 << shift;
+      const int at_l = lane & ((32 >> shift) - 1), sub = lane >> (5 - shift);
       AtomRec<Real> o;
-      o.x = L.x[lane];
-      o.y = L.y[lane];
-      o.z = L.z[lane];
-      o.tf = L.tf[lane];
-      const int orow = L.row[lane], opar = L.par[lane], entry = L.entry[lane], ja = o.tf & kHeavyAtom;
-      const int otag = TAGGED ? L.tag[lane] : 0;
-      const bool valid = lane < m;
+      o.x = L.x[at_l];
+      o.y = L.y[at_l];
+      o.z = L.z[at_l];
+      o.tf = L.tf[at_l];
+      const int entry = L.entry[at_l], ja = o.tf & kHeavyAtom;
+      const bool valid = at_l < m;
       const bool special = valid && entry != -2;
       const bool any_special = __any_sync(0xffffffffu, special);
       for (int rt = 0; rt < a.nocc; rt += 32) {
@@ -1010,13 +1016,15 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
         // bit i: row rt + i and this lane's atom are a pair in reach (near)
         // with weight 0.2 (four): no branch or vote in the rows' loads
         unsigned near = 0, four = 0;
-#pragma unroll 4
-        for (int i = 0; i < nr; ++i) {
-          const AtomRec<Real> r = s.hpacked[a.hb + rt + i];
+        const unsigned mine = valid ? 0xffffffffu >> (32 - nr) : 0u;  // rows
+#pragma unroll (GRAD ? 1 : 4)
+        for (int i0 = 0; i0 < nr; i0 += rep) {
+          const int i = i0 + sub;
+          const AtomRec<Real> r = s.hpacked[a.hb + rt + min(i, nr - 1)];
           const Real dv[3] = {r.x - o.x, r.y - o.y, r.z - o.z};
           near |= (lkb_within(lkb_dot(dv, dv), k.max_dis) ? 1u : 0u) << i;
         }
-        if (!valid) near = 0;
+        near &= mine;
         if (any_special) {
           unsigned out = 0;
           const uint2* masks = nullptr;  // of the word that holds this atom, by row atom
@@ -1027,9 +1035,10 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
           } else if (PMASK && special) {
             masks = s.pmask + s.cp_moff[entry] + (int64_t)(ja >> 5) * a.n_atoms;
           }
-#pragma unroll 4
-          for (int i = 0; i < nr; ++i) {
-            const int ra = __shfl_sync(0xffffffffu, rtf, i) & kHeavyAtom;
+#pragma unroll (GRAD ? 1 : 4)
+          for (int i0 = 0; i0 < nr; i0 += rep) {
+            const int i = i0 + sub;
+            const int ra = __shfl_sync(0xffffffffu, rtf, i) & kHeavyAtom;  // past nr: 0
             uint2 mk = make_uint2(0u, 0u);
             if (masks) mk = masks[ra * stride];
             out |= ((mk.x >> (ja & 31)) & 1u) << i;
@@ -1041,7 +1050,7 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
             const bool partner = special && entry >= 0;
             unsigned far = 0x3f3f3f3fu;
             if (partner) {
-              const int bt2 = (opar - ja) / s.A, nc2 = s.bt_n_conn[bt2];
+              const int bt2 = (L.par[at_l] - ja) / s.A, nc2 = s.bt_n_conn[bt2];
               const uint8_t* seps = s.cp_seps + (int64_t)entry * 16;
               const uint32_t cj = load_cpd(s, bt2, nc2, ja);
               for (int u = 0; u < nc1; ++u) {
@@ -1053,7 +1062,8 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
             }
             if (__any_sync(0xffffffffu, partner)) {
               const uint32_t c0 = lane < nr ? load_cpd(s, a.bt, nc1, rtf & kHeavyAtom) : 0u;
-              for (int i = 0; i < nr; ++i) {
+              for (int i0 = 0; i0 < nr; i0 += rep) {
+                const int i = i0 + sub;
                 const uint32_t ci = __shfl_sync(0xffffffffu, c0, i);
                 int sep = 5;
                 for (int u = 0; u < nc1; ++u)
@@ -1075,7 +1085,7 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
         for (;;) {
           const bool act = (there | back) != 0, bk = there == 0;
           const int i = act ? __ffs(bk ? back : there) - 1 : 0;
-          const bool bridged = bk ? (bridge_rows >> i) & 1u : (o.tf & kHeavyBridges) != 0;
+          const bool bridged = bk ? (bridge_rows >> i) & 1u : (L.tf[at_l] & kHeavyBridges) != 0;
           const unsigned m1 = __ballot_sync(0xffffffffu, act && bridged);
           const unsigned m0 = __ballot_sync(0xffffffffu, act && !bridged);
           if ((m0 | m1) == 0) break;
@@ -1085,7 +1095,7 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
               back &= back - 1;
             else
               there &= there - 1;
-            const int rr = a.off + ra, rpar = a.bt * s.A + ra;
+            const int rr = a.off + ra, rpar = a.bt * s.A + ra, orow = L.row[at_l], opar = L.par[at_l];
             LkbQueue<TAGGED>& Q = q.qs[bridged ? 1 : 0];
             const int at = (bridged ? q.nq[1] : q.nq[0]) + __popc((bridged ? m1 : m0) & q.lt_mask);
             Q.rp[at] = bk ? orow : rr;
@@ -1093,7 +1103,7 @@ __device__ __forceinline__ void lkb_walk(const ScoreArgs<Real>& s, const LkbArgs
             Q.pi[at] = bk ? opar : rpar;
             Q.oi[at] = bk ? rpar : opar;
             Q.sep[at] = (four >> i) & 1u ? 4 : 6;
-            if (TAGGED) Q.tag[at] = otag;
+            if (TAGGED) Q.tag[at] = L.tag[at_l];
           }
           q.nq[0] += __popc(m0);
           q.nq[1] += __popc(m1);
