@@ -757,6 +757,11 @@ struct Lkb4 {
 #ifndef TMOL_B200_LKB_MIN_CTAS
 #define TMOL_B200_LKB_MIN_CTAS 2
 #endif
+// The float64 adjoint does not fit in the 128 registers that two CTAs per SM
+// leave a thread (it spilled a kilobyte): one, 16 x 150 residues, gradient 355
+// us with two, 251 with one.  Float keeps two (one: 30% slower).
+template <typename Real, bool GRAD>
+constexpr int lkb_min_ctas = sizeof(Real) == 8 && GRAD ? 1 : TMOL_B200_LKB_MIN_CTAS;
 
 template <typename Real, bool GRAD, typename Queue>
 __device__ TMOL_B200_LKB_DRAIN_ATTR Lkb4<Real> lkb_drain(const LkbEval<Real> ev, const Queue& q, int n, int lane,
@@ -1177,7 +1182,7 @@ __device__ __forceinline__ void lkb_flush_counts(const ScoreArgs<Real>& s, const
 // COUNT: the work counters (registers and instructions in the pair loop),
 // compiled into a separate instantiation used on request
 template <typename Real, bool GRAD, bool BLOCK_PAIR, bool COUNT>
-__global__ void __launch_bounds__(256, TMOL_B200_LKB_MIN_CTAS) lkb_score_kernel(ScoreArgs<Real> s, LkbArgs<Real> k, int items_per_ticket) {
+__global__ void __launch_bounds__(256, lkb_min_ctas<Real, GRAD>) lkb_score_kernel(ScoreArgs<Real> s, LkbArgs<Real> k, int items_per_ticket) {
   if (s.done && *s.done) return;  // a speculative gradient was taken
   // [warp][plain, bridged]; block-pair mode tags queued pairs with their
   // block pair (p * B + b1) * B + b2
@@ -1278,7 +1283,7 @@ __global__ void __launch_bounds__(256, TMOL_B200_LKB_MIN_CTAS) lkb_score_kernel(
 // dTdV[t * n_pairs + d].  Queued pairs carry d, so the queues fill across
 // rotamer pairs and items (a rotamer pair has few pairs in reach).
 template <typename Real, bool GRAD, bool COUNT>
-__global__ void __launch_bounds__(256, TMOL_B200_LKB_MIN_CTAS)
+__global__ void __launch_bounds__(256, lkb_min_ctas<Real, GRAD>)
     lkb_rotamer_kernel(ScoreArgs<Real> s, LkbArgs<Real> k, RotArgs ra, const Real* rot_spheres) {
   __shared__ LkbQueue<true> queues[LKB_MAX_WARPS][2];
   __shared__ LkbList<Real, true> lists[LKB_MAX_WARPS];
