@@ -389,3 +389,44 @@ def test_lkball_lists(block_pair, scale):
     close(E, numpy.asarray(Eo).reshape(E.shape), 1e-9)
     assert numpy.array_equal(nbr.cpu().numpy(), nbro)
     close(dx, dxo, 1e-9)
+
+
+def wide_block_pose_stack():
+    """Poses with a block of more than 32 heavy atoms, alone and bonded to
+    small ones, and with lists of at most eight and sixteen."""
+    from exotic_blocks import big_block_type
+    from tmol_b200.chem.restypes import ChemicalDatabase, PackedBlockTypes, ResidueTypeSet
+    from tmol_b200.pose.builder import PoseTopology, build_pose_stack
+
+    wide = big_block_type("BIG70", 70, False, 5)
+    pbt = PackedBlockTypes(
+        ChemicalDatabase.get_default(), list(ResidueTypeSet.get_default().types.values()) + [wide]
+    )
+    rng = numpy.random.default_rng(3)
+    topologies, coords = [], []
+    for names in (["BIG70"], ["ALA:nterm", "BIG70", "GLY", "SER:cterm"], ["BIG70", "BIG70"], ["GLY"], ["ALA", "GLY"]):
+        bonds = [(i, "up", i + 1, "down") for i in range(len(names) - 1)]
+        n = sum(pbt.active_block_types[pbt.bt_index[x]].n_atoms for x in names)
+        steps = rng.normal(size=(n, 3))
+        walk = numpy.cumsum(1.5 * steps / numpy.linalg.norm(steps, axis=1, keepdims=True), axis=0)
+        topologies.append(PoseTopology(names, bonds))
+        coords.append(0.6 * walk + rng.normal(scale=0.3, size=walk.shape))
+    return build_pose_stack(topologies, coords, pbt=pbt)
+
+
+@pytest.mark.parametrize("block_pair", [False, True])
+def test_lkball_wide_blocks(block_pair):
+    """The walk where the rows take several tiles of 32 and where a list is
+    short enough for two or four lanes an atom; tolerances as above."""
+    from tests.test_gpu_lkball import gpu_run
+    from tests.test_lkball_oracle import oracle_run
+    from tmol_b200.score.lkball_energy_term import LKBallEnergyTerm
+
+    ps = wide_block_pose_stack()
+    _, E, dx, nbr = gpu_run(ps, LKBallEnergyTerm(), torch.float64, block_pair)
+    _, Eo, dxo, nbro = oracle_run(ps, True)
+    if block_pair:
+        E = E.sum((2, 3))
+    close(E, numpy.asarray(Eo).reshape(E.shape), 1e-9)
+    assert numpy.array_equal(nbr.cpu().numpy(), nbro)
+    close(dx, dxo, 1e-9)
